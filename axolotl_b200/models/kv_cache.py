@@ -29,6 +29,9 @@ class KVCache:
         kq, vq = qkv[:, Hq * D:(Hq + Hk) * D], qkv[:, (Hq + Hk) * D:]
         if meta.decode:
             # one new token per active sequence: row i of qkv belongs to sequence meta.seq[i]
+            if qkv.is_cuda:      # the attention kernel appends the new k / v rows itself
+                return Fn.decode_attention_append(qkv, self.k[layer], self.v[layer], meta.seq, meta.lens_after, Hq, Hk, D,
+                                                  scale, window)
             self.k[layer, meta.seq, meta.pos] = kq
             self.v[layer, meta.seq, meta.pos] = vq
             if meta.all_rows:

@@ -729,6 +729,23 @@ def flash_varlen(qkv, meta: AttnMeta, Hq, Hk, D, scale=None, Dv=None, softcap=0.
                      getattr(meta, "window", 0), softcap, sinks).reshape(T, Hq * Dv)
 
 
+def _decode_launch(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window, append, pos=None, inv_freq=None, attn_scale=1.0):
+    B = qkv.shape[0]
+    out = torch.empty((B, Hq * D), dtype=qkv.dtype, device=qkv.device)
+    _lib.check_rc(_lib.cuda_lib().axb_decode_attn(
+        qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, k_cache.data_ptr(), v_cache.data_ptr(), _lib.ptr(seq),
+        lens.data_ptr(), _lib.ptr(pos), _lib.ptr(inv_freq), attn_scale, out.data_ptr(), out.stride(0), B, Hq, Hk, D,
+        k_cache.shape[1], scale, int(window or 0), int(append), 0, _lib.stream_ptr()), "decode_attn")
+    return out
+
+
+@torch.no_grad()
+def decode_attention_append(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window=0):
+    """``decode_attention`` that also stores the new token's k / v (taken from ``qkv``) at position ``lens[b] - 1`` of
+    cache row ``seq[b]`` (int64 on the device), in the same launch. CUDA only."""
+    return _decode_launch(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window, append=True)
+
+
 @torch.no_grad()
 def decode_attention(qkv, k_cache, v_cache, lens, Hq, Hk, D, scale=None, window=0):
     """Attention of ONE new token per sequence against its KV cache (generation).
@@ -741,12 +758,9 @@ def decode_attention(qkv, k_cache, v_cache, lens, Hq, Hk, D, scale=None, window=
     scale = 1.0 / math.sqrt(D) if scale is None else scale
     B = qkv.shape[0]
     if qkv.is_cuda:
-        lib = _lib.cuda_lib()
-        out = torch.empty((B, Hq * D), dtype=qkv.dtype, device=qkv.device)
-        _lib.check_rc(lib.axb_decode_attn(qkv.data_ptr(), qkv.stride(0), 0, k_cache.data_ptr(), v_cache.data_ptr(),
-                                          lens.data_ptr(), out.data_ptr(), out.stride(0), B, Hq, Hk, D,
-                                          k_cache.shape[1], scale, int(window or 0), _lib.stream_ptr()), "decode_attn")
-        return out
+        if v_cache.data_ptr() % 16:        # the kernel streams both caches in 16-byte pieces
+            v_cache = v_cache.clone()
+        return _decode_launch(qkv, k_cache, v_cache, None, lens, Hq, Hk, D, scale, window, append=False)
     q = qkv[:, : Hq * D].reshape(B, Hk, Hq // Hk, D).float()
     out = torch.empty(B, Hq * D, dtype=qkv.dtype)
     for b in range(B):

@@ -1,0 +1,94 @@
+"""Kernels of a generation step against plain PyTorch: decode attention over the KV cache."""
+import math
+
+import pytest
+import torch
+
+from axolotl_b200.ops import functional as Fn
+
+pytestmark = pytest.mark.gpu
+
+
+def _rotate(x, pos, inv_freq):
+    a = pos.float()[:, None, None] * inv_freq
+    c, s = a.cos(), a.sin()
+    h = x.shape[-1] // 2
+    x1, x2 = x[..., :h].float(), x[..., h:].float()
+    return torch.cat([x1 * c - x2 * s, x2 * c + x1 * s], -1).to(x.dtype)
+
+
+def _reference(q, k, v, scale, first, n):
+    """fp32 attention of [Hk, G, D] queries over rows first..n of [rows, Hk, D] caches."""
+    kk, vv = (t[first:n].float().transpose(0, 1) for t in (k, v))
+    return (torch.softmax(q.float() @ kk.transpose(1, 2) * scale, -1) @ vv).reshape(-1)
+
+
+@pytest.mark.parametrize("D,Hq,Hk", [(64, 8, 8), (64, 32, 4), (128, 32, 8), (128, 32, 2), (256, 8, 2), (128, 15, 3)])
+@pytest.mark.parametrize("splits", [0, 1, 2, 8])
+@pytest.mark.parametrize("window", [0, 33])
+@pytest.mark.parametrize("append,rope", [(False, False), (True, False), (True, True)])
+def test_decode_attention_splits_append_and_rope(D, Hq, Hk, splits, window, append, rope):
+    """Lengths at the edges of a warp's 16-position tile and of a cluster's stride; cache rows in another order than the
+    queries; rows past the end hold NaN, which must not reach the result. Bound: the output is one bf16 rounding of an
+    fp32 result (2^-8 of its largest element covers it with the rotated operands' own rounding)."""
+    from axolotl_b200.ops import _lib
+
+    torch.manual_seed(D + Hq + splits)
+    lens = [1, 2, 15, 16, 17, 64, 65, 500, 511]
+    B, cap = len(lens), 520
+    W = (Hq + 2 * Hk) * D
+    qkv = torch.randn(B, W + 8, device="cuda").bfloat16()[:, :W]       # a row stride of its own
+    kc, vc = (torch.randn(B, cap, Hk * D, device="cuda").bfloat16() for _ in range(2))
+    seq = torch.randperm(B, device="cuda")
+    n = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for b in range(B):
+        kc[seq[b], lens[b]:], vc[seq[b], lens[b]:] = float("nan"), float("nan")
+        if append:
+            kc[seq[b], lens[b] - 1], vc[seq[b], lens[b] - 1] = float("nan"), float("nan")
+    pos = (n - 1).contiguous()
+    inv = 1.0 / (10000.0 ** (torch.arange(0, D, 2, device="cuda").float() / D))
+    scale = 1.0 / math.sqrt(D)
+    out = torch.full((B, Hq * D), 7.0, device="cuda", dtype=torch.bfloat16)
+    k0, v0 = kc.clone(), vc.clone()
+    _lib.check_rc(_lib.cuda_lib().axb_decode_attn(
+        qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, kc.data_ptr(), vc.data_ptr(), seq.data_ptr(), n.data_ptr(),
+        pos.data_ptr(), inv.data_ptr() if rope else None, 1.0, out.data_ptr(), out.stride(0), B, Hq, Hk, D, cap, scale, window,
+        int(append), splits, _lib.stream_ptr()), "decode_attn")
+    q = qkv[:, :Hq * D].reshape(B, Hq, D)
+    k = qkv[:, Hq * D:(Hq + Hk) * D].reshape(B, Hk, D)
+    v = qkv[:, (Hq + Hk) * D:].reshape(B, Hk, D)
+    if rope:
+        q, k = _rotate(q, pos, inv), _rotate(k, pos, inv)
+    for b in range(B):
+        if append:
+            k0[seq[b], lens[b] - 1], v0[seq[b], lens[b] - 1] = k[b].reshape(-1), v[b].reshape(-1)
+        ref = _reference(q[b].view(Hk, Hq // Hk, D), k0[seq[b]].view(cap, Hk, D), v0[seq[b]].view(cap, Hk, D), scale,
+                         max(0, lens[b] - window) if window else 0, lens[b])
+        assert torch.isfinite(out[b].float()).all()
+        assert (out[b].float() - ref).abs().max() <= 2 ** -8 * max(1.0, ref.abs().max().item()), lens[b]
+    if append:      # the new rows are in the cache (a rotated value may round the other way), every other row is untouched
+        torch.testing.assert_close(vc, v0, rtol=0, atol=0, equal_nan=True)
+        torch.testing.assert_close(kc, k0, rtol=2 ** -7, atol=2 ** -7 if rope else 0, equal_nan=True)
+
+
+def test_cached_step_on_a_subset_of_the_sequences():
+    """``KVCache.attend`` with query rows that belong to some of the cache's sequences, in another order."""
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _DecodeMeta
+    from axolotl_b200.models.transformer import CausalLM
+
+    m = CausalLM(preset("tiny-llama", num_hidden_layers=1), dtype=torch.bfloat16, device="cuda").init_weights(0)
+    a = m.layers[0].self_attn
+    cache = KVCache(m, 5, 40)
+    cache.k.normal_()
+    cache.v.normal_()
+    k0, v0 = cache.k[0].clone(), cache.v[0].clone()
+    seq = torch.tensor([3, 0, 4], device="cuda")
+    pos = torch.tensor([7, 0, 39], device="cuda")
+    qkv = torch.randn(3, (a.Hq + 2 * a.Hk) * a.D, device="cuda").bfloat16()
+    out = cache.attend(0, qkv, _DecodeMeta(cache, seq, pos, False), a.Hq, a.Hk, a.D, a.scale)
+    nq, nk = a.Hq * a.D, a.Hk * a.D
+    k0[seq, pos], v0[seq, pos] = qkv[:, nq:nq + nk], qkv[:, nq + nk:]
+    assert torch.equal(cache.k[0], k0) and torch.equal(cache.v[0], v0)
+    ref = Fn.decode_attention(qkv.cpu(), k0[seq].cpu(), v0[seq].cpu(), (pos + 1).int().cpu(), a.Hq, a.Hk, a.D, a.scale)
+    assert (out.cpu().float() - ref.float()).abs().max() <= 2 ** -7 * max(1.0, ref.abs().max().item())
