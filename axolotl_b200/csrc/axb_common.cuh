@@ -278,6 +278,30 @@ AXB_DEVICE void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
+// ------------------------------------------------------------------ programmatic dependent launch
+// A kernel launched with the programmatic-serialization attribute may start while its predecessor still runs; it must
+// call pdl_wait() before it touches anything the predecessor writes or reads. Both are no-ops in a plain launch.
+AXB_DEVICE void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+AXB_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ------------------------------------------------------------------ distributed shared memory
+AXB_DEVICE uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+AXB_DEVICE float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+AXB_DEVICE float4 ld_cluster_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 // ------------------------------------------------------------------ CTA pairs (cta_group::2)
 AXB_DEVICE uint32_t cluster_ctarank() {
   uint32_t r;
@@ -391,8 +415,42 @@ AXB_DEVICE float2 unpack_bf16x2(uint32_t u) {
 }
 
 // ------------------------------------------------------------------ host helpers
+#include <atomic>
 #include <cstdio>
 #include <mutex>
+// Raises a kernel's dynamic shared memory limit, once per device (`done`: one flag word per kernel).
+inline int axb_allow_smem(const void* kern, int bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return (int)e;
+}
+// Launch attributes of a clustered and / or dependent launch (cluster = CTAs per cluster along x, 0 = none).
+struct AxbLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  AxbLaunch(dim3 grid, unsigned threads, size_t smem, cudaStream_t st, int cluster, bool pdl) {
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    if (cluster > 0) {
+      at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      at[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+      at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+      ++cfg.numAttrs;
+    }
+    if (pdl) {
+      at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+      ++cfg.numAttrs;
+    }
+  }
+};
 typedef CUresult (*AxbEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                      const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                      const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

@@ -76,23 +76,6 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint3
   const float2 h = unpack_bf16x2(hi);
   lo = pack_bf16x2(x - h.x, y - h.y);
 }
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
 template <int D>
 struct DecCfg {
   static constexpr int ROWB = D * 2;                       // bytes of one cache row of a head
@@ -119,6 +102,7 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
   float* gL = gM + DEC_MAX_SPLITS * C::STAT;
   float* sCS = gL + 2 * DEC_MAX_SPLITS * C::STAT;          // cos | sin of the new position
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_launch_dependents();
   const int kvh = blockIdx.y, b = blockIdx.z;
   const int rank = (int)cluster_ctarank(), nsplit = (int)cluster_nctarank();
   const int G = p.Hq / p.Hk;
@@ -153,6 +137,8 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
   int tile = rank * DEC_W + warp;
 #pragma unroll
   for (int s = 0; s < C::STAGES - 1; ++s) load_tile(tile + s * step, s);
+
+  pdl_wait();            // the rows of the cache above are older than the kernel this launch may overlap; qkv is not
 
   // ---- query rows (and the new k / v row), rotated on the way when asked
   const __nv_bfloat16* qrow = p.qkv + (long long)b * p.ld;
@@ -361,23 +347,13 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
 }
 
 template <int D>
-int launch_decode(const DecodeParams& p, int B, int splits, cudaStream_t st) {
+int launch_decode(const DecodeParams& p, int B, int splits, bool pdl, cudaStream_t st) {
   using C = DecCfg<D>;
   auto kern = decode_attn_kernel<D>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-  if (e != cudaSuccess) return (int)e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)splits, (unsigned)p.Hk, (unsigned)B);
-  cfg.blockDim = dim3(DEC_T);
-  cfg.dynamicSmemBytes = C::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)splits;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, p);
+  static std::atomic<unsigned long long> allowed{0};
+  if (const int rc = axb_allow_smem((const void*)kern, C::SMEM, allowed)) return rc;
+  AxbLaunch l(dim3((unsigned)splits, (unsigned)p.Hk, (unsigned)B), DEC_T, C::SMEM, st, splits, pdl);
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, kern, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -400,11 +376,12 @@ int pick_splits(int B, int Hk, long long max_len) {
 // lens[b]: live positions of sequence b including the new token; out: [B, out_ld >= Hq*D].
 // append: the new token's k / v (columns k_col0 / v_col0 of qkv) are stored at position lens[b] - 1 and attended to;
 // otherwise that position is read from the cache. inv_freq [D/2] + pos [B]: q (and the appended k) are rotated here.
-// splits: 0 = chosen by pick_splits.
+// splits: 0 = chosen by pick_splits. pdl: the launch may overlap the end of its predecessor on the stream, which must not
+// write the caches or lens.
 extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
                                const long long* seq, const int* lens, const int* pos, const float* inv_freq, float attn_scale,
                                void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len, float scale,
-                               int window, int append, int splits, void* stream) {
+                               int window, int append, int splits, int pdl, void* stream) {
   if (B <= 0) return 0;
   if (Hk <= 0 || Hq % Hk || Hq / Hk > MAX_G || B > 65535) return -2;
   if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -3;
@@ -432,8 +409,8 @@ extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_
   p.append = append;
   if (splits == 0) splits = pick_splits(B, Hk, max_len);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (D == 64) return launch_decode<64>(p, B, splits, st);
-  if (D == 128) return launch_decode<128>(p, B, splits, st);
-  if (D == 256) return launch_decode<256>(p, B, splits, st);
+  if (D == 64) return launch_decode<64>(p, B, splits, pdl != 0, st);
+  if (D == 128) return launch_decode<128>(p, B, splits, pdl != 0, st);
+  if (D == 256) return launch_decode<256>(p, B, splits, pdl != 0, st);
   return -2;
 }

@@ -84,9 +84,13 @@ _CUDA_SIGS = {
     "axb_rmsnorm_gated_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp],
     "axb_entropy": [vp, vp, vp, i64, i32, i64, f32, vp],
     # qkv, ld, q_col0, k_col0, v_col0, k_cache, v_cache, seq, lens, pos, inv_freq, attn_scale, out, out_ld, B, Hq, Hk, D,
-    # max_len, scale, window, append, splits, stream
+    # max_len, scale, window, append, splits, pdl, stream
     "axb_decode_attn": [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, f32, vp, i64, i32, i32, i32, i32, i64, f32, i32, i32,
-                        i32, vp],
+                        i32, i32, vp],
+    # P, ldp, S, lds, C, ldc, R, N, K, P2, ldp2, S2, lds2, K2, alpha, bias, out_mode, out_f32, glu_kind, glu_limit, p_dep,
+    # splits, pdl, status, stream
+    "axb_gemm_skinny": [vp, i64, vp, i64, vp, i64, i32, i32, i32, vp, i64, vp, i64, i32, f32, vp, i32, i32, i32, f32, i32, i32,
+                        i32, vp, vp],
     "axb_sinkgd_step": [vp, i32, vp, vp, vp, i32, i32, i32, f32, f32, f32, vp],
     "axb_embedding_fwd": [vp, vp, vp, i64, i32, i64, vp],
     "axb_embedding_bwd": [vp, vp, vp, i64, i32, i64, vp],

@@ -735,7 +735,7 @@ def _decode_launch(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window, a
     _lib.check_rc(_lib.cuda_lib().axb_decode_attn(
         qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, k_cache.data_ptr(), v_cache.data_ptr(), _lib.ptr(seq),
         lens.data_ptr(), _lib.ptr(pos), _lib.ptr(inv_freq), attn_scale, out.data_ptr(), out.stride(0), B, Hq, Hk, D,
-        k_cache.shape[1], scale, int(window or 0), int(append), 0, _lib.stream_ptr()), "decode_attn")
+        k_cache.shape[1], scale, int(window or 0), int(append), 0, 0, _lib.stream_ptr()), "decode_attn")
     return out
 
 

@@ -135,6 +135,15 @@ def gemm(
         _glu_launch(lib, glu, a, int(trans_a), b.data_ptr(), b.stride(0), int(trans_b), out, M, N, K, a2, b2, K2,
                     alpha, (None, 0, 0, 0, None, 0))
         return out
+    if bn is None and _use_skinny(M, N, K, trans_a, trans_b, out, out_mode, c_in, beta):
+        rows, cols = (M, N) if N <= 64 else (N, M)      # the long side is the kernel's 128-row operand
+        p, s, p2, s2, mode = (a, b, a2, b2, 1) if N <= 64 else (b, a, b2, a2, 0)
+        rc = lib.axb_gemm_skinny(
+            p.data_ptr(), p.stride(0), s.data_ptr(), s.stride(0), out.data_ptr(), out.stride(0), rows, cols, K,
+            _lib.ptr(p2), p2.stride(0) if p2 is not None else 0, _lib.ptr(s2), s2.stride(0) if s2 is not None else 0, K2,
+            float(alpha), None, mode, out_mode, 0, 0.0, 1, 0, 0, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
+        _lib.check_rc(rc, "axb_gemm_skinny")
+        return out
     if bn is None:
         bn = _pick_bn(M, N)
     if not accumulate and _use_pair(M, N, bn):
@@ -189,6 +198,19 @@ def _glu_launch(lib, glu, a, trans_a, b_ptr, ldb, trans_b, out, M, N, K, a2, b2,
             _lib.ptr(b2), b2.stride(0) if b2 is not None else 0, K2, float(alpha), 2, int(kind),
             float(limit or 0.0), None, 0, *pf, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
     _lib.check_rc(rc, "axb_gemm_bf16_pair_glu")
+
+
+def _use_skinny(M, N, K, trans_a, trans_b, out, out_mode, c_in, beta) -> bool:
+    """The split-K cluster kernel of csrc/gemm_skinny.cu serves products with one side of a few columns, where 128-row tiles
+    leave most SMs without a CTA. Either N <= 64 (x A^T of an adapter; the old kernel / this one, microseconds with the L2
+    flushed: 512 x 4096 by 48 28.7 / 16.4, 960 x 14336 by 16 71.7 / 20.5, 8192 x 14336 by 16 75.8 / 55) up to the 8192 rows
+    that were measured, or M <= 128 (a generation step; 64 x 4096 by 6144 28.6 / 24.6, 64 x 14336 by 4096 72.5 / 36.9), but
+    above 32 rows only while the weight has fewer than 148 tiles of 128 rows (128 x 4096 by 128256 203.6 / 227.3)."""
+    if trans_a or trans_b or out_mode > 1 or (c_in is not None and beta != 0.0) or K < 512 or out.stride(1) != 1:
+        return False
+    if N <= 64:
+        return 128 < M <= 8192
+    return N >= 512 and (M <= 32 or (M <= 128 and (N + 127) // 128 < _SM))
 
 
 def _use_pair(M, N, bn) -> bool:

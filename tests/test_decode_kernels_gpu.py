@@ -53,7 +53,7 @@ def test_decode_attention_splits_append_and_rope(D, Hq, Hk, splits, window, appe
     _lib.check_rc(_lib.cuda_lib().axb_decode_attn(
         qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, kc.data_ptr(), vc.data_ptr(), seq.data_ptr(), n.data_ptr(),
         pos.data_ptr(), inv.data_ptr() if rope else None, 1.0, out.data_ptr(), out.stride(0), B, Hq, Hk, D, cap, scale, window,
-        int(append), splits, _lib.stream_ptr()), "decode_attn")
+        int(append), splits, 0, _lib.stream_ptr()), "decode_attn")
     q = qkv[:, :Hq * D].reshape(B, Hq, D)
     k = qkv[:, Hq * D:(Hq + Hk) * D].reshape(B, Hk, D)
     v = qkv[:, (Hq + Hk) * D:].reshape(B, Hk, D)
@@ -92,3 +92,46 @@ def test_cached_step_on_a_subset_of_the_sequences():
     assert torch.equal(cache.k[0], k0) and torch.equal(cache.v[0], v0)
     ref = Fn.decode_attention(qkv.cpu(), k0[seq].cpu(), v0[seq].cpu(), (pos + 1).int().cpu(), a.Hq, a.Hk, a.D, a.scale)
     assert (out.cpu().float() - ref.float()).abs().max() <= 2 ** -7 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("R,N,K,K2", [(128, 1, 64, 0), (200, 5, 72, 16), (1000, 17, 520, 48), (6144, 64, 4096, 0), (129, 100, 640, 8),
+                                      (384, 256, 1032, 64)])
+@pytest.mark.parametrize("splits", [0, 1, 3, 8])
+@pytest.mark.parametrize("mode,f32", [(0, False), (0, True), (1, False), (1, True), (2, False)])
+def test_skinny_gemm(R, N, K, K2, splits, mode, f32):
+    """Remainders of the 128-row tile, of the 64-wide K block and of the short side, all cluster sizes. fp32 sums in another
+    order: 2^-20 of the accumulated magnitude; bf16 results one rounding more (2^-8)."""
+    from axolotl_b200.ops import _lib
+
+    torch.manual_seed(R + N)
+    if mode == 2:
+        R = (R + 63) // 64 * 64
+    rows = 2 * R if mode == 2 else R
+    P, S = torch.randn(rows, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    P2 = torch.randn(rows, K2, device="cuda").bfloat16() if K2 else None
+    S2 = torch.randn(N, K2, device="cuda").bfloat16() if K2 else None
+    bias = torch.randn(R, device="cuda").bfloat16() if mode == 0 else None
+    acc = S.double() @ P.double().t()
+    mag = S.double().abs() @ P.double().abs().t()
+    if K2:
+        acc, mag = acc + S2.double() @ P2.double().t(), mag + S2.double().abs() @ P2.double().abs().t()
+    acc, mag = acc * 0.5, mag * 0.5
+    if bias is not None:
+        acc = acc + bias.double()
+    if mode == 2:
+        g, u = acc.chunk(2, -1)
+        ref = torch.nn.functional.silu(g) * u
+        tol = 2 ** -8 * ref.abs() + 2 ** -8 * (1 + g.abs() + u.abs()) * 2 ** -6 + 2 ** -14 * mag.chunk(2, -1)[0]
+    else:
+        ref, tol = acc, 2 ** -20 * mag + (0 if f32 else 2 ** -8 * acc.abs())
+    if mode == 1:
+        ref, tol = ref.t(), tol.t()
+    ld = ref.shape[1] + 3                                  # an odd output stride
+    buf = torch.full((ref.shape[0], ld), 7.0, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+    _lib.check_rc(_lib.cuda_lib().axb_gemm_skinny(
+        P.data_ptr(), K, S.data_ptr(), K, buf.data_ptr(), ld, R, N, K, _lib.ptr(P2), K2, _lib.ptr(S2), K2, K2, 0.5,
+        _lib.ptr(bias), mode, int(f32), 0, 0.0, 1, splits, 0, _lib.status_word().data_ptr(), _lib.stream_ptr()), "gemm_skinny")
+    _lib.check_status()
+    out = buf[:, :ref.shape[1]].double()
+    assert ((out - ref).abs() <= tol + 1e-30).all(), ((out - ref).abs() - tol).max()
+    assert (buf[:, ref.shape[1]:] == 7.0).all()
