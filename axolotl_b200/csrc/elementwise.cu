@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(NORM_T)
                        __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H,
                        float eps, float w_offset) {
   __shared__ float sh[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * H;
   const __nv_bfloat16* rr = res ? res + row * H : nullptr;
@@ -776,15 +778,25 @@ inline int grid_for(long long work, int threads, int cap = 148 * 16) {
 
 #define ST(s) reinterpret_cast<cudaStream_t>(s)
 
+static int rmsnorm_fwd_launch(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
+                              long long rows, int H, float eps, float w_offset, bool pdl, void* stream) {
+  if (H % 8) return -2;
+  if (rows <= 0) return 0;
+  AxbLaunch l(dim3((unsigned)rows), NORM_T, 0, ST(stream), 0, pdl);
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, rmsnorm_fwd_kernel, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
+                                           (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd, H, eps,
+                                           w_offset);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
 extern "C" int axb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y,
                                void* res_out, float* rstd, long long rows, int H, float eps,
                                float w_offset, void* stream) {
-  if (H % 8) return -2;
-  if (rows <= 0) return 0;
-  rmsnorm_fwd_kernel<<<(unsigned)rows, NORM_T, 0, ST(stream)>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
-      (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd, H, eps, w_offset);
-  return (int)cudaGetLastError();
+  return rmsnorm_fwd_launch(x, res, w, y, res_out, rstd, rows, H, eps, w_offset, false, stream);
+}
+// the same as a dependent launch: it may start before its predecessor on the stream has finished, and waits for it
+extern "C" int axb_rmsnorm_fwd_pdl(const void* x, const void* res, const void* w, void* y, void* res_out, long long rows,
+                                   int H, float eps, float w_offset, void* stream) {
+  return rmsnorm_fwd_launch(x, res, w, y, res_out, nullptr, rows, H, eps, w_offset, true, stream);
 }
 extern "C" int axb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd,
                                const void* dres, void* dx, float* dw, long long rows, int H,

@@ -21,6 +21,7 @@ from torch.utils.checkpoint import checkpoint
 from ..ops import functional as Fn
 from ..ops.lora import glu_mlp, linear
 from .config import ModelConfig
+from .decode_step import DecodeStep
 from .layers import FusedLinear, RMSNorm, adapters_enabled, make_norm
 
 IGNORE_INDEX = -100
@@ -799,13 +800,17 @@ class CausalLM(nn.Module):
         if captured is not None and 0 in capture_hidden:
             captured[0] = h
         hooks = self.hooks
+        step = DecodeStep.of(self, h, pos, attn_meta) if getattr(attn_meta, "kv_cache", None) is not None else None
         nvtx = self.nvtx and h.is_cuda
         for i, layer in enumerate(self.layers):
             if nvtx:
                 torch.cuda.nvtx.range_push(f"layer{i}")
             if hooks is not None:
                 hooks.pre_layer(i)
-            if self.gradient_checkpointing and self.training and torch.is_grad_enabled():
+            done = step.layer(layer, h, residual, inv_freq, self.attn_scale) if step is not None else None
+            if done is not None:
+                h, residual, aux = done
+            elif self.gradient_checkpointing and self.training and torch.is_grad_enabled():
                 if self.ckpt_store is not None:
                     from ..train.activation_memory import offloaded_checkpoint
 

@@ -135,3 +135,82 @@ def test_skinny_gemm(R, N, K, K2, splits, mode, f32):
     out = buf[:, :ref.shape[1]].double()
     assert ((out - ref).abs() <= tol + 1e-30).all(), ((out - ref).abs() - tol).max()
     assert (buf[:, ref.shape[1]:] == 7.0).all()
+
+
+_STEP_CASES = {
+    "llama": dict(),
+    "qwen3 q/k norms": dict(model_type="qwen3", head_dim=64),
+    "qwen2 biases": dict(model_type="qwen2", attention_bias=True),
+    "gelu, odd width": dict(hidden_act="gelu_pytorch_tanh", intermediate_size=360),
+    "window": dict(model_type="mistral", extra=dict(sliding_window=24)),
+    "wide groups": dict(num_attention_heads=8, num_key_value_heads=1, head_dim=128),
+}
+
+
+@pytest.mark.parametrize("name", sorted(_STEP_CASES))
+@pytest.mark.parametrize("batch,lora", [(1, False), (8, True), (33, False), (128, True)])
+def test_decode_layers_in_one_call_match_the_operator_path(name, batch, lora, monkeypatch):
+    """Hidden states, logits and cache of a step against the layer-by-layer operators; both round every intermediate to bf16,
+    so the difference is a few roundings (2^-8 each) of a normalised stream through three layers."""
+    from axolotl_b200.models import decode_step
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _DecodeMeta
+    from axolotl_b200.models.lora import ALL_LINEAR, LoraSpec, inject_lora
+    from axolotl_b200.models.transformer import CausalLM
+
+    torch.manual_seed(3)
+    cfg = preset("tiny-llama", vocab_size=512, num_hidden_layers=3, **_STEP_CASES[name])
+    m = CausalLM(cfg, dtype=torch.bfloat16, device="cuda").init_weights(0)
+    if lora:
+        inject_lora(m, LoraSpec(r=8, lora_alpha=16, target_modules=[t for t in ALL_LINEAR if t != "k_proj"]))
+    with torch.no_grad():
+        for n, p in m.named_parameters():
+            if "lora_B" in n or n.endswith("bias"):
+                p.normal_(0, 0.05)
+        for f in m.modules():
+            if getattr(f, "lora_B", None) is not None:     # off-diagonal blocks stay zero
+                keep = torch.zeros_like(f.lora_B)
+                for r0, rows, c0, cols in f.lora_blocks:
+                    keep[r0:r0 + rows, c0:c0 + cols] = 1
+                f.lora_B.mul_(keep)
+    m.refresh_lora_shadows()
+    m.eval()
+    lens = torch.randint(0, 60, (batch,))
+    pos = lens.cuda()
+    seq = torch.randperm(batch, device="cuda")
+    tok = torch.randint(0, 512, (batch,), device="cuda")
+    outs = []
+    k, v = torch.randn(2, 3, batch, 64, m.layers[0].self_attn.Hk * m.layers[0].self_attn.D, device="cuda").bfloat16()
+    for fused in (True, False):
+        cache = KVCache(m, batch, 64)
+        cache.k.copy_(k)
+        cache.v.copy_(v)
+        calls = []
+        if not fused:
+            monkeypatch.setattr(decode_step.DecodeStep, "of", staticmethod(lambda *a: None))
+        else:
+            real = decode_step.DecodeStep.layer
+            monkeypatch.setattr(decode_step.DecodeStep, "layer", lambda self, *a: calls.append(real(self, *a)) or calls[-1])
+        with torch.no_grad():
+            o = m(tok[None], pos.int()[None], attn_meta=_DecodeMeta(cache, seq, pos, False), return_logits=True, capture_hidden=[1, 2])
+        outs.append((o.logits.float(), o.hidden_states.float(), o.captured[2].float(), cache.k.float(), cache.v.float()))
+        if fused:
+            assert len(calls) == 3 and all(c is not None for c in calls)
+            monkeypatch.undo()
+    for a, b in zip(*outs):
+        assert ((a - b).norm() / b.norm()).item() < 0.012 and torch.isfinite(a).all()
+
+
+def test_decode_step_leaves_other_layers_to_their_own_forward():
+    """A forward hook, an expert layer and a disabled adapter: each keeps (or regains) the path that honours it."""
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import generate_cached
+    from axolotl_b200.models.transformer import CausalLM
+
+    m = CausalLM(preset("tiny-llama", vocab_size=512), dtype=torch.bfloat16, device="cuda").init_weights(0)
+    a = generate_cached(m, [[1, 5, 9], [7, 8]], 6)
+    seen = []
+    h = m.layers[1].mlp.down_proj.register_forward_hook(lambda mod, i, o: seen.append(o.shape[0]))
+    b = generate_cached(m, [[1, 5, 9], [7, 8]], 6)
+    h.remove()
+    assert len(seen) == 6 and a == b
