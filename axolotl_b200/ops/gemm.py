@@ -22,14 +22,23 @@ USE_PAIR = os.environ.get("AXB_GEMM_PAIR", "1") != "0"
 USE_GLU_EPILOGUE = os.environ.get("AXB_GLU_EPILOGUE", "1") != "0"
 
 
-def _pick_bn(M: int, N: int) -> int:
-    m_tiles = (M + 127) // 128
-    for bn in (256, 128, 64):
-        if bn > 64 and N <= bn // 2:
+def _pick_tile(M: int, N: int) -> tuple[int, bool]:
+    """(tile width, whether the CTA-pair kernel runs it): the choice with the least waves x time per wave. A K block of one
+    wave takes about the same 0.31 us with 128 x 64 and 128 x 128 tiles, 0.40 us with 128 x 256 (one CTA per SM each) and
+    0.34 us with the pair kernel's 256 x 256 (74 SM pairs), measured at K = 32000 with the L2 flushed; what decides is how
+    many waves a tile needs. 960 x 32000 by 4096: 580 / 304 / 200 / 173 us (10, 4, 2, 1 waves with 64, 128, 256, pair);
+    320 x 32000 by 4096: 292 / 157 / 196 / 163 us; 640 x 4096 by 14336: 163 / 93 / 73 / 77 us. Ties go to the wider tile,
+    which reads less."""
+    best = None
+    for bn, rows, slots, cost, pair in ((256, 256, _SM // 2, 1.10, True), (256, 128, _SM, 1.30, False), (128, 128, _SM, 1.0, False),
+                                        (64, 128, _SM, 0.99, False)):
+        if (pair and not USE_PAIR) or (bn > 64 and N <= bn // 2) or (pair and (M <= 128 or N < 256)):
             continue
-        if m_tiles * ((N + bn - 1) // bn) >= _SM or bn == 64:
-            return bn
-    return 64
+        tiles = -(-M // rows) * -(-N // bn)
+        t = -(-tiles // slots) * cost
+        if best is None or t < best[0]:
+            best = (t, bn, pair)
+    return best[1], best[2]
 
 
 def _row_major_2d(t: torch.Tensor) -> torch.Tensor:
@@ -144,9 +153,12 @@ def gemm(
             float(alpha), None, mode, out_mode, 0, 0.0, 1, 0, 0, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
         _lib.check_rc(rc, "axb_gemm_skinny")
         return out
-    if bn is None:
+    pair = False
+    if bn is None and accumulate:
         bn = _pick_bn(M, N)
-    if not accumulate and _use_pair(M, N, bn):
+    elif bn is None:
+        bn, pair = _pick_tile(M, N)
+    if pair:
         rc = lib.axb_gemm_bf16_pair(
             a.data_ptr(), a.stride(0), int(trans_a), b.data_ptr(), b.stride(0), int(trans_b),
             out.data_ptr(), out.stride(0), _lib.ptr(c_in), c_in.stride(0) if c_in is not None else 0, M, N, K,
@@ -172,9 +184,9 @@ def gemm(
 
 def glu_fusable(M: int, I: int, device) -> bool:
     """Whether the GLU epilogues of the CTA-pair kernel serve an MLP with ``M`` token rows and ``I``
-    intermediate columns (enough 256-row tiles for the 74 SM pairs, whole 32-column chunks)."""
-    return (USE_PAIR and USE_GLU_EPILOGUE and device.type == "cuda" and M >= 512 and I % 32 == 0
-            and ((M + 255) // 256) * ((I + 255) // 256) >= 74)
+    intermediate columns (whole 32-column chunks; more than one 128-row tile, below that the short-side kernel is the
+    faster one). They save a pass over gate|up whatever the number of tiles."""
+    return USE_PAIR and USE_GLU_EPILOGUE and device.type == "cuda" and M > 128 and I % 32 == 0 and I >= 256
 
 
 def _glu_launch(lib, glu, a, trans_a, b_ptr, ldb, trans_b, out, M, N, K, a2, b2, K2, alpha, pf):
@@ -214,9 +226,18 @@ def _use_skinny(M, N, K, trans_a, trans_b, out, out_mode, c_in, beta) -> bool:
 
 
 def _use_pair(M, N, bn) -> bool:
-    """The 2-CTA kernel (256x256 tile per SM pair, each CTA stages half of B) wins once there are
-    enough 256x256 tiles for the 74 SM pairs; small or skinny problems keep the 1-CTA kernel."""
-    return USE_PAIR and bn == 256 and M >= 512 and N >= 512 and ((M + 255) // 256) * ((N + 255) // 256) >= 74
+    return bn == 256 and _pick_tile(M, N)[1]
+
+
+def _pick_bn(M, N) -> int:
+    """Tile width of a split-K product (the split factor fills the SMs)."""
+    m_tiles = (M + 127) // 128
+    for bn in (256, 128, 64):
+        if bn > 64 and N <= bn // 2:
+            continue
+        if m_tiles * ((N + bn - 1) // bn) >= _SM or bn == 64:
+            return bn
+    return 64
 
 
 def pick_splits(out_tiles: int, k_blocks: int) -> int:
@@ -248,8 +269,9 @@ def _gemm_allgather(a, b_shard, info, *, trans_a, trans_b, a2, b2, alpha, beta, 
     out_mode = 0 if out_dtype == torch.bfloat16 else 1
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+    pair = False
     if bn is None:
-        bn = _pick_bn(M, N)
+        bn, pair = _pick_tile(M, N)
     ctx = info.ctx
     staging, plans = ctx.acquire(info, backward=trans_b)
     plan = None
@@ -267,7 +289,7 @@ def _gemm_allgather(a, b_shard, info, *, trans_a, trans_b, a2, b2, alpha, beta, 
         pf = (None, 0, 0, 0, None, 0)
     if glu is not None:
         _glu_launch(lib, glu, a, 0, staging.data_ptr(), cols, int(trans_b), out, M, N, K, a2, b2, K2, alpha, pf)
-    elif _use_pair(M, N, bn):
+    elif pair:
         rc = lib.axb_gemm_bf16_pair(
             a.data_ptr(), a.stride(0), 0, staging.data_ptr(), cols, int(trans_b), out.data_ptr(), out.stride(0),
             _lib.ptr(c_in), c_in.stride(0) if c_in is not None else 0, M, N, K,

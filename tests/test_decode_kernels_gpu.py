@@ -214,3 +214,29 @@ def test_decode_step_leaves_other_layers_to_their_own_forward():
     b = generate_cached(m, [[1, 5, 9], [7, 8]], 6)
     h.remove()
     assert len(seen) == 6 and a == b
+
+
+@pytest.mark.parametrize("M,N", [(129, 256), (129, 4096), (256, 320), (257, 2056), (300, 1000), (511, 4096), (640, 14336)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("c_in", [False, True])
+def test_gemm_tiles_chosen_below_512_rows(M, N, ta, tb, c_in):
+    """Problems that the CTA-pair kernel used to refuse: few rows, few tiles, ragged edges, all operand layouts and the
+    accumulating epilogue. fp32 sums of 264 products: 2^-20 of their magnitude."""
+    from axolotl_b200.ops import _lib
+    from axolotl_b200.ops.gemm import _pick_tile, gemm
+
+    torch.manual_seed(M + N)
+    K = 264
+    if (ta and M % 8) or (tb and N % 8):
+        pytest.skip("a transposed operand needs 16-byte rows")
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    aa, bb = a.t().contiguous() if ta else a, b.t().contiguous() if tb else b
+    ref, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    c = torch.randn(M, N, device="cuda") if c_in else None
+    want = ref + c.double() if c_in else ref
+    out = gemm(aa, bb, trans_a=ta, trans_b=tb, out_dtype=torch.float32, c_in=c, beta=1.0 if c_in else 0.0)
+    assert ((out.double() - want).abs() <= 2 ** -20 * (mag + want.abs())).all(), _pick_tile(M, N)
+    if not c_in:
+        o16 = gemm(aa, bb, trans_a=ta, trans_b=tb)
+        assert ((o16.double() - ref).abs() <= 2 ** -20 * mag + 2 ** -8 * ref.abs()).all()
+    _lib.check_status()
