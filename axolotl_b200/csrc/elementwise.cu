@@ -59,6 +59,13 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
          d = unpack_bf16x2(u.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+  const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+__device__ __forceinline__ uint4 packed8(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   uint4 u;
   u.x = pack_bf16x2(f[0], f[1]);
@@ -70,7 +77,10 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 
 // ---------------------------------------------------------------------------------- RMSNorm
 // h = x (+ res);  res_out = h (optional);  y = h * rstd * (w + w_offset)
+// Bound: HBM. A thread owns NV 16-byte vectors of a row (NV = 0: any number, in a loop), all requested before the first is
+// used, and keeps them packed while the row is summed: 8192 x 4096 with a residual 60 -> 49 us (4 x 67 MB, L2 flushed).
 constexpr int NORM_T = 256;
+template <int NV>
 __global__ void __launch_bounds__(NORM_T)
     rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
@@ -83,59 +93,189 @@ __global__ void __launch_bounds__(NORM_T)
   const __nv_bfloat16* xr = x + row * H;
   const __nv_bfloat16* rr = res ? res + row * H : nullptr;
   float ss = 0.f;
-  // H <= 8 * NORM_T * 4 supported by keeping up to 4 vectors per thread in registers
-  float cache[4][8];
-  int nv = 0;
-  for (int i = threadIdx.x * 8; i < H; i += NORM_T * 8, ++nv) {
-    float f[8];
-    load8(xr + i, f);
+  auto add = [&](uint4 a, uint4 b, float (&f)[8]) {        // x (+ res)
+    unpack8(a, f);
     if (rr) {
       float g[8];
-      load8(rr + i, g);
+      unpack8(b, g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += g[j];
     }
-    if (res_out) {
-      // round the residual stream to bf16 first so forward and backward see the same h (in
-      // registers: a store followed by a load of the same address would wait for a trip to L2)
-      uint4 u;
-      u.x = pack_bf16x2(f[0], f[1]);
-      u.y = pack_bf16x2(f[2], f[3]);
-      u.z = pack_bf16x2(f[4], f[5]);
-      u.w = pack_bf16x2(f[6], f[7]);
-      *reinterpret_cast<uint4*>(res_out + row * H + i) = u;
-      const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-      f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+  };
+  if constexpr (NV > 0) {
+    uint4 a[NV], b[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = (k * NORM_T + threadIdx.x) * 8;
+      a[k] = b[k] = make_uint4(0, 0, 0, 0);
+      if (i < H) {
+        a[k] = *reinterpret_cast<const uint4*>(xr + i);
+        if (rr) b[k] = *reinterpret_cast<const uint4*>(rr + i);
+      }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      ss += f[j] * f[j];
-      if (nv < 4) cache[nv][j] = f[j];
-    }
-  }
-  ss = block_sum<NORM_T>(ss, sh);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-  int k = 0;
-  for (int i = threadIdx.x * 8; i < H; i += NORM_T * 8, ++k) {
-    float f[8], wv[8];
-    if (k < 4) {
+    for (int k = 0; k < NV; ++k) {
+      const int i = (k * NORM_T + threadIdx.x) * 8;
+      float f[8];
+      add(a[k], b[k], f);
+      if (res_out) {
+        // the residual stream is rounded to bf16 first so that forward and backward see the same h
+        a[k] = packed8(f);
+        if (i < H) *reinterpret_cast<uint4*>(res_out + row * H + i) = a[k];
+        unpack8(a[k], f);
+      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = cache[k][j];
-    } else {
-      load8((res_out ? res_out + row * H : xr) + i, f);
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
     }
-    load8(w + i, wv);
+    ss = block_sum<NORM_T>(ss, sh);
+    const float rstd = rsqrtf(ss / H + eps);
+    if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * (wv[j] + w_offset);
-    store8(y + row * H + i, f);
+    for (int k = 0; k < NV; ++k) {
+      const int i = (k * NORM_T + threadIdx.x) * 8;
+      if (i >= H) continue;
+      float f[8], wv[8];
+      if (res_out) unpack8(a[k], f);
+      else add(a[k], b[k], f);
+      load8(w + i, wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * (wv[j] + w_offset);
+      store8(y + row * H + i, f);
+    }
+  } else {
+    for (int i = threadIdx.x * 8; i < H; i += NORM_T * 8) {
+      float f[8];
+      add(*reinterpret_cast<const uint4*>(xr + i), rr ? *reinterpret_cast<const uint4*>(rr + i) : make_uint4(0, 0, 0, 0), f);
+      if (res_out) {
+        const uint4 u = packed8(f);
+        *reinterpret_cast<uint4*>(res_out + row * H + i) = u;
+        unpack8(u, f);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+    ss = block_sum<NORM_T>(ss, sh);
+    const float rstd = rsqrtf(ss / H + eps);
+    if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
+    for (int i = threadIdx.x * 8; i < H; i += NORM_T * 8) {
+      float f[8], wv[8];
+      if (res_out) load8(res_out + row * H + i, f);
+      else add(*reinterpret_cast<const uint4*>(xr + i), rr ? *reinterpret_cast<const uint4*>(rr + i) : make_uint4(0, 0, 0, 0), f);
+      load8(w + i, wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * (wv[j] + w_offset);
+      store8(y + row * H + i, f);
+    }
   }
 }
 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres). Each thread owns fixed columns, so the
 // weight gradient is accumulated in registers over the rows of the block and flushed once.
+// Bound: HBM. The blocks stay resident and walk over rows; the three inputs of the next row are requested before the
+// present row's reduction, so that a block always has loads in flight, and the row is read once (packed in registers). The
+// flush goes through shared memory, whole 128-byte lines per warp: the strided atomics of eight blocks per SM cost more
+// than the pass itself. 8192 x 4096 83 -> 54 us; 4096 x 2048 with a weight gradient 115 -> 28 us (L2 flushed).
+template <int NV, bool DW>
 __global__ void __launch_bounds__(NORM_T)
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
+                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
+                       const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                       float* __restrict__ dw, int H, int rows, float w_offset) {
+  __shared__ float sh[2][NORM_T / 32];
+  __shared__ float s_dw[DW ? NORM_T * 8 : 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float dw_acc[DW ? NV : 1][8];
+  if (DW) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dw_acc[k][j] = 0.f;
+  }
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 wv[NV], a[NV], b[NV], d[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = (k * NORM_T + threadIdx.x) * 8;
+    wv[k] = i < H ? *reinterpret_cast<const uint4*>(w + i) : zero;
+  }
+  float rstd = 0.f;
+  auto fetch = [&](long long row) {
+    rstd = rstd_in[row];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = (k * NORM_T + threadIdx.x) * 8;
+      a[k] = b[k] = d[k] = zero;
+      if (i < H) {
+        a[k] = *reinterpret_cast<const uint4*>(dy + row * H + i);
+        b[k] = *reinterpret_cast<const uint4*>(h + row * H + i);
+        if (dres) d[k] = *reinterpret_cast<const uint4*>(dres + row * H + i);
+      }
+    }
+  };
+  long long row = blockIdx.x;
+  if (row < rows) fetch(row);
+  int turn = 0;
+  for (; row < rows; row += gridDim.x, turn ^= 1) {
+    uint4 ca[NV], cb[NV], cd[NV];
+    const float rs = rstd;
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      ca[k] = a[k];
+      cb[k] = b[k];
+      cd[k] = d[k];
+      float fa[8], fb[8], fw[8];
+      unpack8(ca[k], fa);
+      unpack8(cb[k], fb);
+      unpack8(wv[k], fw);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dot += fa[j] * (fw[j] + w_offset) * fb[j] * rs;
+    }
+    if (row + gridDim.x < rows) fetch(row + gridDim.x);
+    dot = warp_sum(dot);
+    if (lane == 0) sh[turn][warp] = dot;        // two slots in turn: one barrier per row
+    __syncthreads();
+    dot = 0.f;
+#pragma unroll
+    for (int q = 0; q < NORM_T / 32; ++q) dot += sh[turn][q];
+    dot /= H;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = (k * NORM_T + threadIdx.x) * 8;
+      if (i >= H) continue;
+      float fa[8], fb[8], fw[8], o[8];
+      unpack8(ca[k], fa);
+      unpack8(cb[k], fb);
+      unpack8(wv[k], fw);
+      unpack8(cd[k], o);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = fb[j] * rs;
+        const float g = rs * (fa[j] * (fw[j] + w_offset) - xhat * dot);
+        if (DW) dw_acc[k][j] += fa[j] * xhat;
+        o[j] = dres ? o[j] + g : g;
+      }
+      store8(dx + row * H + i, o);
+    }
+  }
+  if constexpr (DW) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s_dw[threadIdx.x * 8 + j] = dw_acc[k][j];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = k * NORM_T * 8 + j * NORM_T + threadIdx.x;
+        if (i < H) atomicAdd(dw + i, s_dw[j * NORM_T + threadIdx.x]);
+      }
+    }
+  }
+}
+// rows wider than 4 x 2048 elements: the first four vectors of a thread accumulate their weight gradient in registers
+__global__ void __launch_bounds__(NORM_T)
+    rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                        float* __restrict__ dw, int H, int rows, float w_offset) {
@@ -783,7 +923,9 @@ static int rmsnorm_fwd_launch(const void* x, const void* res, const void* w, voi
   if (H % 8) return -2;
   if (rows <= 0) return 0;
   AxbLaunch l(dim3((unsigned)rows), NORM_T, 0, ST(stream), 0, pdl);
-  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, rmsnorm_fwd_kernel, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
+  const int nv = (H / 8 + NORM_T - 1) / NORM_T;
+  auto kern = nv == 1 ? rmsnorm_fwd_kernel<1> : (nv == 2 ? rmsnorm_fwd_kernel<2> : (nv <= 4 ? rmsnorm_fwd_kernel<4> : rmsnorm_fwd_kernel<0>));
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, kern, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
                                            (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd, H, eps,
                                            w_offset);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
@@ -803,8 +945,17 @@ extern "C" int axb_rmsnorm_bwd(const void* dy, const void* h, const void* w, con
                                float w_offset, void* stream) {
   if (H % 8) return -2;
   if (rows <= 0) return 0;
-  const int grid = rows < 148 * 8 ? (int)rows : 148 * 8;
-  rmsnorm_bwd_kernel<<<grid, NORM_T, 0, ST(stream)>>>(
+  const int nv = (H / 8 + NORM_T - 1) / NORM_T;
+  auto kern = rmsnorm_bwd_wide_kernel;
+  int per_sm = 8;
+  if (nv <= 4) {
+    kern = nv == 1 ? (dw ? rmsnorm_bwd_kernel<1, true> : rmsnorm_bwd_kernel<1, false>)
+         : nv == 2 ? (dw ? rmsnorm_bwd_kernel<2, true> : rmsnorm_bwd_kernel<2, false>)
+                   : (dw ? rmsnorm_bwd_kernel<4, true> : rmsnorm_bwd_kernel<4, false>);
+    per_sm = nv == 4 ? 2 : 4;      // resident blocks: their row loops keep the loads in flight, more only add flushes
+  }
+  const int grid = rows < 148 * per_sm ? (int)rows : 148 * per_sm;
+  kern<<<grid, NORM_T, 0, ST(stream)>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd,
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw, H, (int)rows, w_offset);
   return (int)cudaGetLastError();
