@@ -44,3 +44,28 @@ def test_rmsnorm_kernels(H, rows, res, dw):
     if dw:
         t = dyd * xh
         assert ((g.double() - g0 - t.sum(0)).abs() <= 2 ** -18 * (t.abs().sum(0) + g0.abs())).all()
+
+
+@pytest.mark.parametrize("D,Hq,Hk", [(64, 3, 1), (64, 9, 9), (64, 16, 2), (128, 12, 2), (128, 5, 5)])
+@pytest.mark.parametrize("lens", [[1], [31, 2], [33, 64, 130], [400, 257]])
+@pytest.mark.parametrize("window,causal", [(0, True), (70, True), (0, False)])
+def test_attention_head_and_token_remainders(D, Hq, Hk, lens, window, causal):
+    """Head counts that are not multiples of a block's, odd and even groups, lengths around the 32-, 64-, 128- and 256-row
+    tiles: output and gradients against fp32 autograd. bf16 operands, probabilities and gradients: 2^-6 of the largest
+    element, 2^-7 in the norm."""
+    torch.manual_seed(D + Hq)
+    T = sum(lens)
+    qkv = torch.randn(T, (Hq + 2 * Hk) * D, device="cuda").bfloat16().requires_grad_(True)
+    do = torch.randn(T, Hq * D, device="cuda").bfloat16()
+    meta = Fn.AttnMeta(np.concatenate([[0], np.cumsum(lens)]), "cuda", causal)
+    meta = meta.windowed(window) if window else meta
+    o = Fn.flash_varlen(qkv, meta, Hq, Hk, D)
+    (g,) = torch.autograd.grad(o, qkv, do)
+    x = qkv.detach().float().requires_grad_(True)
+    q, k, v = (t.reshape(T, -1, D) for t in x.split([Hq * D, Hk * D, Hk * D], -1))
+    ref = Fn._attn_ref(q, k, v, meta.cu_seqlens_host, D ** -0.5, causal, window).reshape(T, -1)
+    (gr,) = torch.autograd.grad(ref, x, do.float())
+    for a, b in ((o.detach().float(), ref.detach()), (g.float(), gr)):
+        assert ((a - b).abs() <= 2 ** -6 * b.abs().max()).all()
+        assert ((a - b).norm() / b.norm()).item() < 2 ** -7
+    _lib.check_status()
