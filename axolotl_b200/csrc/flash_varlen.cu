@@ -5,8 +5,8 @@
 // projection buffer [T, (Hq + 2*Hk) * D] (bf16), documents are delimited by a host-built tile
 // table (one entry per (document, 128-row tile)), so no [S,S] mask and no cross-document
 // attention ever exists. Both kernels are warp-specialised:
-//   warp 0: TMA producer, warp 1: tcgen05.mma issuer, warps 2-5: softmax / gradient math
-// with S, P.V (forward) and S^T, dP^T, dK, dV, dQ^T (backward) accumulators living in TMEM.
+//   warp 0: TMA producer, warp 1: tcgen05.mma issuer, warps 2-9: softmax / gradient math
+// with S, P, O (forward) and S^T, dP^T, dK, dV, dQ^T (backward) accumulators living in TMEM.
 //
 // Replaces flash-attn varlen (FA2/FA4) that the reference reaches through HF's
 // flash_attention_2 interface (src/axolotl/monkeypatch/attention/flash_attn_4.py:37-111) and its
@@ -16,7 +16,6 @@
 
 namespace {
 
-constexpr int kThreads = 192;
 constexpr int HALF_BYTES = 128 * 128;  // 128 rows x 128 B (64 bf16) swizzled tile
 
 struct AttnParams {
@@ -49,6 +48,8 @@ struct AttnParams {
   // backward: the q heads of one kv head may be split over `kv_split` CTAs (load balance for wide
   // GQA groups); their dK / dV partial tiles are then reduce-added into a pre-zeroed buffer
   int kv_split;
+  // forward: the two units of a CTA. 0: one unit, 1: two q heads of a kv head, 2: two neighbouring q tiles of a head
+  int pair_mode;
 };
 
 AXB_DEVICE float fast_exp2(float x) {
@@ -65,70 +66,82 @@ AXB_DEVICE uint32_t sw128_chunk_off(int row, int chunk) {
 // =====================================================================================
 // Forward
 // =====================================================================================
+// A CTA works on two 128-row units of queries against one stream of K / V tiles: two q heads of the same kv head at the same
+// rows (GQA groups of even size), or two neighbouring q tiles of one head. Each unit has its own softmax warpgroup and its own
+// S and O in TMEM, [S0 | S1 | O0 | O1]; while one warpgroup exponentiates, the tensor core runs the other unit's P.V and next
+// scores, and K / V are read once for both. P (bf16) overwrites the first half of its S columns and is the TMEM operand of
+// P.V, so it never passes through shared memory. O accumulates in TMEM; it is rescaled only when a row's maximum has grown by
+// more than 2^8 (P then stays below 2^8, its relative rounding and the fp32 sums are what they were), which a row meets a
+// handful of times: l and P use the same reference maximum, so the result does not depend on when that happens.
+// Bound: exponentials (16 per clock and SM against 1024 clocks of MMA per 128 x 128 block) and the MMA stream, about level.
+// One 16384-token document, 32 / 8 heads of 128: 3.02 -> 1.87 ms (730 -> 1180 TFLOP/s) against one softmax warpgroup with O in
+// registers and P through shared memory; 4 x 2048 267 -> 184 us; 11 x 707 windowed, 64 heads of 64, 229 -> 155 us.
+// TMA warp, MMA warp, two idle warps (they complete the warpgroup that gives registers away), 2 x 4 softmax warps. A row of S
+// is held in 128 registers: the 384 x 168 registers of the launch are split 128 x 40 + 256 x 232.
+constexpr int kFwdThreads = 384;
 template <int D>
 struct FwdCfg {
   static constexpr int HALVES = D / 64;
   static constexpr int TILE_BYTES = HALVES * HALF_BYTES;  // Q / K / V tile of 128 rows
-  static constexpr int P_BYTES = 2 * HALF_BYTES;          // P [128 x 128]
   static constexpr int KV_STAGES = 2;
-  static constexpr int SMEM = TILE_BYTES * (1 + 2 * KV_STAGES) + P_BYTES + 1024 + 256;
+  static constexpr int SMEM = TILE_BYTES * (2 + 2 * KV_STAGES) + 1024 + 256;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int S_COL = 0;      // S buffers: 2 x 128 columns
-  static constexpr int PV_COL = 256;   // PV buffers: 2 x D columns
+  static constexpr int O_COL = 256;    // O of unit u at O_COL + u * D; S (and P) of unit u at u * 128
 };
 
 template <int D>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kFwdThreads, 1)
     flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_qkv,
                      const AttnParams p) {
   using C = FwdCfg<D>;
   const int tile_id = blockIdx.y;
   if (tile_id >= p.n_tiles) return;
-  const int head = blockIdx.x;
-  const int kv_head = head / (p.Hq / p.Hk);
   const int4 ti = p.tiles[tile_id];
   const int doc_start = ti.x, doc_len = ti.y, q0 = ti.z;
   if (!AXB_INDEX_OK(AXB_SITE_ATTN_TILE, (long long)doc_start + doc_len - 1, p.kv_rows) || !AXB_INDEX_OK(AXB_SITE_ATTN_TILE, q0, doc_len)) return;
+  if (p.pair_mode == 2 && (q0 & 128)) return;   // the tile above takes these rows along
   const bool bidir = ti.w & 1;  // every token of the document sees the whole document
   const int win = bidir ? 0 : (ti.w >> 1);  // sliding window: row q sees kv rows (q - win, q]; 0 = unlimited
-  const int kv_end = bidir ? doc_len : min(q0 + 128, doc_len);
-  const int jb0 = win > 0 ? max(0, q0 - win + 1) / 128 : 0;  // first kv block any row of the tile can see
-  const int n_blocks = (kv_end + 127) / 128 - jb0;           // kv blocks visited: jb0 .. jb0 + n_blocks - 1
+  const int head0 = p.pair_mode == 1 ? 2 * (int)blockIdx.x : (int)blockIdx.x;
+  const int kv_head = head0 / (p.Hq / p.Hk);
+  const int jb0 = win > 0 ? max(0, q0 - win + 1) / 128 : 0;  // first kv block any row of the first unit can see
+  // kv blocks jb0 .. jb0 + n - 1 of a unit (0: no such unit)
+  auto blocks_of = [&](int unit) -> int {
+    if (unit == 1 && (p.pair_mode == 0 || (p.pair_mode == 2 && q0 + 128 >= doc_len))) return 0;
+    const int top = p.pair_mode == 2 && unit == 1 ? q0 + 256 : q0 + 128;
+    return ((bidir ? doc_len : min(top, doc_len)) + 127) / 128 - jb0;
+  };
+  const int n_u0 = blocks_of(0), n_u1 = blocks_of(1), n_max = max(n_u0, n_u1);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + C::TILE_BYTES;
+  uint8_t* sQ = smem;                                // [2 units]
+  uint8_t* sK = sQ + 2 * C::TILE_BYTES;
   uint8_t* sV = sK + C::KV_STAGES * C::TILE_BYTES;
-  uint8_t* sP = sV + C::KV_STAGES * C::TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + C::P_BYTES);
-  uint64_t* q_full = bars + 0;
-  uint64_t* k_full = bars + 1;    // [2]
-  uint64_t* v_full = bars + 3;    // [2]
-  uint64_t* kv_empty = bars + 5;  // [2]
-  uint64_t* s_full = bars + 7;    // [2]
-  uint64_t* s_empty = bars + 9;   // [2]
-  uint64_t* p_full = bars + 11;
-  uint64_t* p_empty = bars + 12;
-  uint64_t* pv_full = bars + 13;   // [2]
-  uint64_t* pv_empty = bars + 15;  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + C::KV_STAGES * C::TILE_BYTES);
+  uint64_t* q_full = bars + 0;    // [unit]
+  uint64_t* k_full = bars + 2;    // [stage]
+  uint64_t* v_full = bars + 4;    // [stage]
+  uint64_t* k_empty = bars + 6;   // [stage]
+  uint64_t* v_empty = bars + 8;   // [stage]
+  uint64_t* s_full = bars + 10;   // [unit]  scores ready; every MMA issued before them has retired, P.V of the block before included
+  uint64_t* p_full = bars + 12;   // [unit]  P written (S read, O rescaled)
+  uint64_t* o_full = bars + 14;   // [unit]  O final
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
       mbar_init(&k_full[s], 1);
       mbar_init(&v_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_empty[s], 1);
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_empty[s], 128);
-      mbar_init(&pv_full[s], 1);
-      mbar_init(&pv_empty[s], 128);
+      mbar_init(&p_full[s], 128);
+      mbar_init(&o_full[s], 1);
     }
-    mbar_init(p_full, 128);
-    mbar_init(p_empty, 1);
     mbar_fence_init();
     tma_prefetch_desc(&tm_qkv);
   }
@@ -141,220 +154,188 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(q_full, C::TILE_BYTES);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 0 && lane == 0) {
+      auto load = [&](uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int col, int row) {
+        mbar_expect_tx(bar, C::TILE_BYTES);
 #pragma unroll
-      for (int h = 0; h < C::HALVES; ++h)
-        tma_load_2d(sQ + h * HALF_BYTES, &tm_q, q_full, p.q_col0 + head * D + h * 64,
-                    doc_start + q0 - p.q_row_off);
-      for (int j = 0; j < n_blocks; ++j) {
+        for (int h = 0; h < C::HALVES; ++h) tma_load_2d(dst + h * HALF_BYTES, m, bar, col + h * 64, row);
+      };
+      const int qrow = doc_start + q0 - p.q_row_off;
+      load(sQ, &tm_q, &q_full[0], p.q_col0 + head0 * D, qrow);
+      for (int j = 0; j < n_max; ++j) {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&kv_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
-        mbar_expect_tx(&k_full[st], C::TILE_BYTES);
-#pragma unroll
-        for (int h = 0; h < C::HALVES; ++h)
-          tma_load_2d(sK + st * C::TILE_BYTES + h * HALF_BYTES, &tm_qkv, &k_full[st],
-                      p.k_col0 + kv_head * D + h * 64, doc_start + (jb0 + j) * 128);
-        mbar_expect_tx(&v_full[st], C::TILE_BYTES);
-#pragma unroll
-        for (int h = 0; h < C::HALVES; ++h)
-          tma_load_2d(sV + st * C::TILE_BYTES + h * HALF_BYTES, &tm_qkv, &v_full[st],
-                      p.v_col0 + kv_head * D + h * 64, doc_start + (jb0 + j) * 128);
+        const int row = doc_start + (jb0 + j) * 128;
+        if (!mbar_wait(&k_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+        load(sK + st * C::TILE_BYTES, &tm_qkv, &k_full[st], p.k_col0 + kv_head * D, row);
+        if (j == 0 && n_u1 > 0)
+          load(sQ + C::TILE_BYTES, &tm_q, &q_full[1], p.q_col0 + (p.pair_mode == 1 ? head0 + 1 : head0) * D,
+               p.pair_mode == 2 ? qrow + 128 : qrow);
+        if (!mbar_wait(&v_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+        load(sV + st * C::TILE_BYTES, &tm_qkv, &v_full[st], p.v_col0 + kv_head * D, row);
       }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    } else if (warp == 1 && lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);  // Q (K-major) x K (K-major)
-      constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);   // P (K-major) x V (MN-major)
-      const uint32_t q_addr = smem_u32(sQ);
-      const uint32_t p_addr = smem_u32(sP);
-      bool ok = mbar_wait(q_full, 0, p.status, AXB_TIMEOUT_FULL);
-      auto issue_s = [&](int j) -> bool {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&k_full[st], ph, p.status, AXB_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(&s_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + st * C::TILE_BYTES);
+      constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);   // P (TMEM) x V (MN-major)
+      auto issue_s = [&](int u, int j) {
+        const uint32_t q_addr = smem_u32(sQ + u * C::TILE_BYTES), k_addr = smem_u32(sK + (j & 1) * C::TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + C::S_COL + st * 128, make_smem_desc_sw128(q_addr + off, 16, 1024),
+          umma_f16(tmem_base + u * 128, make_smem_desc_sw128(q_addr + off, 16, 1024),
                    make_smem_desc_sw128(k_addr + off, 16, 1024), idesc_s, kk > 0);
         }
-        umma_commit(&s_full[st]);
-        return true;
+        umma_commit(&s_full[u]);
       };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (j + 1 < n_blocks) {
-          ok = issue_s(j + 1);
-          if (!ok) break;
-        }
-        if (!mbar_wait(p_full, j & 1, p.status, AXB_TIMEOUT_GENERIC)) break;
-        if (!mbar_wait(&v_full[st], ph, p.status, AXB_TIMEOUT_FULL)) break;
-        if (!mbar_wait(&pv_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        const uint32_t v_addr = smem_u32(sV + st * C::TILE_BYTES);
+      auto issue_pv = [&](int u, int j) {
+        const uint32_t v_addr = smem_u32(sV + (j & 1) * C::TILE_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {  // 128 kv rows / 16
-          const uint32_t poff = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + C::PV_COL + st * D, make_smem_desc_sw128(p_addr + poff, 16, 1024),
-                   make_smem_desc_sw128(v_addr + kk * 2048, HALF_BYTES, 1024), idesc_pv, kk > 0);
+        for (int kk = 0; kk < 8; ++kk)   // 128 kv rows / 16: 8 TMEM columns of P each
+          umma_f16_ts(tmem_base + C::O_COL + u * D, tmem_base + u * 128 + kk * 8,
+                      make_smem_desc_sw128(v_addr + kk * 2048, HALF_BYTES, 1024), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+      };
+      bool ok = mbar_wait(&q_full[0], 0, p.status, AXB_TIMEOUT_FULL) && mbar_wait(&k_full[0], 0, p.status, AXB_TIMEOUT_FULL);
+      if (ok) {
+        tc_fence_after();
+        issue_s(0, 0);
+        if (n_u1 > 0) {
+          ok = mbar_wait(&q_full[1], 0, p.status, AXB_TIMEOUT_FULL);
+          if (ok) {
+            tc_fence_after();
+            issue_s(1, 0);
+          }
         }
-        umma_commit(&pv_full[st]);
-        umma_commit(&kv_empty[st]);
-        umma_commit(p_empty);
+        umma_commit(&k_empty[0]);
+      }
+      for (int j = 0; j < n_max && ok; ++j) {
+        const int st = j & 1, nst = st ^ 1;
+        bool v_ready = false, k_ready = false;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int n_u = u == 0 ? n_u0 : n_u1;
+          if (j >= n_u || !ok) continue;
+          ok = mbar_wait(&p_full[u], j & 1, p.status, AXB_TIMEOUT_GENERIC);
+          if (ok && !v_ready) ok = mbar_wait(&v_full[st], (j >> 1) & 1, p.status, AXB_TIMEOUT_FULL);
+          if (!ok) break;
+          v_ready = true;
+          tc_fence_after();
+          issue_pv(u, j);
+          if (j == n_u - 1) umma_commit(&o_full[u]);
+          if (j + 1 < n_u) {
+            if (!k_ready) ok = mbar_wait(&k_full[nst], ((j + 1) >> 1) & 1, p.status, AXB_TIMEOUT_FULL);
+            if (!ok) break;
+            k_ready = true;
+            tc_fence_after();
+            issue_s(u, j + 1);     // over P(j), which the P.V before it has read
+          }
+        }
+        if (!ok) break;
+        umma_commit(&v_empty[st]);
+        if (j + 1 < n_max) umma_commit(&k_empty[nst]);
       }
     }
   } else {
-    // ---------------------------------------------------------------- softmax warps
+    // ---------------------------------------------------------------- softmax warpgroups
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int u = (warp - 4) >> 2;
     const int lg = warp & 3;
-    const int r = lg * 32 + lane;  // row inside the tile
-    const int q_idx = q0 + r;
+    const int r = lg * 32 + lane;  // row inside the unit
+    const int n_u = u == 0 ? n_u0 : n_u1;
+    const int qu0 = p.pair_mode == 2 ? q0 + u * 128 : q0;
+    const int head = p.pair_mode == 1 ? head0 + u : head0;
+    const int q_idx = qu0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
-    float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
-    float o[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) o[i] = 0.f;
+    const uint32_t s_addr = tmem_base + lane_off + u * 128, o_addr = tmem_base + lane_off + C::O_COL + u * D;
+    float m = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      const int st = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[st], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+    for (int j = 0; j < n_u && ok; ++j) {
+      if (!mbar_wait(&s_full[u], j & 1, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      const uint32_t s_addr = tmem_base + lane_off + C::S_COL + st * 128;
+      uint32_t sr[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, sr[c]);
+      tmem_ld_wait();
       const int kv0 = (jb0 + j) * 128;
-      const bool need_mask = (j == n_blocks - 1) || (win > 0 && kv0 < q0 + 128 - win);
-      const int lim = (bidir ? doc_len - 1 : min(q_idx, doc_len - 1)) - kv0;  // columns <= lim are visible
-      const int lo = win > 0 ? q_idx - win + 1 - kv0 : -(1 << 30);            // columns >= lo are visible
-      float mx = -INFINITY;
-      // two compiled variants of each pass: interior blocks carry no per-element compares
-      auto max_pass = [&](auto masked) {
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t sr[32];
-          tmem_ld_32x32(s_addr + c * 32, sr);
-          tmem_ld_wait();
+      if ((j == n_u - 1) || (win > 0 && kv0 < qu0 + 128 - win)) {
+        const int lim = (bidir ? doc_len - 1 : min(q_idx, doc_len - 1)) - kv0;  // columns <= lim are visible
+        const int lo = win > 0 ? q_idx - win + 1 - kv0 : -(1 << 30);            // columns >= lo are visible
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float v = __uint_as_float(sr[i]);
-            if constexpr (decltype(masked)::value) {
-              if (c * 32 + i > lim || c * 32 + i < lo) v = -INFINITY;
-            }
-            mx = fmaxf(mx, v);
-          }
-        }
-      };
-      if (need_mask) max_pass(std::true_type{});
-      else max_pass(std::false_type{});
-      const float m_new = fmaxf(m, mx * p.sl2);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = fast_exp2(m - m_use);
-      if (!mbar_wait(p_empty, (j & 1) ^ 1, p.status, AXB_TIMEOUT_GENERIC)) {
-        ok = false;
-        break;
-      }
-      float rowsum = 0.f;
-      auto p_pass = [&](auto masked) {
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t sr[32];
-          tmem_ld_32x32(s_addr + c * 32, sr);
-          tmem_ld_wait();
-          uint32_t pk[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float v0 = __uint_as_float(sr[i]), v1 = __uint_as_float(sr[i + 1]);
-            float p0 = fast_exp2(v0 * p.sl2 - m_use), p1 = fast_exp2(v1 * p.sl2 - m_use);
-            if constexpr (decltype(masked)::value) {
-              if (c * 32 + i > lim || c * 32 + i < lo) p0 = 0.f;
-              if (c * 32 + i + 1 > lim || c * 32 + i + 1 < lo) p1 = 0.f;
-            }
-            rowsum += p0 + p1;
-            pk[i >> 1] = pack_bf16x2(p0, p1);
-          }
-          // columns [c*32, c*32+32) -> half c/2, 16-byte chunks (c%2)*4 .. +3
-          uint8_t* pbase = sP + (c >> 1) * HALF_BYTES;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 val = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
-            *reinterpret_cast<uint4*>(pbase + sw128_chunk_off(r, (c & 1) * 4 + q)) = val;
-          }
-        }
-      };
-      if (need_mask) p_pass(std::true_type{});
-      else p_pass(std::false_type{});
-      tc_fence_before();
-      mbar_arrive(&s_empty[st]);
-      fence_proxy_async_smem();
-      mbar_arrive(p_full);
-      l = l * alpha + rowsum;
-      m = m_new;
-      if (j > 0) {
-        const int pst = (j - 1) & 1;
-        const uint32_t pph = ((j - 1) >> 1) & 1;
-        if (!mbar_wait(&pv_full[pst], pph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t pv_addr = tmem_base + lane_off + C::PV_COL + pst * D;
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t vr[32];
-          tmem_ld_32x32(pv_addr + c * 32, vr);
-          tmem_ld_wait();
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            o[c * 32 + i] = o[c * 32 + i] * alpha_prev + __uint_as_float(vr[i]);
-        }
-        tc_fence_before();
-        mbar_arrive(&pv_empty[pst]);
+            if (c * 32 + i > lim || c * 32 + i < lo) sr[c][i] = 0xff800000u;    // -inf
       }
-      alpha_prev = alpha;
-    }
-    if (ok && n_blocks > 0) {
-      const int pst = (n_blocks - 1) & 1;
-      const uint32_t pph = ((n_blocks - 1) >> 1) & 1;
-      if (mbar_wait(&pv_full[pst], pph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-        tc_fence_after();
-        const uint32_t pv_addr = tmem_base + lane_off + C::PV_COL + pst * D;
-        const float inv_l = l > 0.f ? 1.f / l : 0.f;
-        const long long lrow = (long long)doc_start + q_idx - p.q_row_off;  // row in the local buffers
-        const bool row_ok = q_idx < doc_len && lrow >= 0 && lrow < p.q_rows;
-        __nv_bfloat16* orow = p.out + lrow * p.out_ld + (long long)head * D;
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sr[c][i]));
+      const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.sl2);
+      if (j == 0) {
+        m = m_new;
+      } else if (__any_sync(0xffffffffu, m_new > m + 8.f)) {
+        const float m_next = m_new > m + 8.f ? m_new : m;
+        const float alpha = m_next == m ? 1.f : fast_exp2(m - m_next);
+        m = m_next;
+        l *= alpha;
+#pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
-          uint32_t vr[32];
-          tmem_ld_32x32(pv_addr + c * 32, vr);
+          uint32_t o[32];
+          tmem_ld_32x32(o_addr + c * 32, o);
           tmem_ld_wait();
-          if (row_ok) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float f[8];
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x32(o_addr + c * 32, o);
+        }
+      }
+      const float m_use = m == -INFINITY ? 0.f : m;    // no visible column so far: every P is exp2(-inf) = 0
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-              for (int i = 0; i < 8; ++i)
-                f[i] = (o[c * 32 + q * 8 + i] * alpha_prev + __uint_as_float(vr[q * 8 + i])) *
-                       inv_l;
-              uint4 u;
-              u.x = pack_bf16x2(f[0], f[1]);
-              u.y = pack_bf16x2(f[2], f[3]);
-              u.z = pack_bf16x2(f[4], f[5]);
-              u.w = pack_bf16x2(f[6], f[7]);
-              *reinterpret_cast<uint4*>(orow + c * 32 + q * 8) = u;
-            }
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float p0 = fast_exp2(fmaf(__uint_as_float(sr[c][i]), p.sl2, -m_use));
+          const float p1 = fast_exp2(fmaf(__uint_as_float(sr[c][i + 1]), p.sl2, -m_use));
+          sum[i & 2] += p0;
+          sum[(i & 2) + 1] += p1;
+          pk[i >> 1] = pack_bf16x2(p0, p1);
+        }
+        tmem_st_32x16(s_addr + c * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&p_full[u]);
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    }
+    if (ok && n_u > 0 && mbar_wait(&o_full[u], 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      tc_fence_after();
+      const float inv_l = l > 0.f ? 1.f / l : 0.f;
+      const long long lrow = (long long)doc_start + q_idx - p.q_row_off;  // row in the local buffers
+      const bool row_ok = q_idx < doc_len && lrow >= 0 && lrow < p.q_rows;
+      __nv_bfloat16* orow = p.out + lrow * p.out_ld + (long long)head * D;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(o_addr + c * 32, o);
+        tmem_ld_wait();
+        if (row_ok) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(o[q * 8 + i]) * inv_l;
+            *reinterpret_cast<uint4*>(orow + c * 32 + q * 8) =
+                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
           }
         }
-        if (row_ok) p.lse2[(long long)head * p.q_rows + lrow] = m + log2f(l);
       }
+      if (row_ok) p.lse2[(long long)head * p.q_rows + lrow] = m + log2f(l);
     }
   }
   tc_fence_before();
@@ -824,8 +805,8 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tm, const AttnParams& p
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  dim3 grid(p.Hq, p.n_tiles);
-  kern<<<grid, kThreads, C::SMEM, st>>>(tq, tm, p);
+  dim3 grid(p.pair_mode == 1 ? p.Hq / 2 : p.Hq, p.n_tiles);
+  kern<<<grid, kFwdThreads, C::SMEM, st>>>(tq, tm, p);
   return (int)cudaGetLastError();
 }
 template <int D>
@@ -884,6 +865,12 @@ int flash_fwd_impl(const AttnGeom& g, int Hq, int Hk, int D, int q_col0, int k_c
   p.sl2 = softmax_scale * 1.4426950408889634f;
   p.scale = softmax_scale;
   p.status = status;
+  // Two heads share K / V and have the same blocks, so they pair wherever the group is even. Odd groups pair neighbouring q
+  // tiles; a table that holds only the tiles of a rank's rows may lack one of the two, so those run single units.
+  p.pair_mode = (Hq / Hk) % 2 == 0 ? 1 : (g.q_rows == g.kv_rows && g.q_row_off == 0 ? 2 : 0);
+  // A pair takes about 1.25 times a single unit's time, so with fewer pairs than three quarters of the SMs single units
+  // finish first (6 heads, 500 + 300 tokens: 18 us single, 23 us paired; 8 heads, 2 x 2048: 44 / 47 us).
+  if (2ll * 111 > (long long)Hq * n_tiles) p.pair_mode = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return D == 128 ? launch_fwd<128>(tq, tkv, p, st) : launch_fwd<64>(tq, tkv, p, st);
 }
