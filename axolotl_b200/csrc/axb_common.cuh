@@ -81,6 +81,13 @@ AXB_DEVICE bool elect_one() {
   return pred != 0;
 }
 
+// Issuing loops (TMA, MMA). The WHOLE warp walks them and one elected lane issues: with the loop inside `if (lane == 0)` the
+// compiler cannot keep addresses, descriptors and barrier words in uniform registers, and the moves to them bound the loop,
+// about 0.3 us for the four MMAs of a K block (128 x 64 and 128 x 128 tiles took the same time). For that the warp index has
+// to be known uniform, and every wait has to end the same way for all lanes.
+AXB_DEVICE int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+AXB_DEVICE bool warp_all(bool x) { return __all_sync(0xffffffffu, x); }
+
 // ------------------------------------------------------------------ mbarrier
 AXB_DEVICE void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

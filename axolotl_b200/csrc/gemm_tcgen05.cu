@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* tempty_bar = bars + 2 * C::STAGES + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
 
   const int n_workers = (int)gridDim.x - p.g_ctas - p.r_ctas;  // CTAs that run GEMM tiles
@@ -402,27 +402,27 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += n_workers) {
-        int m_blk, n_blk, split;
-        decode_tile(tile, num_m, num_n, p.splits, m_blk, n_blk, split, p.group_m);
-        const int kb0 = (int)((long long)nk_total * split / p.splits);
-        const int kb1 = (int)((long long)nk_total * (split + 1) / p.splits);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += n_workers) {
+      int m_blk, n_blk, split;
+      decode_tile(tile, num_m, num_n, p.splits, m_blk, n_blk, split, p.group_m);
+      const int kb0 = (int)((long long)nk_total * split / p.splits);
+      const int kb1 = (int)((long long)nk_total * (split + 1) / p.splits);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!warp_all(mbar_wait(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
+          ok = false;
+          break;
+        }
+        const bool ext = kb >= nk_main;
+        const CUtensorMap* ma = ext ? &tmA2 : &tmA;
+        const CUtensorMap* mb = ext ? &tmB2 : &tmB;
+        const int k0 = (ext ? kb - nk_main : kb) * BK;
+        uint8_t* a_dst = sA + stage * C::A_BYTES;
+        uint8_t* b_dst = sB + stage * C::B_BYTES;
+        if (elect_one()) {
           mbar_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-          const bool ext = kb >= nk_main;
-          const CUtensorMap* ma = ext ? &tmA2 : &tmA;
-          const CUtensorMap* mb = ext ? &tmB2 : &tmB;
-          const int k0 = (ext ? kb - nk_main : kb) * BK;
-          uint8_t* a_dst = sA + stage * C::A_BYTES;
-          uint8_t* b_dst = sB + stage * C::B_BYTES;
           if (!A_MN) {
             tma_load_2d(a_dst, ma, &full_bar[stage], k0, m_blk * BM);
           } else {
@@ -437,59 +437,56 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int c = 0; c < BN / 64; ++c)
               tma_load_2d(b_dst + c * 8192, mb, &full_bar[stage], n_blk * BN + c * 64, k0);
           }
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++stage == C::STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += n_workers, ++it) {
-        int m_blk, n_blk, split;
-        decode_tile(tile, num_m, num_n, p.splits, m_blk, n_blk, split, p.group_m);
-        const int kb0 = (int)((long long)nk_total * split / p.splits);
-        const int kb1 = (int)((long long)nk_total * (split + 1) / p.splits);
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) {
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr uint32_t a_step = (A_MN ? 2048 : 32) / 16, b_step = (B_MN ? 2048 : 32) / 16;
+    const uint64_t da_base = make_smem_desc_sw128(smem_u32(sA), A_MN ? 8192 : 16, 1024);
+    const uint64_t db_base = make_smem_desc_sw128(smem_u32(sB), B_MN ? 8192 : 16, 1024);
+    int stage = 0;
+    uint32_t phase = 0;
+    int it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += n_workers, ++it) {
+      int m_blk, n_blk, split;
+      decode_tile(tile, num_m, num_n, p.splits, m_blk, n_blk, split, p.group_m);
+      const int kb0 = (int)((long long)nk_total * split / p.splits);
+      const int kb1 = (int)((long long)nk_total * (split + 1) / p.splits);
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      if (!warp_all(mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!warp_all(mbar_wait(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL))) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * C::A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * C::B_BYTES);
+        const uint64_t da = da_base + (uint32_t)(stage * (C::A_BYTES / 16)), db = db_base + (uint32_t)(stage * (C::B_BYTES / 16));
+        if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + kk * 32, 16, 1024);
-            umma_f16(d_tmem, da, db, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_f16(d_tmem, da + kk * a_step, db + kk * b_step, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
           umma_commit(&empty_bar[stage]);  // releases the smem stage when these MMAs retire
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
+        __syncwarp();
+        if (++stage == C::STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&tfull_bar[acc]);   // (a split without K blocks commits too)
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue warps
@@ -951,7 +948,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * P_STAGES + 4);
   uint64_t* epi_bar = bars + 24;                   // [epilogue warp][slot]: "gate|up chunk landed" (GLU backward)
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const int n_workers = (int)gridDim.x - p.g_ctas;  // even; gather CTAs come in whole clusters
   if ((int)blockIdx.x >= n_workers) {
@@ -995,31 +992,31 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
-        int m_blk, n_blk, split;
-        decode_tile(tile, num_m, num_n, 1, m_blk, n_blk, split, p.group_m);
-        for (int kb = 0; kb < nk_total; ++kb) {
-          if (!mbar_wait_backoff(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY, p.prod_sleep_ns)) {
-            ok = false;
-            break;
-          }
-          // One "full" barrier per stage, in the leader CTA: the leader expects the bytes of BOTH CTAs'
-          // loads, and the partner's loads credit that barrier directly (cta_group::2 TMA). No relay,
-          // no remote arrive, no fence on the critical path.
-          const uint32_t fb = mapa_u32(smem_u32(&full_bar[stage]), 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters) {
+      int m_blk, n_blk, split;
+      decode_tile(tile, num_m, num_n, 1, m_blk, n_blk, split, p.group_m);
+      const int m0 = m_blk * 256 + (int)rank * 128;
+      const int n0 = p.epi == 1 ? (int)rank * p.N + n_blk * 128 : n_blk * 256 + (int)rank * 128;
+      for (int kb = 0; kb < nk_total; ++kb) {
+        if (!warp_all(mbar_wait_backoff(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY, p.prod_sleep_ns))) {
+          ok = false;
+          break;
+        }
+        // One "full" barrier per stage, in the leader CTA: the leader expects the bytes of BOTH CTAs'
+        // loads, and the partner's loads credit that barrier directly (cta_group::2 TMA). No relay,
+        // no remote arrive, no fence on the critical path.
+        const uint32_t fb = mapa_u32(smem_u32(&full_bar[stage]), 0);
+        const bool ext = kb >= nk_main;
+        const CUtensorMap* ma = ext ? &tmA2 : &tmA;
+        const CUtensorMap* mb = ext ? &tmB2 : &tmB;
+        const int k0 = (ext ? kb - nk_main : kb) * BK;
+        uint8_t* a_dst = sA + stage * P_A_BYTES;
+        uint8_t* b_dst = sB + stage * P_B_BYTES;
+        if (elect_one()) {
           if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * P_STAGE_BYTES);
-          const bool ext = kb >= nk_main;
-          const CUtensorMap* ma = ext ? &tmA2 : &tmA;
-          const CUtensorMap* mb = ext ? &tmB2 : &tmB;
-          const int k0 = (ext ? kb - nk_main : kb) * BK;
-          uint8_t* a_dst = sA + stage * P_A_BYTES;
-          uint8_t* b_dst = sB + stage * P_B_BYTES;
-          const int m0 = m_blk * 256 + (int)rank * 128;
-          const int n0 = p.epi == 1 ? (int)rank * p.N + n_blk * 128 : n_blk * 256 + (int)rank * 128;
           if (!A_MN) {
             tma_load_2d_pair(a_dst, ma, fb, k0, m0);
           } else {
@@ -1032,17 +1029,21 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_2d_pair(b_dst, mb, fb, n0, k0);
             tma_load_2d_pair(b_dst + 8192, mb, fb, n0 + 64, k0);
           }
-          if (++stage == P_STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++stage == P_STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (rank 0 only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(256, 256, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t a_step = (A_MN ? 2048 : 32) / 16, b_step = (B_MN ? 2048 : 32) / 16;
+      const uint64_t da_base = make_smem_desc_sw128(smem_u32(sA), A_MN ? 8192 : 16, 1024);
+      const uint64_t db_base = make_smem_desc_sw128(smem_u32(sB), B_MN ? 8192 : 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -1050,33 +1051,29 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int tile = cluster_id; tile < total_tiles && ok; tile += n_clusters, ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait_spin(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) break;
+        if (!warp_all(mbar_wait_spin(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * 256;
         for (int kb = 0; kb < nk_total; ++kb) {
-          if (!mbar_wait_spin(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
+          if (!warp_all(mbar_wait_spin(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL))) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * P_A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * P_B_BYTES);
+          const uint64_t da = da_base + (uint32_t)(stage * (P_A_BYTES / 16)), db = db_base + (uint32_t)(stage * (P_B_BYTES / 16));
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + kk * 32, 16, 1024);
-            umma_f16_pair(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk)
+              umma_f16_pair(d_tmem, da + kk * a_step, db + kk * b_step, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_commit_pair_mc(&empty_bar[stage]);  // frees the stage in both CTAs (commit multicast)
+            if (kb == nk_total - 1) umma_commit_pair_mc(&tfull_bar[acc]);
           }
-          umma_commit_pair_mc(&empty_bar[stage]);  // frees the stage in both CTAs (commit multicast)
+          __syncwarp();
           if (++stage == P_STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (!ok) break;
-        umma_commit_pair_mc(&tfull_bar[acc]);
       }
     }
   } else {

@@ -8,8 +8,8 @@
 // one fp32 scale per expert; W2 / A2 (the LoRA K-extension) are bf16. Rows are expert-sorted and padded to
 // 128-row blocks (blk_expert[b] = expert of block b), exactly as in grouped_gemm.cu.
 //
-// Per k block the TMA producer brings the bf16 A tiles and the PACKED weight tile (4 KB instead of 16 KB)
-// into shared memory; four converter warps expand the nibbles and write the bf16 tile in the
+// Per k block TMA brings the bf16 A tiles and the PACKED weight tile (4 KB instead of 16 KB)
+// into shared memory; converter warps expand the nibbles and write the bf16 tile in the
 // 128-byte-swizzled layout tcgen05.mma reads; the MMA warp accumulates in TMEM; four epilogue warps store
 // the result. One decoded weight tile feeds TWO 128-row blocks of the same expert (256 rows per pass), which
 // halves the decode work per FLOP. The decode builds, per 16-value scale group, the eight products
@@ -28,12 +28,31 @@ constexpr int BM = 128;
 constexpr int BN = 128;
 constexpr int BK = 64;
 constexpr int W4_CONV_WARPS = 8;
-constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS;   // TMA, MMA, 4 epilogue warps, 8 converter warps
-constexpr int W4_STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2;   // one 128-row A tile; a stage holds two
+constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (A), MMA, 4 epilogue warps, 8 converter warps, TMA (weights)
+// Three rings of their own: the packed weights are small and run eight k blocks ahead, so a converter never waits for memory;
+// a slot of the decoded tile is only held from its decode to its MMA, and a slot of A from its load to its MMA.
+// The converters work in four groups of two warps, each on a k block of its own, so that four chains (packed tile seen ->
+// decode -> stores -> proxy fence -> arrival) run side by side.
+constexpr int SA = 4, SB = 4, SR = 8;  // slots: A (two 128-row tiles), decoded B, packed B
+constexpr int CGROUPS = 4, CG_WARPS = W4_CONV_WARPS / CGROUPS, CG_UNITS = 256 / (32 * CG_WARPS);
+constexpr int A_BYTES = BM * BK * 2;   // one 128-row A tile; a slot holds two
 constexpr int B_BYTES = BN * BK * 2;
 constexpr int RAW_BYTES = 4096;   // FWD: 128 rows x 32 bytes; DX: 64 rows x 64 bytes
-constexpr int W4_SMEM = W4_STAGES * (2 * A_BYTES + B_BYTES + RAW_BYTES) + 1024 + 256;
+constexpr int W4_SMEM = SA * 2 * A_BYTES + SB * B_BYTES + SR * RAW_BYTES + 1024 + 512;
+static_assert(W4_SMEM <= 227 * 1024, "");
+
+// position in a ring of N slots
+template <int N>
+struct Ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  AXB_DEVICE void next() {
+    if (++slot == N) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+};
 
 // E4M3 byte -> fp32, branch free: the 7 magnitude bits placed at the top of an fp32 mantissa / the bottom of
 // its exponent give value x 2^-120 (subnormal inputs included), and 0x7F / 0xFF are NaN. Same value as
@@ -162,18 +181,21 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
                          const W4Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* sA = smem;                                   // [stage][2][128 x 64]
-  uint8_t* sB = smem + W4_STAGES * 2 * A_BYTES;
-  uint8_t* sRaw = sB + W4_STAGES * B_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + W4_STAGES * RAW_BYTES);
-  uint64_t* raw_full = bars;                    // TMA landed: A tiles + packed weights (or the bf16 LoRA tile)
-  uint64_t* full_bar = bars + W4_STAGES;        // converters done: the bf16 B tile is in place (one arrival per warp)
-  uint64_t* empty_bar = bars + 2 * W4_STAGES;   // MMAs retired
-  uint64_t* tfull_bar = bars + 3 * W4_STAGES;
-  uint64_t* tempty_bar = bars + 3 * W4_STAGES + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * W4_STAGES + 4);
+  uint8_t* sA = smem;                                   // [slot][2][128 x 64]
+  uint8_t* sB = smem + SA * 2 * A_BYTES;
+  uint8_t* sRaw = sB + SB * B_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + SR * RAW_BYTES);
+  uint64_t* a_full = bars;                      // A tiles landed
+  uint64_t* a_empty = a_full + SA;              // their MMAs retired
+  uint64_t* b_full = a_empty + SA;              // bf16 B tile in place (one arrival per warp of its group; the LoRA tile by TMA)
+  uint64_t* b_empty = b_full + SB;
+  uint64_t* r_full = b_empty + SB;              // packed weights landed
+  uint64_t* r_empty = r_full + SR;              // read by its group
+  uint64_t* tfull_bar = r_empty + SR;
+  uint64_t* tempty_bar = tfull_bar + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int n_blocks = *p.n_blocks;
   const int num_n = (p.N + BN - 1) / BN;
   const int nk_main = (p.K + BK - 1) / BK, nk_ext = (p.K2 + BK - 1) / BK;
@@ -181,10 +203,17 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
   const int total = ((n_blocks + 1) / 2) * num_n;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < W4_STAGES; ++s) {
-      mbar_init(&raw_full[s], 1);
-      mbar_init(&full_bar[s], W4_CONV_WARPS);
-      mbar_init(&empty_bar[s], 1);
+    for (int s = 0; s < SA; ++s) {
+      mbar_init(&a_full[s], 1);
+      mbar_init(&a_empty[s], 1);
+    }
+    for (int s = 0; s < SB; ++s) {
+      mbar_init(&b_full[s], CG_WARPS);
+      mbar_init(&b_empty[s], 1);
+    }
+    for (int s = 0; s < SR; ++s) {
+      mbar_init(&r_full[s], 1);
+      mbar_init(&r_empty[s], CG_WARPS);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
@@ -204,97 +233,103 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-        for (int sub = 0; sub < 2 && ok; ++sub) {
-          Pass ps;
-          if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
-          const uint32_t a_bytes = ps.two ? 2 * A_BYTES : A_BYTES;
-          for (int kb = 0; kb < nk; ++kb) {
-            if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
-              ok = false;
-              break;
-            }
-            const bool ext = kb >= nk_main;
-            uint8_t* a_dst = sA + stage * 2 * A_BYTES;
-            const CUtensorMap* ma = ext ? &tmA2 : &tmA;
-            const int ka = ext ? (kb - nk_main) * BK : kb * BK;
-            mbar_expect_tx(&raw_full[stage], a_bytes + (ext ? B_BYTES : RAW_BYTES));
-            tma_load_2d(a_dst, ma, &raw_full[stage], ka, ps.blk * BM);
-            if (ps.two) tma_load_2d(a_dst + A_BYTES, ma, &raw_full[stage], ka, (ps.blk + 1) * BM);
-            if (!ext) {
-              if (!DX) tma_load_3d(sRaw + stage * RAW_BYTES, &tmQ, &raw_full[stage], kb * (BK / 2), ps.n0, ps.e);   // [128 n, 32 B of k]
-              else tma_load_3d(sRaw + stage * RAW_BYTES, &tmQ, &raw_full[stage], ps.n0 / 2, kb * BK, ps.e);         // [64 n, 64 B of k]
-            } else {
-              uint8_t* b_dst = sB + stage * B_BYTES;
-              if (!DX) {
-                tma_load_3d(b_dst, &tmB2, &raw_full[stage], ka, ps.n0, ps.e);
-              } else {
-                tma_load_3d(b_dst, &tmB2, &raw_full[stage], ps.n0, ka, ps.e);
-                tma_load_3d(b_dst + 8192, &tmB2, &raw_full[stage], ps.n0 + 64, ka, ps.e);
-              }
-            }
-            if (++stage == W4_STAGES) {
-              stage = 0;
-              phase ^= 1;
-            }
+    // ------------------------------------------------------------ A tiles
+    Ring<SA> ra;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+      for (int sub = 0; sub < 2 && ok; ++sub) {
+        Pass ps;
+        if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
+        const uint32_t a_bytes = ps.two ? 2 * A_BYTES : A_BYTES;
+        for (int kb = 0; kb < nk; ++kb, ra.next()) {
+          if (!warp_all(mbar_wait(&a_empty[ra.slot], ra.phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
+            ok = false;
+            break;
           }
+          const bool ext = kb >= nk_main;
+          uint8_t* a_dst = sA + ra.slot * 2 * A_BYTES;
+          const CUtensorMap* ma = ext ? &tmA2 : &tmA;
+          const int ka = ext ? (kb - nk_main) * BK : kb * BK;
+          if (elect_one()) {
+            mbar_expect_tx(&a_full[ra.slot], a_bytes);
+            tma_load_2d(a_dst, ma, &a_full[ra.slot], ka, ps.blk * BM);
+            if (ps.two) tma_load_2d(a_dst + A_BYTES, ma, &a_full[ra.slot], ka, (ps.blk + 1) * BM);
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else if (warp == W4_THREADS / 32 - 1) {
+    // ------------------------------------------------------------ packed weights
+    Ring<SR> rr;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+      for (int sub = 0; sub < 2 && ok; ++sub) {
+        Pass ps;
+        if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
+        for (int kb = 0; kb < nk_main; ++kb, rr.next()) {
+          if (!warp_all(mbar_wait(&r_empty[rr.slot], rr.phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
+            ok = false;
+            break;
+          }
+          if (elect_one()) {
+            mbar_expect_tx(&r_full[rr.slot], RAW_BYTES);
+            if (!DX) tma_load_3d(sRaw + rr.slot * RAW_BYTES, &tmQ, &r_full[rr.slot], kb * (BK / 2), ps.n0, ps.e);   // [128 n, 32 B of k]
+            else tma_load_3d(sRaw + rr.slot * RAW_BYTES, &tmQ, &r_full[rr.slot], ps.n0 / 2, kb * BK, ps.e);         // [64 n, 64 B of k]
+          }
+          __syncwarp();
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, 0, DX ? 1 : 0);
-      int stage = 0, it = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-        for (int sub = 0; sub < 2 && ok; ++sub) {
-          Pass ps;
-          if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
-          const int acc = it & 1;
-          if (!mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) {
+    // ------------------------------------------------------------ MMA issue
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, 0, DX ? 1 : 0);
+    const uint64_t da_base = make_smem_desc_sw128(smem_u32(sA), 16, 1024);
+    const uint64_t db_base = DX ? make_smem_desc_sw128(smem_u32(sB), 8192, 1024) : make_smem_desc_sw128(smem_u32(sB), 16, 1024);
+    Ring<SA> ra;
+    Ring<SB> rb;
+    int it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+      for (int sub = 0; sub < 2 && ok; ++sub) {
+        Pass ps;
+        if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
+        const int acc = it & 1;
+        if (!warp_all(mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * 2 * BN;
+        for (int kb = 0; kb < nk; ++kb, ra.next(), rb.next()) {
+          if (!warp_all(mbar_wait(&a_full[ra.slot], ra.phase, p.status, AXB_TIMEOUT_FULL) &&
+                        mbar_wait(&b_full[rb.slot], rb.phase, p.status, AXB_TIMEOUT_FULL))) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d_tmem = tmem_base + acc * 2 * BN;
-          for (int kb = 0; kb < nk; ++kb) {
-            // raw_full: the TMA writes (A tiles, LoRA B tile) observed by this thread itself; full_bar: the decoded tile
-            if (!mbar_wait(&raw_full[stage], phase, p.status, AXB_TIMEOUT_FULL) ||
-                !mbar_wait(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t a_addr = smem_u32(sA + stage * 2 * A_BYTES), b_addr = smem_u32(sB + stage * B_BYTES);
+          const uint64_t da = da_base + (uint32_t)(ra.slot * (2 * A_BYTES / 16)), db = db_base + (uint32_t)(rb.slot * (B_BYTES / 16));
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk) {
-              const uint64_t db = DX ? make_smem_desc_sw128(b_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + kk * 32, 16, 1024);
+              const uint64_t dbk = db + kk * (DX ? 2048 / 16 : 32 / 16);
               const uint32_t accum = (kb > 0 || kk > 0) ? 1u : 0u;
-              umma_f16(d_tmem, make_smem_desc_sw128(a_addr + kk * 32, 16, 1024), db, idesc, accum);
-              if (ps.two) umma_f16(d_tmem + BN, make_smem_desc_sw128(a_addr + A_BYTES + kk * 32, 16, 1024), db, idesc, accum);
+              umma_f16(d_tmem, da + kk * 2, dbk, idesc, accum);
+              if (ps.two) umma_f16(d_tmem + BN, da + A_BYTES / 16 + kk * 2, dbk, idesc, accum);
             }
-            umma_commit(&empty_bar[stage]);
-            if (++stage == W4_STAGES) {
-              stage = 0;
-              phase ^= 1;
-            }
+            umma_commit(&a_empty[ra.slot]);
+            umma_commit(&b_empty[rb.slot]);
+            if (kb == nk - 1) umma_commit(&tfull_bar[acc]);
           }
-          if (!ok) break;
-          umma_commit(&tfull_bar[acc]);
-          ++it;
+          __syncwarp();
         }
+        ++it;
       }
     }
   } else if (warp >= 6) {
     // ------------------------------------------------------------ converters: packed tile -> bf16 B tile
-    // 256 threads; thread ct reads 16 packed bytes (32 codes, 2 scale groups) at raw + ct * 16 and writes four
-    // 16-byte chunks of the swizzled bf16 tile. Two warps per scheduler hide each other's latencies.
+    // A k block is 256 units of 16 packed bytes (32 codes, 2 scale groups); thread t of a group takes units t, t + 64, ...
+    // Unit ct lies at raw + ct * 16 and becomes four 16-byte chunks of the swizzled bf16 tile.
     //   FWD: raw tile [128 n][32 B]: weight row n0 + ct / 2, codes 32 * (ct & 1) .. + 31 of k block kb
     //        -> K-major row ct / 2, chunks 4 * (ct & 1) .. + 3.
     //   DX : raw tile [64 wn][64 B]: weight row kb * 64 + ct / 4, columns n0 + 64 * half + 32 * part .. + 31
@@ -302,12 +337,10 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
     // Shared-memory accesses are conflict free: the loads are contiguous, and the eight lanes of a store phase
     // hit eight different 16-byte chunk positions (rows differ in swizzle bits 0-1 or bit 0, `part` flips bit 2,
     // and in dX the odd half walks its chunks in the order 2, 3, 0, 1, which flips bit 1).
-    const int ct = threadIdx.x - 192;   // 0..255
+    const int cw = warp - 6, grp = cw / CG_WARPS, gt = (cw % CG_WARPS) * 32 + lane;
     const long long sc_row_bytes = p.Wk / 16;
-    const int part = ct & 1;
-    const int r = DX ? (ct >> 2) : (ct >> 1), half = DX ? ((ct >> 1) & 1) : 0;
-    int stage = 0;
-    uint32_t phase = 0;
+    const int part = gt & 1, half = DX ? ((gt >> 1) & 1) : 0;      // the same for all units of a thread
+    long long cb = 0, cr = 0;                                     // k blocks (of B, of packed weights) before this pass
     bool ok = true;
     for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
       for (int sub = 0; sub < 2 && ok; ++sub) {
@@ -315,79 +348,96 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
         const float g = p.pts[ps.e];
         const uint8_t* sc_base = p.scale + (long long)ps.e * p.Wn * sc_row_bytes;
-        // Block scales (2 bytes per thread and k block) are fetched FOUR k blocks ahead: a global load that misses
-        // the small L1 left beside 200 KB of shared memory takes longer than one k block. Forward: one 16-byte
-        // load covers four k blocks of this thread's weight row; dX: a new weight row per k block.
-        const bool vec_ok = !DX && (sc_row_bytes & 15) == 0;
-        auto load_group = [&](int kb0, uint32_t (&out)[4]) {
+        // the two E4M3 bytes of each unit, requested one turn (four k blocks) ahead and looked at when they are needed
+        auto load_scales = [&](int kb, uint32_t (&out)[CG_UNITS]) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) out[j] = 0u;
-          if (kb0 >= nk_main) return;
-          if (!DX) {
-            const int n = ps.n0 + r;
-            if (n >= p.Wn) return;
-            const uint8_t* row = sc_base + (long long)n * sc_row_bytes;
-            if (vec_ok && kb0 * 4 + 16 <= sc_row_bytes) {
-              const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + kb0 * 4));
-              out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+          for (int u = 0; u < CG_UNITS; ++u) {
+            out[u] = 0u;
+            const int ct = gt + u * (256 / CG_UNITS);
+            if (kb >= nk_main) continue;
+            if (!DX) {
+              const int n = ps.n0 + (ct >> 1);
+              if (n < p.Wn) out[u] = __ldg(reinterpret_cast<const unsigned short*>(sc_base + (long long)n * sc_row_bytes + kb * 4 + part * 2));
             } else {
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (kb0 + j < nk_main) out[j] = __ldg(reinterpret_cast<const uint32_t*>(row + (kb0 + j) * 4));
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) out[j] = (out[j] >> (part * 16)) & 0xFFFFu;
-          } else {
-            const int k0 = ps.n0 + half * 64 + part * 32;
-            if (k0 >= p.Wk) return;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int wn = (kb0 + j) * BK + r;
-              if (kb0 + j < nk_main && wn < p.Wn)
-                out[j] = __ldg(reinterpret_cast<const unsigned short*>(sc_base + (long long)wn * sc_row_bytes + k0 / 16));
+              const int k0 = ps.n0 + half * 64 + part * 32, wn = kb * BK + (ct >> 2);
+              if (k0 < p.Wk && wn < p.Wn)
+                out[u] = __ldg(reinterpret_cast<const unsigned short*>(sc_base + (long long)wn * sc_row_bytes + k0 / 16));
             }
           }
         };
-        uint32_t cur[4], nxt[4];
-        load_group(0, cur);
-        for (int kb0 = 0; kb0 < nk && ok; kb0 += 4) {
-          load_group(kb0 + 4, nxt);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int kb = kb0 + j;
-            if (kb >= nk) break;
-            if (!mbar_wait(&raw_full[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
+        // this group's k blocks of the pass: every fourth of the whole sequence
+        int kb = (int)((grp - cb) & (CGROUPS - 1));
+        uint32_t cur[CG_UNITS], nxt[CG_UNITS];
+        load_scales(kb, cur);
+        for (; kb < nk && ok; kb += CGROUPS) {
+          load_scales(kb + CGROUPS, nxt);
+          const long long ib = cb + kb, ir = cr + kb;
+          const int bslot = (int)(ib % SB), rslot = (int)(ir % SR);
+          const uint32_t bphase = (uint32_t)(ib / SB) & 1, rphase = (uint32_t)(ir / SR) & 1;
+          if (kb < nk_main) {
+            if (!mbar_wait(&r_full[rslot], rphase, p.status, AXB_TIMEOUT_FULL)) {
               ok = false;
               break;
             }
-            if (kb < nk_main) {
-              uint4 w = *reinterpret_cast<const uint4*>(sRaw + stage * RAW_BYTES + ct * 16);
-              uint32_t sc2 = cur[j];                    // two E4M3 bytes: codes 0-15 and 16-31 of this thread
-              uint8_t* dst_row = sB + stage * B_BYTES + half * 8192 + r * 128;
-              int pos = (part * 4) ^ (r & 7);           // chunk position of this thread's first chunk
+            uint4 w[CG_UNITS];
+#pragma unroll
+            for (int u = 0; u < CG_UNITS; ++u)
+              w[u] = *reinterpret_cast<const uint4*>(sRaw + rslot * RAW_BYTES + (gt + u * (256 / CG_UNITS)) * 16);
+            if (!mbar_wait(&b_empty[bslot], bphase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
+              ok = false;
+              break;
+            }
+#pragma unroll
+            for (int u = 0; u < CG_UNITS; ++u) {
+              const int ct = gt + u * (256 / CG_UNITS), r = DX ? (ct >> 2) : (ct >> 1);
+              uint32_t sc2 = cur[u];
+              int pos = (part * 4) ^ (r & 7);           // chunk position of this unit's first chunk
               if (DX && half) {
-                w = make_uint4(w.z, w.w, w.x, w.y);
+                w[u] = make_uint4(w[u].z, w[u].w, w[u].x, w[u].y);
                 sc2 = ((sc2 >> 8) | (sc2 << 8)) & 0xFFFFu;
                 pos ^= 2;
               }
+              uint8_t* dst_row = sB + bslot * B_BYTES + half * 8192 + r * 128;
               Lut t = make_lut(e4m3_to_float(sc2 & 0xFF) * g);
-              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 0) << 4)) = decode8(w.x, t);
-              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 1) << 4)) = decode8(w.y, t);
+              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 0) << 4)) = decode8(w[u].x, t);
+              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 1) << 4)) = decode8(w[u].y, t);
               t = make_lut(e4m3_to_float(sc2 >> 8) * g);
-              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 2) << 4)) = decode8(w.z, t);
-              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 3) << 4)) = decode8(w.w, t);
-              fence_proxy_async_smem();
+              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 2) << 4)) = decode8(w[u].z, t);
+              *reinterpret_cast<uint4*>(dst_row + ((pos ^ 3) << 4)) = decode8(w[u].w, t);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(&b_full[bslot]);
+              mbar_arrive(&r_empty[rslot]);
+            }
+          } else {                                    // the LoRA tile comes by TMA, on the group's first arrival
+            if (!mbar_wait(&b_empty[bslot], bphase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
+              ok = false;
+              break;
+            }
+            if (lane == 0) {
+              if (cw % CG_WARPS == 0) {
+                const int ka = (kb - nk_main) * BK;
+                uint8_t* b_dst = sB + bslot * B_BYTES;
+                mbar_expect_tx(&b_full[bslot], B_BYTES);
+                if (!DX) {
+                  tma_load_3d(b_dst, &tmB2, &b_full[bslot], ka, ps.n0, ps.e);
+                } else {
+                  tma_load_3d(b_dst, &tmB2, &b_full[bslot], ps.n0, ka, ps.e);
+                  tma_load_3d(b_dst + 8192, &tmB2, &b_full[bslot], ps.n0 + 64, ka, ps.e);
+                }
+              } else {
+                mbar_arrive(&b_full[bslot]);
+              }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full_bar[stage]);
-            if (++stage == W4_STAGES) {
-              stage = 0;
-              phase ^= 1;
-            }
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
+          for (int u = 0; u < CG_UNITS; ++u) cur[u] = nxt[u];
         }
+        cb += nk;
+        cr += nk_main;
       }
     }
   } else {
