@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   uint64_t* o_full = bars + 14;   // [unit]  O final
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&q_full[s], 1);
@@ -156,11 +156,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
       auto load = [&](uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int col, int row) {
-        mbar_expect_tx(bar, C::TILE_BYTES);
+        if (elect_one()) {
+          mbar_expect_tx(bar, C::TILE_BYTES);
 #pragma unroll
-        for (int h = 0; h < C::HALVES; ++h) tma_load_2d(dst + h * HALF_BYTES, m, bar, col + h * 64, row);
+          for (int h = 0; h < C::HALVES; ++h) tma_load_2d(dst + h * HALF_BYTES, m, bar, col + h * 64, row);
+        }
+        __syncwarp();
       };
       const int qrow = doc_start + q0 - p.q_row_off;
       load(sQ, &tm_q, &q_full[0], p.q_col0 + head0 * D, qrow);
@@ -168,46 +171,59 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
         const int row = doc_start + (jb0 + j) * 128;
-        if (!mbar_wait(&k_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+        if (!warp_all(mbar_wait(&k_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
         load(sK + st * C::TILE_BYTES, &tm_qkv, &k_full[st], p.k_col0 + kv_head * D, row);
         if (j == 0 && n_u1 > 0)
           load(sQ + C::TILE_BYTES, &tm_q, &q_full[1], p.q_col0 + (p.pair_mode == 1 ? head0 + 1 : head0) * D,
                p.pair_mode == 2 ? qrow + 128 : qrow);
-        if (!mbar_wait(&v_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+        if (!warp_all(mbar_wait(&v_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
         load(sV + st * C::TILE_BYTES, &tm_qkv, &v_full[st], p.v_col0 + kv_head * D, row);
       }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);  // Q (K-major) x K (K-major)
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);   // P (TMEM) x V (MN-major)
+      const uint64_t dq_base = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dk_base = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t dv_base = make_smem_desc_sw128(smem_u32(sV), HALF_BYTES, 1024);
+      constexpr uint32_t TILE16 = C::TILE_BYTES / 16;
       auto issue_s = [&](int u, int j) {
-        const uint32_t q_addr = smem_u32(sQ + u * C::TILE_BYTES), k_addr = smem_u32(sK + (j & 1) * C::TILE_BYTES);
+        const uint64_t dq = dq_base + (uint32_t)u * TILE16, dk = dk_base + (uint32_t)(j & 1) * TILE16;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + u * 128, make_smem_desc_sw128(q_addr + off, 16, 1024),
-                   make_smem_desc_sw128(k_addr + off, 16, 1024), idesc_s, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
+            umma_f16(tmem_base + u * 128, dq + off, dk + off, idesc_s, kk > 0);
+          }
+          umma_commit(&s_full[u]);
         }
-        umma_commit(&s_full[u]);
+        __syncwarp();
       };
-      auto issue_pv = [&](int u, int j) {
-        const uint32_t v_addr = smem_u32(sV + (j & 1) * C::TILE_BYTES);
+      auto issue_pv = [&](int u, int j, bool last) {
+        const uint64_t dv = dv_base + (uint32_t)(j & 1) * TILE16;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)   // 128 kv rows / 16: 8 TMEM columns of P each
-          umma_f16_ts(tmem_base + C::O_COL + u * D, tmem_base + u * 128 + kk * 8,
-                      make_smem_desc_sw128(v_addr + kk * 2048, HALF_BYTES, 1024), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk)   // 128 kv rows / 16: 8 TMEM columns of P each
+            umma_f16_ts(tmem_base + C::O_COL + u * D, tmem_base + u * 128 + kk * 8, dv + kk * (2048 / 16), idesc_pv,
+                        (j > 0 || kk > 0) ? 1u : 0u);
+          if (last) umma_commit(&o_full[u]);
+        }
+        __syncwarp();
       };
-      bool ok = mbar_wait(&q_full[0], 0, p.status, AXB_TIMEOUT_FULL) && mbar_wait(&k_full[0], 0, p.status, AXB_TIMEOUT_FULL);
+      auto commit = [&](uint64_t* bar) {
+        if (elect_one()) umma_commit(bar);
+        __syncwarp();
+      };
+      bool ok = warp_all(mbar_wait(&q_full[0], 0, p.status, AXB_TIMEOUT_FULL) && mbar_wait(&k_full[0], 0, p.status, AXB_TIMEOUT_FULL));
       if (ok) {
         tc_fence_after();
         issue_s(0, 0);
         if (n_u1 > 0) {
-          ok = mbar_wait(&q_full[1], 0, p.status, AXB_TIMEOUT_FULL);
+          ok = warp_all(mbar_wait(&q_full[1], 0, p.status, AXB_TIMEOUT_FULL));
           if (ok) {
             tc_fence_after();
             issue_s(1, 0);
           }
         }
-        umma_commit(&k_empty[0]);
+        commit(&k_empty[0]);
       }
       for (int j = 0; j < n_max && ok; ++j) {
         const int st = j & 1, nst = st ^ 1;
@@ -218,13 +234,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           if (j >= n_u || !ok) continue;
           ok = mbar_wait(&p_full[u], j & 1, p.status, AXB_TIMEOUT_GENERIC);
           if (ok && !v_ready) ok = mbar_wait(&v_full[st], (j >> 1) & 1, p.status, AXB_TIMEOUT_FULL);
+          ok = warp_all(ok);
           if (!ok) break;
           v_ready = true;
           tc_fence_after();
-          issue_pv(u, j);
-          if (j == n_u - 1) umma_commit(&o_full[u]);
+          issue_pv(u, j, j == n_u - 1);
           if (j + 1 < n_u) {
-            if (!k_ready) ok = mbar_wait(&k_full[nst], ((j + 1) >> 1) & 1, p.status, AXB_TIMEOUT_FULL);
+            if (!k_ready) ok = warp_all(mbar_wait(&k_full[nst], ((j + 1) >> 1) & 1, p.status, AXB_TIMEOUT_FULL));
             if (!ok) break;
             k_ready = true;
             tc_fence_after();
@@ -232,8 +248,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           }
         }
         if (!ok) break;
-        umma_commit(&v_empty[st]);
-        if (j + 1 < n_max) umma_commit(&k_empty[nst]);
+        commit(&v_empty[st]);
+        if (j + 1 < n_max) commit(&k_empty[nst]);
       }
     }
   } else {
@@ -471,7 +487,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   uint64_t* acc_full = bars + 15; // dK / dV final
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < C::STAGES; ++s) {
@@ -497,102 +513,110 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * C::KV_BYTES);
 #pragma unroll
       for (int h = 0; h < C::HALVES; ++h) {
-        tma_load_2d(sK + h * HALF_BYTES, &tm_kv, kv_full, p.k_col0 + kv_head * D + h * 64,
-                    doc_start + kv0);
-        tma_load_2d(sV + h * HALF_BYTES, &tm_kv, kv_full, p.v_col0 + kv_head * D + h * 64,
-                    doc_start + kv0);
+        tma_load_2d(sK + h * HALF_BYTES, &tm_kv, kv_full, p.k_col0 + kv_head * D + h * 64, doc_start + kv0);
+        tma_load_2d(sV + h * HALF_BYTES, &tm_kv, kv_full, p.v_col0 + kv_head * D + h * 64, doc_start + kv0);
       }
-      for (int it = 0; it < n_iter; ++it) {
-        const int st = it % C::STAGES;
-        const uint32_t ph = (it / C::STAGES) & 1;
-        const int head = head0 + it / n_qt;
-        const int qrow = doc_start + (q_first + it % n_qt) * 64 - p.q_row_off;
-        if (!mbar_wait(&q_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+    }
+    __syncwarp();
+    int st = 0, qt = 0, head = head0;
+    uint32_t ph = 0;
+    for (int it = 0; it < n_iter; ++it) {
+      const int qrow = doc_start + (q_first + qt) * 64 - p.q_row_off;
+      if (!warp_all(mbar_wait(&q_empty[st], ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
         mbar_expect_tx(&q_full[st], 2 * C::Q_BYTES);
 #pragma unroll
         for (int h = 0; h < C::HALVES; ++h) {
-          tma_load_2d(sQ + st * C::Q_BYTES + h * C::Q_HALF, &tm_q, &q_full[st],
-                      p.q_col0 + head * D + h * 64, qrow);
-          tma_load_2d(sdO + st * C::Q_BYTES + h * C::Q_HALF, &tm_do, &q_full[st],
-                      head * D + h * 64, qrow);
+          tma_load_2d(sQ + st * C::Q_BYTES + h * C::Q_HALF, &tm_q, &q_full[st], p.q_col0 + head * D + h * 64, qrow);
+          tma_load_2d(sdO + st * C::Q_BYTES + h * C::Q_HALF, &tm_do, &q_full[st], head * D + h * 64, qrow);
         }
+      }
+      __syncwarp();
+      if (++qt == n_qt) {
+        qt = 0;
+        ++head;
+      }
+      if (++st == C::STAGES) {
+        st = 0;
+        ph ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);  // K/V (K-major) x Q/dO (K-major)
-      constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);  // P^T/dS^T x dO/Q (MN-major)
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, 1, 1);  // K^T (MN) x dS^T (MN)
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-      const uint32_t pt_addr = smem_u32(sPT), dst_addr = smem_u32(sdST);
-      bool ok = mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL);
-      // S^T(i) = K . Q(i)^T and dP^T(i) = V . dO(i)^T into TMEM buffer i & 1
-      auto issue_scores = [&](int i) -> bool {
-        const int st = i % C::STAGES, b = i & 1;
-        const uint32_t ph = (i / C::STAGES) & 1;
-        if (!mbar_wait(&q_full[st], ph, p.status, AXB_TIMEOUT_FULL)) return false;
-        // buffer b was last used by iteration i - 2: its dQ^T must have been drained
-        if (i >= 2 && !mbar_wait(&st_free[b], ((i - 2) >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))
-          return false;
-        tc_fence_after();
-        const uint32_t q_addr = smem_u32(sQ + st * C::Q_BYTES);
-        const uint32_t do_addr = smem_u32(sdO + st * C::Q_BYTES);
+    constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);  // K/V (K-major) x Q/dO (K-major)
+    constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);  // P^T/dS^T x dO/Q (MN-major)
+    constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, 1, 1);  // K^T (MN) x dS^T (MN)
+    constexpr uint32_t Q16 = C::Q_BYTES / 16, PT16 = C::PT_BYTES / 16;
+    const uint64_t dk_k = make_smem_desc_sw128(smem_u32(sK), 16, 1024), dk_mn = make_smem_desc_sw128(smem_u32(sK), HALF_BYTES, 1024);
+    const uint64_t dv_k = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
+    const uint64_t dq_k = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dq_mn = make_smem_desc_sw128(smem_u32(sQ), C::Q_HALF, 1024);
+    const uint64_t do_k = make_smem_desc_sw128(smem_u32(sdO), 16, 1024), do_mn = make_smem_desc_sw128(smem_u32(sdO), C::Q_HALF, 1024);
+    const uint64_t pt_k = make_smem_desc_sw128(smem_u32(sPT), 16, 1024), ds_k = make_smem_desc_sw128(smem_u32(sdST), 16, 1024);
+    const uint64_t ds_mn = make_smem_desc_sw128(smem_u32(sdST), HALF_BYTES, 1024);
+    bool ok = warp_all(mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL));
+    int s_st = 0;             // stage and phase of the next scores
+    uint32_t s_ph = 0;
+    // S^T(i) = K . Q(i)^T and dP^T(i) = V . dO(i)^T into TMEM buffer i & 1
+    auto issue_scores = [&](int i) -> bool {
+      const int b = i & 1;
+      bool fine = mbar_wait(&q_full[s_st], s_ph, p.status, AXB_TIMEOUT_FULL);
+      // buffer b was last used by iteration i - 2: its dQ^T must have been drained
+      if (fine && i >= 2) fine = mbar_wait(&st_free[b], ((i - 2) >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY);
+      if (!warp_all(fine)) return false;
+      tc_fence_after();
+      const uint64_t dq = dq_k + (uint32_t)s_st * Q16, dd = do_k + (uint32_t)s_st * Q16;
+      const uint32_t col = tmem_base + 128 * b;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {  // reduce over d
-          const uint32_t koff = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          const uint32_t qoff = (kk / 4) * C::Q_HALF + (kk % 4) * 32;
-          umma_f16(tmem_base + C::ST_COL + 128 * b, make_smem_desc_sw128(k_addr + koff, 16, 1024),
-                   make_smem_desc_sw128(q_addr + qoff, 16, 1024), idesc_st, kk > 0);
+          const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * C::Q_HALF + (kk % 4) * 32) / 16;
+          umma_f16(col + C::ST_COL, dk_k + koff, dq + qoff, idesc_st, kk > 0);
         }
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t koff = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          const uint32_t qoff = (kk / 4) * C::Q_HALF + (kk % 4) * 32;
-          umma_f16(tmem_base + C::DPT_COL + 128 * b, make_smem_desc_sw128(v_addr + koff, 16, 1024),
-                   make_smem_desc_sw128(do_addr + qoff, 16, 1024), idesc_st, kk > 0);
+          const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * C::Q_HALF + (kk % 4) * 32) / 16;
+          umma_f16(col + C::DPT_COL, dv_k + koff, dd + qoff, idesc_st, kk > 0);
         }
         umma_commit(&s_full[b]);
-        return true;
-      };
-      ok = ok && issue_scores(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int st = it % C::STAGES, b = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        if (it + 1 < n_iter && !issue_scores(it + 1)) break;   // keeps the tensor core busy during softmax(it)
-        const uint32_t q_addr = smem_u32(sQ + st * C::Q_BYTES);
-        const uint32_t do_addr = smem_u32(sdO + st * C::Q_BYTES);
-        const uint32_t ptb = pt_addr + b * C::PT_BYTES, dstb = dst_addr + b * C::PT_BYTES;
-        if (!mbar_wait(&pt_full[b], ph, p.status, AXB_TIMEOUT_GENERIC)) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      if (++s_st == C::STAGES) {
+        s_st = 0;
+        s_ph ^= 1;
+      }
+      return true;
+    };
+    ok = ok && issue_scores(0);
+    int st = 0;
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const int b = it & 1;
+      const uint32_t ph = (it >> 1) & 1;
+      if (it + 1 < n_iter && !issue_scores(it + 1)) break;   // keeps the tensor core busy during softmax(it)
+      const uint64_t dq = dq_mn + (uint32_t)st * Q16, dd = do_mn + (uint32_t)st * Q16;
+      const uint64_t pt = pt_k + (uint32_t)b * PT16, ds = ds_k + (uint32_t)b * PT16, dst = ds_mn + (uint32_t)b * PT16;
+      if (!warp_all(mbar_wait(&pt_full[b], ph, p.status, AXB_TIMEOUT_GENERIC))) break;
+      tc_fence_after();
+      if (elect_one()) {
         // reduce over the 64 q rows of this tile: 4 K-steps of 16
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          // dV += P^T . dO   (B = dO tile, MN-major: chunk stride = one 64x64 half)
-          umma_f16(tmem_base + C::DV_COL, make_smem_desc_sw128(ptb + kk * 32, 16, 1024),
-                   make_smem_desc_sw128(do_addr + kk * 2048, C::Q_HALF, 1024), idesc_acc,
-                   (it > 0 || kk > 0));
-        }
+        for (int kk = 0; kk < 4; ++kk)   // dV += P^T . dO   (B = dO tile, MN-major: chunk stride = one 64x64 half)
+          umma_f16(tmem_base + C::DV_COL, pt + kk * 2, dd + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          umma_f16(tmem_base + C::DK_COL, make_smem_desc_sw128(dstb + kk * 32, 16, 1024),
-                   make_smem_desc_sw128(q_addr + kk * 2048, C::Q_HALF, 1024), idesc_acc,
-                   (it > 0 || kk > 0));
-        }
+        for (int kk = 0; kk < 4; ++kk)
+          umma_f16(tmem_base + C::DK_COL, ds + kk * 2, dq + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
         umma_commit(&q_empty[st]);
         // dQ^T [d, q] = K^T . dS^T over the 128 kv rows (8 K-steps of 16), into the columns of S^T(b)
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          umma_f16(tmem_base + C::ST_COL + 128 * b,
-                   make_smem_desc_sw128(k_addr + kk * 2048, HALF_BYTES, 1024),
-                   make_smem_desc_sw128(dstb + kk * 2048, HALF_BYTES, 1024), idesc_dq, kk > 0);
-        }
+        for (int kk = 0; kk < 8; ++kk)
+          umma_f16(tmem_base + C::ST_COL + 128 * b, dk_mn + kk * (2048 / 16), dst + kk * (2048 / 16), idesc_dq, kk > 0);
         umma_commit(&dq_full[b]);
+        if (it == n_iter - 1) umma_commit(acc_full);
       }
-      umma_commit(acc_full);
+      __syncwarp();
+      if (++st == C::STAGES) st = 0;
     }
   } else {
     const int lg = warp & 3;

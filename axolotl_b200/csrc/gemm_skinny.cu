@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(SK_T)
   uint64_t* empty = full + C::STAGES;
   uint64_t* done = empty + C::STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int rank = (int)cluster_ctarank(), cs = (int)cluster_nctarank();
   const int tile = blockIdx.x / cs;
   const bool glu = p.out_mode == 2;
@@ -87,65 +87,72 @@ __global__ void __launch_bounds__(SK_T)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      auto load_p = [&](int kb, int s) {
-        const bool ext = kb >= nk_main;
-        const int k0 = (ext ? kb - nk_main : kb) * SK_BK;
-        uint8_t* dst = smem + s * C::STAGE;
-        const CUtensorMap* m = ext ? &tmP2 : &tmP;
-        if (glu) {
-          tma_load_2d(dst, m, &full[s], k0, tile * 64);
-          tma_load_2d(dst + SK_P_BYTES / 2, m, &full[s], k0, p.R + tile * 64);
-        } else {
-          tma_load_2d(dst, m, &full[s], k0, tile * SK_BM);
-        }
-      };
-      auto load_s = [&](int kb, int s) {
-        const bool ext = kb >= nk_main;
-        tma_load_2d(smem + s * C::STAGE + SK_P_BYTES, ext ? &tmS2 : &tmS, &full[s], (ext ? kb - nk_main : kb) * SK_BK, 0);
-      };
-      if (p.p_dep) pdl_wait();
-      const int pre = min(C::STAGES, kb1 - kb0);
-      for (int i = 0; i < pre; ++i) {
+    auto load_p = [&](int kb, int s) {
+      const bool ext = kb >= nk_main;
+      const int k0 = (ext ? kb - nk_main : kb) * SK_BK;
+      uint8_t* dst = smem + s * C::STAGE;
+      const CUtensorMap* m = ext ? &tmP2 : &tmP;
+      if (glu) {
+        tma_load_2d(dst, m, &full[s], k0, tile * 64);
+        tma_load_2d(dst + SK_P_BYTES / 2, m, &full[s], k0, p.R + tile * 64);
+      } else {
+        tma_load_2d(dst, m, &full[s], k0, tile * SK_BM);
+      }
+    };
+    auto load_s = [&](int kb, int s) {
+      const bool ext = kb >= nk_main;
+      tma_load_2d(smem + s * C::STAGE + SK_P_BYTES, ext ? &tmS2 : &tmS, &full[s], (ext ? kb - nk_main : kb) * SK_BK, 0);
+    };
+    if (p.p_dep) pdl_wait();
+    const int pre = min(C::STAGES, kb1 - kb0);
+    for (int i = 0; i < pre; ++i) {
+      if (elect_one()) {
         mbar_expect_tx(&full[i], C::STAGE);
         load_p(kb0 + i, i);
       }
-      pdl_wait();
-      for (int i = 0; i < pre; ++i) load_s(kb0 + i, i);
-      int s = 0;
-      uint32_t phase = 0;              // stage s is refilled once its first contents have been consumed
-      for (int kb = kb0 + pre; kb < kb1; ++kb) {
-        if (!mbar_wait(&empty[s], phase, p.status, AXB_TIMEOUT_EMPTY)) break;
+      __syncwarp();
+    }
+    pdl_wait();
+    for (int i = 0; i < pre; ++i) {
+      if (elect_one()) load_s(kb0 + i, i);
+      __syncwarp();
+    }
+    int s = 0;
+    uint32_t phase = 0;              // stage s is refilled once its first contents have been consumed
+    for (int kb = kb0 + pre; kb < kb1; ++kb) {
+      if (!warp_all(mbar_wait(&empty[s], phase, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
         mbar_expect_tx(&full[s], C::STAGE);
         load_p(kb, s);
         load_s(kb, s);
-        if (++s == C::STAGES) {
-          s = 0;
-          phase ^= 1;
-        }
+      }
+      __syncwarp();
+      if (++s == C::STAGES) {
+        s = 0;
+        phase ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(SK_BM, NT, 0, 0);
-      int s = 0;
-      uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full[s], phase, p.status, AXB_TIMEOUT_FULL)) break;
-        tc_fence_after();
-        const uint32_t a = smem_u32(smem + s * C::STAGE), b = a + SK_P_BYTES;
+    constexpr uint32_t idesc = make_idesc_bf16(SK_BM, NT, 0, 0);
+    const uint64_t base = make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+    int s = 0;
+    uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!warp_all(mbar_wait(&full[s], phase, p.status, AXB_TIMEOUT_FULL))) break;
+      tc_fence_after();
+      const uint64_t a = base + (uint32_t)(s * (C::STAGE / 16)), b = a + SK_P_BYTES / 16;
+      if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < SK_BK / 16; ++kk)
-          umma_f16(tmem, make_smem_desc_sw128(a + kk * 32, 16, 1024), make_smem_desc_sw128(b + kk * 32, 16, 1024), idesc,
-                   (kb > kb0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < SK_BK / 16; ++kk) umma_f16(tmem, a + kk * 2, b + kk * 2, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
         umma_commit(&empty[s]);
-        if (++s == C::STAGES) {
-          s = 0;
-          phase ^= 1;
-        }
       }
-      umma_commit(done);
+      __syncwarp();
+      if (++s == C::STAGES) {
+        s = 0;
+        phase ^= 1;
+      }
     }
+    if (elect_one()) umma_commit(done);
   }
   __syncwarp();
   mbar_wait(done, 0, p.status, AXB_TIMEOUT_TMEM_FULL);

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* tempty_bar = bars + 2 * C::STAGES + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const int n_blocks = MODE == GRAM ? 0 : *p.n_blocks;
 
@@ -141,25 +141,25 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      Tile t;
-      for (int tile = blockIdx.x; ok && decode<BN, MODE>(p, tile, n_blocks, t); tile += gridDim.x) {
-        const int nk = t.nk_main + t.nk_ext;
-        for (int kb = 0; kb < nk; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    Tile t;
+    for (int tile = blockIdx.x; ok && decode<BN, MODE>(p, tile, n_blocks, t); tile += gridDim.x) {
+      const int nk = t.nk_main + t.nk_ext;
+      for (int kb = 0; kb < nk; ++kb) {
+        if (!warp_all(mbar_wait(&empty_bar[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
+          ok = false;
+          break;
+        }
+        const bool ext = kb >= t.nk_main;
+        const CUtensorMap* ma = ext ? &tmA2 : &tmA;
+        const CUtensorMap* mb = ext ? &tmB2 : &tmB;
+        const int k = ext ? (kb - t.nk_main) * BK : t.k0 + kb * BK;
+        uint8_t* a_dst = sA + stage * C::A_BYTES;
+        uint8_t* b_dst = sB + stage * C::B_BYTES;
+        if (elect_one()) {
           mbar_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-          const bool ext = kb >= t.nk_main;
-          const CUtensorMap* ma = ext ? &tmA2 : &tmA;
-          const CUtensorMap* mb = ext ? &tmB2 : &tmB;
-          const int k = ext ? (kb - t.nk_main) * BK : t.k0 + kb * BK;
-          uint8_t* a_dst = sA + stage * C::A_BYTES;
-          uint8_t* b_dst = sB + stage * C::B_BYTES;
           if (!A_MN) {
             tma_load_2d(a_dst, ma, &full_bar[stage], k, t.m0);
           } else {
@@ -174,54 +174,52 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int c = 0; c < BN / 64; ++c)
               tma_load_3d(b_dst + c * 8192, mb, &full_bar[stage], t.n0 + c * 64, k, t.zb);
           }
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++stage == C::STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      bool ok = true;
-      Tile t;
-      for (int tile = blockIdx.x; ok && decode<BN, MODE>(p, tile, n_blocks, t); tile += gridDim.x) {
-        const int nk = t.nk_main + t.nk_ext;
-        if (nk == 0) continue;
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        ++it;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < nk; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * C::A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * C::B_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_addr + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_addr + kk * 32, 16, 1024);
-            umma_f16(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+    constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr uint32_t a_step = (A_MN ? 2048 : 32) / 16, b_step = (B_MN ? 2048 : 32) / 16;
+    const uint64_t da_base = make_smem_desc_sw128(smem_u32(sA), A_MN ? 8192 : 16, 1024);
+    const uint64_t db_base = make_smem_desc_sw128(smem_u32(sB), B_MN ? 8192 : 16, 1024);
+    int stage = 0;
+    uint32_t phase = 0;
+    int it = 0;
+    bool ok = true;
+    Tile t;
+    for (int tile = blockIdx.x; ok && decode<BN, MODE>(p, tile, n_blocks, t); tile += gridDim.x) {
+      const int nk = t.nk_main + t.nk_ext;
+      if (nk == 0) continue;
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      ++it;
+      if (!warp_all(mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = 0; kb < nk; ++kb) {
+        if (!warp_all(mbar_wait(&full_bar[stage], phase, p.status, AXB_TIMEOUT_FULL))) {
+          ok = false;
+          break;
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
+        tc_fence_after();
+        const uint64_t da = da_base + (uint32_t)(stage * (C::A_BYTES / 16)), db = db_base + (uint32_t)(stage * (C::B_BYTES / 16));
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma_f16(d_tmem, da + kk * a_step, db + kk * b_step, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(&empty_bar[stage]);
+          if (kb == nk - 1) umma_commit(&tfull_bar[acc]);
+        }
+        __syncwarp();
+        if (++stage == C::STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
     }
   } else {

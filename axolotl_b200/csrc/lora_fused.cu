@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1)
   uint64_t* t_done = bars + 15;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int t_chunk = blockIdx.x / p.n_splits, split = blockIdx.x % p.n_splits;
   const int row0 = t_chunk * LF_ROWS;
   const int nb0 = (int)((long long)p.n_blocks * split / p.n_splits);
@@ -93,89 +93,92 @@ __global__ void __launch_bounds__(LF_THREADS, 1)
   // TMEM columns: t accumulators [sub * 64, +Rpad), dB accumulators [256 + buf * 64, +Rpad)
   if (nb1 > nb0 && n_sub > 0) {
     if (warp == 0) {
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(xa_full, n_sub * LF_SMALL_BYTES);
         for (int s = 0; s < n_sub; ++s) {
           tma_load_2d(sXA + s * LF_SMALL_BYTES, &tmXA, xa_full, 0, row0 + s * 128);
           tma_load_2d(sXA + s * LF_SMALL_BYTES + 8192, &tmXA, xa_full, 0, row0 + s * 128 + 64);
         }
-        int stage = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int nb = nb0, i = 0; nb < nb1 && ok; ++nb, ++i) {
-          const int bb = i & 1;
-          if (!mbar_wait(&b_empty[bb], ((i >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+      }
+      __syncwarp();
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int nb = nb0, i = 0; nb < nb1 && ok; ++nb, ++i) {
+        const int bb = i & 1;
+        if (!warp_all(mbar_wait(&b_empty[bb], ((i >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+        if (elect_one()) {
           mbar_expect_tx(&b_full[bb], LF_SMALL_BYTES);
           tma_load_2d(sB + bb * LF_SMALL_BYTES, &tmB, &b_full[bb], 0, nb * 128);
           tma_load_2d(sB + bb * LF_SMALL_BYTES + 8192, &tmB, &b_full[bb], 0, nb * 128 + 64);
-          for (int s = 0; s < n_sub; ++s) {
-            if (!mbar_wait(&dy_empty[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY)) {
-              ok = false;
-              break;
-            }
+        }
+        __syncwarp();
+        for (int s = 0; s < n_sub; ++s) {
+          if (!warp_all(mbar_wait(&dy_empty[stage], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
+            ok = false;
+            break;
+          }
+          uint8_t* dst = sDY + stage * LF_DY_BYTES;
+          if (elect_one()) {
             mbar_expect_tx(&dy_full[stage], LF_DY_BYTES);
-            uint8_t* dst = sDY + stage * LF_DY_BYTES;
             tma_load_2d(dst, &tmDY, &dy_full[stage], nb * 128, row0 + s * 128);
             tma_load_2d(dst + 16384, &tmDY, &dy_full[stage], nb * 128 + 64, row0 + s * 128);
-            if (++stage == LF_DY_STAGES) {
-              stage = 0;
-              phase ^= 1;
-            }
+          }
+          __syncwarp();
+          if (++stage == LF_DY_STAGES) {
+            stage = 0;
+            phase ^= 1;
           }
         }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
-        const uint32_t idesc1 = make_idesc_bf16(128, p.Rpad, 0, 1);   // A = dY tile K-major, B = B tile MN-major
-        const uint32_t idesc2 = make_idesc_bf16(128, p.Rpad, 1, 1);   // A = dY tile read MN-major, B = xa MN-major
-        bool ok = mbar_wait(xa_full, 0, p.status, AXB_TIMEOUT_FULL);
-        int stage = 0;
-        uint32_t phase = 0;
-        for (int nb = nb0, i = 0; nb < nb1 && ok; ++nb, ++i) {
-          const int bb = i & 1;
-          const uint32_t use = (i >> 1) & 1;
-          if (!mbar_wait(&b_full[bb], use, p.status, AXB_TIMEOUT_FULL) ||
-              !mbar_wait(&db_empty[bb], use ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) {
+      const uint32_t idesc1 = make_idesc_bf16(128, p.Rpad, 0, 1);   // A = dY tile K-major, B = B tile MN-major
+      const uint32_t idesc2 = make_idesc_bf16(128, p.Rpad, 1, 1);   // A = dY tile read MN-major, B = xa MN-major
+      const uint64_t dy_k = make_smem_desc_sw128(smem_u32(sDY), 16, 1024), dy_mn = make_smem_desc_sw128(smem_u32(sDY), 16384, 1024);
+      const uint64_t b_mn = make_smem_desc_sw128(smem_u32(sB), 8192, 1024), xa_mn = make_smem_desc_sw128(smem_u32(sXA), 8192, 1024);
+      bool ok = warp_all(mbar_wait(xa_full, 0, p.status, AXB_TIMEOUT_FULL));
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int nb = nb0, i = 0; nb < nb1 && ok; ++nb, ++i) {
+        const int bb = i & 1;
+        const uint32_t use = (i >> 1) & 1;
+        ok = warp_all(mbar_wait(&b_full[bb], use, p.status, AXB_TIMEOUT_FULL) &&
+                      mbar_wait(&db_empty[bb], use ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY));
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t db1 = b_mn + (uint32_t)(bb * (LF_SMALL_BYTES / 16));
+        const uint32_t d_db = tmem_base + 256 + bb * 64;
+        for (int s = 0; s < n_sub; ++s) {
+          if (!warp_all(mbar_wait(&dy_full[stage], phase, p.status, AXB_TIMEOUT_FULL))) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t b_addr = smem_u32(sB + bb * LF_SMALL_BYTES);
-          const uint32_t d_db = tmem_base + 256 + bb * 64;
-          for (int s = 0; s < n_sub; ++s) {
-            if (!mbar_wait(&dy_full[stage], phase, p.status, AXB_TIMEOUT_FULL)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t a_addr = smem_u32(sDY + stage * LF_DY_BYTES);
-            const uint32_t xa_addr = smem_u32(sXA + s * LF_SMALL_BYTES);
-            const uint32_t d_t = tmem_base + s * 64;
+          const uint64_t da1 = dy_k + (uint32_t)(stage * (LF_DY_BYTES / 16)), da2 = dy_mn + (uint32_t)(stage * (LF_DY_BYTES / 16));
+          const uint64_t db2 = xa_mn + (uint32_t)(s * (LF_SMALL_BYTES / 16));
+          const uint32_t d_t = tmem_base + s * 64;
+          if (elect_one()) {
             // t[s] += dY(128 x 128) . B(128 x R): k runs over the 128 columns of the tile (two 64-column halves)
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-              const uint64_t da = make_smem_desc_sw128(a_addr + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-              const uint64_t db = make_smem_desc_sw128(b_addr + kk * 2048, 8192, 1024);
-              umma_f16(d_t, da, db, idesc1, (i > 0 || kk > 0) ? 1u : 0u);
-            }
+            for (int kk = 0; kk < 8; ++kk)
+              umma_f16(d_t, da1 + ((kk >> 2) * 16384 + (kk & 3) * 32) / 16, db1 + kk * (2048 / 16), idesc1, (i > 0 || kk > 0) ? 1u : 0u);
             // dB[nb] += dY^T(128 cols x 128 rows) . xa(128 rows x R): k runs over the 128 token rows
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-              const uint64_t da = make_smem_desc_sw128(a_addr + kk * 2048, 16384, 1024);
-              const uint64_t db = make_smem_desc_sw128(xa_addr + kk * 2048, 8192, 1024);
-              umma_f16(d_db, da, db, idesc2, (s > 0 || kk > 0) ? 1u : 0u);
-            }
+            for (int kk = 0; kk < 8; ++kk)
+              umma_f16(d_db, da2 + kk * (2048 / 16), db2 + kk * (2048 / 16), idesc2, (s > 0 || kk > 0) ? 1u : 0u);
             umma_commit(&dy_empty[stage]);
-            if (++stage == LF_DY_STAGES) {
-              stage = 0;
-              phase ^= 1;
+            if (s == n_sub - 1) {
+              umma_commit(&db_full[bb]);
+              umma_commit(&b_empty[bb]);
+              if (nb == nb1 - 1) umma_commit(t_done);
             }
           }
-          if (!ok) break;
-          umma_commit(&db_full[bb]);
-          umma_commit(&b_empty[bb]);
+          __syncwarp();
+          if (++stage == LF_DY_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        if (ok) umma_commit(t_done);
       }
     } else {
       const int lg = warp & 3;   // TMEM lanes [32 lg, 32 lg + 32)
