@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(192, 1)
   uint64_t* pv_empty = bars + 13; // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     mbar_init(k_full, 1);
@@ -134,68 +134,79 @@ __global__ void __launch_bounds__(192, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, C::QK_BYTES);
 #pragma unroll
       for (int h = 0; h < DQK / 64; ++h)
         tma_load_2d(sQ + h * HALF_BYTES, &tm_q, q_full, p.q_col0 + head * DQK + h * 64, doc_start + q0);
-      for (int j = 0; j < n_blocks; ++j) {
-        const uint32_t ph = j & 1;
-        if (!mbar_wait(k_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+    }
+    __syncwarp();
+    for (int j = 0; j < n_blocks; ++j) {
+      const uint32_t ph = j & 1;
+      if (!warp_all(mbar_wait(k_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
         mbar_expect_tx(k_full, C::QK_BYTES);
 #pragma unroll
         for (int h = 0; h < DQK / 64; ++h)
           tma_load_2d(sK + h * HALF_BYTES, &tm_kv, k_full, p.k_col0 + kv_head * DQK + h * 64, doc_start + (jb0 + j) * 128);
-        if (!mbar_wait(v_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+      }
+      __syncwarp();
+      if (!warp_all(mbar_wait(v_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
         mbar_expect_tx(v_full, C::V_BYTES);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           tma_load_2d(sV + h * HALF_BYTES, &tm_kv, v_full, p.v_col0 + kv_head * DV + part * 128 + h * 64,
                       doc_start + (jb0 + j) * 128);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
-      const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV), p_addr = smem_u32(sP);
-      bool ok = mbar_wait(q_full, 0, p.status, AXB_TIMEOUT_FULL);
-      auto issue_s = [&](int j) -> bool {
-        const int b = j & 1;
-        if (!mbar_wait(k_full, j & 1, p.status, AXB_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(&s_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
+    constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
+    const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dk = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
+    const uint64_t dv = make_smem_desc_sw128(smem_u32(sV), HALF_BYTES, 1024), dp = make_smem_desc_sw128(smem_u32(sP), 16, 1024);
+    bool ok = warp_all(mbar_wait(q_full, 0, p.status, AXB_TIMEOUT_FULL));
+    auto issue_s = [&](int j) -> bool {
+      const int b = j & 1;
+      if (!warp_all(mbar_wait(k_full, j & 1, p.status, AXB_TIMEOUT_FULL) &&
+                    mbar_wait(&s_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)))
+        return false;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {
-          const uint32_t off = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + b * 128, make_smem_desc_sw128(q_addr + off, 16, 1024),
-                   make_smem_desc_sw128(k_addr + off, 16, 1024), idesc_s, kk > 0);
+          const uint32_t off = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
+          umma_f16(tmem_base + b * 128, dq + off, dk + off, idesc_s, kk > 0);
         }
         umma_commit(&s_full[b]);
         umma_commit(k_empty);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        const int b = j & 1;
-        if (j + 1 < n_blocks) {
-          ok = issue_s(j + 1);
-          if (!ok) break;
-        }
-        if (!mbar_wait(p_full, j & 1, p.status, AXB_TIMEOUT_GENERIC)) break;
-        if (!mbar_wait(v_full, j & 1, p.status, AXB_TIMEOUT_FULL)) break;
-        if (!mbar_wait(&pv_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    if (ok) ok = issue_s(0);
+    for (int j = 0; j < n_blocks && ok; ++j) {
+      const int b = j & 1;
+      if (j + 1 < n_blocks) {
+        ok = issue_s(j + 1);
+        if (!ok) break;
+      }
+      if (!warp_all(mbar_wait(p_full, j & 1, p.status, AXB_TIMEOUT_GENERIC) && mbar_wait(v_full, j & 1, p.status, AXB_TIMEOUT_FULL) &&
+                    mbar_wait(&pv_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)))
+        break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t poff = (kk / 4) * HALF_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + 256 + b * 128, make_smem_desc_sw128(p_addr + poff, 16, 1024),
-                   make_smem_desc_sw128(v_addr + kk * 2048, HALF_BYTES, 1024), idesc_pv, kk > 0);
+          const uint32_t poff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
+          umma_f16(tmem_base + 256 + b * 128, dp + poff, dv + kk * (2048 / 16), idesc_pv, kk > 0);
         }
         umma_commit(&pv_full[b]);
         umma_commit(v_empty);
         umma_commit(p_empty);
       }
+      __syncwarp();
     }
   } else {
     const int lg = warp & 3;
@@ -352,8 +363,12 @@ struct WBwd {
   static constexpr int ST_COL = 0, DPT_COL = 64, DV_COL = 128, DK_COL = 256;
 };
 
+// Two softmax warpgroups share every q tile, 32 columns each: with nothing double-buffered (shared memory is full) an iteration
+// is a chain of scores -> P^T, dS^T -> dQ^T, and the second group halves its middle. lse / delta are requested an iteration
+// early, Q / dO are handed back before dQ^T runs, and the columns of dQ^T once they are in registers.
+constexpr int WBWD_THREADS = 320;
 template <int DQK, int DV, bool SOFTCAP>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(WBWD_THREADS, 1)
     flash_wide_bwd_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_q,
                           const __grid_constant__ CUtensorMap tm_do, const WideParams p) {
   using C = WBwd<DQK, DV>;
@@ -399,15 +414,15 @@ __global__ void __launch_bounds__(192, 1)
   uint64_t* acc_full = bars + 7;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
     mbar_init(s_full, 1);
-    mbar_init(pt_full, 128);
+    mbar_init(pt_full, 256);
     mbar_init(dq_full, 1);
-    mbar_init(st_free, 128);
+    mbar_init(st_free, 256);
     mbar_init(acc_full, 1);
     mbar_fence_init();
   }
@@ -421,7 +436,7 @@ __global__ void __launch_bounds__(192, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, C::K_BYTES + C::V_BYTES);
 #pragma unroll
       for (int h = 0; h < DQK / 64; ++h)
@@ -429,10 +444,13 @@ __global__ void __launch_bounds__(192, 1)
 #pragma unroll
       for (int h = 0; h < DV / 64; ++h)
         tma_load_2d(sV + h * HALF_BYTES, &tm_kv, kv_full, p.v_col0 + kv_head * DV + h * 64, doc_start + kv0);
-      for (int it = 0; it < n_iter; ++it) {
-        const int head = head0 + it / n_qt;
-        const int qrow = doc_start + (q_first + it % n_qt) * 64;
-        if (!mbar_wait(q_empty, (it & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY)) break;
+    }
+    __syncwarp();
+    int qt = 0, head = head0;
+    for (int it = 0; it < n_iter; ++it) {
+      const int qrow = doc_start + (q_first + qt) * 64;
+      if (!warp_all(mbar_wait(q_empty, (it & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
         mbar_expect_tx(q_full, C::Q_BYTES + C::DO_BYTES);
 #pragma unroll
         for (int h = 0; h < DQK / 64; ++h)
@@ -441,83 +459,98 @@ __global__ void __launch_bounds__(192, 1)
         for (int h = 0; h < DV / 64; ++h)
           tma_load_2d(sdO + h * QH_BYTES, &tm_do, q_full, head * DV + h * 64, qrow);
       }
+      __syncwarp();
+      if (++qt == n_qt) {
+        qt = 0;
+        ++head;
+      }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);
-      constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1);
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, 1, 1);
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sdO);
-      const uint32_t pt_addr = smem_u32(sPT), dst_addr = smem_u32(sdST);
-      bool ok = mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const uint32_t ph = it & 1;
-        if (!mbar_wait(q_full, ph, p.status, AXB_TIMEOUT_FULL)) break;
-        // the S^T columns carried dQ^T of the previous iteration: it must have been drained
-        if (it > 0 && !mbar_wait(st_free, (it - 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
+    constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);
+    constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1);
+    constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, 1, 1);
+    const uint64_t dk_k = make_smem_desc_sw128(smem_u32(sK), 16, 1024), dv_k = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
+    const uint64_t dq_k = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), do_k = make_smem_desc_sw128(smem_u32(sdO), 16, 1024);
+    const uint64_t pt_k = make_smem_desc_sw128(smem_u32(sPT), 16, 1024), ds_k = make_smem_desc_sw128(smem_u32(sdST), 16, 1024);
+    const uint64_t do_mn = make_smem_desc_sw128(smem_u32(sdO) + (vpart / 64) * QH_BYTES, QH_BYTES, 1024);
+    const uint64_t dq_mn = make_smem_desc_sw128(smem_u32(sQ) + (kpart / 64) * QH_BYTES, QH_BYTES, 1024);
+    const uint64_t dk_mn = make_smem_desc_sw128(smem_u32(sK) + (kpart / 64) * HALF_BYTES, HALF_BYTES, 1024);
+    const uint64_t ds_mn = make_smem_desc_sw128(smem_u32(sdST), HALF_BYTES, 1024);
+    bool ok = warp_all(mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL));
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const uint32_t ph = it & 1;
+      bool fine = mbar_wait(q_full, ph, p.status, AXB_TIMEOUT_FULL);
+      // the S^T columns carried dQ^T of the previous iteration: it must have been drained
+      if (fine && it > 0) fine = mbar_wait(st_free, (it - 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY);
+      if (!warp_all(fine)) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < DQK / 16; ++kk) {
-          const uint32_t koff = (kk / 4) * HALF_BYTES + (kk % 4) * 32, qoff = (kk / 4) * QH_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + C::ST_COL, make_smem_desc_sw128(k_addr + koff, 16, 1024),
-                   make_smem_desc_sw128(q_addr + qoff, 16, 1024), idesc_st, kk > 0);
+          const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * QH_BYTES + (kk % 4) * 32) / 16;
+          umma_f16(tmem_base + C::ST_COL, dk_k + koff, dq_k + qoff, idesc_st, kk > 0);
         }
 #pragma unroll
         for (int kk = 0; kk < DV / 16; ++kk) {
-          const uint32_t koff = (kk / 4) * HALF_BYTES + (kk % 4) * 32, qoff = (kk / 4) * QH_BYTES + (kk % 4) * 32;
-          umma_f16(tmem_base + C::DPT_COL, make_smem_desc_sw128(v_addr + koff, 16, 1024),
-                   make_smem_desc_sw128(do_addr + qoff, 16, 1024), idesc_st, kk > 0);
+          const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * QH_BYTES + (kk % 4) * 32) / 16;
+          umma_f16(tmem_base + C::DPT_COL, dv_k + koff, do_k + qoff, idesc_st, kk > 0);
         }
         umma_commit(s_full);
-        if (!mbar_wait(pt_full, ph, p.status, AXB_TIMEOUT_GENERIC)) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      if (!warp_all(mbar_wait(pt_full, ph, p.status, AXB_TIMEOUT_GENERIC))) break;
+      tc_fence_after();
+      if (elect_one()) {
         if (has_v) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_f16(tmem_base + C::DV_COL, make_smem_desc_sw128(pt_addr + kk * 32, 16, 1024),
-                     make_smem_desc_sw128(do_addr + (vpart / 64) * QH_BYTES + kk * 2048, QH_BYTES, 1024), idesc_acc,
-                     (it > 0 || kk > 0));
+            umma_f16(tmem_base + C::DV_COL, pt_k + kk * 2, do_mn + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
         }
         if (has_k) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_f16(tmem_base + C::DK_COL, make_smem_desc_sw128(dst_addr + kk * 32, 16, 1024),
-                     make_smem_desc_sw128(q_addr + (kpart / 64) * QH_BYTES + kk * 2048, QH_BYTES, 1024), idesc_acc,
-                     (it > 0 || kk > 0));
+            umma_f16(tmem_base + C::DK_COL, ds_k + kk * 2, dq_mn + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
+        }
+        umma_commit(q_empty);   // Q and dO of this iteration are consumed: the next ones load beside dQ^T
+        if (has_k) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_f16(tmem_base + C::ST_COL, make_smem_desc_sw128(k_addr + (kpart / 64) * HALF_BYTES + kk * 2048, HALF_BYTES, 1024),
-                     make_smem_desc_sw128(dst_addr + kk * 2048, HALF_BYTES, 1024), idesc_dq, kk > 0);
+            umma_f16(tmem_base + C::ST_COL, dk_mn + kk * (2048 / 16), ds_mn + kk * (2048 / 16), idesc_dq, kk > 0);
         }
-        umma_commit(q_empty);   // Q, dO, P^T, dS^T of this iteration are consumed
-        umma_commit(dq_full);
+        umma_commit(dq_full);   // ... and P^T, dS^T
+        if (it == n_iter - 1) umma_commit(acc_full);
       }
-      umma_commit(acc_full);
+      __syncwarp();
     }
   } else {
     const int lg = warp & 3;
     const int r = lg * 32 + lane;   // kv row of the tile (S^T, dP^T, dK, dV) or column of the part (dQ^T)
-    const int tid = threadIdx.x - 64;
+    const int grp = (warp - 2) >> 2;   // columns [32 grp, 32 grp + 32) of every q tile
+    const int tid = threadIdx.x - 64 - grp * 128;
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
     bool ok = true;
+    // -lse or delta * scale of one of this group's 32 q rows, requested an iteration ahead (rows outside: P = 0)
+    auto fetch_row = [&](int it) -> float {
+      float val = tid < 32 ? -INFINITY : 0.f;
+      if (tid >= 64 || it >= n_iter) return val;
+      const int q = (q_first + it % n_qt) * 64 + grp * 32 + (tid & 31);
+      const long long row = (long long)doc_start + q;
+      if (q < doc_len && row < p.T) {
+        const long long off = (long long)(head0 + it / n_qt) * p.T + row;
+        val = tid < 32 ? -p.lse2[off] : p.delta[off] * p.scale;
+      }
+      return val;
+    };
+    float row_val = fetch_row(0);
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t ph = it & 1;
       const int head = head0 + it / n_qt;
       const int qt0 = (q_first + it % n_qt) * 64;
-      asm volatile("bar.sync 1, 128;" ::: "memory");   // everyone finished reading the previous lse / delta
-      {
-        const int i = tid & 63;
-        const int q = qt0 + i;
-        float val = tid < 64 ? -INFINITY : 0.f;
-        const long long row = (long long)doc_start + q;
-        if (q < doc_len && row < p.T) {
-          const long long off = (long long)head * p.T + row;
-          val = tid < 64 ? -p.lse2[off] : p.delta[off] * p.scale;
-        }
-        (tid < 64 ? s_lse : s_delta)[i] = val;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");   // the group finished reading the previous lse / delta
+      if (tid < 64) (tid < 32 ? s_lse : s_delta)[grp * 32 + (tid & 31)] = row_val;
+      row_val = fetch_row(it + 1);
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
       if (!mbar_wait(s_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
@@ -526,8 +559,8 @@ __global__ void __launch_bounds__(192, 1)
       const bool row_in_doc = kv_idx < doc_len;
       const int q_lo = row_in_doc ? (bidir ? -(1 << 30) : kv_idx) : (1 << 30);
       const int q_hi = win > 0 ? kv_idx + win - 1 : (1 << 30);
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      {
+        const int c = grp;
         uint32_t sr[32], dr[32];
         tmem_ld_32x32(tmem_base + lane_off + C::ST_COL + c * 32, sr);
         tmem_ld_32x32(tmem_base + lane_off + C::DPT_COL + c * 32, dr);
@@ -576,20 +609,20 @@ __global__ void __launch_bounds__(192, 1)
         int i_hi = min(64, doc_len - qt0);
         if (row0 + i_hi > p.T) i_hi = (int)(p.T - row0);
         float* col = p.dq_acc + row0 * p.dq_ld + (long long)head * DQK + kpart + r;
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          uint32_t qr[32];
-          tmem_ld_32x32(tmem_base + lane_off + C::ST_COL + c * 32, qr);
-          tmem_ld_wait();
-          if (r >= k_lo) {
+        uint32_t qr[32];
+        tmem_ld_32x32(tmem_base + lane_off + C::ST_COL + grp * 32, qr);
+        tmem_ld_wait();
+        tc_fence_before();
+        mbar_arrive(st_free);        // the next scores may overwrite the columns while the sums leave
+        if (r >= k_lo) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i < i_hi) atomicAdd(col + (long long)(c * 32 + i) * p.dq_ld, __uint_as_float(qr[i]));
-          }
+          for (int i = 0; i < 32; ++i)
+            if (grp * 32 + i < i_hi) atomicAdd(col + (long long)(grp * 32 + i) * p.dq_ld, __uint_as_float(qr[i]));
         }
+      } else {
+        tc_fence_before();
+        mbar_arrive(st_free);
       }
-      tc_fence_before();
-      mbar_arrive(st_free);
     }
     if (ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
@@ -598,7 +631,7 @@ __global__ void __launch_bounds__(192, 1)
       __nv_bfloat16* krow = p.dkv + grow * p.dkv_ld + p.dk_col0 + (long long)kv_head * DQK + kpart;
       __nv_bfloat16* vrow = p.dkv + grow * p.dkv_ld + p.dv_col0 + (long long)kv_head * DV + vpart;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 2 * grp; c < 2 * grp + 2; ++c) {
         uint32_t a[32], b[32];
         tmem_ld_32x32(tmem_base + lane_off + C::DK_COL + c * 32, a);
         tmem_ld_32x32(tmem_base + lane_off + C::DV_COL + c * 32, b);
@@ -696,7 +729,7 @@ int launch_wide_bwd(const CUtensorMap& tkv, const CUtensorMap& tq, const CUtenso
   constexpr int pk = (DQK + 127) / 128, pv = (DV + 127) / 128;
   constexpr int parts = pk > pv ? pk : pv;
   dim3 grid(p.Hk, p.n_tiles, parts);
-  kern<<<grid, 192, C::SMEM, st>>>(tkv, tq, tdo, p);
+  kern<<<grid, WBWD_THREADS, C::SMEM, st>>>(tkv, tq, tdo, p);
   return (int)cudaGetLastError();
 }
 
