@@ -456,6 +456,15 @@ AXB_DEVICE float2 unpack_bf16x2(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
+// Row `lane` of a 32-row staging tile with 128-byte rows (64 bf16) and the 128-byte swizzle the
+// tensor map expects: 16-byte chunk j of row r sits at chunk position j ^ (r & 7). The tile base is
+// 1024-byte aligned.
+AXB_DEVICE void stage_row128(uint8_t* tile, int lane, const uint4 (&w)[8]) {
+  uint8_t* rowp = tile + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) = w[j];
+}
+
 // ------------------------------------------------------------------ host helpers
 #include <atomic>
 #include <cstdio>

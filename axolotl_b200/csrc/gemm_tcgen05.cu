@@ -93,15 +93,7 @@ struct GemmParams {
 
 int g_epi_sleep_ns = 64, g_prod_sleep_ns = 0, g_pair_group_m = 0, g_pair_tma_store = 1, g_pair_band_mb = 32;
 
-// Row `lane` of a 32-row staging tile with 128-byte rows (64 bf16) and the 128-byte swizzle the
-// tensor map expects: 16-byte chunk j of row r sits at chunk position j ^ (r & 7). The tile base is
-// 1024-byte aligned.
-__device__ __forceinline__ void stage_row128(uint8_t* tile, int lane, const uint4 (&w)[8]) {
-  uint8_t* rowp = tile + lane * 128;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(rowp + ((j ^ (lane & 7)) << 4)) = w[j];
-}
-// Same for 64-byte rows (32 bf16) and the 64-byte swizzle: chunk j of row r sits at j ^ ((r >> 1) & 3).
+// stage_row128 for 64-byte rows (32 bf16) and the 64-byte swizzle: chunk j of row r sits at j ^ ((r >> 1) & 3).
 __device__ __forceinline__ void stage_row64(uint8_t* tile, int lane, const uint4 (&w)[4]) {
   uint8_t* rowp = tile + lane * 64;
 #pragma unroll

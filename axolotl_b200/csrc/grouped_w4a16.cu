@@ -29,16 +29,17 @@ constexpr int BN = 128;
 constexpr int BK = 64;
 constexpr int W4_CONV_WARPS = 8;
 constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (A), MMA, 4 epilogue warps, 8 converter warps, TMA (weights)
-// Three rings of their own: the packed weights are small and run eight k blocks ahead, so a converter never waits for memory;
+// Three rings of their own: the packed weights are small and run four k blocks ahead of the decode;
 // a slot of the decoded tile is only held from its decode to its MMA, and a slot of A from its load to its MMA.
 // The converters work in four groups of two warps, each on a k block of its own, so that four chains (packed tile seen ->
 // decode -> stores -> proxy fence -> arrival) run side by side.
-constexpr int SA = 4, SB = 4, SR = 8;  // slots: A (two 128-row tiles), decoded B, packed B
+constexpr int SA = 4, SB = 4, SR = 4;  // slots: A (two 128-row tiles), decoded B, packed B
 constexpr int CGROUPS = 4, CG_WARPS = W4_CONV_WARPS / CGROUPS, CG_UNITS = 256 / (32 * CG_WARPS);
 constexpr int A_BYTES = BM * BK * 2;   // one 128-row A tile; a slot holds two
 constexpr int B_BYTES = BN * BK * 2;
 constexpr int RAW_BYTES = 4096;   // FWD: 128 rows x 32 bytes; DX: 64 rows x 64 bytes
-constexpr int W4_SMEM = SA * 2 * A_BYTES + SB * B_BYTES + SR * RAW_BYTES + 1024 + 512;
+constexpr int EPI_BYTES = 4096;   // per epilogue warp: 32 rows x 64 bf16 columns on their way out
+constexpr int W4_SMEM = SA * 2 * A_BYTES + SB * B_BYTES + SR * RAW_BYTES + 4 * EPI_BYTES + 1024 + 512;
 static_assert(W4_SMEM <= 227 * 1024, "");
 
 // position in a ring of N slots
@@ -119,6 +120,7 @@ struct W4Params {
   long long ldc;
   float alpha;
   int out_mode;   // 0 bf16, 1 fp32
+  int tma_store;  // bf16 rows leave through staging tiles and TMA stores (row stores of 32 lanes, a line each, held up the converters)
   const uint8_t* scale;   // [E, Wn, Wk / 16] e4m3 bytes
   const float* pts;       // [E]
   const int* blk_expert;
@@ -178,13 +180,14 @@ template <bool DX>
 __global__ void __launch_bounds__(W4_THREADS, 1)
     grouped_w4a16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmQ,
                          const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
-                         const W4Params p) {
+                         const __grid_constant__ CUtensorMap tmC, const W4Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;                                   // [slot][2][128 x 64]
   uint8_t* sB = smem + SA * 2 * A_BYTES;
   uint8_t* sRaw = sB + SB * B_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + SR * RAW_BYTES);
+  uint8_t* sEpi = sRaw + SR * RAW_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + 4 * EPI_BYTES);
   uint64_t* a_full = bars;                      // A tiles landed
   uint64_t* a_empty = a_full + SA;              // their MMAs retired
   uint64_t* b_full = a_empty + SA;              // bf16 B tile in place (one arrival per warp of its group; the LoRA tile by TMA)
@@ -456,6 +459,37 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         }
         tc_fence_after();
         for (int h = 0; h <= ps.two; ++h) {
+          if (p.tma_store) {
+            const uint32_t t_row = tmem_base + (uint32_t(lane_group * 32) << 16) + acc * 2 * BN + h * BN;
+            uint8_t* tile_out = sEpi + lane_group * EPI_BYTES;
+#pragma unroll 1
+            for (int c = 0; c < BN / 64; ++c) {
+              if (ps.n0 + c * 64 >= p.N) break;
+              uint32_t r[2][32];
+              tmem_ld_32x32(t_row + c * 64, r[0]);
+              tmem_ld_32x32(t_row + c * 64 + 32, r[1]);
+              tmem_ld_wait();
+              uint4 w[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const uint32_t* v = &r[q >> 2][(q & 3) * 8];
+                w[q] = make_uint4(pack_bf16x2(__uint_as_float(v[0]) * p.alpha, __uint_as_float(v[1]) * p.alpha),
+                                  pack_bf16x2(__uint_as_float(v[2]) * p.alpha, __uint_as_float(v[3]) * p.alpha),
+                                  pack_bf16x2(__uint_as_float(v[4]) * p.alpha, __uint_as_float(v[5]) * p.alpha),
+                                  pack_bf16x2(__uint_as_float(v[6]) * p.alpha, __uint_as_float(v[7]) * p.alpha));
+              }
+              if (lane == 0) bulk_wait_group_read<0>();
+              __syncwarp();
+              stage_row128(tile_out, lane, w);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_store_2d(&tmC, tile_out, ps.n0 + c * 64, (ps.blk + h) * BM + lane_group * 32);
+                bulk_commit_group();
+              }
+            }
+            continue;
+          }
           const long long row = (long long)(ps.blk + h) * BM + lane_group * 32 + lane;
           const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + acc * 2 * BN + h * BN;
 #pragma unroll 1
@@ -493,6 +527,7 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         ++it;
       }
     }
+    if (lane == 0) bulk_wait_group<0>();
   }
 
   tc_fence_before();
@@ -518,7 +553,7 @@ extern "C" int axb_grouped_gemm_w4a16(const void* A, long long lda, const void* 
   if ((lda & 7) || (Wk & 63) || (Wn & 7) || (K2 > 0 && ((lda2 & 7) || (K2 & 7))) || out_mode < 0 || out_mode > 1) return -2;
   const unsigned long long rows = (unsigned long long)max_blocks * BM;
   const int Ka = trans_w ? Wn : Wk, N = trans_w ? Wk : Wn;
-  CUtensorMap tA, tQ, tA2, tB2;
+  CUtensorMap tA, tQ, tA2, tB2, tC;
   int rc = axb_make_tmap_2d(&tA, A, rows, Ka, lda, BM, 64);
   rc |= trans_w ? make_tmap_u8_3d(&tQ, qdata, E, Wn, Wk / 2, 64, 64) : make_tmap_u8_3d(&tQ, qdata, E, Wn, Wk / 2, 128, 32);
   if (K2 > 0) {
@@ -529,8 +564,12 @@ extern "C" int axb_grouped_gemm_w4a16(const void* A, long long lda, const void* 
     tA2 = tA;
     tB2 = tA;
   }
+  const bool tma_store = out_mode == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  tC = tA;
+  if (tma_store) rc |= axb_make_tmap_2d(&tC, C, rows, N, ldc, 32, 64);
   if (rc) return -4;
   W4Params p = {};
+  p.tma_store = tma_store;
   p.N = N; p.K = Ka; p.K2 = K2 > 0 ? K2 : 0; p.Wn = Wn; p.Wk = Wk; p.E = E;
   p.C = C; p.ldc = ldc; p.alpha = alpha; p.out_mode = out_mode;
   p.scale = reinterpret_cast<const uint8_t*>(scale); p.pts = pts;
@@ -549,7 +588,7 @@ extern "C" int axb_grouped_gemm_w4a16(const void* A, long long lda, const void* 
       if (e != cudaSuccess) return (int)e;
       set = true;
     }
-    grouped_w4a16_kernel<true><<<grid, W4_THREADS, W4_SMEM, st>>>(tA, tQ, tA2, tB2, p);
+    grouped_w4a16_kernel<true><<<grid, W4_THREADS, W4_SMEM, st>>>(tA, tQ, tA2, tB2, tC, p);
   } else {
     static bool set = false;
     if (!set) {
@@ -557,7 +596,7 @@ extern "C" int axb_grouped_gemm_w4a16(const void* A, long long lda, const void* 
       if (e != cudaSuccess) return (int)e;
       set = true;
     }
-    grouped_w4a16_kernel<false><<<grid, W4_THREADS, W4_SMEM, st>>>(tA, tQ, tA2, tB2, p);
+    grouped_w4a16_kernel<false><<<grid, W4_THREADS, W4_SMEM, st>>>(tA, tQ, tA2, tB2, tC, p);
   }
   return (int)cudaGetLastError();
 }
