@@ -34,13 +34,16 @@ constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (A), MMA, 4 e
 // The converters work in four groups of two warps, each on a k block of its own, so that four chains (packed tile seen ->
 // decode -> stores -> proxy fence -> arrival) run side by side.
 constexpr int SA = 4, SB = 4, SR = 4;  // slots: A (two 128-row tiles), decoded B, packed B
+// Every group owns one slot of the packed and one of the decoded ring (k block i of the whole sequence belongs to group, slot
+// i % 4), so that a slot's waits are made in order by the same warps: a wait for a phase whose predecessor has not completed
+// would see the parity it asks for and pass.
 constexpr int CGROUPS = 4, CG_WARPS = W4_CONV_WARPS / CGROUPS, CG_UNITS = 256 / (32 * CG_WARPS);
 constexpr int A_BYTES = BM * BK * 2;   // one 128-row A tile; a slot holds two
 constexpr int B_BYTES = BN * BK * 2;
 constexpr int RAW_BYTES = 4096;   // FWD: 128 rows x 32 bytes; DX: 64 rows x 64 bytes
 constexpr int EPI_BYTES = 4096;   // per epilogue warp: 32 rows x 64 bf16 columns on their way out
 constexpr int W4_SMEM = SA * 2 * A_BYTES + SB * B_BYTES + SR * RAW_BYTES + 4 * EPI_BYTES + 1024 + 512;
-static_assert(W4_SMEM <= 227 * 1024, "");
+static_assert(W4_SMEM <= 227 * 1024 && SB == CGROUPS && SR == CGROUPS, "");
 
 // position in a ring of N slots
 template <int N>
@@ -270,12 +273,14 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
       for (int sub = 0; sub < 2 && ok; ++sub) {
         Pass ps;
         if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
-        for (int kb = 0; kb < nk_main; ++kb, rr.next()) {
+        for (int kb = 0; kb < nk; ++kb, rr.next()) {
           if (!warp_all(mbar_wait(&r_empty[rr.slot], rr.phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
             ok = false;
             break;
           }
-          if (elect_one()) {
+          if (kb >= nk_main) {          // a LoRA block has no packed weights: its slot only keeps the order
+            if (elect_one()) mbar_arrive(&r_full[rr.slot]);
+          } else if (elect_one()) {
             mbar_expect_tx(&r_full[rr.slot], RAW_BYTES);
             if (!DX) tma_load_3d(sRaw + rr.slot * RAW_BYTES, &tmQ, &r_full[rr.slot], kb * (BK / 2), ps.n0, ps.e);   // [128 n, 32 B of k]
             else tma_load_3d(sRaw + rr.slot * RAW_BYTES, &tmQ, &r_full[rr.slot], ps.n0 / 2, kb * BK, ps.e);         // [64 n, 64 B of k]
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
     const int cw = warp - 6, grp = cw / CG_WARPS, gt = (cw % CG_WARPS) * 32 + lane;
     const long long sc_row_bytes = p.Wk / 16;
     const int part = gt & 1, half = DX ? ((gt >> 1) & 1) : 0;      // the same for all units of a thread
-    long long cb = 0, cr = 0;                                     // k blocks (of B, of packed weights) before this pass
+    long long cb = 0;                                             // k blocks before this pass
     bool ok = true;
     for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
       for (int sub = 0; sub < 2 && ok; ++sub) {
@@ -374,14 +379,13 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         load_scales(kb, cur);
         for (; kb < nk && ok; kb += CGROUPS) {
           load_scales(kb + CGROUPS, nxt);
-          const long long ib = cb + kb, ir = cr + kb;
-          const int bslot = (int)(ib % SB), rslot = (int)(ir % SR);
-          const uint32_t bphase = (uint32_t)(ib / SB) & 1, rphase = (uint32_t)(ir / SR) & 1;
+          const int bslot = grp, rslot = grp;
+          const uint32_t bphase = (uint32_t)((cb + kb) / CGROUPS) & 1;
+          if (!mbar_wait(&r_full[rslot], bphase, p.status, AXB_TIMEOUT_FULL)) {
+            ok = false;
+            break;
+          }
           if (kb < nk_main) {
-            if (!mbar_wait(&r_full[rslot], rphase, p.status, AXB_TIMEOUT_FULL)) {
-              ok = false;
-              break;
-            }
             uint4 w[CG_UNITS];
 #pragma unroll
             for (int u = 0; u < CG_UNITS; ++u)
@@ -420,6 +424,7 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
               break;
             }
             if (lane == 0) {
+              mbar_arrive(&r_empty[rslot]);
               if (cw % CG_WARPS == 0) {
                 const int ka = (kb - nk_main) * BK;
                 uint8_t* b_dst = sB + bslot * B_BYTES;
@@ -440,7 +445,6 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
           for (int u = 0; u < CG_UNITS; ++u) cur[u] = nxt[u];
         }
         cb += nk;
-        cr += nk_main;
       }
     }
   } else {
