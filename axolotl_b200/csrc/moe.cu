@@ -80,55 +80,189 @@ __global__ void nvfp4_dequant_kernel(const uint8_t* __restrict__ q, const uint8_
   }
 }
 
-// Local dispatch: out[r, :] = row_token[r] >= 0 ? scale[r] * x[row_token[r], :] : 0 for every row of
-// the padded expert-sorted layout (one warp per row; pad rows are written as zeros).
+// ---- Layout of a routed batch: the T * k slots sorted by expert, every expert's rows padded to whole 128-row blocks, slots of
+// an expert in slot order. Three launches (count, place, scatter) instead of two dozen tensor operations around a sort, whose
+// issue cost exceeded the expert GEMMs of a short batch.
+constexpr int RL_T = 1024;        // slots per block of the counting and scattering kernels
+constexpr int RL_MAX_E = 1024;
+
+__global__ void __launch_bounds__(RL_T) route_count_kernel(const long long* __restrict__ expert, int* __restrict__ hist, int n, int E) {
+  extern __shared__ int h[];      // [E]
+  for (int e = threadIdx.x; e < E; e += RL_T) h[e] = 0;
+  __syncthreads();
+  const int i = blockIdx.x * RL_T + threadIdx.x;
+  if (i < n) {
+    const long long e = expert[i];
+    if (e >= 0 && e < E) atomicAdd(&h[e], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += RL_T) hist[(long long)blockIdx.x * E + e] = h[e];
+}
+
+// hist[b][e] becomes the padded row of the first slot of expert e in block b
+__global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__ hist, int blocks, int E, int max_blocks,
+                                                               int* __restrict__ seg_start, int* __restrict__ seg_rows,
+                                                               int* __restrict__ blk_expert, int* __restrict__ n_blocks) {
+  __shared__ int warp_sum[32];
+  __shared__ int first[RL_MAX_E + 1];     // first 128-row block of every expert
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+  int count = 0;
+  if (e < E) {
+#pragma unroll 8
+    for (int b = 0; b < blocks; ++b) count += hist[(long long)b * E + e];
+  }
+  const int nb = (count + 127) / 128;
+  int incl = nb;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int v = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    warp_sum[lane] = v;
+  }
+  __syncthreads();
+  const int start = incl - nb + (warp ? warp_sum[warp - 1] : 0);
+  if (e < E) {
+    first[e] = start;
+    if (e == E - 1) {
+      first[E] = start + nb;
+      *n_blocks = start + nb;
+    }
+    seg_start[e] = start * 128;
+    seg_rows[e] = nb * 128;
+    int row = start * 128;
+    for (int b = 0; b < blocks; ++b) {
+      const int c = hist[(long long)b * E + e];
+      hist[(long long)b * E + e] = row;
+      row += c;
+    }
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < max_blocks; b += RL_MAX_E) {   // the expert whose blocks hold b; the last one beyond them
+    int lo = 0, hi = E - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (first[mid + 1] > b) hi = mid;
+      else lo = mid + 1;
+    }
+    blk_expert[b] = lo;
+  }
+}
+
+__global__ void __launch_bounds__(RL_T) route_scatter_kernel(const long long* __restrict__ expert, const int* __restrict__ base,
+                                                             int* __restrict__ slot_row, int* __restrict__ row_slot, int n, int E) {
+  extern __shared__ unsigned short c[];   // [32 warps][E]: slots of the expert in the warps before
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 32 * E; i += RL_T) c[i] = 0;
+  __syncthreads();
+  const int i = blockIdx.x * RL_T + threadIdx.x;
+  const long long e64 = i < n ? expert[i] : -1;
+  const int e = e64 >= 0 && e64 < E ? (int)e64 : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, e);
+  const int rank = __popc(same & ((1u << lane) - 1u));
+  if (e >= 0 && rank == 0) c[warp * E + e] = (unsigned short)__popc(same);
+  __syncthreads();
+  for (int q = threadIdx.x; q < E; q += RL_T) {
+    unsigned run = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) {
+      const unsigned v = c[w * E + q];
+      c[w * E + q] = (unsigned short)run;
+      run += v;
+    }
+  }
+  __syncthreads();
+  if (e >= 0) {
+    const int row = base[(long long)blockIdx.x * E + e] + c[warp * E + e] + rank;
+    slot_row[i] = row;
+    row_slot[row] = i;
+  } else if (i < n) {
+    slot_row[i] = 0;
+  }
+}
+
+// Local dispatch: out[r, :] = scale * x[token of row r, :], zeros in pad rows. The token of a row is row_token[r] (scale
+// row_scale[r]) or, with k > 0, row_token[r] / k (row_token then holds slots; scale row_scale[slot]). One warp per row; eight
+// vectors of a row are requested before the first is stored.
 __global__ void moe_dispatch_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_token,
                                          const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ out,
-                                         long long n_rows, int width) {
+                                         long long n_rows, int width, int k) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long r = w; r < n_rows; r += n_warps) {
-    const int tok = row_token[r];
+    const int id = row_token[r];
     __nv_bfloat16* d = out + r * width;
-    if (tok < 0) {
+    if (id < 0) {
       for (int c = lane * 8; c < width; c += 256) *reinterpret_cast<uint4*>(d + c) = make_uint4(0, 0, 0, 0);
       continue;
     }
-    const __nv_bfloat16* s = x + (long long)tok * width;
-    const float g = row_scale ? row_scale[r] : 1.f;
-    for (int c = lane * 8; c < width; c += 256) {
-      uint4 v = *reinterpret_cast<const uint4*>(s + c);
-      if (row_scale) {
-        uint32_t in[4] = {v.x, v.y, v.z, v.w};
+    const __nv_bfloat16* s = x + (long long)(k > 0 ? id / k : id) * width;
+    const float g = row_scale ? row_scale[k > 0 ? (long long)id : r] : 1.f;
+    for (int c0 = 0; c0 < width; c0 += 8 * 256) {
+      uint4 v[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack_bf16x2(in[e]);
-          in[e] = pack_bf16x2(f.x * g, f.y * g);
-        }
-        v = make_uint4(in[0], in[1], in[2], in[3]);
+      for (int q = 0; q < 8; ++q) {
+        const int c = c0 + q * 256 + lane * 8;
+        v[q] = c < width ? *reinterpret_cast<const uint4*>(s + c) : make_uint4(0, 0, 0, 0);
       }
-      *reinterpret_cast<uint4*>(d + c) = v;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int c = c0 + q * 256 + lane * 8;
+        if (c >= width) break;
+        if (row_scale) {
+          uint32_t in[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = unpack_bf16x2(in[e]);
+            in[e] = pack_bf16x2(f.x * g, f.y * g);
+          }
+          v[q] = make_uint4(in[0], in[1], in[2], in[3]);
+        }
+        *reinterpret_cast<uint4*>(d + c) = v[q];
+      }
     }
   }
 }
 
-// Local combine: out[t, :] = sum_j w[t, j] * ys[slot_row[t, j], :] (fp32 accumulation, no atomics).
-template <int TOPK_MAX>
+// Local combine: out[t, :] = sum_j w[t, j] * ys[slot_row[t, j], :] (fp32 accumulation in slot order, no atomics). One warp per
+// (token, 256 columns); the rows of eight slots are requested together (a warp per token with one load at a time took 30 us
+// for 333 tokens).
 __global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ slot_row,
                                         const float* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                         long long n_tokens, int k, int width) {
-  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  const int chunks = (width + 255) / 256;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long t = wid; t < n_tokens; t += n_warps) {
-    for (int c = lane * 8; c < width; c += 256) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int j = 0; j < k; ++j) {
-        const int r = slot_row[t * k + j];
-        const float g = w ? w[t * k + j] : 1.f;
-        const uint4 v = *reinterpret_cast<const uint4*>(ys + (long long)r * width + c);
-        const uint32_t in[4] = {v.x, v.y, v.z, v.w};
+  for (long long it = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_tokens * chunks; it += n_warps) {
+    const long long t = it / chunks;
+    const int c = (int)(it - t * chunks) * 256 + lane * 8;
+    const bool in_row = c < width;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int j0 = 0; j0 < k; j0 += 8) {
+      const int mine = j0 + (lane & 7);
+      const int my_row = mine < k ? slot_row[t * k + mine] : 0;
+      const float my_w = mine < k ? (w ? w[t * k + mine] : 1.f) : 0.f;
+      uint4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = __shfl_sync(0xffffffffu, my_row, j);
+        v[j] = in_row && j0 + j < k ? *reinterpret_cast<const uint4*>(ys + (long long)r * width + c) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float g = __shfl_sync(0xffffffffu, my_w, j);
+        if (j0 + j >= k) break;
+        const uint32_t in[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 f = unpack_bf16x2(in[e]);
@@ -136,14 +270,16 @@ __global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ ys, co
           acc[2 * e + 1] += g * f.y;
         }
       }
+    }
+    if (in_row)
       *reinterpret_cast<uint4*>(out + t * width + c) =
           make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
                      pack_bf16x2(acc[6], acc[7]));
-    }
   }
 }
 
-// dw[t, j] = <dy[t, :], ys[slot_row[t, j], :]>  (gradient of the routing weights; one warp per slot)
+// dw[t, j] = <dy[t, :], ys[slot_row[t, j], :]>  (gradient of the routing weights; one warp per slot, eight vectors of each row
+// in flight)
 __global__ void moe_combine_dw_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ ys,
                                       const int* __restrict__ slot_row, float* __restrict__ dw, long long n_slots,
                                       int k, int width) {
@@ -154,13 +290,25 @@ __global__ void moe_combine_dw_kernel(const __nv_bfloat16* __restrict__ dy, cons
     const __nv_bfloat16* a = dy + (sl / k) * width;
     const __nv_bfloat16* b = ys + (long long)slot_row[sl] * width;
     float acc = 0.f;
-    for (int c = lane * 8; c < width; c += 256) {
-      const uint4 va = *reinterpret_cast<const uint4*>(a + c), vb = *reinterpret_cast<const uint4*>(b + c);
-      const uint32_t ia[4] = {va.x, va.y, va.z, va.w}, ib[4] = {vb.x, vb.y, vb.z, vb.w};
+    for (int c0 = lane * 8; c0 < width; c0 += 8 * 256) {
+      uint4 va[8], vb[8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 fa = unpack_bf16x2(ia[e]), fb = unpack_bf16x2(ib[e]);
-        acc += fa.x * fb.x + fa.y * fb.y;
+      for (int q = 0; q < 8; ++q) {
+        const int c = c0 + q * 256;
+        va[q] = vb[q] = make_uint4(0, 0, 0, 0);
+        if (c < width) {
+          va[q] = *reinterpret_cast<const uint4*>(a + c);
+          vb[q] = *reinterpret_cast<const uint4*>(b + c);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t ia[4] = {va[q].x, va[q].y, va[q].z, va[q].w}, ib[4] = {vb[q].x, vb[q].y, vb[q].z, vb[q].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 fa = unpack_bf16x2(ia[e]), fb = unpack_bf16x2(ib[e]);
+          acc += fa.x * fb.x + fa.y * fb.y;
+        }
       }
     }
 #pragma unroll
@@ -397,13 +545,36 @@ static int rows_grid(long long n_rows) {
   return (int)(want > 148 * 8 ? 148 * 8 : (want < 1 ? 1 : want));
 }
 
-// out [n_rows, width] bf16; row_token int32 [n_rows] (-1 = zero row); row_scale fp32 [n_rows] or NULL
+// Layout of a routed batch. expert [n] (n = T * k slots, expert ids), E <= 1024; slot_row [n], row_slot [max_blocks * 128] (slot of
+// a padded row, -1 = pad), seg_start / seg_rows [E], blk_expert [max_blocks], n_blocks [1]; scratch: ceil(n / 1024) * E ints.
+// max_blocks >= ceil(n / 128) + E.
+extern "C" int axb_moe_route_layout(const long long* expert, int n, int E, int max_blocks, int* slot_row, int* row_slot,
+                                    int* seg_start, int* seg_rows, int* blk_expert, int* n_blocks, int* scratch, void* stream) {
+  if (E < 1 || E > RL_MAX_E || n < 0 || max_blocks < (n + 127) / 128 + E) return -2;
+  cudaError_t e = cudaMemsetAsync(row_slot, 0xff, (size_t)max_blocks * 128 * sizeof(int), ST(stream));
+  if (e != cudaSuccess) return (int)e;
+  const int blocks = (n + RL_T - 1) / RL_T;
+  if (blocks > 0) route_count_kernel<<<blocks, RL_T, E * (int)sizeof(int), ST(stream)>>>(expert, scratch, n, E);
+  route_place_kernel<<<1, RL_MAX_E, 0, ST(stream)>>>(scratch, blocks, E, max_blocks, seg_start, seg_rows, blk_expert, n_blocks);
+  if (blocks > 0) {
+    const int smem = 32 * E * (int)sizeof(unsigned short);      // at most 64 KB
+    if (smem > 48 * 1024) {
+      static std::atomic<unsigned long long> allowed{0};
+      if (const int rc = axb_allow_smem((const void*)route_scatter_kernel, 64 * 1024, allowed)) return rc;
+    }
+    route_scatter_kernel<<<blocks, RL_T, smem, ST(stream)>>>(expert, scratch, slot_row, row_slot, n, E);
+  }
+  return (int)cudaGetLastError();
+}
+
+// out [n_rows, width] bf16. k == 0: row_token int32 [n_rows] (-1 = zero row), row_scale fp32 [n_rows] or NULL; k > 0: row_token
+// holds slots (token = slot / k) and row_scale is indexed by the slot
 extern "C" int axb_moe_dispatch_rows(const void* x, const int* row_token, const float* row_scale, void* out,
-                                     long long n_rows, int width, void* stream) {
+                                     long long n_rows, int width, int k, void* stream) {
   if (width % 8) return -2;
   if (n_rows <= 0) return 0;
   moe_dispatch_rows_kernel<<<rows_grid(n_rows), 256, 0, ST(stream)>>>(
-      (const __nv_bfloat16*)x, row_token, row_scale, (__nv_bfloat16*)out, n_rows, width);
+      (const __nv_bfloat16*)x, row_token, row_scale, (__nv_bfloat16*)out, n_rows, width, k);
   return (int)cudaGetLastError();
 }
 
@@ -412,7 +583,7 @@ extern "C" int axb_moe_combine_rows(const void* ys, const int* slot_row, const f
                                     long long n_tokens, int k, int width, void* stream) {
   if (width % 8) return -2;
   if (n_tokens <= 0) return 0;
-  moe_combine_rows_kernel<16><<<rows_grid(n_tokens), 256, 0, ST(stream)>>>(
+  moe_combine_rows_kernel<<<rows_grid(n_tokens * ((width + 255) / 256)), 256, 0, ST(stream)>>>(
       (const __nv_bfloat16*)ys, slot_row, w, (__nv_bfloat16*)out, n_tokens, k, width);
   return (int)cudaGetLastError();
 }

@@ -33,7 +33,9 @@ _CUDA_SIGS = {
     "axb_gemm_set_backoff": [i32, i32],
     "axb_gemm_set_pair_tuning": [i32, i32, i32],
     "axb_nvfp4_dequant": [vp, vp, vp, vp, i64, i64, vp],
-    "axb_moe_dispatch_rows": [vp, vp, vp, vp, i64, i32, vp],
+    "axb_moe_dispatch_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
+    # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, scratch, stream
+    "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp],
     "axb_moe_combine_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_moe_combine_dw": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_nf4_dequant": [vp, vp, vp, i64, i32, vp],

@@ -279,29 +279,46 @@ class _GroupedProj(torch.autograd.Function):
 
 
 class RoutedLayout(GroupLayout):
-    """Layout of a local (single-rank) MoE layer built from the router's top-k choice ``idx`` [T, k]:
-    adds the slot <-> padded-row maps used by the dispatch / combine kernels."""
+    """Layout of a local (single-rank) MoE layer built from the router's top-k choice ``idx`` [T, k] (int64):
+    adds the slot <-> padded-row maps used by the dispatch / combine kernels (``row_slot``: slot of a padded row, -1 in
+    pad rows; ``slot_row``: its inverse). Built by three kernels of csrc/moe.cu, without a host round trip."""
 
     def __init__(self, idx: torch.Tensor, E: int):
         T, k = idx.shape
-        flat_e = idx.reshape(-1)
-        order = torch.argsort(flat_e, stable=True)
-        # torch.bincount synchronises with the host (it sizes its output from the data): count with a
-        # scatter-add instead so the layer stays free of host round trips
-        counts = torch.zeros(E, dtype=torch.int64, device=idx.device).scatter_add_(0, flat_e, torch.ones_like(flat_e))
-        super().__init__(counts, T * k)
+        n = T * k
+        flat_e = idx.reshape(-1).to(torch.int64).contiguous()
         self.k = k
-        self.slot_row = torch.empty(T * k, dtype=torch.int32, device=idx.device)
-        self.slot_row[order] = self.dest.to(torch.int32)
-        self.row_token = torch.full((self.max_rows,), -1, dtype=torch.int32, device=idx.device)
-        self.row_token[self.dest] = (order // k).to(torch.int32)
+        if E > 1024:               # more experts than the placing kernel has threads
+            order = torch.argsort(flat_e, stable=True)
+            super().__init__(torch.zeros(E, dtype=torch.int64, device=idx.device).scatter_add_(0, flat_e, torch.ones_like(flat_e)), n)
+            self.slot_row = torch.empty(n, dtype=torch.int32, device=idx.device)
+            self.slot_row[order] = self.dest.to(torch.int32)
+            self.row_slot = torch.full((self.max_rows,), -1, dtype=torch.int32, device=idx.device)
+            self.row_slot[self.dest] = order.to(torch.int32)
+            return
+        self.E, self.n_rows = E, n
+        self.max_blocks = (n + BLOCK - 1) // BLOCK + E
+        self.max_rows = self.max_blocks * BLOCK
+        chunks = (n + 1023) // 1024
+        sizes = [n, self.max_rows, E, E, self.max_blocks, 1, chunks * E]
+        at = [0]
+        for s in sizes:
+            at.append(at[-1] + (s + 3) // 4 * 4)
+        buf = torch.empty(at[-1], dtype=torch.int32, device=idx.device)
+        (self.slot_row, self.row_slot, self.seg_start, self.seg_rows, self.blk_expert, self.n_blocks,
+         scratch) = (buf[a:a + s] for a, s in zip(at, sizes))
+        _lib.check_rc(_lib.cuda_lib().axb_moe_route_layout(
+            flat_e.data_ptr(), n, E, self.max_blocks, self.slot_row.data_ptr(), self.row_slot.data_ptr(), self.seg_start.data_ptr(),
+            self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), scratch.data_ptr(), _lib.stream_ptr()),
+            "moe_route_layout")
 
 
-def _dispatch_rows(x, row_token, row_scale, n_rows):
-    out = torch.empty((n_rows, x.shape[1]), dtype=x.dtype, device=x.device)
+def _dispatch_rows(x, lay, slot_scale):
+    """Rows of ``x`` [T, H] in the padded layout, each times its slot's entry of ``slot_scale`` [T, k] (fp32, optional)."""
+    out = torch.empty((lay.max_rows, x.shape[1]), dtype=x.dtype, device=x.device)
     _lib.check_rc(_lib.cuda_lib().axb_moe_dispatch_rows(
-        x.data_ptr(), row_token.data_ptr(), row_scale.data_ptr() if row_scale is not None else None, out.data_ptr(),
-        n_rows, x.shape[1], _lib.stream_ptr()), "moe_dispatch_rows")
+        x.data_ptr(), lay.row_slot.data_ptr(), slot_scale.data_ptr() if slot_scale is not None else None, out.data_ptr(),
+        lay.max_rows, x.shape[1], lay.k, _lib.stream_ptr()), "moe_dispatch_rows")
     return out
 
 
@@ -319,7 +336,7 @@ class _LocalDispatch(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, lay):
         ctx.lay, ctx.T = lay, x.shape[0]
-        return _dispatch_rows(x.contiguous(), lay.row_token, None, lay.max_rows)
+        return _dispatch_rows(x.contiguous(), lay, None)
 
     @staticmethod
     def backward(ctx, dxp):
@@ -343,9 +360,7 @@ class _LocalCombine(torch.autograd.Function):
         ys, wf = ctx.saved_tensors
         lay = ctx.lay
         dy = dy.contiguous()
-        row_scale = torch.zeros(lay.max_rows, dtype=torch.float32, device=dy.device)
-        row_scale[lay.slot_row.long()] = wf.reshape(-1)
-        dys = _dispatch_rows(dy, lay.row_token, row_scale, lay.max_rows)
+        dys = _dispatch_rows(dy, lay, wf)
         dw = None
         if ctx.needs_input_grad[1]:
             dw = torch.empty(wf.shape, dtype=torch.float32, device=dy.device)

@@ -1,0 +1,67 @@
+"""Layout of a routed batch, dispatch and combine kernels against plain PyTorch."""
+import pytest
+import torch
+
+from axolotl_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (3, 2, 8), (333, 8, 128), (128, 8, 8), (1025, 1, 5), (700, 6, 160), (200, 4, 1024), (40, 2, 1500)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_routed_layout(T, k, E, skew):
+    """Slot counts at the edges of the 1024-slot blocks and of warps, experts without slots, one expert with all of them,
+    expert counts at and above the placing kernel's threads: the layout of a stable sort, exactly."""
+    from axolotl_b200.ops.grouped import BLOCK, RoutedLayout
+
+    torch.manual_seed(T + E)
+    idx = torch.stack([torch.randperm(E)[:k] if E >= k else torch.zeros(k, dtype=torch.long) for _ in range(T)])
+    if skew:
+        idx = (idx * 0 + E - 1) if E < 8 else idx % max(1, E // 4)
+    lay = RoutedLayout(idx.cuda(), E)
+    flat = idx.reshape(-1)
+    counts = torch.bincount(flat, minlength=E)
+    padded = (counts + BLOCK - 1) // BLOCK * BLOCK
+    start = padded.cumsum(0) - padded
+    order = torch.argsort(flat, stable=True)
+    dest = torch.cat([torch.arange(int(c)) + int(s) for c, s in zip(counts, start)])
+    slot_row = torch.empty(T * k, dtype=torch.long)
+    slot_row[order] = dest
+    row_slot = torch.full((lay.max_rows,), -1, dtype=torch.long)
+    row_slot[dest] = order
+    nb = int(padded.sum()) // BLOCK
+    assert int(lay.n_blocks) == nb and lay.max_rows >= nb * BLOCK
+    assert torch.equal(lay.slot_row.long().cpu(), slot_row) and torch.equal(lay.row_slot.long().cpu(), row_slot)
+    assert torch.equal(lay.seg_rows.long().cpu(), padded) and torch.equal(lay.seg_start.long().cpu(), start)
+    blk = torch.searchsorted(padded.cumsum(0), torch.arange(lay.max_blocks) * BLOCK, right=True).clamp(max=E - 1)
+    assert torch.equal(lay.blk_expert.long().cpu(), blk)
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 3, 256), (37, 8, 2048), (19, 9, 2056), (3, 16, 264)])
+def test_dispatch_and_combine_rows(T, k, H):
+    """Widths around the 256-column chunks and eight vectors in flight, more than eight slots per token. One bf16 rounding of
+    an fp32 sum (2^-8); the weight gradient is an fp32 dot product (2^-18 of its magnitude)."""
+    from axolotl_b200.ops.grouped import RoutedLayout, _combine_rows, _dispatch_rows
+
+    torch.manual_seed(T + H)
+    E = 16
+    idx = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).cuda()
+    lay = RoutedLayout(idx, E)
+    x, w = torch.randn(T, H, device="cuda").bfloat16(), torch.rand(T, k, device="cuda")
+    rows = lay.row_slot.long()
+    live = rows >= 0
+    for scale in (None, w):
+        out = _dispatch_rows(x, lay, scale)
+        ref = x[rows.clamp(min=0) // k].float() * (scale.reshape(-1)[rows.clamp(min=0)][:, None] if scale is not None else 1.0)
+        assert torch.equal(out, torch.where(live[:, None], ref.bfloat16(), torch.zeros_like(out)))
+    ys = torch.randn(lay.max_rows, H, device="cuda").bfloat16()
+    for scale in (None, w):
+        out = _combine_rows(ys, lay.slot_row, scale, T, k)
+        ref = (ys[lay.slot_row.long()].view(T, k, H).double() * (scale.double()[..., None] if scale is not None else 1.0)).sum(1)
+        assert ((out.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()
+    dw = torch.empty(T, k, device="cuda")
+    dy = torch.randn(T, H, device="cuda").bfloat16()
+    _lib.check_rc(_lib.cuda_lib().axb_moe_combine_dw(dy.data_ptr(), ys.data_ptr(), lay.slot_row.data_ptr(), dw.data_ptr(), T * k, k, H,
+                                                     _lib.stream_ptr()), "moe_combine_dw")
+    prod = dy.double()[:, None] * ys[lay.slot_row.long()].view(T, k, H).double()
+    assert ((dw.double() - prod.sum(-1)).abs() <= 2 ** -18 * prod.abs().sum(-1)).all()
