@@ -375,12 +375,16 @@ __global__ void rope_qk_kernel(__nv_bfloat16* __restrict__ qkv, const int* __res
   }
 }
 
-// Fast path without q/k norm: one warp per token. Each lane computes the sine / cosine of its two
-// angles ONCE and reuses them for every q and k head of the token (the angles depend on the position
+// Fast path without q/k norm: one warp per (token, group of heads). Each lane computes the sine / cosine of its two
+// angles ONCE and reuses them for the group's heads (the angles depend on the position
 // only), and moves bf16 pairs (4-byte accesses, 128 B per warp instruction). sign = -1 is the
 // inverse rotation, i.e. the backward pass.
+// Bound: latency for short batches, HBM for long ones. Four heads are loaded before the first is stored (in place, the
+// compiler cannot move a load above an earlier store), and heads are spread over blockIdx.y while there are few tokens:
+// 960 rows of 40 heads 15.6 -> 5.7 us, 8192 rows 38 -> 32 us (one warp walking all heads of a row, one head at a time, before).
 // `rot` <= D: only the first `rot` dimensions of a head rotate (partial rotary embeddings: pairs (j, j + rot / 2));
 // the rest of the head passes through untouched.
+constexpr int ROPE_H = 4;
 __global__ void rope_fast_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos,
                                  const float* __restrict__ inv_freq, int T, int nh, int D,
                                  long long row_stride, float sign, float attn_scale, int rot) {
@@ -391,6 +395,7 @@ __global__ void rope_fast_kernel(__nv_bfloat16* __restrict__ qkv, const int* __r
   const int half = rot >> 1;
   const float ps = (float)pos[t];
   __nv_bfloat16* row = qkv + t * row_stride;
+  const int groups = (nh + ROPE_H - 1) / ROPE_H;
   for (int j = 2 * lane; j < half; j += 64) {
     float s0, c0, s1, c1;
     sincosf(ps * inv_freq[j], &s0, &c0);
@@ -399,15 +404,31 @@ __global__ void rope_fast_kernel(__nv_bfloat16* __restrict__ qkv, const int* __r
     s1 *= sign * attn_scale;
     c0 *= attn_scale;
     c1 *= attn_scale;
-#pragma unroll 4
-    for (int hd = 0; hd < nh; ++hd) {
-      uint32_t* pa = reinterpret_cast<uint32_t*>(row + (long long)hd * D + j);
-      uint32_t* pb = reinterpret_cast<uint32_t*>(row + (long long)hd * D + half + j);
-      const float2 a = unpack_bf16x2(*pa), b = unpack_bf16x2(*pb);
-      *pa = pack_bf16x2(a.x * c0 - b.x * s0, a.y * c1 - b.y * s1);
-      *pb = pack_bf16x2(b.x * c0 + a.x * s0, b.y * c1 + a.y * s1);
+    for (int g = blockIdx.y; g < groups; g += gridDim.y) {
+      uint32_t* p0 = reinterpret_cast<uint32_t*>(row + (long long)g * ROPE_H * D + j);
+      uint32_t ua[ROPE_H], ub[ROPE_H];
+#pragma unroll
+      for (int h = 0; h < ROPE_H; ++h) {
+        if (g * ROPE_H + h >= nh) break;
+        ua[h] = p0[(h * D) >> 1];
+        ub[h] = p0[(h * D + half) >> 1];
+      }
+#pragma unroll
+      for (int h = 0; h < ROPE_H; ++h) {
+        if (g * ROPE_H + h >= nh) break;
+        const float2 a = unpack_bf16x2(ua[h]), b = unpack_bf16x2(ub[h]);
+        p0[(h * D) >> 1] = pack_bf16x2(a.x * c0 - b.x * s0, a.y * c1 - b.y * s1);
+        p0[(h * D + half) >> 1] = pack_bf16x2(b.x * c0 + a.x * s0, b.y * c1 + a.y * s1);
+      }
     }
   }
+}
+// eight blocks per SM, but never more head groups than there are
+static dim3 rope_grid(int T, int nh) {
+  const int bx = (T + 7) / 8, groups = (nh + ROPE_H - 1) / ROPE_H;
+  int by = (148 * 8 + bx - 1) / bx;
+  if (by > groups) by = groups;
+  return dim3((unsigned)bx, (unsigned)(by < 1 ? 1 : by));
 }
 
 // Backward of (per-head RMSNorm ->) RoPE for the fused q/k gradient buffer, in place.
@@ -966,7 +987,7 @@ extern "C" int axb_rope_qk(void* qkv, const int* pos, const float* inv_freq, int
                            void* stream) {
   if (T <= 0) return 0;
   if (!qn_w && !kn_w && (D % 4) == 0 && (row_stride % 2) == 0) {
-    rope_fast_kernel<<<(unsigned)((T + 7) / 8), 256, 0, ST(stream)>>>((__nv_bfloat16*)qkv, pos, inv_freq, T, Hq + Hk, D,
+    rope_fast_kernel<<<rope_grid(T, Hq + Hk), 256, 0, ST(stream)>>>((__nv_bfloat16*)qkv, pos, inv_freq, T, Hq + Hk, D,
                                                                      row_stride, sign, attn_scale, D);
     return (int)cudaGetLastError();
   }
@@ -983,7 +1004,7 @@ extern "C" int axb_rope_partial(void* qkv, const int* pos, const float* inv_freq
                                 long long row_stride, float sign, float attn_scale, void* stream) {
   if (T <= 0) return 0;
   if (rot <= 0 || rot > D || (rot & 3) || (row_stride & 1) || (D & 1)) return -2;
-  rope_fast_kernel<<<(unsigned)((T + 7) / 8), 256, 0, ST(stream)>>>((__nv_bfloat16*)qkv, pos, inv_freq, T, n_heads, D,
+  rope_fast_kernel<<<rope_grid(T, n_heads), 256, 0, ST(stream)>>>((__nv_bfloat16*)qkv, pos, inv_freq, T, n_heads, D,
                                                                    row_stride, sign, attn_scale, rot);
   return (int)cudaGetLastError();
 }
@@ -995,7 +1016,7 @@ extern "C" int axb_rope_qk_bwd(void* dqkv, const void* x_pre, const int* pos,
   if (T <= 0) return 0;
   if (D > 512) return -2;
   if (!qn_w && !kn_w && (D % 4) == 0 && (row_stride % 2) == 0) {
-    rope_fast_kernel<<<(unsigned)((T + 7) / 8), 256, 0, ST(stream)>>>((__nv_bfloat16*)dqkv, pos, inv_freq, T, Hq + Hk, D,
+    rope_fast_kernel<<<rope_grid(T, Hq + Hk), 256, 0, ST(stream)>>>((__nv_bfloat16*)dqkv, pos, inv_freq, T, Hq + Hk, D,
                                                                      row_stride, -1.f, attn_scale, D);
     return (int)cudaGetLastError();
   }

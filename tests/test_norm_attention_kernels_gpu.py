@@ -69,3 +69,24 @@ def test_attention_head_and_token_remainders(D, Hq, Hk, lens, window, causal):
         assert ((a - b).abs() <= 2 ** -6 * b.abs().max()).all()
         assert ((a - b).norm() / b.norm()).item() < 2 ** -7
     _lib.check_status()
+
+
+@pytest.mark.parametrize("T,nh,D,rot", [(1, 1, 64, 64), (3, 5, 128, 128), (9, 40, 128, 128), (700, 36, 64, 64), (2500, 10, 256, 128)])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_rope_head_groups(T, nh, D, rot, sign):
+    """Head counts around the groups of four, few and many tokens (heads over blockIdx.y or not), partial rotation, a row
+    stride of its own; the columns behind the heads stay untouched. One bf16 rounding of an fp32 rotation; the angle's own
+    rounding (2^-24 of up to T radians) is far below it."""
+    torch.manual_seed(T + nh)
+    buf = torch.randn(T, nh * D + 24, device="cuda").bfloat16()
+    want = buf.clone()
+    pos = torch.randint(0, max(2, T), (T,), dtype=torch.int32, device="cuda")
+    inv = 1.0 / (10000.0 ** (torch.arange(0, rot, 2, device="cuda").float() / rot))
+    _lib.check_rc(_lib.cuda_lib().axb_rope_partial(buf.data_ptr(), pos.data_ptr(), inv.data_ptr(), T, nh, D, rot, buf.stride(0), sign, 1.0,
+                                                   _lib.stream_ptr()), "rope_partial")
+    x = want[:, :nh * D].reshape(T, nh, D).double()
+    ang = (pos.float()[:, None, None] * inv).double()
+    a, b = x[..., :rot // 2], x[..., rot // 2:rot]
+    r = torch.cat([a * ang.cos() - sign * b * ang.sin(), b * ang.cos() + sign * a * ang.sin(), x[..., rot:]], -1).reshape(T, -1)
+    assert ((buf[:, :nh * D].double() - r).abs() <= 2 ** -8 * r.abs() + 2 ** -12).all()
+    assert torch.equal(buf[:, nh * D:], want[:, nh * D:])
