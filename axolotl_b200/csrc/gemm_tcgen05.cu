@@ -46,7 +46,7 @@ struct GemmParams {
   const void* Cin;
   long long ldc, ldcin;
   float alpha, beta;
-  int out_mode;  // 0: bf16 store, 1: fp32 store, 2: fp32 atomic add (split-K)
+  int out_mode;  // 0: bf16 store, 1: fp32 store, 2: fp32 atomic add (split-K), 6: the same into C^T (C[n * ldc + m])
   int splits;
   int group_m;  // m tiles per rasterisation band (the A rows of a band stay L2 resident)
   int* status;
@@ -586,6 +586,9 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
             }
           }
+        } else if (p.out_mode == 6) {     // a warp's 32 rows are consecutive in memory: whole lines per instruction
+          float* ccol = reinterpret_cast<float*>(p.C) + (long long)col0 * p.ldc + row;
+          for (int j = 0; j < 32 && col0 + j < p.N; ++j) atomicAdd(ccol + (long long)j * p.ldc, v[j]);
         } else {
           float* crow = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
           for (int j = 0; j < 32 && col0 + j < p.N; ++j) atomicAdd(crow + j, v[j]);
@@ -687,7 +690,7 @@ int gemm_entry(const void* A, long long lda, int a_mn, const void* B, long long 
   if (M <= 0 || N <= 0 || (K <= 0 && K2 <= 0)) return 0;
   if ((lda & 7) || (ldb & 7) || (K2 > 0 && ((lda2 & 7) || (ldb2 & 7)))) return -2;
   if (splits < 1) splits = 1;
-  if (splits > 1 && out_mode != 2) return -3;
+  if (splits > 1 && out_mode != 2 && out_mode != 6) return -3;
   CUtensorMap tA, tB, tA2, tB2;
   int rc = 0;
   // K-major operand [R, K]: box [BM|BN rows, 64 cols]; MN-major operand [K, R]: box [64, 64].
@@ -749,7 +752,8 @@ __global__ void __launch_bounds__(kThreads, 1) gather_only_kernel(const GemmPara
 //   a_mn = 0: A is [M,K] row-major (lda);  a_mn = 1: A is stored transposed, [K,M] row-major.
 //   b_mn = 0: B is [N,K] row-major (ldb);  b_mn = 1: B is stored transposed, [K,N] row-major.
 //   A2/B2 (optional, K2 > 0) use the same storage convention as A/B.
-//   out_mode 0: bf16 C, 1: fp32 C, 2: fp32 atomic accumulate into C (required when splits > 1).
+//   out_mode 0: bf16 C, 1: fp32 C, 2: fp32 atomic accumulate into C (2 or 6 when splits > 1), 6: the same into C [N, M] = the
+//   transposed result.
 //   bn: tile width 64 / 128 / 256. Leading dimensions must be multiples of 8 elements.
 // Returns 0 or a CUDA / driver error code; asynchronous device-side wait timeouts land in *status.
 extern "C" int axb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb,

@@ -240,3 +240,21 @@ def test_gemm_tiles_chosen_below_512_rows(M, N, ta, tb, c_in):
         o16 = gemm(aa, bb, trans_a=ta, trans_b=tb)
         assert ((o16.double() - ref).abs() <= 2 ** -20 * mag + 2 ** -8 * ref.abs()).all()
     _lib.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 512, 256), (16, 4096, 8192), (48, 1000, 960), (64, 14336, 328), (40, 777 * 8, 1000)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_gemm_accumulates_the_transposed_tile(M, N, K, splits):
+    """t^T x into a strided fp32 buffer with a short first side. Atomic fp32 sums in any order: 2^-20 of their magnitude."""
+    from axolotl_b200.ops import _lib
+    from axolotl_b200.ops.gemm import gemm
+
+    torch.manual_seed(M + N)
+    t, x = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    buf = torch.randn(M, N + 4, device="cuda")
+    c0 = buf.clone()
+    gemm(t, x, trans_a=True, trans_b=True, out=buf[:, :N], accumulate=True, splits=splits, alpha=0.5)
+    _lib.check_status()
+    ref = c0[:, :N].double() + 0.5 * (t.double().t() @ x.double())
+    mag = c0[:, :N].double().abs() + 0.5 * (t.double().abs().t() @ x.double().abs())
+    assert ((buf[:, :N].double() - ref).abs() <= 2 ** -20 * mag).all() and torch.equal(buf[:, N:], c0[:, N:])
