@@ -11,6 +11,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ..ops import _lib
 from ..ops import functional as Fn
 
 
@@ -38,8 +39,17 @@ class KVCache:
                 return Fn.decode_attention(qkv, self.k[layer], self.v[layer], meta.lens_after, Hq, Hk, D, scale, window)
             return Fn.decode_attention(qkv, self.k[layer, meta.seq], self.v[layer, meta.seq], meta.lens_after,
                                        Hq, Hk, D, scale, window)
-        self.k[layer, meta.seq, meta.pos] = kq         # prefill: packed prompt rows -> (sequence, position)
-        self.v[layer, meta.seq, meta.pos] = vq
+        # prefill: packed prompt rows -> (sequence, position)
+        if (qkv.is_cuda and qkv.dtype == self.k.dtype == torch.bfloat16 and self.width % 8 == 0 and qkv.stride(1) == 1
+                and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and meta.seq.dtype == meta.pos.dtype == torch.int64
+                and meta.seq.is_contiguous() and meta.pos.is_contiguous() and meta.seq.shape == meta.pos.shape == qkv.shape[:1]
+                and not (torch.is_grad_enabled() and qkv.requires_grad)):
+            _lib.check_rc(_lib.cuda_lib().axb_kv_append(
+                qkv.data_ptr(), qkv.stride(0), Hq * D, (Hq + Hk) * D, self.k[layer].data_ptr(), self.v[layer].data_ptr(),
+                meta.seq.data_ptr(), meta.pos.data_ptr(), qkv.shape[0], self.width, self.B, self.max_len, _lib.stream_ptr()), "kv_append")
+        else:
+            self.k[layer, meta.seq, meta.pos] = kq
+            self.v[layer, meta.seq, meta.pos] = vq
         return Fn.flash_varlen(qkv, meta.attn.windowed(window) if window else meta.attn, Hq, Hk, D, scale)
 
 

@@ -258,3 +258,19 @@ def test_gemm_accumulates_the_transposed_tile(M, N, K, splits):
     ref = c0[:, :N].double() + 0.5 * (t.double().t() @ x.double())
     mag = c0[:, :N].double().abs() + 0.5 * (t.double().abs().t() @ x.double().abs())
     assert ((buf[:, :N].double() - ref).abs() <= 2 ** -20 * mag).all() and torch.equal(buf[:, N:], c0[:, N:])
+
+
+@pytest.mark.parametrize("width", [8, 256, 264, 1024])
+def test_prompt_rows_go_to_their_cache_slots(width):
+    from axolotl_b200.ops import _lib
+
+    T, B, cap = 37, 5, 20
+    qkv = torch.randn(T, 3 * width + 8, device="cuda").bfloat16()
+    slots = torch.randperm(B * cap, device="cuda")[:T]
+    seq, pos = slots // cap, slots % cap
+    kc, vc = torch.randn(2, B, cap, width, device="cuda").bfloat16()
+    k0, v0 = kc.clone(), vc.clone()
+    _lib.check_rc(_lib.cuda_lib().axb_kv_append(qkv.data_ptr(), qkv.stride(0), width, 2 * width, kc.data_ptr(), vc.data_ptr(), seq.data_ptr(),
+                                                pos.data_ptr(), T, width, B, cap, _lib.stream_ptr()), "kv_append")
+    k0[seq, pos], v0[seq, pos] = qkv[:, width:2 * width], qkv[:, 2 * width:3 * width]
+    assert torch.equal(kc, k0) and torch.equal(vc, v0)
