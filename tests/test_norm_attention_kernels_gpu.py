@@ -90,3 +90,38 @@ def test_rope_head_groups(T, nh, D, rot, sign):
     r = torch.cat([a * ang.cos() - sign * b * ang.sin(), b * ang.cos() + sign * a * ang.sin(), x[..., rot:]], -1).reshape(T, -1)
     assert ((buf[:, :nh * D].double() - r).abs() <= 2 ** -8 * r.abs() + 2 ** -12).all()
     assert torch.equal(buf[:, nh * D:], want[:, nh * D:])
+
+
+@pytest.mark.parametrize("V", [5, 264, 8192 + 3, 40960, 40968, 65536 + 7, 128256])
+@pytest.mark.parametrize("cap", [0.0, 5.0])
+def test_ce_row_edges(V, cap):
+    """Both block sizes, tails behind the last vector and partly filled groups of vectors, rows with -inf (masked) logits, an
+    ignored row, the label at either end. The gradient is one bf16 rounding of an fp32 softmax whose exponent (up to ~20, exp
+    within 2^-21) and sum carry below 2^-12."""
+    torch.manual_seed(V)
+    R, ld = 6, (V + 7) // 8 * 8 + 8
+    z = torch.randn(R, ld, device="cuda").mul_(4).bfloat16()
+    z[0, : V // 2] = float("-inf") if not cap else -1e4
+    z[1, 1:V] = float("-inf") if not cap else -1e4      # one finite logit
+    lab = torch.tensor([V - 1, 0, -100, V // 2, V - 1, 0], device="cuda")
+    want = z.clone()
+    loss, lse = torch.empty(2, R, device="cuda")
+    args = (z.data_ptr(), lab.data_ptr(), loss.data_ptr(), lse.data_ptr(), R, V, ld, 0.5, -100, 1)
+    lib = _lib.cuda_lib()
+    _lib.check_rc(lib.axb_ce_fwd_bwd_softcap(*args, cap, _lib.stream_ptr()) if cap else lib.axb_ce_fwd_bwd(*args, _lib.stream_ptr()), "ce")
+    x = want[:, :V].double()
+    t = torch.tanh(x / cap) if cap else x
+    e = cap * t if cap else x
+    ref_lse = torch.logsumexp(e, -1)
+    g = torch.exp(e - ref_lse[:, None])
+    keep = lab != -100
+    idx = lab.clamp_min(0)
+    g[torch.arange(R), idx] -= 1.0
+    if cap:
+        g = g * (1 - t * t)
+    g = torch.where(keep[:, None], 0.5 * g, torch.zeros_like(g))
+    assert ((lse - ref_lse).abs() <= 2 ** -19 * (1 + ref_lse.abs())).all()
+    ref_loss = torch.where(keep, ref_lse - e[torch.arange(R), idx], torch.zeros_like(ref_lse))
+    assert ((loss - ref_loss).abs() <= 2 ** -18 * (1 + ref_lse.abs())).all()
+    assert ((z[:, :V].double() - g).abs() <= (2 ** -8 + 2 ** -12) * g.abs() + 2 ** -20).all()
+    assert torch.equal(z[:, V:], want[:, V:])
