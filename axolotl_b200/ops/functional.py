@@ -378,10 +378,22 @@ def token_entropy(logits, temperature=1.0, return_lse=False):
 
 
 # --------------------------------------------------------------------------------------- embedding
+def _flat_grad(p):
+    """The optimizer's fp32 gradient buffer of a bf16 CUDA parameter that the kernels may add into, else None."""
+    g = getattr(p, "_axb_grad", None)
+    ok = (g is not None and p.is_cuda and p.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.device == p.device
+          and g.shape == p.shape and g.is_contiguous())
+    return g if ok else None
+
+
 class _Embedding(torch.autograd.Function):
+    """The table's gradient is added to the optimizer's fp32 buffer where the table has one: no dense gradient of its own, which
+    would be filled, rounded to bf16, widened and added (five passes over the table for a few thousand rows)."""
+
     @staticmethod
     def forward(ctx, table, ids):
         ctx.save_for_backward(ids)
+        ctx.table = table if isinstance(table, torch.nn.Parameter) else None
         ctx.tshape = table.shape
         ctx.tdtype = table.dtype
         if not table.is_cuda:
@@ -405,12 +417,13 @@ class _Embedding(torch.autograd.Function):
             g.index_add_(0, ids.reshape(-1), dout.reshape(-1, H).float())
             return g.to(ctx.tdtype), None
         lib = _lib.cuda_lib()
-        g = torch.zeros(V, H, dtype=torch.float32, device=dout.device)
+        tgt = _flat_grad(ctx.table)
+        g = tgt if tgt is not None else torch.zeros(V, H, dtype=torch.float32, device=dout.device)
         d2 = dout.reshape(-1, H).contiguous()
         flat = ids.reshape(-1).contiguous()
         _lib.check_rc(lib.axb_embedding_bwd(d2.data_ptr(), flat.data_ptr(), g.data_ptr(),
                                             flat.numel(), H, V, _lib.stream_ptr()), "embedding_bwd")
-        return g.to(ctx.tdtype), None
+        return (None if tgt is not None else g.to(ctx.tdtype)), None
 
 
 def embedding(table, ids):
@@ -790,7 +803,7 @@ class _LinearCE(torch.autograd.Function):
         V = w.shape[0]
         need_dw = w.requires_grad
         dh = torch.empty_like(h)
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device) if need_dw else None
+        dw = None
         losses = torch.empty(T, dtype=torch.float32, device=h.device)
         lib = _lib.cuda_lib() if h.is_cuda else None
         for r0 in range(0, T, chunk_rows):
@@ -829,16 +842,30 @@ class _LinearCE(torch.autograd.Function):
             gemm(dlogits, w, trans_b=True, out=dh[r0:r1])
             if need_dw:
                 sp = pick_splits(((V + 127) // 128) * ((H + 255) // 256), (r1 - r0 + 63) // 64)
-                gemm(dlogits, hc, trans_a=True, trans_b=True, out=dw, accumulate=True, splits=sp)
+                if dw is None and h.is_cuda and sp <= 1:     # the first chunk writes, the others add
+                    dw = torch.empty(w.shape, dtype=torch.float32, device=w.device)
+                    gemm(dlogits, hc, trans_a=True, trans_b=True, out=dw, out_dtype=torch.float32)
+                else:
+                    if dw is None:
+                        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+                    gemm(dlogits, hc, trans_a=True, trans_b=True, out=dw, accumulate=True, splits=sp)
+        if need_dw and dw is None:
+            dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
         ctx.save_for_backward(dh, dw)
         ctx.w_dtype = w.dtype
+        ctx.w = w if isinstance(w, torch.nn.Parameter) else None
         return losses.sum() / denom
 
     @staticmethod
     def backward(ctx, gout):
         dh, dw = ctx.saved_tensors
-        return (dh * gout.to(dh.dtype), (dw * gout).to(ctx.w_dtype) if dw is not None else None,
-                None, None, None, None, None, None)
+        dx = dh * gout.to(dh.dtype)
+        tgt = _flat_grad(ctx.w) if dw is not None and dw.is_contiguous() else None
+        if tgt is not None:      # straight into the optimizer's fp32 buffer
+            _lib.check_rc(_lib.cuda_lib().axb_axpy_f32(tgt.data_ptr(), dw.data_ptr(), gout.float().data_ptr(), dw.numel(),
+                                                       _lib.stream_ptr()), "axpy_f32")
+            dw = None
+        return dx, (dw * gout).to(ctx.w_dtype) if dw is not None else None, None, None, None, None, None, None
 
 
 def linear_cross_entropy(hidden, lm_head_weight, labels, num_items=None, chunk_rows=2048,

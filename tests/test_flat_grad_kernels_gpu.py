@@ -1,0 +1,79 @@
+"""Flat fp32 gradient buffers: embedding and loss-head gradients added in place, square sum, AdamW."""
+import math
+
+import pytest
+import torch
+
+from axolotl_b200.ops import _lib
+from axolotl_b200.ops import functional as Fn
+from axolotl_b200.ops.optim import adamw_step_, grad_sumsq
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H", [8, 2048, 1036, 33])
+@pytest.mark.parametrize("off", [0, 1])
+def test_embedding_bwd_forms(H, off):
+    """16-byte and element form (width or table off the grid), ids of a ragged batch with repeats. fp32 sums in any order."""
+    torch.manual_seed(H)
+    T, V = 301, 50
+    d = torch.randn(T, H, device="cuda").bfloat16()
+    ids = torch.randint(0, V, (T,), device="cuda")
+    buf = torch.randn(V * H + off + 3, device="cuda")
+    tab = buf[off:off + V * H].view(V, H)
+    ref = tab.double().index_add(0, ids, d.double())
+    mag = tab.double().abs().index_add(0, ids, d.double().abs())
+    rest = buf[off + V * H:].clone()
+    _lib.check_rc(_lib.cuda_lib().axb_embedding_bwd(d.data_ptr(), ids.data_ptr(), tab.data_ptr(), T, H, V, _lib.stream_ptr()), "embedding_bwd")
+    assert ((tab.double() - ref).abs() <= 2 ** -20 * mag).all() and torch.equal(buf[off + V * H:], rest)
+
+
+@pytest.mark.parametrize("n", [1, 3, 1024, 5_000_003])
+@pytest.mark.parametrize("off", [0, 1])
+def test_flat_sumsq_axpy_adamw(n, off):
+    """Vector body and element tail, aligned and not. n terms summed by at most 2^13 steps per lane: 2^-12 for the sum."""
+    torch.manual_seed(n)
+    big = torch.randn(4, n + off, device="cuda")
+    flat = [torch.empty(n + off, device="cuda").copy_(b)[off:] for b in big]
+    p, g, m, v = flat
+    v.abs_()
+    ss = grad_sumsq(g, None)
+    assert math.isclose(float(ss), float(g.double().pow(2).sum()), rel_tol=2 ** -12)
+    y, want = torch.randn(n + off, device="cuda")[off:], None
+    want = y.double() + 0.75 * g.double()
+    _lib.check_rc(_lib.cuda_lib().axb_axpy_f32(y.data_ptr(), g.data_ptr(), torch.full((), 0.75, device="cuda").data_ptr(), n,
+                                               _lib.stream_ptr()), "axpy")
+    assert ((y.double() - want).abs() <= 2 ** -23 * (want.abs() + g.abs())).all()
+    lr, b1, b2, eps, wd, step = 1e-2, 0.9, 0.95, 1e-6, 0.1, 3
+    P, G, M, W = (t.double() for t in (p, g, m, v))
+    M = b1 * M + (1 - b1) * G
+    W = b2 * W + (1 - b2) * G * G
+    upd = lr * (M / (1 - b1 ** step)) / ((W / (1 - b2 ** step)).sqrt() + eps)
+    ref = P * (1 - lr * wd) - upd
+    copy = torch.empty(n + off, device="cuda", dtype=torch.bfloat16)[off:]
+    adamw_step_(p, g, m, v, lr=lr, beta1=b1, beta2=b2, eps=eps, weight_decay=wd, step=step, bf16_copy=copy)
+    # a handful of fp32 roundings (1 - beta in fp32: 2^-24 / 0.05) of operands of these magnitudes
+    assert ((p.double() - ref).abs() <= 2 ** -19 * (P.abs() + upd.abs() + lr)).all()
+    assert torch.equal(copy, p.bfloat16())
+
+
+@pytest.mark.parametrize("T,V", [(64, 512), (640, 4096)])
+def test_head_and_table_gradients_reach_the_flat_buffer(T, V):
+    """With an optimizer buffer the gradients are added to it (twice here, two chunks), without one they come back rounded to bf16."""
+    torch.manual_seed(T)
+    H = 256
+    ids, labels = torch.randint(0, V, (2, T), device="cuda")
+    tab0, w0 = (torch.randn(V, H, device="cuda") * 0.1).bfloat16(), (torch.randn(V, H, device="cuda") * 0.1).bfloat16()
+    def run(flat):
+        tab, w = torch.nn.Parameter(tab0.clone()), torch.nn.Parameter(w0.clone())
+        if flat:
+            tab._axb_grad, w._axb_grad = torch.ones(2, V, H, device="cuda")
+        for _ in range(2 if flat else 1):
+            (Fn.linear_cross_entropy(Fn.embedding(tab, ids), w, labels, chunk_rows=T // 2) * 3.0).backward()
+        if flat:
+            assert tab.grad is None and w.grad is None
+            return tab._axb_grad.sub(1).div(2), w._axb_grad.sub(1).div(2)
+        return tab.grad.float(), w.grad.float()
+    for a, b in zip(run(True), run(False)):
+        # one bf16 rounding of the returned gradient; the buffer's ones cost 2^-23 of themselves per addition
+        assert ((a - b).abs() <= 2 ** -8 * b.abs() + 2 ** -20).all()
