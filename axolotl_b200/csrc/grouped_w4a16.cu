@@ -27,12 +27,13 @@ namespace {
 constexpr int BM = 128;
 constexpr int BN = 128;
 constexpr int BK = 64;
-constexpr int W4_CONV_WARPS = 8;
-constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (A), MMA, 4 epilogue warps, 8 converter warps, TMA (weights)
+constexpr int W4_CONV_WARPS = 16;
+constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (A), MMA, 4 epilogue warps, converters, TMA (weights)
 // Three rings of their own: the packed weights are small and run four k blocks ahead of the decode;
 // a slot of the decoded tile is only held from its decode to its MMA, and a slot of A from its load to its MMA.
-// The converters work in four groups of two warps, each on a k block of its own, so that four chains (packed tile seen ->
-// decode -> stores -> proxy fence -> arrival) run side by side.
+// The converters work in four groups of four warps, each on a k block of its own, so that four chains (packed tile seen ->
+// decode -> stores -> proxy fence -> arrival) run side by side. Two warps a group left the decode's dependent instructions
+// uncovered: 512 rows of each of 128 experts, 2048 -> 1536 393 -> 366 us, 768 -> 2048 220 -> 199.
 constexpr int SA = 4, SB = 4, SR = 4;  // slots: A (two 128-row tiles), decoded B, packed B
 // Every group owns one slot of the packed and one of the decoded ring (k block i of the whole sequence belongs to group, slot
 // i % 4), so that a slot's waits are made in order by the same warps: a wait for a phase whose predecessor has not completed
@@ -43,8 +44,14 @@ constexpr int B_BYTES = BN * BK * 2;
 constexpr int RAW_BYTES = 4096;   // FWD: 128 rows x 32 bytes; DX: 64 rows x 64 bytes
 constexpr int EPI_BYTES = 4096;   // per epilogue warp: 32 rows x 64 bf16 columns on their way out
 constexpr int W4_SMEM = SA * 2 * A_BYTES + SB * B_BYTES + SR * RAW_BYTES + 4 * EPI_BYTES + 1024 + 512;
-static_assert(W4_SMEM <= 227 * 1024 && SB == CGROUPS && SR == CGROUPS, "");
+static_assert(W4_SMEM <= 227 * 1024 && SB == CGROUPS && SR % CGROUPS == 0, "");
 
+constexpr int PF = 8;                  // k blocks between a packed tile's L2 prefetch and its load
+AXB_DEVICE void tma_prefetch_3d(const CUtensorMap* tmap, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0),
+               "r"(c1), "r"(c2)
+               : "memory");
+}
 // position in a ring of N slots
 template <int N>
 struct Ring {
@@ -267,6 +274,28 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
     }
   } else if (warp == W4_THREADS / 32 - 1) {
     // ------------------------------------------------------------ packed weights
+    // They come from DRAM, and four slots do not cover that latency where an expert has few rows: a second walk over the same
+    // sequence asks for them PF k blocks earlier, into L2 (20 rows of each of 128 experts, 2048 -> 1536: 221 -> 190 us,
+    // 768 -> 2048: 109 -> 94; 16 blocks ahead is no better; with 512 rows an expert it makes no difference). More slots would do
+    // the same and cost the A ring one.
+    int pt = blockIdx.x, psub = 0, pkb = 0;
+    Pass pp;
+    bool live = pt < total && get_pass(p.blk_expert, n_blocks, num_n, p.E, pt, 0, pp);
+    auto prefetch_step = [&]() {
+      if (!live) return;
+      if (pkb < nk_main && elect_one()) {
+        if (!DX) tma_prefetch_3d(&tmQ, pkb * (BK / 2), pp.n0, pp.e);
+        else tma_prefetch_3d(&tmQ, pp.n0 / 2, pkb * BK, pp.e);
+      }
+      __syncwarp();
+      if (++pkb < nk) return;
+      pkb = 0;
+      do {
+        if (++psub == 2) psub = 0, pt += gridDim.x;
+        live = pt < total;
+      } while (live && !get_pass(p.blk_expert, n_blocks, num_n, p.E, pt, psub, pp));
+    };
+    for (int i = 0; i < PF; ++i) prefetch_step();
     Ring<SR> rr;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
@@ -274,6 +303,7 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         Pass ps;
         if (!get_pass(p.blk_expert, n_blocks, num_n, p.E, tile, sub, ps)) continue;
         for (int kb = 0; kb < nk; ++kb, rr.next()) {
+          prefetch_step();
           if (!warp_all(mbar_wait(&r_empty[rr.slot], rr.phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) {
             ok = false;
             break;
@@ -336,7 +366,7 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
     }
   } else if (warp >= 6) {
     // ------------------------------------------------------------ converters: packed tile -> bf16 B tile
-    // A k block is 256 units of 16 packed bytes (32 codes, 2 scale groups); thread t of a group takes units t, t + 64, ...
+    // A k block is 256 units of 16 packed bytes (32 codes, 2 scale groups); thread t of a group takes units t, t + 128
     // Unit ct lies at raw + ct * 16 and becomes four 16-byte chunks of the swizzled bf16 tile.
     //   FWD: raw tile [128 n][32 B]: weight row n0 + ct / 2, codes 32 * (ct & 1) .. + 31 of k block kb
     //        -> K-major row ct / 2, chunks 4 * (ct & 1) .. + 3.
@@ -379,9 +409,9 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
         load_scales(kb, cur);
         for (; kb < nk && ok; kb += CGROUPS) {
           load_scales(kb + CGROUPS, nxt);
-          const int bslot = grp, rslot = grp;
-          const uint32_t bphase = (uint32_t)((cb + kb) / CGROUPS) & 1;
-          if (!mbar_wait(&r_full[rslot], bphase, p.status, AXB_TIMEOUT_FULL)) {
+          const int bslot = grp, rslot = (int)((cb + kb) % SR);
+          const uint32_t bphase = (uint32_t)((cb + kb) / SB) & 1, rphase = (uint32_t)((cb + kb) / SR) & 1;
+          if (!mbar_wait(&r_full[rslot], rphase, p.status, AXB_TIMEOUT_FULL)) {
             ok = false;
             break;
           }
