@@ -99,6 +99,7 @@ _CUDA_SIGS = {
     "axb_embedding_bwd": [vp, vp, vp, i64, i32, i64, vp],
     "axb_ce_fwd_bwd": [vp, vp, vp, vp, i64, i32, i64, f32, i64, i32, vp],
     "axb_ce_fwd_bwd_softcap": [vp, vp, vp, vp, i64, i32, i64, f32, i64, i32, f32, vp],
+    "axb_transpose": [vp, vp, i64, i64, i32, vp],
     "axb_axpy_f32": [vp, vp, vp, i64, vp],
     "axb_sumsq": [vp, i64, vp, vp],
     "axb_adamw": [vp, vp, vp, vp, vp, i64, f32, f32, f32, f32, f32, f32, f32, vp, f32, f32, vp],

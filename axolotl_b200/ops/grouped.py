@@ -194,7 +194,11 @@ def _adapter_operands(experts, which, A, B, E):
         return hit[3], hit[4]
     r = A.shape[0] // E
     A16 = A.detach().to(torch.bfloat16).view(E, r, -1).contiguous()
-    Bt16 = B.detach().view(-1, r, E).permute(2, 0, 1).to(torch.bfloat16).contiguous()
+    if B.is_cuda and B.dtype == torch.float32 and B.is_contiguous():      # [N * r, E] -> [E, N * r]
+        Bt16 = torch.empty((E, B.numel() // (r * E), r), dtype=torch.bfloat16, device=B.device)
+        _lib.check_rc(_lib.cuda_lib().axb_transpose(B.data_ptr(), Bt16.data_ptr(), B.numel() // E, E, 0, _lib.stream_ptr()), "transpose")
+    else:
+        Bt16 = B.detach().view(-1, r, E).permute(2, 0, 1).to(torch.bfloat16).contiguous()
     cache[which] = (_PARAM_EPOCH[0], A, B, A16, Bt16, torch.is_grad_enabled())
     return A16, Bt16
 
@@ -259,12 +263,19 @@ class _GroupedProj(torch.autograd.Function):
                 dA = grouped_gram(dt, x, lay, torch.empty((E, r, x.shape[1]), dtype=torch.float32,
                                                           device=x.device)).view(E * r, -1).to(A.dtype)
             dBt = grouped_gram(dy, t, lay, torch.empty((E, dy.shape[1], r), dtype=torch.float32, device=x.device))
-            dB_full = dBt.permute(1, 2, 0).reshape(B.shape)                      # [N, r, E] -> [N, r*E]
             gB = _grad_buffer(B)
-            if gB is not None:
-                gB.add_(dB_full)
+            tgt = gB if gB is not None else torch.empty(B.shape, dtype=torch.float32, device=dy.device)
+            if dBt.is_cuda and tgt.dtype == torch.float32 and tgt.is_contiguous():       # [E, N * r] -> [N, r * E]
+                _lib.check_rc(_lib.cuda_lib().axb_transpose(dBt.data_ptr(), tgt.data_ptr(), E, dBt.numel() // E,
+                                                            1 if gB is not None else 2, _lib.stream_ptr()), "transpose")
+                if gB is None:
+                    dB = tgt.to(B.dtype)
             else:
-                dB = dB_full.to(B.dtype)
+                dB_full = dBt.permute(1, 2, 0).reshape(B.shape)
+                if gB is not None:
+                    gB.add_(dB_full)
+                else:
+                    dB = dB_full.to(B.dtype)
         else:
             (x,) = ctx.saved_tensors
             dx = mm(dy)

@@ -65,3 +65,16 @@ def test_dispatch_and_combine_rows(T, k, H):
                                                      _lib.stream_ptr()), "moe_combine_dw")
     prod = dy.double()[:, None] * ys[lay.slot_row.long()].view(T, k, H).double()
     assert ((dw.double() - prod.sum(-1)).abs() <= 2 ** -18 * prod.abs().sum(-1)).all()
+
+
+@pytest.mark.parametrize("R,C", [(1, 1), (63, 65), (64, 64), (130, 7), (8, 24576), (4099, 128)])
+def test_transpose_modes(R, C):
+    """Tile edges; the bf16 form is one rounding, the fp32 forms are exact."""
+    from axolotl_b200.ops import _lib
+
+    a = torch.randn(R, C, device="cuda")
+    base = torch.randn(C, R, device="cuda")
+    for mode, dst, want in ((0, torch.empty(C, R, device="cuda", dtype=torch.bfloat16), a.t().bfloat16()),
+                            (1, base.clone(), base + a.t()), (2, torch.empty(C, R, device="cuda"), a.t())):
+        _lib.check_rc(_lib.cuda_lib().axb_transpose(a.data_ptr(), dst.data_ptr(), R, C, mode, _lib.stream_ptr()), "transpose")
+        assert torch.equal(dst, want)
