@@ -70,12 +70,13 @@ AXB_DEVICE uint32_t sw128_chunk_off(int row, int chunk) {
 // rows (GQA groups of even size), or two neighbouring q tiles of one head. Each unit has its own softmax warpgroup and its own
 // S and O in TMEM, [S0 | S1 | O0 | O1]; while one warpgroup exponentiates, the tensor core runs the other unit's P.V and next
 // scores, and K / V are read once for both. P (bf16) overwrites the first half of its S columns and is the TMEM operand of
-// P.V, so it never passes through shared memory. O accumulates in TMEM; it is rescaled only when a row's maximum has grown by
-// more than 2^8 (P then stays below 2^8, its relative rounding and the fp32 sums are what they were), which a row meets a
-// handful of times: l and P use the same reference maximum, so the result does not depend on when that happens.
+// P.V, so it never passes through shared memory. O accumulates in TMEM; a warp rescales its rows when one of them has a new
+// maximum. Waiting until a maximum has grown by 2^8 would spare most of that (one 16384-token document 1.73 ms) and was taken
+// back: with a reference below the maximum the largest P of a row is not exactly one, and rounding it to bf16 makes the error
+// against 64 bits 1.5 % larger for unit normal q and k, 19 % for twice that. Dividing by the sum of the rounded P mends half.
 // Bound: exponentials (16 per clock and SM against 1024 clocks of MMA per 128 x 128 block) and the MMA stream, about level.
-// One 16384-token document, 32 / 8 heads of 128: 3.02 -> 1.87 ms (730 -> 1180 TFLOP/s) against one softmax warpgroup with O in
-// registers and P through shared memory; 4 x 2048 267 -> 184 us; 11 x 707 windowed, 64 heads of 64, 229 -> 155 us.
+// One 16384-token document, 32 / 8 heads of 128: 3.01 -> 1.89 ms (730 -> 1160 TFLOP/s) against one softmax warpgroup with O in
+// registers and P through shared memory; 4 x 2048 268 -> 180 us; 11 x 707, 64 heads of 64, 279 -> 183 us.
 // TMA warp, MMA warp, two idle warps (they complete the warpgroup that gives registers away), 2 x 4 softmax warps. A row of S
 // is held in 128 registers: the 384 x 168 registers of the launch are split 128 x 40 + 256 x 232.
 constexpr int kFwdThreads = 384;
@@ -294,19 +295,23 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.sl2);
       if (j == 0) {
         m = m_new;
-      } else if (__any_sync(0xffffffffu, m_new > m + 8.f)) {
-        const float m_next = m_new > m + 8.f ? m_new : m;
-        const float alpha = m_next == m ? 1.f : fast_exp2(m - m_next);
-        m = m_next;
+      } else if (__any_sync(0xffffffffu, m_new > m)) {
+        const float alpha = m_new == m ? 1.f : fast_exp2(m - m_new);
+        m = m_new;
         l *= alpha;
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(o_addr + c * 32, o);
+        for (int c = 0; c < D / 64; ++c) {
+          uint32_t o[2][32];
+          tmem_ld_32x32(o_addr + c * 64, o[0]);
+          tmem_ld_32x32(o_addr + c * 64 + 32, o[1]);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_32x32(o_addr + c * 32, o);
+          for (int i = 0; i < 32; ++i) {
+            o[0][i] = __float_as_uint(__uint_as_float(o[0][i]) * alpha);
+            o[1][i] = __float_as_uint(__uint_as_float(o[1][i]) * alpha);
+          }
+          tmem_st_32x32(o_addr + c * 64, o[0]);
+          tmem_st_32x32(o_addr + c * 64 + 32, o[1]);
         }
       }
       const float m_use = m == -INFINITY ? 0.f : m;    // no visible column so far: every P is exp2(-inf) = 0
