@@ -4,15 +4,13 @@
 //
 // The 128-wide kernels of flash_varlen.cu keep a whole head in shared memory and TMEM with double buffers;
 // at 256 that does not fit (Q + K + V tiles of 128 rows are 192 KB, dK + dV accumulators are all 512 TMEM
-// columns). Here every CTA produces one 128-column PART of the outputs and contracts S = Q.K^T (and
-// dP = dO.V^T) over the full width:
-//   forward   grid (q head, q tile, v part):   S over Dqk, O[:, part] = P . V[:, part]
-//   backward  grid (kv head, kv tile, part):   S^T, dP^T over the full widths; dV[:, part], dK[:, part] and
-//                                              dQ^T[part, :] for this part only
-// so the score GEMMs are computed once per part (1.4x the minimum FLOPs at 256/256) and nothing else grows.
-// Stages are single-buffered (shared memory is full); the pipeline still overlaps the K load and the next S
-// with the softmax of the current block. Same tile table, same packed fused-projection layout
-// [T, Hq*Dqk | Hk*Dqk | Hk*Dv] and the same bounded waits as flash_varlen.cu.
+// columns).
+//   forward   grid (q head, q tile): Q stays, K and V stream through a ring of 128-column units
+//   backward  grid (kv head, kv tile, part): S^T, dP^T over the full widths; dV[:, part], dK[:, part] and
+//             dQ^T[part, :] of one 128-column PART of the outputs, so the score GEMMs are computed once per part
+//             (1.4x the minimum FLOPs at 256/256) and nothing else grows. Stages are single-buffered.
+// Same tile table, same packed fused-projection layout [T, Hq*Dqk | Hk*Dqk | Hk*Dv] and the same bounded waits as
+// flash_varlen.cu.
 //
 // Takes the place of the reference's flash-attn / SDPA paths for these head sizes
 // (src/axolotl/monkeypatch/attention/flash_attn_4.py:37-111; Gemma attention soft-capping reaches the
@@ -58,24 +56,34 @@ AXB_DEVICE uint32_t sw128_chunk_off(int row, int chunk) {
 }
 
 // =====================================================================================================
-// Forward: 192 threads = TMA warp, MMA warp, 4 softmax warps. One CTA per (q head, 128-row q tile, v part).
+// Forward: 192 threads = TMA warp, MMA warp, 4 softmax warps. One CTA per (q head, 128-row q tile), all of the v head.
+// S is double buffered in TMEM [S0 | S1 | O (Dv)]: the scores of the next block are there when a block's P is done, and the next
+// but one are issued behind its P.V. P (bf16) overwrites the first half of its S columns and is the TMEM operand of P.V. O
+// accumulates in TMEM and is rescaled by a warp that has a row with a new maximum (see flash_varlen.cu).
+// K and V stream through one ring of 128-column units in the order in which the MMA warp reads them: K(0), K(1), V(0), K(2),
+// V(1), ... Q and the ring's five units fill shared memory.
+// Bound: the load latency of a unit against the ring, then the MMA stream (2048 clocks per 128 x 128 block at 256 / 256).
+// 4 documents of 2048, 16 / 8 heads of 256: 363 -> 166 us against one CTA per 128-column part of V with S, softmax and P (through
+// shared memory) done once per part, O in registers and single K / V buffers.
 // =====================================================================================================
-template <int DQK>
+template <int DQK, int DV>
 struct WFwd {
   static constexpr int QK_BYTES = (DQK / 64) * HALF_BYTES;
-  static constexpr int V_BYTES = 2 * HALF_BYTES;   // 128 kv rows x 128 v columns of this part
-  static constexpr int P_BYTES = 2 * HALF_BYTES;
-  static constexpr int SMEM = 2 * QK_BYTES + V_BYTES + P_BYTES + 1024 + 256;
+  static constexpr int KU = (DQK + 127) / 128, VU = DV / 128;   // units of a K / V tile (the last of a 192-wide K is half full)
+  static constexpr int UNIT = 2 * HALF_BYTES, SLOTS = 5;
+  static constexpr int SMEM = QK_BYTES + SLOTS * UNIT + 1024 + 256;
+  static constexpr int O_COL = 256;
+  static_assert(SMEM <= 227 * 1024 && O_COL + DV <= 512, "");
 };
 
 template <int DQK, int DV, bool SOFTCAP>
 __global__ void __launch_bounds__(192, 1)
     flash_wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                           const WideParams p) {
-  using C = WFwd<DQK>;
+  using C = WFwd<DQK, DV>;
   const int tile_id = blockIdx.y;
   if (tile_id >= p.n_tiles) return;
-  const int head = blockIdx.x, part = blockIdx.z;
+  const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hk);
   const int4 ti = p.tiles[tile_id];
   const int doc_start = ti.x, doc_len = ti.y, q0 = ti.z;
@@ -89,43 +97,33 @@ __global__ void __launch_bounds__(192, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
-  uint8_t* sK = sQ + C::QK_BYTES;
-  uint8_t* sV = sK + C::QK_BYTES;
-  uint8_t* sP = sV + C::V_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + C::P_BYTES);
+  uint8_t* sU = sQ + C::QK_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sU + C::SLOTS * C::UNIT);
   uint64_t* q_full = bars + 0;
-  uint64_t* k_full = bars + 1;
-  uint64_t* v_full = bars + 2;
-  uint64_t* k_empty = bars + 3;
-  uint64_t* v_empty = bars + 4;
-  uint64_t* s_full = bars + 5;    // [2]
-  uint64_t* s_empty = bars + 7;   // [2]
-  uint64_t* p_full = bars + 9;
-  uint64_t* p_empty = bars + 10;
-  uint64_t* pv_full = bars + 11;  // [2]
-  uint64_t* pv_empty = bars + 13; // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* u_full = bars + 1;               // [slot] unit landed
+  uint64_t* u_empty = u_full + C::SLOTS;     // [slot] its MMAs retired
+  uint64_t* s_full = u_empty + C::SLOTS;     // [2] scores ready
+  uint64_t* p_full = s_full + 2;             // [2] P written (S read, O rescaled)
+  uint64_t* pv_full = p_full + 2;            // [2] P.V added to O
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_full + 2);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(k_full, 1);
-    mbar_init(v_full, 1);
-    mbar_init(k_empty, 1);
-    mbar_init(v_empty, 1);
+    for (int s = 0; s < C::SLOTS; ++s) {
+      mbar_init(&u_full[s], 1);
+      mbar_init(&u_empty[s], 1);
+    }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_empty[s], 128);
+      mbar_init(&p_full[s], 128);
       mbar_init(&pv_full[s], 1);
-      mbar_init(&pv_empty[s], 128);
     }
-    mbar_init(p_full, 128);
-    mbar_init(p_empty, 1);
     mbar_fence_init();
     tma_prefetch_desc(&tm_kv);
   }
   if (warp == 2) {
-    tmem_alloc(tmem_slot, 512);   // S: 2 x 128 columns at 0; P.V: 2 x 128 columns at 256
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -133,207 +131,210 @@ __global__ void __launch_bounds__(192, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    if (elect_one()) {
-      mbar_expect_tx(q_full, C::QK_BYTES);
-#pragma unroll
-      for (int h = 0; h < DQK / 64; ++h)
-        tma_load_2d(sQ + h * HALF_BYTES, &tm_q, q_full, p.q_col0 + head * DQK + h * 64, doc_start + q0);
-    }
-    __syncwarp();
-    for (int j = 0; j < n_blocks; ++j) {
-      const uint32_t ph = j & 1;
-      if (!warp_all(mbar_wait(k_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+  if (warp < 2) {
+    int slot = 0;                            // both warps walk the units in the same order
+    uint32_t phase = 0;
+    auto advance = [&]() {
+      if (++slot == C::SLOTS) {
+        slot = 0;
+        phase ^= 1;
+      }
+    };
+    if (warp == 0) {
       if (elect_one()) {
-        mbar_expect_tx(k_full, C::QK_BYTES);
+        mbar_expect_tx(q_full, C::QK_BYTES);
 #pragma unroll
         for (int h = 0; h < DQK / 64; ++h)
-          tma_load_2d(sK + h * HALF_BYTES, &tm_kv, k_full, p.k_col0 + kv_head * DQK + h * 64, doc_start + (jb0 + j) * 128);
+          tma_load_2d(sQ + h * HALF_BYTES, &tm_q, q_full, p.q_col0 + head * DQK + h * 64, doc_start + q0);
       }
       __syncwarp();
-      if (!warp_all(mbar_wait(v_empty, ph ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
-      if (elect_one()) {
-        mbar_expect_tx(v_full, C::V_BYTES);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          tma_load_2d(sV + h * HALF_BYTES, &tm_kv, v_full, p.v_col0 + kv_head * DV + part * 128 + h * 64,
-                      doc_start + (jb0 + j) * 128);
-      }
-      __syncwarp();
-    }
-  } else if (warp == 1) {
-    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
-    const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dk = make_smem_desc_sw128(smem_u32(sK), 16, 1024);
-    const uint64_t dv = make_smem_desc_sw128(smem_u32(sV), HALF_BYTES, 1024), dp = make_smem_desc_sw128(smem_u32(sP), 16, 1024);
-    bool ok = warp_all(mbar_wait(q_full, 0, p.status, AXB_TIMEOUT_FULL));
-    auto issue_s = [&](int j) -> bool {
-      const int b = j & 1;
-      if (!warp_all(mbar_wait(k_full, j & 1, p.status, AXB_TIMEOUT_FULL) &&
-                    mbar_wait(&s_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)))
-        return false;
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < DQK / 16; ++kk) {
-          const uint32_t off = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
-          umma_f16(tmem_base + b * 128, dq + off, dk + off, idesc_s, kk > 0);
+      // columns col0 .. col0 + width - 1 of block j, in units
+      auto load = [&](int j, int col0, int width) -> bool {
+        for (int c = 0; c < width; c += 128, advance()) {
+          if (!warp_all(mbar_wait(&u_empty[slot], phase ^ 1, p.status, AXB_TIMEOUT_EMPTY))) return false;
+          const int halves = width - c >= 128 ? 2 : 1;
+          if (elect_one()) {
+            mbar_expect_tx(&u_full[slot], halves * HALF_BYTES);
+            for (int h = 0; h < halves; ++h)
+              tma_load_2d(sU + slot * C::UNIT + h * HALF_BYTES, &tm_kv, &u_full[slot], col0 + c + h * 64, doc_start + (jb0 + j) * 128);
+          }
+          __syncwarp();
         }
-        umma_commit(&s_full[b]);
-        umma_commit(k_empty);
+        return true;
+      };
+      const int kc = p.k_col0 + kv_head * DQK, vc = p.v_col0 + kv_head * DV;
+      bool ok = true;
+      for (int j = 0; j < 2 && j < n_blocks && ok; ++j) ok = load(j, kc, DQK);
+      for (int j = 0; j < n_blocks && ok; ++j) {
+        ok = load(j, vc, DV);
+        if (ok && j + 2 < n_blocks) ok = load(j + 2, kc, DQK);
       }
-      __syncwarp();
-      return true;
-    };
-    if (ok) ok = issue_s(0);
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      const int b = j & 1;
-      if (j + 1 < n_blocks) {
-        ok = issue_s(j + 1);
-        if (!ok) break;
-      }
-      if (!warp_all(mbar_wait(p_full, j & 1, p.status, AXB_TIMEOUT_GENERIC) && mbar_wait(v_full, j & 1, p.status, AXB_TIMEOUT_FULL) &&
-                    mbar_wait(&pv_empty[b], ((j >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY)))
-        break;
-      tc_fence_after();
-      if (elect_one()) {
+    } else {
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
+      constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
+      const uint64_t dq = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dk_base = make_smem_desc_sw128(smem_u32(sU), 16, 1024);
+      const uint64_t dv_base = make_smem_desc_sw128(smem_u32(sU), HALF_BYTES, 1024);
+      auto issue_s = [&](int j) -> bool {
+        const int b = j & 1;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t poff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
-          umma_f16(tmem_base + 256 + b * 128, dp + poff, dv + kk * (2048 / 16), idesc_pv, kk > 0);
+        for (int u = 0; u < C::KU; ++u, advance()) {
+          if (!warp_all(mbar_wait(&u_full[slot], phase, p.status, AXB_TIMEOUT_FULL))) return false;
+          tc_fence_after();
+          const uint64_t dk = dk_base + (uint32_t)(slot * (C::UNIT / 16));
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+              if (u * 128 + kk * 16 >= DQK) break;
+              const uint32_t off = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16;
+              umma_f16(tmem_base + b * 128, dq + u * (C::UNIT / 16) + off, dk + off, idesc_s, u > 0 || kk > 0);
+            }
+            umma_commit(&u_empty[slot]);
+            if (u == C::KU - 1) umma_commit(&s_full[b]);
+          }
+          __syncwarp();
         }
-        umma_commit(&pv_full[b]);
-        umma_commit(v_empty);
-        umma_commit(p_empty);
+        return true;
+      };
+      auto issue_pv = [&](int j) -> bool {
+        const int b = j & 1;
+        if (!warp_all(mbar_wait(&p_full[b], (j >> 1) & 1, p.status, AXB_TIMEOUT_GENERIC))) return false;
+#pragma unroll
+        for (int u = 0; u < C::VU; ++u, advance()) {
+          if (!warp_all(mbar_wait(&u_full[slot], phase, p.status, AXB_TIMEOUT_FULL))) return false;
+          tc_fence_after();
+          const uint64_t dv = dv_base + (uint32_t)(slot * (C::UNIT / 16));
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)       // 128 kv rows / 16: 8 TMEM columns of P each
+              umma_f16_ts(tmem_base + C::O_COL + u * 128, tmem_base + b * 128 + kk * 8, dv + kk * (2048 / 16), idesc_pv, j > 0 || kk > 0);
+            umma_commit(&u_empty[slot]);
+            if (u == C::VU - 1) umma_commit(&pv_full[b]);
+          }
+          __syncwarp();
+        }
+        return true;
+      };
+      bool ok = n_blocks > 0 && warp_all(mbar_wait(q_full, 0, p.status, AXB_TIMEOUT_FULL));
+      for (int j = 0; j < 2 && j < n_blocks && ok; ++j) ok = issue_s(j);
+      for (int j = 0; j < n_blocks && ok; ++j) {
+        ok = issue_pv(j);
+        if (ok && j + 2 < n_blocks) ok = issue_s(j + 2);     // over P(j), which the P.V before it has read
       }
-      __syncwarp();
     }
   } else {
     const int lg = warp & 3;
     const int r = lg * 32 + lane;
     const int q_idx = q0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
-    // effective score in the log2 domain
-    auto eff = [&](float v) -> float {
-      if constexpr (SOFTCAP) return tanhf(v * p.cap_in) * p.cap_out2;
-      else return v * p.sl2;
-    };
-    float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
-    float o[128];
-#pragma unroll
-    for (int i = 0; i < 128; ++i) o[i] = 0.f;
+    const uint32_t o_addr = tmem_base + lane_off + C::O_COL;
+    const float mul = SOFTCAP ? 1.f : p.sl2;      // to the log2 domain (soft-capped scores are brought there first)
+    float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_blocks && ok; ++j) {
       const int b = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[b], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      if (!warp_all(mbar_wait(&s_full[b], (j >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL))) {
         ok = false;
         break;
       }
       tc_fence_after();
       const uint32_t s_addr = tmem_base + lane_off + b * 128;
+      uint32_t sr[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, sr[c]);
+      tmem_ld_wait();
+      if constexpr (SOFTCAP) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sr[c][i] = __float_as_uint(tanhf(__uint_as_float(sr[c][i]) * p.cap_in) * p.cap_out2);
+      }
       const int kv0 = (jb0 + j) * 128;
-      const int lim = (bidir ? doc_len - 1 : min(q_idx, doc_len - 1)) - kv0;
-      const int lo = win > 0 ? q_idx - win + 1 - kv0 : -(1 << 30);
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t sr[32];
-        tmem_ld_32x32(s_addr + c * 32, sr);
-        tmem_ld_wait();
+      if (kv0 + 127 > (bidir ? doc_len - 1 : min(q0, doc_len - 1)) || (win > 0 && kv0 < q0 + 128 - win)) {
+        const int lim = (bidir ? doc_len - 1 : min(q_idx, doc_len - 1)) - kv0;  // columns <= lim are visible
+        const int lo = win > 0 ? q_idx - win + 1 - kv0 : -(1 << 30);            // columns >= lo are visible
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float v = __uint_as_float(sr[i]);
-          if (c * 32 + i > lim || c * 32 + i < lo) v = -INFINITY;
-          mx = fmaxf(mx, v);
-        }
-      }
-      const float m_new = fmaxf(m, mx == -INFINITY ? -INFINITY : eff(mx));   // eff is increasing
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = fast_exp2(m - m_use);
-      if (!mbar_wait(p_empty, (j & 1) ^ 1, p.status, AXB_TIMEOUT_GENERIC)) {
-        ok = false;
-        break;
-      }
-      float rowsum = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t sr[32];
-        tmem_ld_32x32(s_addr + c * 32, sr);
-        tmem_ld_wait();
-        uint32_t pk[16];
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0 = fast_exp2(eff(__uint_as_float(sr[i])) - m_use), p1 = fast_exp2(eff(__uint_as_float(sr[i + 1])) - m_use);
-          if (c * 32 + i > lim || c * 32 + i < lo) p0 = 0.f;
-          if (c * 32 + i + 1 > lim || c * 32 + i + 1 < lo) p1 = 0.f;
-          rowsum += p0 + p1;
-          pk[i >> 1] = pack_bf16x2(p0, p1);
-        }
-        uint8_t* pbase = sP + (c >> 1) * HALF_BYTES;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(pbase + sw128_chunk_off(r, (c & 1) * 4 + q)) =
-              make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i > lim || c * 32 + i < lo) sr[c][i] = 0xff800000u;    // -inf
       }
-      tc_fence_before();
-      mbar_arrive(&s_empty[b]);
-      fence_proxy_async_smem();
-      mbar_arrive(p_full);
-      l = l * alpha + rowsum;
-      m = m_new;
-      if (j > 0) {
-        const int pb = (j - 1) & 1;
-        if (!mbar_wait(&pv_full[pb], ((j - 1) >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sr[c][i]));
+      const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul);
+      if (j == 0) {
+        m = m_new;
+      } else if (__any_sync(0xffffffffu, m_new > m)) {
+        // S(j) was issued behind P.V(j - 2): the one after it has to be waited for
+        if (!warp_all(mbar_wait(&pv_full[b ^ 1], ((j - 1) >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL))) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t pv_addr = tmem_base + lane_off + 256 + pb * 128;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t vr[32];
-          tmem_ld_32x32(pv_addr + c * 32, vr);
+        const float alpha = m_new == m ? 1.f : fast_exp2(m - m_new);
+        m = m_new;
+        l *= alpha;
+#pragma unroll 1
+        for (int c = 0; c < DV / 64; ++c) {
+          uint32_t o[2][32];
+          tmem_ld_32x32(o_addr + c * 64, o[0]);
+          tmem_ld_32x32(o_addr + c * 64 + 32, o[1]);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[c * 32 + i] = o[c * 32 + i] * alpha_prev + __uint_as_float(vr[i]);
+          for (int i = 0; i < 32; ++i) {
+            o[0][i] = __float_as_uint(__uint_as_float(o[0][i]) * alpha);
+            o[1][i] = __float_as_uint(__uint_as_float(o[1][i]) * alpha);
+          }
+          tmem_st_32x32(o_addr + c * 64, o[0]);
+          tmem_st_32x32(o_addr + c * 64 + 32, o[1]);
         }
-        tc_fence_before();
-        mbar_arrive(&pv_empty[pb]);
       }
-      alpha_prev = alpha;
+      const float m_use = m == -INFINITY ? 0.f : m;    // no visible column so far: every P is exp2(-inf) = 0
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float p0 = fast_exp2(fmaf(__uint_as_float(sr[c][i]), mul, -m_use));
+          const float p1 = fast_exp2(fmaf(__uint_as_float(sr[c][i + 1]), mul, -m_use));
+          sum[i & 2] += p0;
+          sum[(i & 2) + 1] += p1;
+          pk[i >> 1] = pack_bf16x2(p0, p1);
+        }
+        tmem_st_32x16(s_addr + c * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&p_full[b]);
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
-    if (ok && n_blocks > 0) {
-      const int pb = (n_blocks - 1) & 1;
-      if (mbar_wait(&pv_full[pb], ((n_blocks - 1) >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-        tc_fence_after();
-        const uint32_t pv_addr = tmem_base + lane_off + 256 + pb * 128;
-        const float inv_l = l > 0.f ? 1.f / l : 0.f;
-        const long long row = (long long)doc_start + q_idx;
-        const bool row_ok = q_idx < doc_len && row < p.T;
-        __nv_bfloat16* orow = p.out + row * p.out_ld + (long long)head * DV + part * 128;
+    const int last = n_blocks - 1;
+    if (ok && n_blocks > 0 && warp_all(mbar_wait(&pv_full[last & 1], (last >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL))) {
+      tc_fence_after();
+      const float inv_l = l > 0.f ? 1.f / l : 0.f;
+      const long long row = (long long)doc_start + q_idx;
+      const bool row_ok = q_idx < doc_len && row < p.T;
+      __nv_bfloat16* orow = p.out + row * p.out_ld + (long long)head * DV;
+#pragma unroll 1
+      for (int c = 0; c < DV / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(o_addr + c * 32, o);
+        tmem_ld_wait();
+        if (row_ok) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t vr[32];
-          tmem_ld_32x32(pv_addr + c * 32, vr);
-          tmem_ld_wait();
-          if (row_ok) {
+          for (int q = 0; q < 4; ++q) {
+            float f[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float f[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = (o[c * 32 + q * 8 + i] * alpha_prev + __uint_as_float(vr[q * 8 + i])) * inv_l;
-              uint4 u;
-              u.x = pack_bf16x2(f[0], f[1]);
-              u.y = pack_bf16x2(f[2], f[3]);
-              u.z = pack_bf16x2(f[4], f[5]);
-              u.w = pack_bf16x2(f[6], f[7]);
-              *reinterpret_cast<uint4*>(orow + c * 32 + q * 8) = u;
-            }
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(o[q * 8 + i]) * inv_l;
+            *reinterpret_cast<uint4*>(orow + c * 32 + q * 8) =
+                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
           }
         }
-        if (row_ok && part == 0) p.lse2[(long long)head * p.T + row] = m + log2f(l);
       }
+      if (row_ok) p.lse2[(long long)head * p.T + row] = m + log2f(l);
     }
   }
   tc_fence_before();
@@ -707,12 +708,12 @@ int launch_wide_fwd(const CUtensorMap& tq, const CUtensorMap& tkv, const WidePar
   auto kern = flash_wide_fwd_kernel<DQK, DV, SC>;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WFwd<DQK>::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WFwd<DQK, DV>::SMEM);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  dim3 grid(p.Hq, p.n_tiles, DV / 128);
-  kern<<<grid, 192, WFwd<DQK>::SMEM, st>>>(tq, tkv, p);
+  dim3 grid(p.Hq, p.n_tiles);
+  kern<<<grid, 192, WFwd<DQK, DV>::SMEM, st>>>(tq, tkv, p);
   return (int)cudaGetLastError();
 }
 template <int DQK, int DV, bool SC>

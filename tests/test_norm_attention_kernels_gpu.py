@@ -125,3 +125,30 @@ def test_ce_row_edges(V, cap):
     assert ((loss - ref_loss).abs() <= 2 ** -18 * (1 + ref_lse.abs())).all()
     assert ((z[:, :V].double() - g).abs() <= (2 ** -8 + 2 ** -12) * g.abs() + 2 ** -20).all()
     assert torch.equal(z[:, V:], want[:, V:])
+
+
+@pytest.mark.parametrize("D,Dv", [(64, 64), (128, 128), (256, 256), (192, 128)])
+@pytest.mark.parametrize("scale", [1.0, 3.0])
+@pytest.mark.parametrize("docs", [[0, 1, 130, 1100], [0, 640]])
+def test_attention_output_is_rounded_like_a_maximum_referenced_softmax(D, Dv, scale, docs):
+    """Rising row maxima over several key blocks (every block of the ring, O rescaled), flat and peaked rows. P is rounded to
+    bf16 against the row's own maximum so far: the error is at most that of P (2^-9 relative, its root mean square 2^-9 /
+    sqrt(3) with the largest P exact) and of the output (the same), 2^-9 together; 1.15 for the spread."""
+    from axolotl_b200.ops import functional as Fn
+
+    torch.manual_seed(D)
+    T, Hq, Hk = docs[-1], 4, 2
+    qkv = torch.randn(T, Hq * D + Hk * (D + Dv), device="cuda")
+    qkv[:, : (Hq + Hk) * D] *= scale
+    qkv = qkv.bfloat16()
+    out = Fn.flash_varlen(qkv, Fn.AttnMeta(docs, "cuda"), Hq, Hk, D, Dv=Dv)
+    _lib.check_status()
+    q, k, v = (t.double() for t in qkv.split([Hq * D, Hk * D, Hk * Dv], 1))
+    ref = torch.empty(T, Hq, Dv, dtype=torch.double, device="cuda")
+    for a, b in zip(docs, docs[1:]):
+        for h in range(Hq):
+            g = h // (Hq // Hk)
+            s = q[a:b, h * D:(h + 1) * D] @ k[a:b, g * D:(g + 1) * D].t() / D ** 0.5
+            s = s.masked_fill(torch.ones_like(s, dtype=torch.bool).triu(1), float("-inf"))
+            ref[a:b, h] = torch.softmax(s, -1) @ v[a:b, g * Dv:(g + 1) * Dv]
+    assert (out.double().view_as(ref) - ref).norm() <= 1.15 * 2 ** -9 * ref.norm()
