@@ -19,11 +19,9 @@ SKINNY_SPLITS = int(__import__("os").environ.get("AXB_LORA_SKINNY_SPLITS", "0"))
 
 
 def skinny_gemm(a, b, *, trans_b=False, alpha=1.0):
-    """``alpha * a @ op(b)^T`` for an output only a few columns wide ([T, R], R = adapter rank): with one
-    128-row tile per CTA such a GEMM has T/128 CTAs, too few to pull the wide operand at memory speed, so
-    the K range can be split over several CTAs (fp32 atomics into a zeroed [T, R] buffer, cast once).
-    Off by default (AXB_LORA_SKINNY_SPLITS=2|4 enables it): the Llama-3-8B LoRA step measured 306.6 /
-    307.3 / 307.6 ms with 2 / 4 / no splits on one B200, i.e. no difference beyond run-to-run noise."""
+    """``alpha * a @ op(b)^T`` for an output only a few columns wide ([T, R], R = adapter rank). ``gemm`` takes the
+    short-side kernel for it, which splits K over a cluster. AXB_LORA_SKINNY_SPLITS=2|4 splits it with fp32 atomics into
+    a zeroed [T, R] buffer instead (cast once): no faster before that kernel either."""
     T = a.shape[0]
     R = b.shape[1] if trans_b else b.shape[0]
     K = a.shape[1]
