@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(NT, 1536 / NT)
 #pragma unroll
       for (int j = 0; j < 8; ++j) m = fmaxf(m, f[j]);   // tanh is increasing: only the maximum is capped
     }
-    const float b = rebase(m == -INFINITY ? m : eff(m));
+    const float b = rebase(eff(m));             // capped, a group of -inf is a group of -cap: finite terms like all others
     float part = 0.f;                           // summed on its own: a long row loses less
 #pragma unroll
     for (int k = 0; k < CE_U; ++k) {

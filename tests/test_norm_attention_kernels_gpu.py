@@ -127,6 +127,29 @@ def test_ce_row_edges(V, cap):
     assert torch.equal(z[:, V:], want[:, V:])
 
 
+@pytest.mark.parametrize("V", [5, 264, 8192 + 3, 40960, 40968, 128256])
+def test_capped_ce_counts_masked_logits(V):
+    """cap * tanh(-inf) = -cap is an ordinary term of the sum: all logits -inf but one (at either end, so that the groups
+    before and behind a finite one hold nothing else), all of them, and a masked label. Bounds as in ``test_ce_row_edges``."""
+    cap, R, ld = 5.0, 4, (V + 7) // 8 * 8
+    z = torch.full((R, ld), float("-inf"), device="cuda").bfloat16()
+    z[0, 0], z[1, V - 1], z[3, V // 2] = 1.0, 1.0, 7.0
+    lab = torch.tensor([0, V - 1, V // 2, 0], device="cuda")
+    x = z[:, :V].double()
+    loss, lse = torch.empty(2, R, device="cuda")
+    _lib.check_rc(_lib.cuda_lib().axb_ce_fwd_bwd_softcap(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), lse.data_ptr(), R, V, ld, 0.5, -100, 1,
+                                                         cap, _lib.stream_ptr()), "ce")
+    t = torch.tanh(x / cap)
+    ref_lse = torch.logsumexp(cap * t, -1)
+    g = torch.exp(cap * t - ref_lse[:, None])
+    ref_loss = ref_lse - cap * t[torch.arange(R), lab]
+    g[torch.arange(R), lab] -= 1.0
+    g = 0.5 * g * (1 - t * t)
+    assert ((lse - ref_lse).abs() <= 2 ** -19 * (1 + ref_lse.abs())).all()
+    assert ((loss - ref_loss).abs() <= 2 ** -18 * (1 + ref_lse.abs())).all()
+    assert ((z[:, :V].double() - g).abs() <= (2 ** -8 + 2 ** -12) * g.abs() + 2 ** -20).all()
+
+
 @pytest.mark.parametrize("D,Dv", [(64, 64), (128, 128), (256, 256), (192, 128)])
 @pytest.mark.parametrize("scale", [1.0, 3.0])
 @pytest.mark.parametrize("docs", [[0, 1, 130, 1100], [0, 640]])
