@@ -120,8 +120,9 @@ class DecodeStep:
             return None
         if _nn._global_forward_hooks or _nn._global_forward_pre_hooks:
             return None
-        if meta.lens_after.dtype != torch.int32 or meta.seq.dtype != torch.int64 or pos.dtype != torch.int32:
-            return None
+        for t, dtype in ((meta.seq, torch.int64), (meta.lens_after, torch.int32), (pos, torch.int32)):     # one per row, as the kernels read them
+            if not torch.is_tensor(t) or t.dtype != dtype or t.device != h.device or t.shape != h.shape[:1]:
+                return None
         return DecodeStep(h, pos, meta)
 
     def __init__(self, h, pos, meta):

@@ -15,6 +15,21 @@ from ..ops import _lib
 from ..ops import functional as Fn
 
 
+def _row_ids(t, n, device, dtype=torch.int64):
+    """``t`` as the kernels read it, ``n`` contiguous integers on ``device``. Takes what an indexed store takes: any integer
+    dtype, stride and device, a list, a mask, one value for all rows; anything else raises."""
+    if torch.is_tensor(t) and t.dtype == dtype and t.shape == (n,) and t.device == device and t.is_contiguous():
+        return t
+    t = torch.as_tensor(t, device=device)
+    if t.dtype in (torch.bool, torch.uint8):
+        t = t.nonzero().squeeze(1)
+    elif t.dtype not in (torch.int32, torch.int64):
+        raise IndexError(f"cache rows and lengths are integers, got {t.dtype}")
+    if t.dim() > 1 or t.numel() not in (1, n):
+        raise IndexError(f"{tuple(t.shape)} cache rows or lengths for {n} new tokens")
+    return t.to(dtype).expand(n).contiguous()
+
+
 class KVCache:
     def __init__(self, model, batch: int, max_len: int):
         cfg = model.config
@@ -30,9 +45,11 @@ class KVCache:
         kq, vq = qkv[:, Hq * D:(Hq + Hk) * D], qkv[:, (Hq + Hk) * D:]
         if meta.decode:
             # one new token per active sequence: row i of qkv belongs to sequence meta.seq[i]
-            if qkv.is_cuda:      # the attention kernel appends the new k / v rows itself
-                return Fn.decode_attention_append(qkv, self.k[layer], self.v[layer], meta.seq, meta.lens_after, Hq, Hk, D,
-                                                  scale, window)
+            k, v, n = self.k[layer], self.v[layer], qkv.shape[0]
+            if qkv.is_cuda and Hk * D == self.width and (k.data_ptr() | v.data_ptr()) % 16 == 0:
+                # the attention kernel appends the new k / v rows itself
+                return Fn.decode_attention_append(qkv, k, v, _row_ids(meta.seq, n, qkv.device),
+                                                  _row_ids(meta.lens_after, n, qkv.device, torch.int32), Hq, Hk, D, scale, window)
             self.k[layer, meta.seq, meta.pos] = kq
             self.v[layer, meta.seq, meta.pos] = vq
             if meta.all_rows:

@@ -94,6 +94,58 @@ def test_cached_step_on_a_subset_of_the_sequences():
     assert (out.cpu().float() - ref.float()).abs().max() <= 2 ** -7 * max(1.0, ref.abs().max().item())
 
 
+_SEQ_FORMS = {
+    "int32": lambda t: t.int(),
+    "strided": lambda t: torch.stack([t, t.flip(0)], 1)[:, 0],
+    "host": lambda t: t.cpu(),
+    "list": lambda t: t.tolist(),
+}
+
+
+@pytest.mark.parametrize("form", sorted(_SEQ_FORMS))
+@pytest.mark.parametrize("whole_model", [False, True])
+def test_cached_step_takes_the_sequence_ids_of_an_indexed_store(form, whole_model):
+    """Sequence ids of another integer type, stride or device than the kernel's own: the same result and the same cache, bit for bit."""
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _DecodeMeta
+    from axolotl_b200.models.transformer import CausalLM
+
+    torch.manual_seed(1)
+    m = CausalLM(preset("tiny-llama", vocab_size=512, num_hidden_layers=1), dtype=torch.bfloat16, device="cuda").init_weights(0).eval()
+    a = m.layers[0].self_attn
+    ids = torch.tensor([3, 0, 4, 1], device="cuda")
+    pos = torch.tensor([7, 0, 39, 12], device="cuda")
+    qkv = torch.randn(4, (a.Hq + 2 * a.Hk) * a.D, device="cuda").bfloat16()
+    kv = torch.randn(2, 1, 5, 40, a.Hk * a.D, device="cuda").bfloat16()
+    got = []
+    for seq in (ids, _SEQ_FORMS[form](ids)):
+        cache = KVCache(m, 5, 40)
+        cache.k.copy_(kv[0])
+        cache.v.copy_(kv[1])
+        meta = _DecodeMeta(cache, seq, pos, False)
+        with torch.no_grad():
+            if whole_model:    # a step of another form than the one-call layers take runs operator by operator: a rounding apart
+                out = m(torch.arange(4, device="cuda")[None], pos.int()[None], attn_meta=meta, return_logits=False).hidden_states
+            else:
+                out = cache.attend(0, qkv, meta, a.Hq, a.Hk, a.D, a.scale)
+        got.append((out, cache.k, cache.v))
+    for x, y in zip(*got):
+        assert torch.equal(x, y) if not whole_model else ((x.float() - y.float()).norm() <= 0.012 * y.float().norm())
+
+
+@pytest.mark.parametrize("bad", [torch.zeros(4), torch.zeros(3, dtype=torch.long), torch.zeros(4, 1, dtype=torch.long)])
+def test_cached_step_refuses_other_sequence_ids(bad):
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _DecodeMeta
+    from axolotl_b200.models.transformer import CausalLM
+
+    m = CausalLM(preset("tiny-llama", num_hidden_layers=1), dtype=torch.bfloat16, device="cuda")
+    a, cache = m.layers[0].self_attn, KVCache(m, 5, 40)
+    qkv = torch.zeros(4, (a.Hq + 2 * a.Hk) * a.D, device="cuda").bfloat16()
+    with pytest.raises(IndexError):
+        cache.attend(0, qkv, _DecodeMeta(cache, bad.cuda(), torch.arange(4, device="cuda"), False), a.Hq, a.Hk, a.D, a.scale)
+
+
 @pytest.mark.parametrize("R,N,K,K2", [(128, 1, 64, 0), (200, 5, 72, 16), (1000, 17, 520, 48), (6144, 64, 4096, 0), (129, 100, 640, 8),
                                       (384, 256, 1032, 64)])
 @pytest.mark.parametrize("splits", [0, 1, 3, 8])
