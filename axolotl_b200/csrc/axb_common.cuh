@@ -22,6 +22,7 @@ enum AxbStatus : int {
   AXB_TIMEOUT_PEER_FLAG = 5,  // a flag written by another GPU / CTA never arrived
   AXB_BAD_ARGUMENT = 6,
   AXB_TIMEOUT_GENERIC = 7,
+  AXB_BAD_INDEX = 8,  // an index read from device memory was out of range (the access was skipped)
 };
 
 // Bounds-check build (-DAXB_BOUNDS_CHECK, linked as libaxb200_checked.so): every data-dependent index that a
@@ -37,6 +38,8 @@ enum AxbBoundsSite : int {
   AXB_SITE_W4A16_EXPERT = 5,
   AXB_SITE_ATTN_TILE = 6,
   AXB_SITE_DISPATCH_TOKEN = 7,
+  AXB_SITE_CACHE_ROW = 8,
+  AXB_SITE_CACHE_POS = 9,
 };
 #ifdef AXB_BOUNDS_CHECK
 extern __device__ unsigned long long axb_bounds_record[4];   // site, index, limit, count (bounds_check.cu)
@@ -53,6 +56,16 @@ AXB_DEVICE bool axb_index_ok(int site, long long idx, long long limit) {
 #else
 #define AXB_INDEX_OK(site, idx, limit) true
 #endif
+// For indexes of STORES, which would overwrite other data: checked in every build. An index out of range is reported (once per
+// caller that asks for it) through the status word and, in the bounds-check build, the record above; the caller skips the access.
+AXB_DEVICE bool axb_index_checked(int site, long long idx, long long limit, bool report, int* status) {
+  if (idx >= 0 && idx < limit) return true;
+  if (report) {
+    (void)AXB_INDEX_OK(site, idx, limit);
+    if (status) atomicCAS(status, AXB_OK, AXB_BAD_INDEX);
+  }
+  return false;
+}
 
 // wait budget in nanoseconds of %globaltimer (2 s: far above any legitimate wait)
 #ifndef AXB_WAIT_BUDGET_NS

@@ -14,7 +14,8 @@
 //
 // Optional, for a generation step: the kernel rotates q and the new k itself (rotary embedding, `inv_freq` != null) and
 // appends the new k / v row to the cache (`append`). Only cluster rank 0 stores the row; the warp whose tile holds the
-// new position takes it from shared memory, so no CTA waits for another one's store.
+// new position takes it from shared memory, so no CTA waits for another one's store. Row and position are compared with the
+// cache's: a sequence outside it gets zeros, stores nothing and is reported through the status word.
 //
 // Generation in the reference goes through Hugging Face `generate` with its KV cache and SDPA /
 // flash-attn decode kernels (src/axolotl/cli/inference.py, core/trainers/grpo rollouts).
@@ -42,10 +43,11 @@ struct DecodeParams {
   __nv_bfloat16* out;
   long long out_ld;
   int Hq, Hk;
-  long long max_len;
+  long long max_len, rows;          // positions per cache row, cache rows
   float scale;
   int window;
   int append;
+  int* status;
 };
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
@@ -106,11 +108,18 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
   const int kvh = blockIdx.y, b = blockIdx.z;
   const int rank = (int)cluster_ctarank(), nsplit = (int)cluster_nctarank();
   const int G = p.Hq / p.Hk;
-  const int n = p.lens[b];
+  int n = p.lens[b];
+  long long crow = p.seq ? p.seq[b] : (long long)b, at = n - 1;      // cache row, position of the new token
+  if (crow < 0) crow += p.rows;                            // counted from the end, as an indexed store does
+  if (at < 0 && p.append) at += p.max_len;
+  if (!axb_index_checked(AXB_SITE_CACHE_ROW, crow, p.rows, tid == 0 && kvh == 0 && rank == 0, p.status) ||
+      !axb_index_checked(AXB_SITE_CACHE_POS, max(at, p.append ? at : 0ll), p.max_len, tid == 0 && kvh == 0 && rank == 0, p.status)) {
+    n = 0;                                                 // nothing is read or stored, the result is zero
+    at = -1;
+  }
   const int first = p.window > 0 ? max(0, n - p.window) : 0;
   const int n_load = p.append ? n - 1 : n;                 // the appended row comes from shared memory
   const long long row_elems = (long long)p.Hk * D;
-  const long long crow = p.seq ? p.seq[b] : (long long)b;
   __nv_bfloat16* kb = p.kc + crow * p.max_len * row_elems + (long long)kvh * D;
   __nv_bfloat16* vb = p.vc + crow * p.max_len * row_elems + (long long)kvh * D;
   const int tiles = n > first ? (n - first + DEC_P - 1) / DEC_P : 0;
@@ -180,10 +189,10 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
   if (p.append)
     for (int j = tid; j < D; j += DEC_T) reinterpret_cast<__nv_bfloat16*>(sNew)[D + j] = qrow[p.v_col0 + kvh * D + j];
   __syncthreads();
-  if (p.append && rank == 0 && n > 0) {
+  if (p.append && rank == 0 && at >= 0) {
     for (int j = tid; j < D; j += DEC_T) {
-      kb[(long long)(n - 1) * row_elems + j] = reinterpret_cast<const __nv_bfloat16*>(sNew)[j];
-      vb[(long long)(n - 1) * row_elems + j] = reinterpret_cast<const __nv_bfloat16*>(sNew)[D + j];
+      kb[at * row_elems + j] = reinterpret_cast<const __nv_bfloat16*>(sNew)[j];
+      vb[at * row_elems + j] = reinterpret_cast<const __nv_bfloat16*>(sNew)[D + j];
     }
   }
 
@@ -401,16 +410,16 @@ extern "C" int axb_kv_append(const void* qkv, long long ld, int k_col0, int v_co
 }
 
 // qkv: [B, ld] fused projection of the new tokens (q block at column q_col0; rotated already unless inv_freq is given);
-// k_cache / v_cache: [*, max_len, Hk*D], 16-byte aligned; row b uses cache row seq[b] (seq == null: row b);
+// k_cache / v_cache: [rows, max_len, Hk*D], 16-byte aligned; row b uses cache row seq[b] (seq == null: row b);
 // lens[b]: live positions of sequence b including the new token; out: [B, out_ld >= Hq*D].
 // append: the new token's k / v (columns k_col0 / v_col0 of qkv) are stored at position lens[b] - 1 and attended to;
 // otherwise that position is read from the cache. inv_freq [D/2] + pos [B]: q (and the appended k) are rotated here.
 // splits: 0 = chosen by pick_splits. pdl: the launch may overlap the end of its predecessor on the stream, which must not
-// write the caches or lens.
-extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
-                               const long long* seq, const int* lens, const int* pos, const float* inv_freq, float attn_scale,
-                               void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len, float scale,
-                               int window, int append, int splits, int pdl, void* stream) {
+// write the caches or lens. A cache row outside [-rows, rows) or a length above max_len sets *status (null: not reported).
+extern "C" int axb_cache_attend(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
+                                long long rows, const long long* seq, const int* lens, const int* pos, const float* inv_freq,
+                                float attn_scale, void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len,
+                                float scale, int window, int append, int splits, int pdl, int* status, void* stream) {
   if (B <= 0) return 0;
   if (Hk <= 0 || Hq % Hk || Hq / Hk > MAX_G || B > 65535) return -2;
   if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -3;
@@ -433,13 +442,24 @@ extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_
   p.Hq = Hq;
   p.Hk = Hk;
   p.max_len = max_len;
+  p.rows = rows;
   p.scale = scale;
   p.window = window;
   p.append = append;
+  p.status = status;
   if (splits == 0) splits = pick_splits(B, Hk, max_len);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (D == 64) return launch_decode<64>(p, B, splits, pdl != 0, st);
   if (D == 128) return launch_decode<128>(p, B, splits, pdl != 0, st);
   if (D == 256) return launch_decode<256>(p, B, splits, pdl != 0, st);
   return -2;
+}
+
+// The same for a cache of B rows.
+extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
+                               const long long* seq, const int* lens, const int* pos, const float* inv_freq, float attn_scale,
+                               void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len, float scale,
+                               int window, int append, int splits, int pdl, void* stream) {
+  return axb_cache_attend(qkv, ld, q_col0, k_col0, v_col0, k_cache, v_cache, B, seq, lens, pos, inv_freq, attn_scale, out, out_ld, B,
+                          Hq, Hk, D, max_len, scale, window, append, splits, pdl, nullptr, stream);
 }

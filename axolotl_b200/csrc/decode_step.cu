@@ -14,10 +14,10 @@ extern "C" int axb_gemm_skinny(const void* P, long long ldp, const void* S, long
                                int K, const void* P2, long long ldp2, const void* S2, long long lds2, int K2, float alpha,
                                const void* bias, int out_mode, int out_f32, int glu_kind, float glu_limit, int p_dep, int splits,
                                int pdl, int* status, void* stream);
-extern "C" int axb_decode_attn(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
-                               const long long* seq, const int* lens, const int* pos, const float* inv_freq, float attn_scale,
-                               void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len, float scale,
-                               int window, int append, int splits, int pdl, void* stream);
+extern "C" int axb_cache_attend(const void* qkv, long long ld, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
+                                long long rows, const long long* seq, const int* lens, const int* pos, const float* inv_freq,
+                                float attn_scale, void* out, long long out_ld, int B, int Hq, int Hk, int D, long long max_len,
+                                float scale, int window, int append, int splits, int pdl, int* status, void* stream);
 extern "C" int axb_rope_qk(void* qkv, const int* pos, const float* inv_freq, int T, int Hq, int Hk, int D, long long row_stride,
                            float sign, float attn_scale, const void* qn_w, const void* kn_w, float* rstd_out, float eps,
                            void* stream);
@@ -57,7 +57,7 @@ struct AxbDecodeLayer {
   const int* lens;
   const int* pos;
   const float* inv_freq;
-  long long max_len;
+  long long max_len, rows; // of the cache: positions per row, rows
   int B, Hq, Hk, D, window, glu_kind, chained, pad;
   float eps1, off1, eps2, off2, attn_scale, scale, norm_eps, glu_limit;
   int* status;
@@ -94,9 +94,9 @@ extern "C" int axb_decode_layer(const AxbDecodeLayer* l, void* stream) {
     rc = axb_rope_qk(l->qkv_buf, l->pos, l->inv_freq, B, l->Hq, l->Hk, l->D, W, 1.f, l->attn_scale, l->q_norm, l->k_norm, nullptr,
                      l->norm_eps, stream);
   if (!rc)
-    rc = axb_decode_attn(l->qkv_buf, W, 0, nq, nq + nk, l->k_cache, l->v_cache, l->seq, l->lens, l->pos,
-                         qk_norm ? nullptr : l->inv_freq, l->attn_scale, l->att, nq, B, l->Hq, l->Hk, l->D, l->max_len, l->scale,
-                         l->window, 1, 0, qk_norm ? 0 : 1, stream);
+    rc = axb_cache_attend(l->qkv_buf, W, 0, nq, nq + nk, l->k_cache, l->v_cache, l->rows, l->seq, l->lens, l->pos,
+                          qk_norm ? nullptr : l->inv_freq, l->attn_scale, l->att, nq, B, l->Hq, l->Hk, l->D, l->max_len, l->scale,
+                          l->window, 1, 0, qk_norm ? 0 : 1, l->status, stream);
   if (!rc) rc = project(l->o, l->att, l->y, B, l->low, false, 0, 0.f, l->status, stream);
   if (!rc) rc = axb_rmsnorm_fwd_pdl(l->y, mid, l->norm2, l->xn, l->res_out, B, H, l->eps2, l->off2, stream);
   const int I = l->gate_up.N / 2;

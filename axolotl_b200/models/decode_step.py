@@ -27,7 +27,7 @@ class _Layer(C.Structure):
     _fields_ = ([(n, _Proj) for n in ("qkv", "o", "gate_up", "down")]
                 + [(n, _vp) for n in ("norm1", "norm2", "q_norm", "k_norm", "x", "res_in", "res_mid", "res_out", "y", "xn", "qkv_buf",
                                       "att", "gu", "act", "low", "k_cache", "v_cache", "seq", "lens", "pos", "inv_freq")]
-                + [("max_len", _i64)]
+                + [(n, _i64) for n in ("max_len", "rows")]
                 + [(n, _i32) for n in ("B", "Hq", "Hk", "D", "window", "glu_kind", "chained", "pad")]
                 + [(n, _f32) for n in ("eps1", "off1", "eps2", "off2", "attn_scale", "scale", "norm_eps", "glu_limit")]
                 + [("status", _vp)])
@@ -137,7 +137,7 @@ class DecodeStep:
         self.k_ptr, self.v_ptr, self.layer_bytes = c.k.data_ptr(), c.v.data_ptr(), c.k.stride(0) * 2
         s = self.s = _Layer()
         s.pos, s.seq, s.lens = (t.data_ptr() for t in self.keep)
-        s.B, s.max_len, s.status = self.B, c.max_len, _lib.status_word(h.device).data_ptr()
+        s.B, s.rows, s.max_len, s.status = self.B, c.k.shape[1], c.k.shape[2], _lib.status_word(h.device).data_ptr()
         s.y, s.res_out = self.y.data_ptr(), self.res.data_ptr()
         self.adapters = adapters_enabled()
         self.sized = None

@@ -163,6 +163,8 @@ def generate_cached(model, prompts, max_new_tokens, temperature=0.0, top_p=1.0, 
         logits = Fn_linear(out.hidden_states.reshape(B, -1), model.output_weight())
         cur_len = torch.where(done, cur_len, cur_len + 1)
     model.train(was_training)
+    if dev.type == "cuda":
+        _lib.check_status(dev)                           # a cache row or position out of range, a wait that ran out
     return outs[:n_real]
 
 

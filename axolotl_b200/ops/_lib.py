@@ -86,9 +86,11 @@ _CUDA_SIGS = {
     "axb_rmsnorm_gated_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp],
     "axb_entropy": [vp, vp, vp, i64, i32, i64, f32, vp],
     # qkv, ld, q_col0, k_col0, v_col0, k_cache, v_cache, seq, lens, pos, inv_freq, attn_scale, out, out_ld, B, Hq, Hk, D,
-    # max_len, scale, window, append, splits, pdl, stream
+    # max_len, scale, window, append, splits, pdl, stream; axb_cache_attend: rows behind the caches, status before the stream
     "axb_decode_attn": [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, f32, vp, i64, i32, i32, i32, i32, i64, f32, i32, i32,
                         i32, i32, vp],
+    "axb_cache_attend": [vp, i64, i32, i32, i32, vp, vp, i64, vp, vp, vp, vp, f32, vp, i64, i32, i32, i32, i32, i64, f32, i32, i32,
+                         i32, i32, vp, vp],
     # P, ldp, S, lds, C, ldc, R, N, K, P2, ldp2, S2, lds2, K2, alpha, bias, out_mode, out_f32, glu_kind, glu_limit, p_dep,
     # splits, pdl, status, stream
     "axb_kv_append": [vp, i64, i32, i32, vp, vp, vp, vp, i32, i32, i64, i64, vp],
@@ -184,7 +186,7 @@ _status = {}
 
 
 def status_word(device=None) -> torch.Tensor:
-    """Per-device int32 word that kernels set when a bounded wait ran out."""
+    """Per-device int32 word that kernels set when a bounded wait ran out or a store's index was out of range."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     t = _status.get(key)
@@ -202,6 +204,7 @@ _STATUS_NAMES = {
     5: "peer flag never arrived",
     6: "bad argument",
     7: "generic wait timeout",
+    8: "index out of range (the access was skipped)",
 }
 
 
@@ -210,12 +213,13 @@ class KernelTimeoutError(RuntimeError):
 
 
 def check_status(device=None) -> None:
-    """Synchronising read of the status word; raises when a kernel recorded a timeout."""
+    """Synchronising read of the status word; raises when a kernel recorded a timeout or skipped an access."""
     t = status_word(device)
     code = int(t.item())
     if code != 0:
         t.zero_()
-        raise KernelTimeoutError(f"axolotl_b200 kernel reported status {code}: {_STATUS_NAMES.get(code, '?')}")
+        kind = KernelBoundsError if code == 8 else KernelTimeoutError
+        raise kind(f"axolotl_b200 kernel reported status {code}: {_STATUS_NAMES.get(code, '?')}")
 
 
 class KernelBoundsError(RuntimeError):
@@ -224,7 +228,7 @@ class KernelBoundsError(RuntimeError):
 
 _BOUNDS_SITES = {1: "embedding token id", 2: "embedding-gradient token id", 3: "cross-entropy label",
                  4: "grouped GEMM expert id", 5: "W4A16 grouped GEMM expert id", 6: "attention document tile",
-                 7: "MoE dispatch token index"}
+                 7: "MoE dispatch token index", 8: "KV cache row", 9: "KV cache position"}
 
 
 def bounds_violation():

@@ -745,17 +745,18 @@ def flash_varlen(qkv, meta: AttnMeta, Hq, Hk, D, scale=None, Dv=None, softcap=0.
 def _decode_launch(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window, append, pos=None, inv_freq=None, attn_scale=1.0):
     B = qkv.shape[0]
     out = torch.empty((B, Hq * D), dtype=qkv.dtype, device=qkv.device)
-    _lib.check_rc(_lib.cuda_lib().axb_decode_attn(
-        qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, k_cache.data_ptr(), v_cache.data_ptr(), _lib.ptr(seq),
+    _lib.check_rc(_lib.cuda_lib().axb_cache_attend(
+        qkv.data_ptr(), qkv.stride(0), 0, Hq * D, (Hq + Hk) * D, k_cache.data_ptr(), v_cache.data_ptr(), k_cache.shape[0], _lib.ptr(seq),
         lens.data_ptr(), _lib.ptr(pos), _lib.ptr(inv_freq), attn_scale, out.data_ptr(), out.stride(0), B, Hq, Hk, D,
-        k_cache.shape[1], scale, int(window or 0), int(append), 0, 0, _lib.stream_ptr()), "decode_attn")
+        k_cache.shape[1], scale, int(window or 0), int(append), 0, 0, _lib.status_word(qkv.device).data_ptr(), _lib.stream_ptr()), "decode_attn")
     return out
 
 
 @torch.no_grad()
 def decode_attention_append(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window=0):
     """``decode_attention`` that also stores the new token's k / v (taken from ``qkv``) at position ``lens[b] - 1`` of
-    cache row ``seq[b]`` (int64 on the device), in the same launch. CUDA only."""
+    cache row ``seq[b]`` (int64 on the device), in the same launch. A row or position outside the cache stores nothing, gives
+    zeros and is reported by ``_lib.check_status``. CUDA only."""
     return _decode_launch(qkv, k_cache, v_cache, seq, lens, Hq, Hk, D, scale, window, append=True)
 
 

@@ -146,6 +146,52 @@ def test_cached_step_refuses_other_sequence_ids(bad):
         cache.attend(0, qkv, _DecodeMeta(cache, bad.cuda(), torch.arange(4, device="cuda"), False), a.Hq, a.Hk, a.D, a.scale)
 
 
+def _in_checked_library(test):
+    """Runs a test of this file again with the bounds-check library."""
+    import os
+    import subprocess
+    import sys
+
+    if os.environ.get("AXB_BOUNDS_CHECK") != "1":
+        r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-p", "no:cacheprovider", f"{__file__}::{test}"],
+                           env=dict(os.environ, AXB_BOUNDS_CHECK="1"), capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stdout[-3000:]
+
+
+def test_cached_step_outside_the_cache_stores_nothing():
+    """Positions and rows at and past the cache's ends: only the rows inside are stored (negative ones count from the end, as
+    an indexed store has it), the others give zeros, their neighbours stay as they are, and the status word tells."""
+    from axolotl_b200.ops import _lib
+
+    torch.manual_seed(2)
+    B, cap, Hq, Hk, D = 4, 20, 8, 2, 64
+    big = torch.randn(2, B + 4, cap, Hk * D, device="cuda").bfloat16()      # cache rows 0..3 with two rows around them
+    k, v = big[0, 2:2 + B], big[1, 2:2 + B]
+    seq = torch.tensor([0, 3, -1, 4, -5, 1, 2, 2], device="cuda")
+    pos = torch.tensor([cap, 19, 5, 3, 3, 2 ** 30, -1, -cap - 1], device="cuda")
+    good = {1: (3, 19), 2: (3, 5), 6: (2, 19)}
+    qkv = torch.randn(8, (Hq + 2 * Hk) * D, device="cuda").bfloat16()
+    want = big.clone()
+    for i, (r, p) in good.items():
+        want[0, 2 + r, p], want[1, 2 + r, p] = qkv[i, Hq * D:(Hq + Hk) * D], qkv[i, (Hq + Hk) * D:]
+    out = Fn.decode_attention_append(qkv, k, v, seq, (pos + 1).int(), Hq, Hk, D, D ** -0.5)
+    if _lib.cuda_lib().axb_bounds_check_enabled():
+        v0 = _lib.bounds_violation()
+        assert v0 is not None and v0[0] in ("KV cache row", "KV cache position") and v0[3] == 5, v0
+    with pytest.raises(_lib.KernelBoundsError):
+        _lib.check_status()
+    _lib.check_status()
+    assert torch.equal(big, want)
+    for i in range(8):
+        if i not in (1, 2):
+            assert not out[i].any()
+    i = 2
+    ref = _reference(qkv[i, :Hq * D].view(Hk, Hq // Hk, D), want[0, 5].view(cap, Hk, D), want[1, 5].view(cap, Hk, D), D ** -0.5, 0, 6)
+    assert (out[i].float() - ref).abs().max() <= 2 ** -8 * max(1.0, ref.abs().max().item())
+    assert out[1].any()
+    _in_checked_library("test_cached_step_outside_the_cache_stores_nothing")
+
+
 @pytest.mark.parametrize("R,N,K,K2", [(128, 1, 64, 0), (200, 5, 72, 16), (1000, 17, 520, 48), (6144, 64, 4096, 0), (129, 100, 640, 8),
                                       (384, 256, 1032, 64)])
 @pytest.mark.parametrize("splits", [0, 1, 3, 8])
