@@ -383,13 +383,17 @@ int pick_splits(int B, int Hk, long long max_len) {
 __global__ void __launch_bounds__(256) kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, long long ld, int k_col0, int v_col0,
                                                         __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
                                                         const long long* __restrict__ seq, const long long* __restrict__ pos, int T,
-                                                        int width, long long rows, long long max_len) {
+                                                        int width, long long rows, long long max_len, int* status) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long t = w >> 1;
   if (t >= T) return;
-  const long long b = seq[t], i = pos[t];
-  if (b < 0 || b >= rows || i < 0 || i >= max_len) return;
+  long long b = seq[t], i = pos[t];
+  if (b < 0) b += rows;                        // counted from the end, as an indexed store does
+  if (i < 0) i += max_len;
+  const bool report = lane == 0 && !(w & 1);
+  if (!axb_index_checked(AXB_SITE_CACHE_ROW, b, rows, report, status) || !axb_index_checked(AXB_SITE_CACHE_POS, i, max_len, report, status))
+    return;
   const __nv_bfloat16* src = qkv + t * ld + ((w & 1) ? v_col0 : k_col0);
   __nv_bfloat16* dst = ((w & 1) ? vc : kc) + (b * max_len + i) * width;
 #pragma unroll 4
@@ -398,15 +402,22 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const __nv_bfloat16* __r
 
 }  // namespace
 
-// k_cache / v_cache [rows, max_len, width]; all rows 16-byte aligned, width a multiple of 8
-extern "C" int axb_kv_append(const void* qkv, long long ld, int k_col0, int v_col0, void* k_cache, void* v_cache, const long long* seq,
-                             const long long* pos, int T, int width, long long rows, long long max_len, void* stream) {
+// k_cache / v_cache [rows, max_len, width]; all rows 16-byte aligned, width a multiple of 8. A row outside [-rows, rows) or a
+// position outside [-max_len, max_len) is not stored and sets *status (null: not reported).
+extern "C" int axb_cache_append(const void* qkv, long long ld, int k_col0, int v_col0, void* k_cache, void* v_cache,
+                                const long long* seq, const long long* pos, int T, int width, long long rows, long long max_len,
+                                int* status, void* stream) {
   if (T <= 0) return 0;
   if ((ld & 7) || (k_col0 & 7) || (v_col0 & 7) || (width & 7)) return -2;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -3;
   kv_append_kernel<<<(unsigned)(((long long)T * 2 + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      (const __nv_bfloat16*)qkv, ld, k_col0, v_col0, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, seq, pos, T, width, rows, max_len);
+      (const __nv_bfloat16*)qkv, ld, k_col0, v_col0, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, seq, pos, T, width, rows, max_len,
+      status);
   return (int)cudaGetLastError();
+}
+extern "C" int axb_kv_append(const void* qkv, long long ld, int k_col0, int v_col0, void* k_cache, void* v_cache, const long long* seq,
+                             const long long* pos, int T, int width, long long rows, long long max_len, void* stream) {
+  return axb_cache_append(qkv, ld, k_col0, v_col0, k_cache, v_cache, seq, pos, T, width, rows, max_len, nullptr, stream);
 }
 
 // qkv: [B, ld] fused projection of the new tokens (q block at column q_col0; rotated already unless inv_freq is given);

@@ -57,13 +57,16 @@ class KVCache:
             return Fn.decode_attention(qkv, self.k[layer, meta.seq], self.v[layer, meta.seq], meta.lens_after,
                                        Hq, Hk, D, scale, window)
         # prefill: packed prompt rows -> (sequence, position)
-        if (qkv.is_cuda and qkv.dtype == self.k.dtype == torch.bfloat16 and self.width % 8 == 0 and qkv.stride(1) == 1
-                and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and meta.seq.dtype == meta.pos.dtype == torch.int64
-                and meta.seq.is_contiguous() and meta.pos.is_contiguous() and meta.seq.shape == meta.pos.shape == qkv.shape[:1]
+        k, v = self.k[layer], self.v[layer]
+        if (qkv.is_cuda and qkv.dtype == k.dtype == v.dtype == torch.bfloat16 and Hk * D == self.width and self.width % 8 == 0
+                and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and (qkv.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
+                and k.is_contiguous() and v.is_contiguous()
+                and all(torch.is_tensor(t) and t.dtype == torch.int64 and t.device == qkv.device and t.is_contiguous()
+                        and t.shape == qkv.shape[:1] for t in (meta.seq, meta.pos))
                 and not (torch.is_grad_enabled() and qkv.requires_grad)):
-            _lib.check_rc(_lib.cuda_lib().axb_kv_append(
-                qkv.data_ptr(), qkv.stride(0), Hq * D, (Hq + Hk) * D, self.k[layer].data_ptr(), self.v[layer].data_ptr(),
-                meta.seq.data_ptr(), meta.pos.data_ptr(), qkv.shape[0], self.width, self.B, self.max_len, _lib.stream_ptr()), "kv_append")
+            _lib.check_rc(_lib.cuda_lib().axb_cache_append(
+                qkv.data_ptr(), qkv.stride(0), Hq * D, (Hq + Hk) * D, k.data_ptr(), v.data_ptr(), meta.seq.data_ptr(), meta.pos.data_ptr(),
+                qkv.shape[0], self.width, k.shape[0], k.shape[1], _lib.status_word(qkv.device).data_ptr(), _lib.stream_ptr()), "kv_append")
         else:
             self.k[layer, meta.seq, meta.pos] = kq
             self.v[layer, meta.seq, meta.pos] = vq

@@ -94,6 +94,7 @@ _CUDA_SIGS = {
     # P, ldp, S, lds, C, ldc, R, N, K, P2, ldp2, S2, lds2, K2, alpha, bias, out_mode, out_f32, glu_kind, glu_limit, p_dep,
     # splits, pdl, status, stream
     "axb_kv_append": [vp, i64, i32, i32, vp, vp, vp, vp, i32, i32, i64, i64, vp],
+    "axb_cache_append": [vp, i64, i32, i32, vp, vp, vp, vp, i32, i32, i64, i64, vp, vp],
     "axb_gemm_skinny": [vp, i64, vp, i64, vp, i64, i32, i32, i32, vp, i64, vp, i64, i32, f32, vp, i32, i32, i32, f32, i32, i32,
                         i32, vp, vp],
     "axb_sinkgd_step": [vp, i32, vp, vp, vp, i32, i32, i32, f32, f32, f32, vp],

@@ -372,3 +372,46 @@ def test_prompt_rows_go_to_their_cache_slots(width):
                                                 pos.data_ptr(), T, width, B, cap, _lib.stream_ptr()), "kv_append")
     k0[seq, pos], v0[seq, pos] = qkv[:, width:2 * width], qkv[:, 2 * width:3 * width]
     assert torch.equal(kc, k0) and torch.equal(vc, v0)
+
+
+@pytest.mark.parametrize("form", ["int64", "int32", "host", "list"])
+def test_prompt_rows_take_the_indexes_of_an_indexed_store(form):
+    """Sequence ids and positions of any integer form, negative ones counted from the end; rows of an odd stride."""
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _PrefillMeta
+    from axolotl_b200.models.transformer import CausalLM
+
+    m = CausalLM(preset("tiny-llama", num_hidden_layers=1), dtype=torch.bfloat16, device="cuda")
+    a, cache = m.layers[0].self_attn, KVCache(m, 5, 40)
+    T, nq, nk = 24, a.Hq * a.D, a.Hk * a.D
+    qkv = torch.randn(T, nq + 2 * nk, device="cuda").bfloat16()
+    slots = torch.randperm(200, device="cuda")[:T]
+    seq, pos = slots // 40 - 5 * (slots % 2), slots % 40 - 40 * (slots % 3 == 0)
+    k0, v0 = cache.k.clone(), cache.v.clone()
+    k0[0, seq, pos], v0[0, seq, pos] = qkv[:, nq:nq + nk], qkv[:, nq + nk:]
+    f = {"int64": lambda t: t, "int32": lambda t: t.int(), "host": lambda t: t.cpu(), "list": lambda t: t.tolist()}[form]
+    cache.attend(0, qkv, _PrefillMeta(cache, Fn.AttnMeta([0, T], "cuda"), f(seq), f(pos)), a.Hq, a.Hk, a.D, a.scale)
+    assert torch.equal(cache.k, k0) and torch.equal(cache.v, v0)
+
+
+def test_prompt_rows_outside_the_cache_are_not_stored():
+    from axolotl_b200.ops import _lib
+
+    T, B, cap, width = 6, 4, 20, 64
+    qkv = torch.randn(T, 3 * width, device="cuda").bfloat16()
+    big = torch.randn(2, B + 4, cap, width, device="cuda").bfloat16()
+    k, v = big[0, 2:2 + B], big[1, 2:2 + B]
+    seq = torch.tensor([0, B, -B - 1, 1, 2, 3], device="cuda")
+    pos = torch.tensor([cap, 3, 3, -cap - 1, 2 ** 40, 7], device="cuda")
+    want = big.clone()
+    want[0, 5, 7], want[1, 5, 7] = qkv[5, width:2 * width], qkv[5, 2 * width:]
+    _lib.check_rc(_lib.cuda_lib().axb_cache_append(
+        qkv.data_ptr(), qkv.stride(0), width, 2 * width, k.data_ptr(), v.data_ptr(), seq.data_ptr(), pos.data_ptr(), T, width, B, cap,
+        _lib.status_word().data_ptr(), _lib.stream_ptr()), "kv_append")
+    if _lib.cuda_lib().axb_bounds_check_enabled():
+        v0 = _lib.bounds_violation()
+        assert v0 is not None and v0[0] in ("KV cache row", "KV cache position") and v0[3] == 5, v0
+    with pytest.raises(_lib.KernelBoundsError):
+        _lib.check_status()
+    assert torch.equal(big, want)
+    _in_checked_library("test_prompt_rows_outside_the_cache_are_not_stored")
