@@ -40,6 +40,7 @@ enum AxbBoundsSite : int {
   AXB_SITE_DISPATCH_TOKEN = 7,
   AXB_SITE_CACHE_ROW = 8,
   AXB_SITE_CACHE_POS = 9,
+  AXB_SITE_ROUTE_EXPERT = 10,
 };
 #ifdef AXB_BOUNDS_CHECK
 extern __device__ unsigned long long axb_bounds_record[4];   // site, index, limit, count (bounds_check.cu)

@@ -159,14 +159,15 @@ __global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__
 }
 
 __global__ void __launch_bounds__(RL_T) route_scatter_kernel(const long long* __restrict__ expert, const int* __restrict__ base,
-                                                             int* __restrict__ slot_row, int* __restrict__ row_slot, int n, int E) {
+                                                             int* __restrict__ slot_row, int* __restrict__ row_slot, int n, int E,
+                                                             int* status) {
   extern __shared__ unsigned short c[];   // [32 warps][E]: slots of the expert in the warps before
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < 32 * E; i += RL_T) c[i] = 0;
   __syncthreads();
   const int i = blockIdx.x * RL_T + threadIdx.x;
   const long long e64 = i < n ? expert[i] : -1;
-  const int e = e64 >= 0 && e64 < E ? (int)e64 : -1;
+  const int e = i < n && axb_index_checked(AXB_SITE_ROUTE_EXPERT, e64, E, true, status) ? (int)e64 : -1;
   const unsigned same = __match_any_sync(0xffffffffu, e);
   const int rank = __popc(same & ((1u << lane) - 1u));
   if (e >= 0 && rank == 0) c[warp * E + e] = (unsigned short)__popc(same);
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(RL_T) route_scatter_kernel(const long long* __
     slot_row[i] = row;
     row_slot[row] = i;
   } else if (i < n) {
-    slot_row[i] = 0;
+    slot_row[i] = -1;             // no such expert: combined as zero
   }
 }
 
@@ -234,8 +235,8 @@ __global__ void moe_dispatch_rows_kernel(const __nv_bfloat16* __restrict__ x, co
   }
 }
 
-// Local combine: out[t, :] = sum_j w[t, j] * ys[slot_row[t, j], :] (fp32 accumulation in slot order, no atomics). One warp per
-// (token, 256 columns); the rows of eight slots are requested together (a warp per token with one load at a time took 30 us
+// Local combine: out[t, :] = sum_j w[t, j] * ys[slot_row[t, j], :] (fp32 accumulation in slot order, no atomics; a slot
+// without a row, -1, is zero). One warp per (token, 256 columns); the rows of eight slots are requested together (a warp per token with one load at a time took 30 us
 // for 333 tokens).
 __global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ slot_row,
                                         const float* __restrict__ w, __nv_bfloat16* __restrict__ out,
@@ -250,13 +251,13 @@ __global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ ys, co
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j0 = 0; j0 < k; j0 += 8) {
       const int mine = j0 + (lane & 7);
-      const int my_row = mine < k ? slot_row[t * k + mine] : 0;
-      const float my_w = mine < k ? (w ? w[t * k + mine] : 1.f) : 0.f;
+      const int my_row = mine < k ? slot_row[t * k + mine] : -1;
+      const float my_w = my_row >= 0 ? (w ? w[t * k + mine] : 1.f) : 0.f;
       uint4 v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int r = __shfl_sync(0xffffffffu, my_row, j);
-        v[j] = in_row && j0 + j < k ? *reinterpret_cast<const uint4*>(ys + (long long)r * width + c) : make_uint4(0, 0, 0, 0);
+        v[j] = in_row && r >= 0 ? *reinterpret_cast<const uint4*>(ys + (long long)r * width + c) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -288,7 +289,8 @@ __global__ void moe_combine_dw_kernel(const __nv_bfloat16* __restrict__ dy, cons
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long sl = wid; sl < n_slots; sl += n_warps) {
     const __nv_bfloat16* a = dy + (sl / k) * width;
-    const __nv_bfloat16* b = ys + (long long)slot_row[sl] * width;
+    const int row = slot_row[sl];                 // -1: no row, the gradient is zero
+    const __nv_bfloat16* b = ys + (long long)row * width;
     float acc = 0.f;
     for (int c0 = lane * 8; c0 < width; c0 += 8 * 256) {
       uint4 va[8], vb[8];
@@ -296,7 +298,7 @@ __global__ void moe_combine_dw_kernel(const __nv_bfloat16* __restrict__ dy, cons
       for (int q = 0; q < 8; ++q) {
         const int c = c0 + q * 256;
         va[q] = vb[q] = make_uint4(0, 0, 0, 0);
-        if (c < width) {
+        if (c < width && row >= 0) {
           va[q] = *reinterpret_cast<const uint4*>(a + c);
           vb[q] = *reinterpret_cast<const uint4*>(b + c);
         }
@@ -578,9 +580,10 @@ static int rows_grid(long long n_rows) {
 
 // Layout of a routed batch. expert [n] (n = T * k slots, expert ids), E <= 1024; slot_row [n], row_slot [max_blocks * 128] (slot of
 // a padded row, -1 = pad), seg_start / seg_rows [E], blk_expert [max_blocks], n_blocks [1]; scratch: ceil(n / 1024) * E ints.
-// max_blocks >= ceil(n / 128) + E.
+// max_blocks >= ceil(n / 128) + E. A slot with an expert outside [0, E) has no row (slot_row -1) and sets *status.
 extern "C" int axb_moe_route_layout(const long long* expert, int n, int E, int max_blocks, int* slot_row, int* row_slot,
-                                    int* seg_start, int* seg_rows, int* blk_expert, int* n_blocks, int* scratch, void* stream) {
+                                    int* seg_start, int* seg_rows, int* blk_expert, int* n_blocks, int* scratch, int* status,
+                                    void* stream) {
   if (E < 1 || E > RL_MAX_E || n < 0 || max_blocks < (n + 127) / 128 + E) return -2;
   cudaError_t e = cudaMemsetAsync(row_slot, 0xff, (size_t)max_blocks * 128 * sizeof(int), ST(stream));
   if (e != cudaSuccess) return (int)e;
@@ -593,7 +596,7 @@ extern "C" int axb_moe_route_layout(const long long* expert, int n, int E, int m
       static std::atomic<unsigned long long> allowed{0};
       if (const int rc = axb_allow_smem((const void*)route_scatter_kernel, 64 * 1024, allowed)) return rc;
     }
-    route_scatter_kernel<<<blocks, RL_T, smem, ST(stream)>>>(expert, scratch, slot_row, row_slot, n, E);
+    route_scatter_kernel<<<blocks, RL_T, smem, ST(stream)>>>(expert, scratch, slot_row, row_slot, n, E, status);
   }
   return (int)cudaGetLastError();
 }

@@ -34,8 +34,8 @@ _CUDA_SIGS = {
     "axb_gemm_set_pair_tuning": [i32, i32, i32],
     "axb_nvfp4_dequant": [vp, vp, vp, vp, i64, i64, vp],
     "axb_moe_dispatch_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
-    # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, scratch, stream
-    "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp],
+    # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, scratch, status, stream
+    "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp],
     "axb_moe_combine_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_moe_combine_dw": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_nf4_dequant": [vp, vp, vp, i64, i32, vp],
@@ -229,7 +229,7 @@ class KernelBoundsError(RuntimeError):
 
 _BOUNDS_SITES = {1: "embedding token id", 2: "embedding-gradient token id", 3: "cross-entropy label",
                  4: "grouped GEMM expert id", 5: "W4A16 grouped GEMM expert id", 6: "attention document tile",
-                 7: "MoE dispatch token index", 8: "KV cache row", 9: "KV cache position"}
+                 7: "MoE dispatch token index", 8: "KV cache row", 9: "KV cache position", 10: "MoE routing expert id"}
 
 
 def bounds_violation():

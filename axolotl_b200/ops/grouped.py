@@ -292,7 +292,9 @@ class _GroupedProj(torch.autograd.Function):
 class RoutedLayout(GroupLayout):
     """Layout of a local (single-rank) MoE layer built from the router's top-k choice ``idx`` [T, k] (int64):
     adds the slot <-> padded-row maps used by the dispatch / combine kernels (``row_slot``: slot of a padded row, -1 in
-    pad rows; ``slot_row``: its inverse). Built by three kernels of csrc/moe.cu, without a host round trip."""
+    pad rows; ``slot_row``: its inverse). Built by three kernels of csrc/moe.cu, without a host round trip; a slot whose
+    expert does not exist has no row (``slot_row`` -1), counts as zero in the combination and is reported by
+    ``_lib.check_status``."""
 
     def __init__(self, idx: torch.Tensor, E: int):
         T, k = idx.shape
@@ -320,8 +322,8 @@ class RoutedLayout(GroupLayout):
          scratch) = (buf[a:a + s] for a, s in zip(at, sizes))
         _lib.check_rc(_lib.cuda_lib().axb_moe_route_layout(
             flat_e.data_ptr(), n, E, self.max_blocks, self.slot_row.data_ptr(), self.row_slot.data_ptr(), self.seg_start.data_ptr(),
-            self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), scratch.data_ptr(), _lib.stream_ptr()),
-            "moe_route_layout")
+            self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), scratch.data_ptr(),
+            _lib.status_word(idx.device).data_ptr(), _lib.stream_ptr()), "moe_route_layout")
 
 
 def _dispatch_rows(x, lay, slot_scale):

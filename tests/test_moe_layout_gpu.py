@@ -67,6 +67,37 @@ def test_dispatch_and_combine_rows(T, k, H):
     assert ((dw.double() - prod.sum(-1)).abs() <= 2 ** -18 * prod.abs().sum(-1)).all()
 
 
+def test_slots_of_experts_that_do_not_exist():
+    """They get no row, the others keep theirs; combination and weight gradient take them for zero and the status word tells."""
+    from axolotl_b200.ops.grouped import RoutedLayout, _combine_rows
+
+    torch.manual_seed(0)
+    T, k, E, H = 700, 3, 8, 64
+    idx = torch.randint(0, E, (T, k), device="cuda")
+    clean = RoutedLayout(torch.where(idx == 5, 4, idx), E)      # an expert without rows of its own
+    bad = idx == 5
+    idx = torch.where(bad, torch.tensor([E, -1, 2 ** 40], device="cuda")[torch.arange(k, device="cuda")].expand(T, k), idx)
+    lay = RoutedLayout(idx, E)
+    with pytest.raises(_lib.KernelBoundsError):
+        _lib.check_status()
+    flat = bad.reshape(-1)
+    assert (lay.slot_row[flat] == -1).all() and (lay.slot_row[~flat] >= 0).all()
+    live = lay.row_slot >= 0
+    assert int(live.sum()) == int((~flat).sum())
+    assert torch.equal(lay.slot_row[lay.row_slot[live].long()].long(), live.nonzero().squeeze(1))
+    assert torch.equal(lay.seg_rows[[0, 1, 2, 3, 6, 7]], clean.seg_rows[[0, 1, 2, 3, 6, 7]]) and lay.seg_rows[5] == 0
+    ys, w = torch.randn(lay.max_rows, H, device="cuda").bfloat16(), torch.rand(T, k, device="cuda")
+    rows = ys[lay.slot_row.clamp(min=0).long()].view(T, k, H).double() * (~bad)[..., None]
+    out = _combine_rows(ys, lay.slot_row, w.masked_fill(bad, float("nan")), T, k)
+    ref = (rows * w.double()[..., None]).sum(1)
+    assert ((out.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()
+    dw, dy = torch.empty(T, k, device="cuda"), torch.randn(T, H, device="cuda").bfloat16()
+    _lib.check_rc(_lib.cuda_lib().axb_moe_combine_dw(dy.data_ptr(), ys.data_ptr(), lay.slot_row.data_ptr(), dw.data_ptr(), T * k, k, H,
+                                                     _lib.stream_ptr()), "moe_combine_dw")
+    prod = dy.double()[:, None] * rows
+    assert ((dw.double() - prod.sum(-1)).abs() <= 2 ** -18 * prod.abs().sum(-1)).all()
+
+
 @pytest.mark.parametrize("R,C", [(1, 1), (63, 65), (64, 64), (130, 7), (8, 24576), (4099, 128)])
 def test_transpose_modes(R, C):
     """Tile edges; the bf16 form is one rounding, the fp32 forms are exact."""
