@@ -14,6 +14,7 @@ The segment layout is built on the device: no host synchronisation per layer.
 """
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
@@ -324,6 +325,11 @@ class RoutedLayout(GroupLayout):
             flat_e.data_ptr(), n, E, self.max_blocks, self.slot_row.data_ptr(), self.row_slot.data_ptr(), self.seg_start.data_ptr(),
             self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), scratch.data_ptr(),
             _lib.status_word(idx.device).data_ptr(), _lib.stream_ptr()), "moe_route_layout")
+
+    @functools.cached_property
+    def dest(self):
+        """Padded rows of the slots in expert order: the rows of an expert are ascending in the order of its slots."""
+        return self.slot_row.sort().values.long()
 
 
 def _dispatch_rows(x, lay, slot_scale):

@@ -37,6 +37,20 @@ def test_routed_layout(T, k, E, skew):
     assert torch.equal(lay.blk_expert.long().cpu(), blk)
 
 
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (333, 8, 128), (40, 2, 1500)])
+def test_routed_layout_pads_and_unpads(T, k, E):
+    """The compact form of a routed batch (slots in expert order) through the padded layout and back, exactly."""
+    from axolotl_b200.ops.grouped import RoutedLayout
+
+    idx = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).cuda()
+    lay = RoutedLayout(idx, E)
+    x = torch.randn(T * k, 16, device="cuda").bfloat16()
+    order = torch.argsort(idx.reshape(-1), stable=True)
+    p = lay.pad(x[order])
+    assert torch.equal(lay.unpad(p), x[order]) and torch.equal(p[lay.slot_row.long()], x)
+    assert int((p != 0).any(1).sum()) == T * k
+
+
 @pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 3, 256), (37, 8, 2048), (19, 9, 2056), (3, 16, 264)])
 def test_dispatch_and_combine_rows(T, k, H):
     """Widths around the 256-column chunks and eight vectors in flight, more than eight slots per token. One bf16 rounding of
