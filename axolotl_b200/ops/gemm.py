@@ -169,6 +169,8 @@ def gemm(
         bn = _pick_bn(M, N)
     elif bn is None:
         bn, pair = _pick_tile(M, N)
+    elif not accumulate:
+        pair = _use_pair(M, N, bn)
     if pair:
         rc = lib.axb_gemm_bf16_pair(
             a.data_ptr(), a.stride(0), int(trans_a), b.data_ptr(), b.stride(0), int(trans_b),
@@ -237,7 +239,9 @@ def _use_skinny(M, N, K, trans_a, trans_b, out, out_mode, c_in, beta) -> bool:
 
 
 def _use_pair(M, N, bn) -> bool:
-    return bn == 256 and _pick_tile(M, N)[1]
+    """Whether a tile width that the caller asked for means the CTA-pair kernel (256 x 256 tiles of an SM pair): from 74
+    tiles on, one for every pair. Without a width ``_pick_tile`` decides, for fewer tiles too."""
+    return USE_PAIR and bn == 256 and M >= 512 and N >= 512 and ((M + 255) // 256) * ((N + 255) // 256) >= 74
 
 
 def _pick_bn(M, N) -> int:
@@ -280,9 +284,7 @@ def _gemm_allgather(a, b_shard, info, *, trans_a, trans_b, a2, b2, alpha, beta, 
     out_mode = 0 if out_dtype == torch.bfloat16 else 1
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    pair = False
-    if bn is None:
-        bn, pair = _pick_tile(M, N)
+    bn, pair = _pick_tile(M, N) if bn is None else (bn, _use_pair(M, N, bn))
     ctx = info.ctx
     staging, plans = ctx.acquire(info, backward=trans_b)
     plan = None

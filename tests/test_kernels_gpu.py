@@ -75,6 +75,22 @@ def test_pair_gemm_tma_store_epilogue_matches_row_stores(M, N, K):
     assert bool((guard[M:, :] == 7.0).all()) and bool((guard[:, N:] == 7.0).all())   # nothing beyond the edges
 
 
+@pytest.mark.parametrize("bn,pairs", [(None, 1), (256, 1), (128, 0)])
+def test_gemm_tile_width_and_kernel(bn, pairs, monkeypatch):
+    """A tile width of 256 asked for by the caller takes the CTA-pair kernel, as the chosen one does."""
+    from axolotl_b200.ops import _lib
+    from axolotl_b200.ops.gemm import gemm
+    lib, calls = _lib.cuda_lib(), []
+    real = lib.axb_gemm_bf16_pair
+    monkeypatch.setattr(lib, "axb_gemm_bf16_pair", lambda *a: calls.append(1) or real(*a))
+    a, b = (torch.randn(2560, 64, device=_dev()).bfloat16() for _ in range(2))
+    out = gemm(a, b, bn=bn)
+    _lib.check_status()
+    assert len(calls) == pairs
+    ref = a.double() @ b.double().t()
+    assert ((out.double() - ref).abs() <= 2 ** -20 * (a.double().abs() @ b.double().abs().t()) + 2 ** -8 * ref.abs()).all()
+
+
 def test_gemm_k_extension_and_epilogue():
     from axolotl_b200.ops.gemm import gemm
     torch.manual_seed(2)
