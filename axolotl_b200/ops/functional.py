@@ -378,12 +378,18 @@ def token_entropy(logits, temperature=1.0, return_lse=False):
 
 
 # --------------------------------------------------------------------------------------- embedding
-def _flat_grad(p):
-    """The optimizer's fp32 gradient buffer of a bf16 CUDA parameter that the kernels may add into, else None."""
+def _flat_grad(ctx, i, p):
+    """The optimizer's fp32 gradient buffer of a bf16 CUDA parameter (tensor input ``i`` of the function) that the kernels may
+    add into, else None. A parameter with hooks keeps the gradient that they see, and so does one whose gradient
+    ``torch.autograd.grad`` returns or this backward pass does not accumulate."""
     g = getattr(p, "_axb_grad", None)
-    ok = (g is not None and p.is_cuda and p.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.device == p.device
-          and g.shape == p.shape and g.is_contiguous())
-    return g if ok else None
+    if (g is None or not p.is_cuda or p.dtype != torch.bfloat16 or g.dtype != torch.float32 or g.device != p.device or g.shape != p.shape
+            or not g.is_contiguous() or p._backward_hooks or p._post_accumulate_grad_hooks):
+        return None
+    try:
+        return g if torch._C._will_engine_execute_node(ctx.next_functions[i][0]) else None
+    except RuntimeError:       # the engine runs for autograd.grad and captures this gradient
+        return None
 
 
 class _Embedding(torch.autograd.Function):
@@ -417,7 +423,7 @@ class _Embedding(torch.autograd.Function):
             g.index_add_(0, ids.reshape(-1), dout.reshape(-1, H).float())
             return g.to(ctx.tdtype), None
         lib = _lib.cuda_lib()
-        tgt = _flat_grad(ctx.table)
+        tgt = _flat_grad(ctx, 0, ctx.table)
         g = tgt if tgt is not None else torch.zeros(V, H, dtype=torch.float32, device=dout.device)
         d2 = dout.reshape(-1, H).contiguous()
         flat = ids.reshape(-1).contiguous()
@@ -861,7 +867,7 @@ class _LinearCE(torch.autograd.Function):
     def backward(ctx, gout):
         dh, dw = ctx.saved_tensors
         dx = dh * gout.to(dh.dtype)
-        tgt = _flat_grad(ctx.w) if dw is not None and dw.is_contiguous() else None
+        tgt = _flat_grad(ctx, 1, ctx.w) if dw is not None and dw.is_contiguous() else None
         if tgt is not None:      # straight into the optimizer's fp32 buffer
             _lib.check_rc(_lib.cuda_lib().axb_axpy_f32(tgt.data_ptr(), dw.data_ptr(), gout.float().data_ptr(), dw.numel(),
                                                        _lib.stream_ptr()), "axpy_f32")

@@ -60,6 +60,10 @@ def build_param_groups(named_params, *, weight_decay=0.0, embedding_lr=None, emb
 
 
 class FlatAdamW:
+    """AdamW over flat fp32 buffers. Every parameter gets a view ``_axb_grad`` of the flat gradient, into which the kernels of
+    linear layers, the embedding and the loss head add; the ``.grad`` of a bf16 parameter then stays None. What autograd puts into
+    ``.grad`` all the same (other operators; an embedding or loss head that has hooks) is folded in before the step."""
+
     def __init__(self, groups, lr=1e-4, betas=(0.9, 0.999), eps=1e-8, max_grad_norm=0.0, alloc=None,
                  pad_multiple=8, moment_shard=None):
         self.lr, self.betas, self.eps, self.max_grad_norm = lr, betas, eps, max_grad_norm

@@ -77,3 +77,47 @@ def test_head_and_table_gradients_reach_the_flat_buffer(T, V):
     for a, b in zip(run(True), run(False)):
         # one bf16 rounding of the returned gradient; the buffer's ones cost 2^-23 of themselves per addition
         assert ((a - b).abs() <= 2 ** -8 * b.abs() + 2 ** -20).all()
+
+
+def _loss(tab, w, ids, labels):
+    return Fn.linear_cross_entropy(Fn.embedding(tab, ids), w, labels)
+
+
+@pytest.mark.parametrize("kind", ["hook", "post", "grad", "inputs", "partial"])
+def test_flat_buffer_leaves_hooks_and_partial_backwards_alone(kind):
+    """Hooks on the table or the head see (and may change) their gradient, ``torch.autograd.grad`` returns it, and a backward pass
+    restricted to other inputs adds nothing to the buffers."""
+    torch.manual_seed(0)
+    V, H, T = 512, 256, 64
+    ids, labels = torch.randint(0, V, (2, T), device="cuda")
+    tab, w = (torch.nn.Parameter((torch.randn(V, H, device="cuda") * 0.1).bfloat16()) for _ in range(2))
+    want = torch.autograd.grad(_loss(tab, w, ids, labels), (tab, w))
+    for p in (tab, w):
+        p._axb_grad = torch.zeros(V, H, device="cuda")
+    seen = []
+    if kind == "hook":
+        for p in (tab, w):
+            p.register_hook(lambda g: seen.append(g) or g * 2)
+        _loss(tab, w, ids, labels).backward()
+        assert len(seen) == 2
+        got = tab.grad / 2, w.grad / 2
+    elif kind == "post":
+        for p in (tab, w):
+            p.register_post_accumulate_grad_hook(lambda q: seen.append(q.grad))
+        _loss(tab, w, ids, labels).backward()
+        assert len(seen) == 2
+        got = tab.grad, w.grad
+    elif kind == "grad":
+        got = torch.autograd.grad(_loss(tab, w, ids, labels), (tab, w))
+    elif kind == "inputs":
+        _loss(tab, w, ids, labels).backward(inputs=[tab])
+        assert not w._axb_grad.any() and w.grad is None
+        got = tab._axb_grad.bfloat16(), want[1]
+        tab._axb_grad.zero_()
+    else:
+        h = Fn.embedding(tab, ids).detach().requires_grad_(True)
+        torch.autograd.grad(Fn.linear_cross_entropy(h, w, labels), h)
+        got = want
+    assert not tab._axb_grad.any() and not w._axb_grad.any()
+    for a, b in zip(got, want):
+        assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
