@@ -113,6 +113,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     return ((bidir ? doc_len : min(top, doc_len)) + 127) / 128 - jb0;
   };
   const int n_u0 = blocks_of(0), n_u1 = blocks_of(1), n_max = max(n_u0, n_u1);
+  // The window of the lower tile may begin a block later. Its P is zero in that block and is not multiplied by V, whose rows
+  // there are none of its business (0 x inf is not 0).
+  const int first_u1 = p.pair_mode == 2 && win > 0 ? max(0, q0 + 128 - win + 1) / 128 - jb0 : 0;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -198,13 +201,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         }
         __syncwarp();
       };
-      auto issue_pv = [&](int u, int j, bool last) {
+      auto issue_pv = [&](int u, int j, int first, bool last) {
         const uint64_t dv = dv_base + (uint32_t)(j & 1) * TILE16;
-        if (elect_one()) {
+        if (j >= first && elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)   // 128 kv rows / 16: 8 TMEM columns of P each
             umma_f16_ts(tmem_base + C::O_COL + u * D, tmem_base + u * 128 + kk * 8, dv + kk * (2048 / 16), idesc_pv,
-                        (j > 0 || kk > 0) ? 1u : 0u);
+                        (j > first || kk > 0) ? 1u : 0u);
           if (last) umma_commit(&o_full[u]);
         }
         __syncwarp();
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           if (!ok) break;
           v_ready = true;
           tc_fence_after();
-          issue_pv(u, j, j == n_u - 1);
+          issue_pv(u, j, u == 0 ? 0 : first_u1, j == n_u - 1);
           if (j + 1 < n_u) {
             if (!k_ready) ok = warp_all(mbar_wait(&k_full[nst], ((j + 1) >> 1) & 1, p.status, AXB_TIMEOUT_FULL));
             if (!ok) break;

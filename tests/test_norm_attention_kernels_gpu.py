@@ -175,3 +175,23 @@ def test_attention_output_is_rounded_like_a_maximum_referenced_softmax(D, Dv, sc
             s = s.masked_fill(torch.ones_like(s, dtype=torch.bool).triu(1), float("-inf"))
             ref[a:b, h] = torch.softmax(s, -1) @ v[a:b, g * Dv:(g + 1) * Dv]
     assert (out.double().view_as(ref) - ref).norm() <= 1.15 * 2 ** -9 * ref.norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_windowed_attention_does_not_touch_blocks_outside_the_window(D, bad):
+    """Heads that pair neighbouring q tiles: a non-finite value row reaches the q tiles whose window includes its key block and no
+    other one. The other rows are those of a clean run, bit for bit."""
+    from axolotl_b200.ops import functional as Fn
+
+    torch.manual_seed(D)
+    T, H, win = 4096, 8, 64
+    qkv = torch.randn(T, 3 * H * D, device="cuda").bfloat16()
+    meta = Fn.AttnMeta([0, T], "cuda").windowed(win)
+    clean = Fn.flash_varlen(qkv, meta, H, H, D)
+    qkv[200, 2 * H * D:] = bad
+    out = Fn.flash_varlen(qkv, meta, H, H, D)
+    _lib.check_status()
+    far = torch.ones(T, dtype=torch.bool, device="cuda")
+    far[128:384] = False
+    assert torch.equal(out[far], clean[far]) and torch.isfinite(clean).all()
