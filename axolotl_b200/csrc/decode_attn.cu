@@ -256,16 +256,17 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
     x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 2));
     x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 1));
     x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 2));
-    const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);        // finite: every tile has a live position
-    const float a0 = exp2f(m0 - n0), a1 = exp2f(m1 - n1);
-    m0 = n0;
-    m1 = n1;
+    const float m0_old = m0, m1_old = m1;
+    m0 = fmaxf(m0, x0);
+    m1 = fmaxf(m1, x1);
+    const float b0 = m0 == -INFINITY ? 0.f : m0, b1 = m1 == -INFINITY ? 0.f : m1;    // no finite score so far: every P is 0
+    const float a0 = exp2f(m0_old - b0), a1 = exp2f(m1_old - b1);
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      s[t][0] = exp2f(s[t][0] - m0);
-      s[t][1] = exp2f(s[t][1] - m0);
-      s[t][2] = exp2f(s[t][2] - m1);
-      s[t][3] = exp2f(s[t][3] - m1);
+      s[t][0] = exp2f(s[t][0] - b0);
+      s[t][1] = exp2f(s[t][1] - b0);
+      s[t][2] = exp2f(s[t][2] - b1);
+      s[t][3] = exp2f(s[t][3] - b1);
     }
     l0 = l0 * a0 + ((s[0][0] + s[0][1]) + (s[1][0] + s[1][1]));
     l1 = l1 * a1 + ((s[0][2] + s[0][3]) + (s[1][2] + s[1][3]));

@@ -71,6 +71,28 @@ def test_decode_attention_splits_append_and_rope(D, Hq, Hk, splits, window, appe
         torch.testing.assert_close(kc, k0, rtol=2 ** -7, atol=2 ** -7 if rope else 0, equal_nan=True)
 
 
+@pytest.mark.parametrize("cap,n", [(256, 200), (120, 100)])
+def test_decode_attention_with_scores_of_minus_infinity(cap, n):
+    """A whole 16-position tile (first, middle or last) whose scores are -inf has weight 0, with one CTA per pair and with four."""
+    torch.manual_seed(n)
+    B, Hq, Hk, D = 3, 8, 2, 64
+    qkv = torch.randn(B, (Hq + 2 * Hk) * D, device="cuda").bfloat16()
+    qkv[:, 0:Hq * D:D] = 1.0
+    k, v = torch.randn(2, B, cap, Hk * D, device="cuda").bfloat16()
+    for b, p0 in enumerate((0, 48, n - n % 16)):
+        k[b, p0:p0 + 16, 0::D] = float("-inf")
+    lens = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    scale = D ** -0.5
+    out = Fn.decode_attention(qkv, k, v, lens, Hq, Hk, D, scale)
+    for b in range(B):
+        q = qkv[b, :Hq * D].view(Hk, Hq // Hk, D).float()
+        kk, vv = (t[b, :n].view(n, Hk, D).float().transpose(0, 1) for t in (k, v))
+        s = (q @ kk.transpose(1, 2) * scale)
+        ref = (torch.softmax(s, -1) @ vv).reshape(-1)
+        assert torch.isfinite(ref).all()
+        assert (out[b].float() - ref).abs().max() <= 2 ** -8 * max(1.0, ref.abs().max().item())
+
+
 def test_cached_step_on_a_subset_of_the_sequences():
     """``KVCache.attend`` with query rows that belong to some of the cache's sequences, in another order."""
     from axolotl_b200.models.config import preset
