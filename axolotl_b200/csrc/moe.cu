@@ -191,24 +191,24 @@ __global__ void __launch_bounds__(RL_T) route_scatter_kernel(const long long* __
   }
 }
 
-// Local dispatch: out[r, :] = scale * x[token of row r, :], zeros in pad rows. The token of a row is row_token[r] (scale
-// row_scale[r]) or, with k > 0, row_token[r] / k (row_token then holds slots; scale row_scale[slot]). One warp per row; eight
-// vectors of a row are requested before the first is stored.
-__global__ void moe_dispatch_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_token,
-                                         const float* __restrict__ row_scale, __nv_bfloat16* __restrict__ out,
+// Local dispatch: out[r, :] = scale * x[token of row r, :], zeros in pad rows. Row r holds slot row_slot[r] (-1: a pad row), the
+// slots of token t are t * k .. t * k + k - 1, the scale is slot_scale[slot] (null: 1). One warp per row; eight vectors of a row
+// are requested before the first is stored.
+__global__ void moe_dispatch_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_slot,
+                                         const float* __restrict__ slot_scale, __nv_bfloat16* __restrict__ out,
                                          long long n_rows, int width, int k) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long r = w; r < n_rows; r += n_warps) {
-    const int id = row_token[r];
+    const int id = row_slot[r];
     __nv_bfloat16* d = out + r * width;
     if (id < 0) {
       for (int c = lane * 8; c < width; c += 256) *reinterpret_cast<uint4*>(d + c) = make_uint4(0, 0, 0, 0);
       continue;
     }
-    const __nv_bfloat16* s = x + (long long)(k > 0 ? id / k : id) * width;
-    const float g = row_scale ? row_scale[k > 0 ? (long long)id : r] : 1.f;
+    const __nv_bfloat16* s = x + (long long)(id / k) * width;
+    const float g = slot_scale ? slot_scale[id] : 1.f;
     for (int c0 = 0; c0 < width; c0 += 8 * 256) {
       uint4 v[8];
 #pragma unroll
@@ -220,7 +220,7 @@ __global__ void moe_dispatch_rows_kernel(const __nv_bfloat16* __restrict__ x, co
       for (int q = 0; q < 8; ++q) {
         const int c = c0 + q * 256 + lane * 8;
         if (c >= width) break;
-        if (row_scale) {
+        if (slot_scale) {
           uint32_t in[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -601,14 +601,13 @@ extern "C" int axb_moe_route_layout(const long long* expert, int n, int E, int m
   return (int)cudaGetLastError();
 }
 
-// out [n_rows, width] bf16. k == 0: row_token int32 [n_rows] (-1 = zero row), row_scale fp32 [n_rows] or NULL; k > 0: row_token
-// holds slots (token = slot / k) and row_scale is indexed by the slot
-extern "C" int axb_moe_dispatch_rows(const void* x, const int* row_token, const float* row_scale, void* out,
-                                     long long n_rows, int width, int k, void* stream) {
-  if (width % 8) return -2;
+// out [n_rows, width] bf16, row_slot int32 [n_rows] (-1 = zero row), k slots per token, slot_scale fp32 [tokens * k] or NULL
+extern "C" int axb_moe_dispatch_rows(const void* x, const int* row_slot, const float* slot_scale, void* out, long long n_rows,
+                                     int width, int k, void* stream) {
+  if (width % 8 || k < 1) return -2;
   if (n_rows <= 0) return 0;
   moe_dispatch_rows_kernel<<<rows_grid(n_rows), 256, 0, ST(stream)>>>(
-      (const __nv_bfloat16*)x, row_token, row_scale, (__nv_bfloat16*)out, n_rows, width, k);
+      (const __nv_bfloat16*)x, row_slot, slot_scale, (__nv_bfloat16*)out, n_rows, width, k);
   return (int)cudaGetLastError();
 }
 
