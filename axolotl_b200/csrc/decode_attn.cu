@@ -88,7 +88,7 @@ struct DecCfg {
   static constexpr int Q_BYTES = MAX_G * ROWB;
   static constexpr int NEW_BYTES = 2 * ROWB;
   static constexpr int STAT = DEC_W * MAX_G;               // per-warp row statistics
-  static constexpr int SMEM = RING + Q_BYTES + NEW_BYTES + (2 * STAT + 3 * DEC_MAX_SPLITS * STAT) * 4 + D * 4;
+  static constexpr int SMEM = RING + Q_BYTES + NEW_BYTES + (2 * STAT + 2 * DEC_MAX_SPLITS * STAT) * 4 + D * 4;
 };
 
 template <int D>
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(DEC_T) decode_attn_kernel(const DecodeParams p
   float* sL = sM + C::STAT;
   float* gM = sL + C::STAT;                                // statistics of all warps of the cluster, then weights
   float* gL = gM + DEC_MAX_SPLITS * C::STAT;
-  float* sCS = gL + 2 * DEC_MAX_SPLITS * C::STAT;          // cos | sin of the new position
+  float* sCS = gL + DEC_MAX_SPLITS * C::STAT;              // cos | sin of the new position
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_launch_dependents();
   const int kvh = blockIdx.y, b = blockIdx.z;
