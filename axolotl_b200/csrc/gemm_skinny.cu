@@ -1,4 +1,5 @@
-// GEMM with one long and one short side, for sm_100a: acc[r, n] = sum_k P[r, k] S[n, k] (+ P2 S2^T), N <= 256.
+// GEMM with one long and one short side, for sm_100a: acc[r, n] = sum_k P[r, k] S[n, k] (+ P2 S2^T), N <= 128
+// (up to 256 as two launches).
 //
 //   out_mode 0: C[n, r]  (a generation step or a short row: P = weight, S = tokens, y = x W^T)
 //   out_mode 1: C[r, n]  (the low-rank product x A^T of an adapter: P = tokens, S = A)
@@ -6,7 +7,7 @@
 //               same columns, so that the gated activation needs no pass of its own
 //
 // Bound: one pass over P (HBM). The long side is the 128-row operand of tcgen05.mma, so no tensor-core row is padding and the
-// short side is the MMA's N = 16 .. 256; a 128 x 128-tile kernel reads the same bytes with only R / 128 CTAs, too few to keep
+// short side is the MMA's N = 16 .. 128; a 128 x 128-tile kernel reads the same bytes with only R / 128 CTAs, too few to keep
 // HBM busy. Here the K range of a tile is split over a cluster of up to 8 CTAs and two CTAs share an SM, so that about 200 KB
 // per SM are in flight; the partial tiles meet in distributed shared memory in a fixed order (no atomics, no workspace).
 // In a dependent launch the tiles of P (a weight) are requested before the predecessor has finished.
@@ -35,8 +36,8 @@ template <int NT>
 struct SkCfg {
   static constexpr int S_BYTES = NT * SK_BK * 2;
   static constexpr int STAGE = SK_P_BYTES + S_BYTES;
-  static constexpr int STAGES = NT == 16 ? 5 : (NT == 32 ? 5 : (NT == 64 ? 4 : (NT == 128 ? 3 : 4)));
-  static constexpr int RING = STAGES * STAGE;      // 84 .. 100 KB, NT = 256: 192 KB (one CTA per SM)
+  static constexpr int STAGES = NT <= 32 ? 5 : (NT == 64 ? 4 : 3);
+  static constexpr int RING = STAGES * STAGE;      // 84 .. 100 KB
   static constexpr int SMEM = RING + 1024 + 256;
   static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
   static_assert(NT * SK_BM * 4 <= RING, "the partial tile reuses the ring");
@@ -265,8 +266,8 @@ int launch_skinny(const CUtensorMap& tP, const CUtensorMap& tS, const CUtensorMa
 
 // CTAs per tile: as many as the 2 x 148 resident CTAs hold, at least two K blocks each. Clusters of 5 to 7 CTAs pack badly
 // into the GPCs (6144 x 4096, 8 tokens: 20.5 us with 4, 26.6 us with 6, 24.6 us with 8 CTAs per tile), so only 1 to 4 and 8.
-int pick_splits(int tiles, int nk, int n) {
-  const int slots = n > 128 ? 148 : 296;
+int pick_splits(int tiles, int nk) {
+  const int slots = 296;
   const int sizes[] = {8, 4, 3, 2};
   for (int s : sizes)
     if (tiles * s <= slots && nk >= 2 * s) return s;
@@ -286,7 +287,15 @@ extern "C" int axb_gemm_skinny(const void* P, long long ldp, const void* S, long
   if (N > 256 || out_mode < 0 || out_mode > 2 || splits < 0 || splits > 8) return -2;
   if (out_mode == 2 && (out_f32 || (R % 64) || glu_kind < 0 || glu_kind > 1)) return -2;
   if (K <= 0) return -2;
-  const int NT = N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256)));
+  if (N > 128) {
+    const long long c_off = 128ll * (out_mode == 1 ? 1 : ldc) * (out_f32 ? 4 : 2);
+    const int rc = axb_gemm_skinny(P, ldp, S, lds, C, ldc, R, 128, K, P2, ldp2, S2, lds2, K2, alpha, bias, out_mode, out_f32, glu_kind,
+                                   glu_limit, p_dep, splits, pdl, status, stream);
+    return rc ? rc : axb_gemm_skinny(P, ldp, (const __nv_bfloat16*)S + 128 * lds, lds, (uint8_t*)C + c_off, ldc, R, N - 128, K, P2, ldp2,
+                                     K2 > 0 ? (const __nv_bfloat16*)S2 + 128 * lds2 : nullptr, lds2, K2, alpha, bias, out_mode, out_f32,
+                                     glu_kind, glu_limit, p_dep, splits, pdl, status, stream);
+  }
+  const int NT = N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : 128));
   const int prow = out_mode == 2 ? 64 : SK_BM;
   const uint64_t rows = (uint64_t)R * (out_mode == 2 ? 2 : 1);
   CUtensorMap tP, tS, tP2, tS2;
@@ -316,14 +325,13 @@ extern "C" int axb_gemm_skinny(const void* P, long long ldp, const void* S, long
   p.status = status;
   const int tiles = (R + prow - 1) / prow;
   const int nk = (K + SK_BK - 1) / SK_BK + (p.K2 + SK_BK - 1) / SK_BK;
-  if (splits == 0) splits = pick_splits(tiles, nk, N);
+  if (splits == 0) splits = pick_splits(tiles, nk);
   if (splits > nk) splits = nk;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   switch (NT) {
     case 16: return launch_skinny<16>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
     case 32: return launch_skinny<32>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
     case 64: return launch_skinny<64>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
-    case 128: return launch_skinny<128>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
-    default: return launch_skinny<256>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
+    default: return launch_skinny<128>(tP, tS, tP2, tS2, p, tiles, splits, pdl != 0, st);
   }
 }
