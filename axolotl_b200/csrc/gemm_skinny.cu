@@ -264,13 +264,16 @@ int launch_skinny(const CUtensorMap& tP, const CUtensorMap& tS, const CUtensorMa
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// CTAs per tile: as many as the 2 x 148 resident CTAs hold, at least two K blocks each. Clusters of 5 to 7 CTAs pack badly
-// into the GPCs (6144 x 4096, 8 tokens: 20.5 us with 4, 26.6 us with 6, 24.6 us with 8 CTAs per tile), so only 1 to 4 and 8.
+// CTAs per tile: the largest cluster of which the chip holds one per tile at once, at least two K blocks for each CTA. Two CTAs
+// share an SM but a cluster stays inside one GPC, so that 33 clusters of eight are resident, 70 of four, 92 of three and 148 of
+// two; one more is a second wave (seen as the step in time against the number of tiles; the runtime's occupancy query counts
+// one CTA per SM for clusters). 48 columns, K = 4096: 33 / 35 tiles take 21.5 / 29.5 us with eight CTAs each and 23.5 with
+// four, 74 tiles 37.9 with four and 31.7 with three, 96 tiles 46.1 with three and 37.9 with two. Clusters of 5 to 7 pack
+// badly (6144 x 4096, 8 tokens: 20.5 us with 4, 26.6 us with 6, 24.6 us with 8 CTAs per tile).
 int pick_splits(int tiles, int nk) {
-  const int slots = 296;
-  const int sizes[] = {8, 4, 3, 2};
-  for (int s : sizes)
-    if (tiles * s <= slots && nk >= 2 * s) return s;
+  const int sizes[][2] = {{8, 33}, {4, 70}, {3, 92}, {2, 148}};
+  for (const auto& s : sizes)
+    if (tiles <= s[1] && nk >= 2 * s[0]) return s[0];
   return 1;
 }
 
