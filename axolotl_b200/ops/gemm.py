@@ -227,15 +227,27 @@ def _glu_launch(lib, glu, a, trans_a, b_ptr, ldb, trans_b, out, M, N, K, a2, b2,
 
 def _use_skinny(M, N, K, trans_a, trans_b, out, out_mode, c_in, beta) -> bool:
     """The split-K cluster kernel of csrc/gemm_skinny.cu serves products with one side of a few columns, where 128-row tiles
-    leave most SMs without a CTA. Either N <= 64 (x A^T of an adapter; the old kernel / this one, microseconds with the L2
-    flushed: 512 x 4096 by 48 28.7 / 16.4, 960 x 14336 by 16 71.7 / 20.5, 8192 x 14336 by 16 75.8 / 55) up to the 8192 rows
-    that were measured, or M <= 128 (a generation step; 64 x 4096 by 6144 28.6 / 24.6, 64 x 14336 by 4096 72.5 / 36.9), but
-    above 32 rows only while the weight has fewer than 148 tiles of 128 rows (128 x 4096 by 128256 203.6 / 227.3)."""
+    leave most SMs without a CTA. It gains what the split takes off the K loop and pays for the merge of the partial tiles, which
+    grows with the short side: the lines are multiples of that side, by the CTAs that a tile gets (8 up to 33 tiles of the long
+    side, 4 or 3 up to 92). Microseconds, ordinary tiles / this kernel, L2 flushed:
+
+    N <= 64 (x A^T of an adapter). Up to 31 columns whatever the sizes: 192 x 4096 by 16 23.6 / 11.3, 8192 x 14336 by 16
+    66.6 / 57.3, 65536 x 4096 by 16 109.6 / 104.4, 65536 x 512 by 16 level. Above: 1416 x 1496 by 56 19.3 / 15.3, 1576 x 608 by
+    64 11.3 / 15.3; 8192 x 4096 by 48 29.7 / 27.7, 9216 x 2048 by 32 17.3 / 21.4, 9216 x 4096 by 64 27.9 / 33.7.
+    M <= 128 (a generation step). Up to 16 rows, and 32 with a long K, whatever the weight: 16 x 4096 by 4096 1.35 times as fast,
+    by 128256 1.10 times. Above: 64 x 14336 by 4096 1.54 times, 98 x 2000 by 624 17.4 / 15.3, 116 x 984 by 5192 15.3 / 19.4, 64 x
+    2048 by 8192 0.89 times, 124 x 2608 by 18472 32.3 / 39.1, 128 x 4096 by 128256 0.92 times."""
     if trans_a or trans_b or out_mode > 1 or (c_in is not None and beta != 0.0) or K < 512 or out.stride(1) != 1:
         return False
+    tiles = (max(M, N) + 127) // 128
     if N <= 64:
-        return 128 < M <= 8192
-    return N >= 512 and (M <= 32 or (M <= 128 and (N + 127) // 128 < _SM))
+        return M > 128 and (N < 32 or (K >= 24 * N if tiles <= 33 else tiles <= 92 and K >= 80 * N))
+    if M > 128 or N < 512:
+        return False
+    if M <= 16 or (M <= 32 and K >= 2048):
+        return True
+    pad = 32 if M <= 32 else 64 if M <= 64 else 128      # columns of the kernel's tile
+    return K >= 20 * pad if tiles <= 33 else tiles <= 92 and K >= 40 * pad
 
 
 def _use_pair(M, N, bn) -> bool:

@@ -257,6 +257,25 @@ def test_skinny_gemm(R, N, K, K2, splits, mode, f32):
     assert (buf[:, ref.shape[1]:] == 7.0).all()
 
 
+@pytest.mark.parametrize("M,N,K,skinny", [(129, 31, 512, True), (20000, 16, 512, True), (300, 32, 768, True), (300, 32, 760, False),
+                                          (4224, 64, 1536, True), (4232, 64, 1536, False), (4232, 64, 5120, True), (11784, 64, 5120, False),
+                                          (16, 512, 512, True), (32, 4232, 2048, True), (32, 11784, 1024, False), (64, 4224, 1280, True),
+                                          (64, 4232, 1280, False), (128, 4232, 5120, True), (128, 4232, 5112, False)])
+def test_short_side_products_on_both_sides_of_the_rule(M, N, K, skinny):
+    """Sizes just inside and outside the lines between the short-side kernel and the ordinary tiles. fp32 sums in any order:
+    2^-20 of their magnitude, one bf16 rounding more for the result."""
+    from axolotl_b200.ops import _lib
+    from axolotl_b200.ops.gemm import _use_skinny, gemm
+
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    out = gemm(a, b)
+    assert _use_skinny(M, N, K, False, False, out, 0, None, 0.0) == skinny
+    _lib.check_status()
+    ref, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    assert ((out.double() - ref).abs() <= 2 ** -20 * mag + 2 ** -8 * ref.abs()).all()
+
+
 _STEP_CASES = {
     "llama": dict(),
     "qwen3 q/k norms": dict(model_type="qwen3", head_dim=64),
