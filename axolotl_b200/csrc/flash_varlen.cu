@@ -374,26 +374,29 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // Backward
 // =====================================================================================
 // delta[h][t] = sum_d dO[t,h,d] * O[t,h,d]
-// Bound: one read of dO and O. D / 8 threads of 16 bytes share a (token, head), a block covers 32 tokens x 8 heads so that
-// its results leave as 128-byte rows of delta (one warp per (token, head) took 100 us for 7777 tokens x 64 heads of 64).
-template <int D>
+// Bound: one read of dO and O. D / 8 threads of 16 bytes share a (token, head), a block covers TOK tokens x up to 8 heads so that
+// its results leave as whole sectors of delta (one warp per (token, head) took 100 us for 7777 tokens x 64 heads of 64). 32 tokens
+// while that gives every SM four blocks; below, a block of that size is a chain of up to 16 loads, and 8 tokens shorten it to 4
+// (whole backward pass, heads of 128: 222 tokens, 3 heads 35.8 -> 27.6 us, 960 tokens, 32 heads 84 -> 65).
+template <int D, int TOK>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dout,
                                                          const __nv_bfloat16* __restrict__ out, float* __restrict__ delta,
                                                          long long T, int Hq, long long ld_do, long long ld_o) {
   constexpr int TPR = D / 8, ROWS = 256 / TPR;   // threads per (token, head), pairs per step
-  constexpr int TOK = 32, HEADS = 8;
+  constexpr int HEADS = 8;
   __shared__ float s[HEADS][TOK + 1];
   const long long t0 = (long long)blockIdx.x * TOK;
-  const int h0 = blockIdx.y * HEADS;
-  const int sub = threadIdx.x % TPR, pair0 = threadIdx.x / TPR;
+  const int h0 = blockIdx.y * HEADS, nh = min(HEADS, Hq - h0);
+  const int sub = threadIdx.x % TPR, lane = threadIdx.x & 31, pairs = TOK * nh;
 #pragma unroll 4
-  for (int q = pair0; q < TOK * HEADS; q += ROWS) {     // consecutive pairs: the heads of one token
-    const int h = h0 + q % HEADS;
-    const long long t = t0 + q / HEADS;
+  for (int q0 = (int)(threadIdx.x >> 5) * (32 / TPR); q0 < pairs; q0 += ROWS) {     // the same for all lanes of a warp
+    const int q = q0 + lane / TPR;                       // consecutive pairs: the heads of one token
+    const int h = nh == HEADS ? q % HEADS : q % nh, tq = nh == HEADS ? q / HEADS : q / nh;
+    const long long t = t0 + tq;
     float acc = 0.f;
-    if (t < T && h < Hq) {
-      const uint4 x = *reinterpret_cast<const uint4*>(dout + t * ld_do + (long long)h * D + sub * 8);
-      const uint4 y = *reinterpret_cast<const uint4*>(out + t * ld_o + (long long)h * D + sub * 8);
+    if (q < pairs && t < T) {
+      const uint4 x = *reinterpret_cast<const uint4*>(dout + t * ld_do + (long long)(h0 + h) * D + sub * 8);
+      const uint4 y = *reinterpret_cast<const uint4*>(out + t * ld_o + (long long)(h0 + h) * D + sub * 8);
       const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -403,11 +406,11 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
     }
 #pragma unroll
     for (int o = TPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (sub == 0) s[q % HEADS][q / HEADS] = acc;
+    if (sub == 0 && q < pairs) s[h][tq] = acc;
   }
   __syncthreads();
   const int h = threadIdx.x / TOK, t = threadIdx.x % TOK;
-  if (h0 + h < Hq && t0 + t < T) delta[(long long)(h0 + h) * T + t0 + t] = s[h][t];
+  if (h < nh && t0 + t < T) delta[(long long)(h0 + h) * T + t0 + t] = s[h][t];
 }
 
 // One CTA per (kv tile of 128 rows, kv head). Inner loop over the q heads of the GQA group and
@@ -925,8 +928,11 @@ int flash_bwd_impl(const AttnGeom& g, const void* dout, const void* out, long lo
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, sizeof(float) * T * Hq * D, st);
   if (e != cudaSuccess) return (int)e;
   {
-    const dim3 grid((unsigned)((T + 31) / 32), (unsigned)((Hq + 7) / 8));
-    auto kern = D == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
+    const unsigned hb = (unsigned)((Hq + 7) / 8);
+    const bool few = (T + 31) / 32 * hb < 4 * 148;
+    const dim3 grid((unsigned)(few ? (T + 7) / 8 : (T + 31) / 32), hb);
+    auto kern = D == 128 ? (few ? attn_delta_kernel<128, 8> : attn_delta_kernel<128, 32>)
+                         : (few ? attn_delta_kernel<64, 8> : attn_delta_kernel<64, 32>);
     kern<<<grid, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, T, Hq, o_ld, o_ld);
   }
   AttnParams p = {};
