@@ -22,20 +22,23 @@ USE_PAIR = os.environ.get("AXB_GEMM_PAIR", "1") != "0"
 USE_GLU_EPILOGUE = os.environ.get("AXB_GLU_EPILOGUE", "1") != "0"
 
 
-def _pick_tile(M: int, N: int) -> tuple[int, bool]:
-    """(tile width, whether the CTA-pair kernel runs it): the choice with the least waves x time per wave. A K block of one
-    wave takes about the same 0.31 us with 128 x 64 and 128 x 128 tiles, 0.40 us with 128 x 256 (one CTA per SM each) and
-    0.34 us with the pair kernel's 256 x 256 (74 SM pairs), measured at K = 32000 with the L2 flushed; what decides is how
-    many waves a tile needs. 960 x 32000 by 4096: 580 / 304 / 200 / 173 us (10, 4, 2, 1 waves with 64, 128, 256, pair);
-    320 x 32000 by 4096: 292 / 157 / 196 / 163 us; 640 x 4096 by 14336: 163 / 93 / 73 / 77 us. Ties go to the wider tile,
-    which reads less."""
+# tile width, pair kernel?, rows, tiles at once, microseconds per 64-deep K block, microseconds per tile for bf16 results / fp32
+# results / results added to an operand read by the epilogue (L2 flushed; least squares over 7600 drawn products)
+_TILES = ((256, True, 256, _SM // 2, 0.336, (2.2, 8.7, 25.8)), (256, False, 128, _SM, 0.441, (5.6, 8.6, 24.0)),
+          (128, False, 128, _SM, 0.292, (2.8, 4.3, 11.8)), (64, False, 128, _SM, 0.236, (1.3, 2.1, 5.9)))
+
+
+def _pick_tile(M: int, N: int, k_blocks: int = 64, epilogue: int = 0) -> tuple[int, bool]:
+    """(tile width, whether the CTA-pair kernel runs it): the choice with the least waves x time per wave. Mostly the number
+    of waves decides, 960 x 32000 by 4096 takes 580 / 304 / 200 / 173 us (10, 4, 2, 1 waves with 64, 128, 256, pair); with a
+    short K the epilogue does, which the pair kernel has cheapest in bf16 (TMA stores) and wide tiles have dearest where they read
+    and write fp32: 1568 x 88 by 13712 51 / 44 / 42 / 26 us, 1304 x 96 by 3720 added to fp32 46 / 51 / 64 / 70. Within 0.8 % of the best of the four on average, 2.7 % by waves alone.
+    Ties go to the wider tile, which reads less."""
     best = None
-    for bn, rows, slots, cost, pair in ((256, 256, _SM // 2, 1.10, True), (256, 128, _SM, 1.30, False), (128, 128, _SM, 1.0, False),
-                                        (64, 128, _SM, 0.99, False)):
+    for bn, pair, rows, slots, per_k, per_tile in _TILES:
         if (pair and not USE_PAIR) or (bn > 64 and N <= bn // 2) or (pair and (M <= 128 or N < 256)):
             continue
-        tiles = -(-M // rows) * -(-N // bn)
-        t = -(-tiles // slots) * cost
+        t = -(-(-(-M // rows) * -(-N // bn)) // slots) * (per_k * k_blocks + per_tile[epilogue])
         if best is None or t < best[0]:
             best = (t, bn, pair)
     return best[1], best[2]
@@ -168,7 +171,7 @@ def gemm(
     if bn is None and accumulate:
         bn = _pick_bn(M, N)
     elif bn is None:
-        bn, pair = _pick_tile(M, N)
+        bn, pair = _pick_tile(M, N, (K + 63) // 64 + (K2 + 63) // 64, 2 if c_in is not None and beta != 0.0 else out_mode)
     elif not accumulate:
         pair = _use_pair(M, N, bn)
     if pair:
@@ -296,7 +299,7 @@ def _gemm_allgather(a, b_shard, info, *, trans_a, trans_b, a2, b2, alpha, beta, 
     out_mode = 0 if out_dtype == torch.bfloat16 else 1
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    bn, pair = _pick_tile(M, N) if bn is None else (bn, _use_pair(M, N, bn))
+    bn, pair = _pick_tile(M, N, (K + 63) // 64 + (K2 + 63) // 64, out_mode) if bn is None else (bn, _use_pair(M, N, bn))
     ctx = info.ctx
     staging, plans = ctx.acquire(info, backward=trans_b)
     plan = None

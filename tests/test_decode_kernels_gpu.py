@@ -381,6 +381,28 @@ def test_gemm_tiles_chosen_below_512_rows(M, N, ta, tb, c_in):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("M,N,K,out,tile", [(1568, 2712, 88, 0, (256, True)), (1304, 3720, 96, 2, (64, False)), (200, 300, 136, 1, (64, False)),
+                                            (3824, 264, 920, 2, (128, False)), (300, 37000, 72, 1, (256, False)), (1032, 1056, 392, 0, (256, True))])
+def test_gemm_tiles_by_waves_and_epilogue(M, N, K, out, tile):
+    """Every tile width by its own rule, with the epilogue that decides for it (bf16, fp32, added to fp32). fp32 sums: 2^-20 of
+    their magnitude, one bf16 rounding more for bf16."""
+    from axolotl_b200.ops import _lib
+    from axolotl_b200.ops.gemm import _pick_tile, gemm
+
+    assert _pick_tile(M, N, (K + 63) // 64, out) == tile
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    if out == 2:
+        c = torch.randn(M, N, device="cuda")
+        ref, mag = ref + c.double(), mag + c.double().abs()
+        got = gemm(a, b, out=c, accumulate=True)
+    else:
+        got = gemm(a, b, out_dtype=torch.float32 if out else torch.bfloat16)
+    _lib.check_status()
+    assert ((got.double() - ref).abs() <= 2 ** -20 * mag + (0 if out else 2 ** -8 * ref.abs())).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 512, 256), (16, 4096, 8192), (48, 1000, 960), (64, 14336, 328), (40, 777 * 8, 1000)])
 @pytest.mark.parametrize("splits", [1, 3])
 def test_gemm_accumulates_the_transposed_tile(M, N, K, splits):
