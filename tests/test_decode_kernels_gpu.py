@@ -340,8 +340,88 @@ def test_decode_layers_in_one_call_match_the_operator_path(name, batch, lora, mo
         assert ((a - b).norm() / b.norm()).item() < 0.012 and torch.isfinite(a).all()
 
 
-def test_decode_step_leaves_other_layers_to_their_own_forward():
-    """A forward hook, an expert layer and a disabled adapter: each keeps (or regains) the path that honours it."""
+# (config, adapter, layers that have to run their own forward)
+_OWN_FORWARD = {
+    "experts beside dense layers": (dict(model_type="qwen3_moe", num_experts=8, num_experts_per_tok=2, moe_intermediate_size=128,
+                                         mlp_only_layers=[0, 2]), None, {1}),
+    "adapters disabled": (dict(), dict(), set()),
+    "adapters merged": (dict(), dict(), set()),
+    "magnitude-decomposed adapters": (dict(), dict(use_dora=True), {0, 1, 2}),
+    "square adapters": (dict(), dict(use_mora=True), {0, 1, 2}),
+    "4-bit weight": (dict(), None, {1}),
+    "partial rotation": (dict(extra=dict(partial_rotary_factor=0.5)), None, {0, 1, 2}),
+    "norms on the branch outputs too": (dict(model_type="glm4"), None, {0, 1, 2}),
+    "norms on the branch outputs only": (dict(model_type="olmo2", qk_norm=True), None, {0, 1, 2}),
+    "attention and MLP side by side": (dict(model_type="cohere"), None, {0, 1, 2}),
+    "scaled branches": (dict(model_type="granite", extra=dict(residual_multiplier=0.5)), None, {0, 1, 2}),
+    "a layer without rotation": (dict(model_type="smollm3", extra=dict(no_rope_layers=[1, 0, 1])), None, {1}),
+    "adapter dropout while training": (dict(), dict(lora_dropout=0.3), {0, 1, 2}),
+}
+
+
+@pytest.mark.parametrize("name", sorted(_OWN_FORWARD))
+def test_decode_step_leaves_other_layers_to_their_own_forward(name, monkeypatch):
+    """Layers that are not of the plain form: which of them refuse the one-call form, and the step's result against a step whose
+    layers all run their own forward (a few bf16 roundings apart where some do not)."""
+    from axolotl_b200.models import decode_step
+    from axolotl_b200.models.config import preset
+    from axolotl_b200.models.kv_cache import KVCache, _DecodeMeta
+    from axolotl_b200.models.layers import FusedLinear, disable_adapters
+    from axolotl_b200.models.lora import ALL_LINEAR, LoraSpec, inject_lora
+    from axolotl_b200.models.transformer import CausalLM
+
+    over, adapter, own = _OWN_FORWARD[name]
+    torch.manual_seed(5)
+    m = CausalLM(preset("tiny-llama", vocab_size=512, num_hidden_layers=3, **over), dtype=torch.bfloat16, device="cuda").init_weights(0).eval()
+    if adapter is not None:
+        inject_lora(m, LoraSpec(r=8, lora_alpha=16, target_modules=list(ALL_LINEAR), **adapter))
+        with torch.no_grad():
+            for n, p in m.named_parameters():
+                if "lora_B" in n or "mora_M" in n:
+                    p.normal_(0, 0.05)
+            for f in m.modules():
+                if getattr(f, "lora_B", None) is not None:
+                    keep = torch.zeros_like(f.lora_B)
+                    for r0, rows, c0, cols in f.lora_blocks:
+                        keep[r0:r0 + rows, c0:c0 + cols] = 1
+                    f.lora_B.mul_(keep)
+        m.refresh_lora_shadows()
+    if name == "adapters merged":
+        for f in m.modules():
+            if isinstance(f, FusedLinear):
+                f.merge_lora_()
+    if name == "4-bit weight":
+        m.layers[1].mlp.down_proj.quantize_nf4_()
+    training = name == "adapter dropout while training"
+    m.train(training)
+    pos = torch.randint(0, 60, (8,), device="cuda")
+    tok = torch.randint(0, 512, (8,), device="cuda")
+    at = m.layers[0].self_attn
+    k, v = torch.randn(2, 3, 8, 64, at.Hk * at.D, device="cuda").bfloat16()
+    done, outs = [], []
+    real = decode_step.DecodeStep.layer
+    monkeypatch.setattr(decode_step.DecodeStep, "layer", lambda self, *a: done.append(real(self, *a) if not force else None) or done[-1])
+    for force in (False, True):
+        cache = KVCache(m, 8, 64)
+        cache.k.copy_(k)
+        cache.v.copy_(v)
+        meta = _DecodeMeta(cache, torch.arange(8, device="cuda"), pos, True)
+        with torch.no_grad():
+            if name == "adapters disabled":
+                with disable_adapters():
+                    o = m(tok[None], pos.int()[None], attn_meta=meta, return_logits=True)
+            else:
+                o = m(tok[None], pos.int()[None], attn_meta=meta, return_logits=True)
+        outs.append((o.logits.float(), cache.k.float(), cache.v.float()))
+    assert {i for i in range(3) if done[i] is None} == own and len(done) == 6
+    for a, b in zip(*outs):
+        assert torch.isfinite(a).all()
+        if not training:
+            assert torch.equal(a, b) if len(own) == 3 else ((a - b).norm() <= 0.012 * b.norm())
+
+
+def test_decode_step_leaves_a_hooked_layer_to_its_own_forward():
+    """A forward hook inside a layer is called on every pass."""
     from axolotl_b200.models.config import preset
     from axolotl_b200.models.kv_cache import generate_cached
     from axolotl_b200.models.transformer import CausalLM
