@@ -436,7 +436,7 @@ struct BwdCfg {
   static constexpr int Q_BYTES = HALVES * Q_HALF;       // Q or dO tile: 64 rows
   static constexpr int PT_BYTES = HALF_BYTES;           // P^T / dS^T: [128 kv x 64 q]
   static constexpr int STAGES = 3;                      // Q / dO: the load of a stage hides behind two iterations
-  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + 4 * PT_BYTES + 1024 /*lse+delta*/ + 256 + 1024 /*alignment*/;
+  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + 4 * PT_BYTES + 1024 /*lse+delta*/ + 256;
   static_assert(SMEM <= 227 * 1024, "");
   static constexpr int ST_COL = 0;     // S^T(b) at ST_COL + 128 b, 64 cols; dQ^T(b) aliases it
   static constexpr int DPT_COL = 64;   // dP^T(b) at DPT_COL + 128 b, 64 cols
@@ -478,8 +478,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   const int n_iter = n_qt * group;
   if (n_iter <= 0) return;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];      // no room for slack: the three stages fill the 227 KB at D = 128
   uint8_t* sK = smem;
   uint8_t* sV = sK + C::KV_BYTES;
   uint8_t* sQ = sV + C::KV_BYTES;                    // [STAGES]
