@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(192, 1)
 }
 
 // =====================================================================================================
-// Backward: 192 threads = TMA warp, MMA warp, one softmax warpgroup. One CTA per (kv head, 128-row kv tile,
+// Backward: 320 threads = TMA warp, MMA warp, two softmax warpgroups. One CTA per (kv head, 128-row kv tile,
 // part); loops over the q heads of the GQA group and the 64-row q tiles that see the kv tile. Per iteration
 //   S^T [kv, q] = K . Q^T (over Dqk)      dP^T [kv, q] = V . dO^T (over Dv)
 //   dV[:, part] += P^T . dO[:, part]      dK[:, part] += dS^T . Q[:, part]

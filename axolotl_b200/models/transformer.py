@@ -885,7 +885,7 @@ class CausalLM(nn.Module):
         from .registry import KV_CACHE, Unsupported, get_model_support
 
         sup = get_model_support(self.config.model_type)
-        kernel_ok = (self.config.head_dim in (64, 128) and not self.config.attn_softcap()      # what the decode kernel takes
+        kernel_ok = (self.config.head_dim in (64, 128) and not self.config.attn_softcap()      # (the decode kernel takes 256 too)
                      and not (sup is not None and isinstance(sup.capabilities.get(KV_CACHE), Unsupported)))
         if use_cache and kernel_ok and getattr(self.hooks, "supports_kv_cache", True) is not False:
             from .kv_cache import generate_cached
