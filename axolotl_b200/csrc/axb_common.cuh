@@ -376,6 +376,12 @@ AXB_DEVICE uint32_t mapa_u32(uint32_t smem_addr, uint32_t rank) {
 AXB_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Arrival on the partner's mbarrier that stands for tiles in THIS CTA's shared memory, which this SM's tensor core reads: the lanes
+// that wrote them have each passed fence.proxy.async, so nothing is left to be made visible to the other CTA, and the default
+// scope of the arrival serves. The release.cluster form waits for every access that the SM has in flight, about 0.3 us of a k block.
+AXB_DEVICE void mbar_arrive_partner(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 AXB_DEVICE void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr),
                "r"(bytes)
@@ -390,6 +396,15 @@ AXB_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tmap, uint32
       "{%3, %4}], [%2];"
       :
       : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+      : "memory");
+}
+AXB_DEVICE void tma_load_3d_pair(void* smem_dst, const CUtensorMap* tmap, uint32_t bar_cluster_addr, int c0,
+                                 int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
+      "{%3, %4, %5}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 AXB_DEVICE void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {

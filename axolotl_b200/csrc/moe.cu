@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(RL_T) route_count_kernel(const long long* __re
 // hist[b][e] becomes the padded row of the first slot of expert e in block b
 __global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__ hist, int blocks, int E, int max_blocks,
                                                                int* __restrict__ seg_start, int* __restrict__ seg_rows,
-                                                               int* __restrict__ blk_expert, int* __restrict__ n_blocks) {
-  __shared__ int warp_sum[32];
+                                                               int* __restrict__ blk_expert, int* __restrict__ n_blocks,
+                                                               int4* __restrict__ passes, int* __restrict__ n_pass) {
+  __shared__ unsigned long long warp_sum[32];
   __shared__ int first[RL_MAX_E + 1];     // first 128-row block of every expert
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
   int count = 0;
@@ -111,32 +112,37 @@ __global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__
 #pragma unroll 8
     for (int b = 0; b < blocks; ++b) count += hist[(long long)b * E + e];
   }
-  const int nb = (count + 127) / 128;
-  int incl = nb;
+  // running sums over the experts: blocks of 128 rows (low word), passes of the NVFP4 GEMM over two blocks (high word)
+  const int nb = (count + 127) / 128, np = (nb + 1) / 2;
+  unsigned long long incl = (unsigned long long)np << 32 | (unsigned)nb;
+  const unsigned long long own = incl;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
   if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    int v = warp_sum[lane];
+    unsigned long long v = warp_sum[lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      const unsigned long long u = __shfl_up_sync(0xffffffffu, v, o);
       if (lane >= o) v += u;
     }
     warp_sum[lane] = v;
   }
   __syncthreads();
-  const int start = incl - nb + (warp ? warp_sum[warp - 1] : 0);
+  const unsigned long long before = incl - own + (warp ? warp_sum[warp - 1] : 0);
+  const int start = (int)(unsigned)before, pass0 = (int)(before >> 32);
   if (e < E) {
     first[e] = start;
     if (e == E - 1) {
       first[E] = start + nb;
       *n_blocks = start + nb;
+      *n_pass = pass0 + np;
     }
+    for (int j = 0; j < np; ++j) passes[pass0 + j] = make_int4(start + 2 * j, e, min(256, count - 256 * j), min(2, nb - 2 * j));
     seg_start[e] = start * 128;
     seg_rows[e] = nb * 128;
     int row = start * 128;
@@ -579,17 +585,20 @@ static int rows_grid(long long n_rows) {
 }
 
 // Layout of a routed batch. expert [n] (n = T * k slots, expert ids), E <= 1024; slot_row [n], row_slot [max_blocks * 128] (slot of
-// a padded row, -1 = pad), seg_start / seg_rows [E], blk_expert [max_blocks], n_blocks [1]; scratch: ceil(n / 1024) * E ints.
-// max_blocks >= ceil(n / 128) + E. A slot with an expert outside [0, E) has no row (slot_row -1) and sets *status.
+// a padded row, -1 = pad), seg_start / seg_rows [E], blk_expert [max_blocks], n_blocks [1]; passes [max_blocks, 4], n_pass [1]: the
+// passes of axb_grouped_gemm_w4a16 (first block, expert, rows in use, blocks), `passes` 16-byte aligned; scratch: ceil(n / 1024) * E
+// ints. max_blocks >= ceil(n / 128) + E. A slot with an expert outside [0, E) has no row (slot_row -1) and sets *status.
 extern "C" int axb_moe_route_layout(const long long* expert, int n, int E, int max_blocks, int* slot_row, int* row_slot,
-                                    int* seg_start, int* seg_rows, int* blk_expert, int* n_blocks, int* scratch, int* status,
-                                    void* stream) {
+                                    int* seg_start, int* seg_rows, int* blk_expert, int* n_blocks, int* passes, int* n_pass,
+                                    int* scratch, int* status, void* stream) {
+  if (reinterpret_cast<uintptr_t>(passes) & 15) return -2;
   if (E < 1 || E > RL_MAX_E || n < 0 || max_blocks < (n + 127) / 128 + E) return -2;
   cudaError_t e = cudaMemsetAsync(row_slot, 0xff, (size_t)max_blocks * 128 * sizeof(int), ST(stream));
   if (e != cudaSuccess) return (int)e;
   const int blocks = (n + RL_T - 1) / RL_T;
   if (blocks > 0) route_count_kernel<<<blocks, RL_T, E * (int)sizeof(int), ST(stream)>>>(expert, scratch, n, E);
-  route_place_kernel<<<1, RL_MAX_E, 0, ST(stream)>>>(scratch, blocks, E, max_blocks, seg_start, seg_rows, blk_expert, n_blocks);
+  route_place_kernel<<<1, RL_MAX_E, 0, ST(stream)>>>(scratch, blocks, E, max_blocks, seg_start, seg_rows, blk_expert, n_blocks,
+                                                     reinterpret_cast<int4*>(passes), n_pass);
   if (blocks > 0) {
     const int smem = 32 * E * (int)sizeof(unsigned short);      // at most 64 KB
     if (smem > 48 * 1024) {

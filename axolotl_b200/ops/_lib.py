@@ -34,8 +34,8 @@ _CUDA_SIGS = {
     "axb_gemm_set_pair_tuning": [i32, i32, i32],
     "axb_nvfp4_dequant": [vp, vp, vp, vp, i64, i64, vp],
     "axb_moe_dispatch_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
-    # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, scratch, status, stream
-    "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp],
+    # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, passes, n_pass, scratch, status, stream
+    "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
     "axb_moe_combine_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_moe_combine_dw": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_nf4_dequant": [vp, vp, vp, i64, i32, vp],
@@ -44,7 +44,7 @@ _CUDA_SIGS = {
     # A, lda, W, A2, lda2, W2, C, ldc, E, N, K, K2, trans_w, alpha, out_mode, bn, blk_expert, n_blocks, max_blocks, status, stream
     "axb_grouped_gemm": [vp, i64, vp, vp, i64, vp, vp, i64, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i32, vp, vp],
     # A, lda, B, ldb, C, ldc, c_batch, E, Mg, Ng, rows, alpha, out_mode, bn, seg_start, seg_rows, status, stream
-    # A, lda, qdata, scale, pts, A2, lda2, W2, C, ldc, E, Wn, Wk, K2, trans_w, alpha, out_mode, blk_expert, n_blocks, max_blocks, status, stream
+    # A, lda, qdata, scale, pts, A2, lda2, W2, C, ldc, E, Wn, Wk, K2, trans_w, alpha, out_mode, passes, n_pass, max_blocks, status, stream
     "axb_grouped_gemm_w4a16": [vp, i64, vp, vp, vp, vp, i64, vp, vp, i64, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, vp],
     "axb_flash_wide_fwd": [vp, i64, i64, i32, i32, i32, i32, i32, i32, i32, vp, i32, vp, i64, vp, f32, f32, vp, vp],
     "axb_flash_wide_bwd": [vp, i64, vp, vp, i64, vp, i64, i32, i32, i32, i32, i32, i32, i32, vp, i32, vp, i64, vp, vp,

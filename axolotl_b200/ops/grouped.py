@@ -57,6 +57,18 @@ class GroupLayout:
         self.seg_start = seg_start.to(torch.int32)
         self.seg_rows = padded.to(torch.int32)
 
+    @functools.cached_property
+    def passes(self):
+        """(int32 [max_blocks, 4], count): the passes of the NVFP4 GEMM, (first row block, expert, rows in use, row blocks) of every
+        two row blocks of an expert."""
+        b = torch.arange(self.max_blocks, device=self.blk_expert.device)
+        e = self.blk_expert.long()
+        at = b - self.seg_start[e] // BLOCK                                   # place of the block among its expert's
+        blocks = torch.minimum(self.seg_rows[e] // BLOCK - at, self.n_blocks - b).clamp(max=2)
+        starts = (at % 2 == 0) & (b < self.n_blocks)
+        table = torch.stack([b, e, blocks * BLOCK, blocks], 1).to(torch.int32)
+        return table[torch.argsort(~starts, stable=True)], starts.sum(dtype=torch.int32).view(1)
+
     def pad(self, x_sorted):
         out = x_sorted.new_zeros((self.max_rows, x_sorted.shape[1]))
         return out.index_copy(0, self.dest, x_sorted)
@@ -137,8 +149,8 @@ def grouped_gemm_w4a16(a, q, lay: GroupLayout, *, trans_w=False, a2=None, w2=Non
         a.data_ptr(), a.stride(0), q["qdata"].data_ptr(), q["scale"].data_ptr(), _pts32(q).data_ptr(),
         a2.data_ptr() if a2 is not None else None, a2.stride(0) if a2 is not None else 0,
         w2.data_ptr() if w2 is not None else None, out.data_ptr(), out.stride(0), E, Wn, Wk, K2,
-        1 if trans_w else 0, float(alpha), 0 if out_dtype == torch.bfloat16 else 1, lay.blk_expert.data_ptr(),
-        lay.n_blocks.data_ptr(), lay.max_blocks, _lib.status_word().data_ptr(), _lib.stream_ptr()), "grouped_gemm_w4a16")
+        1 if trans_w else 0, float(alpha), 0 if out_dtype == torch.bfloat16 else 1, lay.passes[0].data_ptr(),
+        lay.passes[1].data_ptr(), lay.max_blocks, _lib.status_word().data_ptr(), _lib.stream_ptr()), "grouped_gemm_w4a16")
     return out
 
 
@@ -314,17 +326,19 @@ class RoutedLayout(GroupLayout):
         self.max_blocks = (n + BLOCK - 1) // BLOCK + E
         self.max_rows = self.max_blocks * BLOCK
         chunks = (n + 1023) // 1024
-        sizes = [n, self.max_rows, E, E, self.max_blocks, 1, chunks * E]
+        sizes = [n, self.max_rows, E, E, self.max_blocks, 1, 4 * self.max_blocks, 1, chunks * E]
         at = [0]
         for s in sizes:
             at.append(at[-1] + (s + 3) // 4 * 4)
         buf = torch.empty(at[-1], dtype=torch.int32, device=idx.device)
-        (self.slot_row, self.row_slot, self.seg_start, self.seg_rows, self.blk_expert, self.n_blocks,
+        (self.slot_row, self.row_slot, self.seg_start, self.seg_rows, self.blk_expert, self.n_blocks, passes, n_pass,
          scratch) = (buf[a:a + s] for a, s in zip(at, sizes))
         _lib.check_rc(_lib.cuda_lib().axb_moe_route_layout(
             flat_e.data_ptr(), n, E, self.max_blocks, self.slot_row.data_ptr(), self.row_slot.data_ptr(), self.seg_start.data_ptr(),
-            self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), scratch.data_ptr(),
+            self.seg_rows.data_ptr(), self.blk_expert.data_ptr(), self.n_blocks.data_ptr(), passes.data_ptr(), n_pass.data_ptr(),
+            scratch.data_ptr(),
             _lib.status_word(idx.device).data_ptr(), _lib.stream_ptr()), "moe_route_layout")
+        self.passes = passes.view(-1, 4), n_pass          # rows in use: the slots alone, the rows that pad a segment are zero
 
     @functools.cached_property
     def dest(self):

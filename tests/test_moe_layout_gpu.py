@@ -3,6 +3,8 @@ import pytest
 import torch
 
 from axolotl_b200.ops import _lib
+from axolotl_b200.ops.grouped import BLOCK, GroupLayout, RoutedLayout, grouped_gemm, grouped_gemm_w4a16
+from axolotl_b200.ops.nvfp4 import dequantize_nvfp4, quantize_nvfp4
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +125,44 @@ def test_transpose_modes(R, C):
                             (1, base.clone(), base + a.t()), (2, torch.empty(C, R, device="cuda"), a.t())):
         _lib.check_rc(_lib.cuda_lib().axb_transpose(a.data_ptr(), dst.data_ptr(), R, C, mode, _lib.stream_ptr()), "transpose")
         assert torch.equal(dst, want)
+
+
+@pytest.mark.parametrize("counts", [[1, 31, 32, 33, 0, 127, 128, 129], [255, 256, 257, 0, 385], [0, 3], [700]])
+def test_passes_of_a_routed_layout(counts):
+    """Every row block is in one pass of its expert; the table that the placing kernel writes holds the passes that the general one
+    gives, with the rows in use instead of whole blocks."""
+    E, T = len(counts), sum(counts)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T)].view(T, 1).cuda()
+    lay = RoutedLayout(idx, E)
+    got, n = lay.passes[0].cpu(), int(lay.passes[1])
+    ref, n_ref = GroupLayout.passes.func(lay)
+    assert n == int(n_ref) == sum(-(-c // 256) for c in counts)
+    assert torch.equal(got[:n, [0, 1, 3]], ref.cpu()[:n, [0, 1, 3]])
+    assert got[:n, 2].tolist() == [min(256, c - a) for c in counts for a in range(0, c, 256)]
+
+
+@pytest.mark.parametrize("N,K,r", [(8, 64, 0), (136, 64, 16), (264, 192, 8), (512, 320, 16)])
+def test_grouped_w4a16_rows_in_use(N, K, r):
+    """Passes of few rows, short sums (fewer k blocks than converter groups), columns that end inside a tile and negative block scales:
+    the bits of the bf16 stack in the grouped GEMM, and zeros in the rows that pad a segment."""
+    counts = [1, 31, 0, 33, 129, 255, 257, 64, 0, 128]
+    E, T = len(counts), sum(counts)
+    torch.manual_seed(N)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).view(T, 1).cuda()
+    lay = RoutedLayout(idx, E)
+    qd, sc, pts = quantize_nvfp4(torch.randn(E, N, K) * 0.05)
+    sc = (sc.float() * torch.where(torch.rand(sc.shape) < 0.1, -1.0, 1.0)).to(sc.dtype)
+    q = {"qdata": qd.cuda(), "scale": sc.cuda(), "pts": pts.cuda()}
+    W = dequantize_nvfp4(q["qdata"], q["scale"], q["pts"])
+    pad = lambda c, s=0.5: torch.where(lay.row_slot[:, None] >= 0, torch.randn(lay.max_rows, c, device="cuda") * s, 0.0).bfloat16()  # noqa: E731
+    x, dy, t = pad(K), pad(N), pad(max(r, 8))
+    A16, Bt = (torch.randn(E, r, K, device="cuda") * 0.05).bfloat16(), (torch.randn(E, N, r, device="cuda") * 0.05).bfloat16()
+    ext = lambda w: dict(a2=t[:, :r].contiguous(), w2=w) if r else {}  # noqa: E731
+    used = int(lay.n_blocks) * BLOCK
+    empty = lay.row_slot[:used] < 0
+    for got, ref in ((grouped_gemm_w4a16(x, q, lay, **ext(Bt)), grouped_gemm(x, W, lay, **ext(Bt))),
+                     (grouped_gemm_w4a16(dy, q, lay, trans_w=True, **ext(A16)), grouped_gemm(dy, W, lay, trans_w=True, **ext(A16)))):
+        _lib.check_status()
+        assert torch.equal(got[:used], ref[:used]) and not got[:used][empty].any()
+    y32 = grouped_gemm_w4a16(x, q, lay, out_dtype=torch.float32)[:used]
+    assert torch.equal(y32.bfloat16(), grouped_gemm(x, W, lay)[:used])
