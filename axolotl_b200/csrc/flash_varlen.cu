@@ -32,7 +32,7 @@ struct AttnParams {
   int* status;
   // backward only
   const float* delta;  // [Hq, T]
-  float* dq_acc;       // [T, Hq*D] fp32, accumulated with atomics
+  float* dq_acc;       // T * Hq * D fp32 in the order of dq_at, accumulated with reductions
   __nv_bfloat16* dkv;  // fused gradient buffer, same layout as qkv (k and v blocks are written)
   long long dkv_ld;
   float scale;
@@ -56,6 +56,29 @@ AXB_DEVICE float fast_exp2(float x) {
   float y;
   asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// two fp32 values in a register pair: one instruction each, rounded like the scalar ones
+AXB_DEVICE uint64_t pack_b32x2(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+AXB_DEVICE uint64_t pack_f32x2(float a, float b) { return pack_b32x2(__float_as_uint(a), __float_as_uint(b)); }
+AXB_DEVICE float2 unpack_f32x2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+AXB_DEVICE uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+AXB_DEVICE uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // byte offset of 8 consecutive bf16 (one 16-byte chunk) inside a [128 x 64] bf16 SW128 tile
@@ -413,6 +436,20 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   if (h < nh && t0 + t < T) delta[(long long)(h0 + h) * T + t0 + t] = s[h][t];
 }
 
+// Where the fp32 sum of dQ[row][col] stands (col = head * D + d, rows of `width`): four rows of a column side by side, so that the
+// thread that owns the column adds them with one 16-byte reduction, and a warp 512 contiguous bytes. The last rows % 4 rows are plain.
+AXB_DEVICE long long dq_at(long long row, long long col, long long width, long long rows4) {
+  return row < rows4 ? (row & ~3ll) * width + col * 4 + (row & 3) : row * width + col;
+}
+AXB_DEVICE void red_add_f32x4(float* to, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(__uint_as_float(a)), "f"(__uint_as_float(b)),
+               "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
+               : "memory");
+}
+AXB_DEVICE void red_add_f32x2(float* to, uint32_t a, uint32_t b) {
+  asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(to), "f"(__uint_as_float(a)), "f"(__uint_as_float(b)) : "memory");
+}
+
 // One CTA per (kv tile of 128 rows, kv head). Inner loop over the q heads of the GQA group and
 // over 64-row q tiles at or below the diagonal. Every MMA has M = 128:
 //   S^T  [kv, q]  = K . Q^T        dP^T [kv, q] = V . dO^T
@@ -427,7 +464,7 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 // exponentials the kernel took the same time. So nothing waits for memory inside the chain: Q / dO run three stages ahead,
 // lse and delta are requested an iteration early, and the columns of dQ^T are handed back once they are in registers, before
 // the sums leave. One 16384-token document, 32 / 8 heads of 128: 8.60 -> 6.31 ms (872 TFLOP/s), 4 x 2048: 0.71 -> 0.56 ms.
-constexpr int kBwdThreads = 320;  // TMA warp, MMA warp, 2 x 4 softmax warps
+constexpr int kBwdThreads = 576;  // TMA warp, MMA warp, 4 x 4 softmax warps
 template <int D>
 struct BwdCfg {
   static constexpr int HALVES = D / 64;
@@ -436,7 +473,7 @@ struct BwdCfg {
   static constexpr int Q_BYTES = HALVES * Q_HALF;       // Q or dO tile: 64 rows
   static constexpr int PT_BYTES = HALF_BYTES;           // P^T / dS^T: [128 kv x 64 q]
   static constexpr int STAGES = 3;                      // Q / dO: the load of a stage hides behind two iterations
-  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + 4 * PT_BYTES + 1024 /*lse+delta*/ + 256;
+  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + 4 * PT_BYTES + 2048 /*lse+delta*/ + 256;
   static_assert(SMEM <= 227 * 1024, "");
   static constexpr int ST_COL = 0;     // S^T(b) at ST_COL + 128 b, 64 cols; dQ^T(b) aliases it
   static constexpr int DPT_COL = 64;   // dP^T(b) at DPT_COL + 128 b, 64 cols
@@ -487,16 +524,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   uint8_t* sdO = sQ + C::STAGES * C::Q_BYTES;        // [STAGES]
   uint8_t* sPT = sdO + C::STAGES * C::Q_BYTES;       // [2]
   uint8_t* sdST = sPT + 2 * C::PT_BYTES;             // [2]
-  float* s_lse = reinterpret_cast<float*>(sdST + 2 * C::PT_BYTES);  // [2][64]
-  float* s_delta = s_lse + 128;                                     // [2][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_delta + 128);
+  float* s_rows = reinterpret_cast<float*>(sdST + 2 * C::PT_BYTES);  // per warpgroup: two buffers of -lse [32], -delta * scale [32]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_rows + 4 * 2 * 64);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;    // [STAGES]  (Q and dO of a stage)
   uint64_t* q_empty = bars + 4;   // [STAGES]
   uint64_t* s_full = bars + 7;    // [2]  S^T(b) and dP^T(b) ready
   uint64_t* pt_full = bars + 9;   // [2]  P^T(b) / dS^T(b) written to smem
-  uint64_t* dq_full = bars + 11;  // [2]  dQ^T(b) ready (and every MMA reading P^T(b)/dS^T(b) retired)
-  uint64_t* st_free = bars + 13;  // [2]  dQ^T(b) in registers: TMEM and smem buffers b reusable
+  uint64_t* dq_full = bars + 11;  // [2]  dQ^T(b) ready (the MMAs that read P^T(b)/dS^T(b) retire before s_full of the next use)
+  uint64_t* st_free = bars + 13;  // [2]  dQ^T(b) in registers: TMEM columns of b reusable
   uint64_t* acc_full = bars + 15; // dK / dV final
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
@@ -509,9 +545,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&s_full[b], 1);
-      mbar_init(&pt_full[b], 128);
+      mbar_init(&pt_full[b], 256);
       mbar_init(&dq_full[b], 1);
-      mbar_init(&st_free[b], 128);
+      mbar_init(&st_free[b], 256);
     }
     mbar_init(acc_full, 1);
     mbar_fence_init();
@@ -613,6 +649,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       if (!warp_all(mbar_wait(&pt_full[b], ph, p.status, AXB_TIMEOUT_GENERIC))) break;
       tc_fence_after();
       if (elect_one()) {
+        // dQ^T [d, q] = K^T . dS^T over the 128 kv rows (8 K-steps of 16), into the columns of S^T(b). First, so that it is drained
+        // while dV and dK run: the next scores but one wait for those columns.
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          umma_f16(tmem_base + C::ST_COL + 128 * b, dk_mn + kk * (2048 / 16), dst + kk * (2048 / 16), idesc_dq, kk > 0);
+        umma_commit(&dq_full[b]);
         // reduce over the 64 q rows of this tile: 4 K-steps of 16
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)   // dV += P^T . dO   (B = dO tile, MN-major: chunk stride = one 64x64 half)
@@ -621,11 +663,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         for (int kk = 0; kk < 4; ++kk)
           umma_f16(tmem_base + C::DK_COL, ds + kk * 2, dq + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
         umma_commit(&q_empty[st]);
-        // dQ^T [d, q] = K^T . dS^T over the 128 kv rows (8 K-steps of 16), into the columns of S^T(b)
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem_base + C::ST_COL + 128 * b, dk_mn + kk * (2048 / 16), dst + kk * (2048 / 16), idesc_dq, kk > 0);
-        umma_commit(&dq_full[b]);
         if (it == n_iter - 1) umma_commit(acc_full);
       }
       __syncwarp();
@@ -633,42 +670,71 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     }
   } else {
     const int lg = warp & 3;
-    const int grp = (warp - 2) >> 2;   // softmax warpgroup: handles iterations with it % 2 == grp
+    const int wg = (warp - 2) >> 2;    // softmax warpgroup: 32 q columns of the iterations with it % 2 == grp
+    const int grp = wg >> 1, c0 = (wg & 1) * 32;
     const int r = lg * 32 + lane;      // kv row in tile (S^T, dP^T, dK, dV) or d row (dQ^T)
-    const int st_tid = threadIdx.x - 64 - grp * 128;  // 0..127 inside the warpgroup
+    const int st_tid = threadIdx.x - 64 - wg * 128;  // 0..127 inside the warpgroup
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
-    const uint32_t st_col = C::ST_COL + 128 * grp, dpt_col = C::DPT_COL + 128 * grp;
+    const uint32_t st_addr = tmem_base + lane_off + C::ST_COL + 128 * grp + c0, dpt_addr = tmem_base + lane_off + C::DPT_COL + 128 * grp + c0;
     uint8_t* my_pt = sPT + grp * C::PT_BYTES;
     uint8_t* my_dst = sdST + grp * C::PT_BYTES;
-    const float* lse = s_lse + grp * 64;
-    const float* dlt = s_delta + grp * 64;
+    float* const rows = s_rows + wg * 128;
     bool ok = true;
-    // -lse (so that P = exp2(S * sl2 + nlse)) or delta * scale of one q row of iteration `it`; rows outside the document
+    // -lse (so that P = exp2(S * sl2 + nlse)) or -delta * scale of one q row of iteration `it`; rows outside the document
     // or outside this rank's q window get nlse = -inf -> P = 0. Requested an iteration ahead: the trip to L2 would stand
     // in the chain from one dQ^T to the next scores otherwise.
     auto fetch_row = [&](int it) -> float {
-      float val = st_tid < 64 ? -INFINITY : 0.f;
-      if (it >= n_iter) return val;
-      const int q = (q_first + it % n_qt) * 64 + (st_tid & 63);
+      float val = st_tid < 32 ? -INFINITY : 0.f;
+      if (it >= n_iter || st_tid >= 64) return val;
+      const int q = (q_first + it % n_qt) * 64 + c0 + (st_tid & 31);
       const long long lrow = (long long)doc_start + q - p.q_row_off;
       if (q < doc_len && lrow >= 0 && lrow < p.q_rows) {
         const long long off = (long long)(head0 + it / n_qt) * p.q_rows + lrow;
-        val = st_tid < 64 ? -p.lse2[off] : p.delta[off] * p.scale;
+        val = st_tid < 32 ? -p.lse2[off] : -p.delta[off] * p.scale;
       }
       return val;
     };
+    // P^T and dS^T of 32 columns, two at a time (packed fp32 arithmetic rounds like the scalar one)
+    const uint64_t sl2 = pack_f32x2(p.sl2, p.sl2), scale2 = pack_f32x2(p.scale, p.scale);
+    auto gradients = [&](auto masked, const uint32_t (&sr)[32], const uint32_t (&dr)[32], const float* nlse, int qc0, int q_lo, int q_hi) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t pk[4], dk[4];
+#pragma unroll
+        for (int i = q * 8; i < q * 8 + 8; i += 4) {
+          const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(nlse + i), ds = *reinterpret_cast<const ulonglong2*>(nlse + 32 + i);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = i + 2 * h;
+            const float2 x = unpack_f32x2(fma_f32x2(pack_b32x2(sr[j], sr[j + 1]), sl2, h ? nl.y : nl.x));
+            float p0 = fast_exp2(x.x), p1 = fast_exp2(x.y);
+            if (decltype(masked)::value) {
+              if (qc0 + j < q_lo || qc0 + j > q_hi) p0 = 0.f;
+              if (qc0 + j + 1 < q_lo || qc0 + j + 1 > q_hi) p1 = 0.f;
+            }
+            const float2 d = unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), fma_f32x2(pack_b32x2(dr[j], dr[j + 1]), scale2, h ? ds.y : ds.x)));
+            pk[((i & 4) >> 1) + h] = pack_bf16x2(p0, p1);
+            dk[((i & 4) >> 1) + h] = pack_bf16x2(d.x, d.y);
+          }
+        }
+        const uint32_t off = sw128_chunk_off(r, c0 / 8 + q);
+        *reinterpret_cast<uint4*>(my_pt + off) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        *reinterpret_cast<uint4*>(my_dst + off) = make_uint4(dk[0], dk[1], dk[2], dk[3]);
+      }
+    };
+    float* const dq_col = p.dq_acc + ((long long)r << 2);      // four rows of a column lie side by side, see dq_at
+    const long long width = (long long)p.Hq * D, rows4 = p.q_rows & ~3;
     float row_val = fetch_row(grp);
+    if (st_tid < 64) rows[st_tid] = row_val;
+    row_val = fetch_row(grp + 2);
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
     for (int it = grp; it < n_iter && ok; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int head = head0 + it / n_qt;
       const int qt0 = (q_first + it % n_qt) * 64;  // doc-relative first q row of the tile
-      // stage lse / delta of the 64 q rows (one buffer per warpgroup; the previous iteration of
-      // this group finished reading it before its threads got here: bar.sync below orders that)
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-      ((st_tid < 64 ? s_lse : s_delta) + grp * 64)[st_tid & 63] = row_val;
-      row_val = fetch_row(it + 2);
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      const int qc0 = qt0 + c0;                    // ... and of this group's columns
+      const float* nlse = rows + ph * 64;
       if (!mbar_wait(&s_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
@@ -676,52 +742,30 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       tc_fence_after();
       // Only tiles that touch the diagonal or the end of the document need per-element masks
       // (q rows outside the document already carry nlse = -inf, i.e. P = 0).
-      const bool need_mask = (!bidir && qt0 < kv0 + 127) || (kv0 + 128 > doc_len) || (win > 0 && qt0 + 63 >= kv0 + win);
-      const bool row_in_doc = kv_idx < doc_len;
-      // q rows that see this thread's kv row: [q_lo, q_hi] (empty for kv rows beyond the document)
-      const int q_lo = row_in_doc ? (bidir ? -(1 << 30) : kv_idx) : (1 << 30);
-      const int q_hi = win > 0 ? kv_idx + win - 1 : (1 << 30);
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      const bool need_mask = (!bidir && qc0 < kv0 + 127) || (kv0 + 128 > doc_len) || (win > 0 && qc0 + 31 >= kv0 + win);
+      {
         uint32_t sr[32], dr[32];
-        tmem_ld_32x32(tmem_base + lane_off + st_col + c * 32, sr);
-        tmem_ld_32x32(tmem_base + lane_off + dpt_col + c * 32, dr);
+        tmem_ld_32x32(st_addr, sr);
+        tmem_ld_32x32(dpt_addr, dr);
         tmem_ld_wait();
-        uint32_t pk[16], dk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 nl = *reinterpret_cast<const float4*>(lse + c * 32 + i);
-          const float4 ds = *reinterpret_cast<const float4*>(dlt + c * 32 + i);
-          const float nlv[4] = {nl.x, nl.y, nl.z, nl.w};
-          const float dsv[4] = {ds.x, ds.y, ds.z, ds.w};
-          float pv[4], dv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float pr = fast_exp2(fmaf(__uint_as_float(sr[i + e]), p.sl2, nlv[e]));
-            if (need_mask) {
-              const int q = qt0 + c * 32 + i + e;
-              if (q < q_lo || q > q_hi) pr = 0.f;
-            }
-            pv[e] = pr;
-            dv[e] = pr * fmaf(__uint_as_float(dr[i + e]), p.scale, -dsv[e]);
-          }
-          pk[i >> 1] = pack_bf16x2(pv[0], pv[1]);
-          pk[(i >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
-          dk[i >> 1] = pack_bf16x2(dv[0], dv[1]);
-          dk[(i >> 1) + 1] = pack_bf16x2(dv[2], dv[3]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t off = sw128_chunk_off(r, c * 4 + q);
-          *reinterpret_cast<uint4*>(my_pt + off) =
-              make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
-          *reinterpret_cast<uint4*>(my_dst + off) =
-              make_uint4(dk[q * 4], dk[q * 4 + 1], dk[q * 4 + 2], dk[q * 4 + 3]);
+        if (need_mask) {
+          const bool row_in_doc = kv_idx < doc_len;
+          // q rows that see this thread's kv row: [q_lo, q_hi] (empty for kv rows beyond the document)
+          const int q_lo = row_in_doc ? (bidir ? -(1 << 30) : kv_idx) : (1 << 30);
+          const int q_hi = win > 0 ? kv_idx + win - 1 : (1 << 30);
+          gradients(std::true_type{}, sr, dr, nlse, qc0, q_lo, q_hi);
+        } else {
+          gradients(std::false_type{}, sr, dr, nlse, 0, 0, 0);
         }
       }
       tc_fence_before();
       fence_proxy_async_smem();
       mbar_arrive(&pt_full[grp]);
+      // lse / delta of this group's next iteration into the other buffer, while the MMAs run; the barrier also says that all warps of
+      // the group have read the present one
+      if (st_tid < 64) rows[(ph ^ 1) * 64 + st_tid] = row_val;
+      row_val = fetch_row(it + 4);
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
       // drain dQ^T: this thread owns d = r (only rows < D are meaningful)
       if (!mbar_wait(&dq_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
@@ -729,36 +773,53 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       }
       tc_fence_after();
       {
-        // valid q columns of this tile: inside the document and inside this rank's q window
-        const long long row0 = (long long)doc_start + qt0 - p.q_row_off;   // local row of column 0
+        // valid q columns of this group: inside the document and inside this rank's q window
+        const long long row0 = (long long)doc_start + qc0 - p.q_row_off;   // local row of column 0
         int i_lo = row0 < 0 ? (int)(-row0) : 0;
-        int i_hi = min(64, doc_len - qt0);
+        int i_hi = min(32, doc_len - qc0);
         if (row0 + i_hi > p.q_rows) i_hi = (int)(p.q_rows - row0);
-        float* col = p.dq_acc + row0 * p.out_ld + (long long)head * D + r;
-        uint32_t qr[64];
-        {
-          uint32_t(&q0)[32] = *reinterpret_cast<uint32_t(*)[32]>(&qr[0]);
-          uint32_t(&q1)[32] = *reinterpret_cast<uint32_t(*)[32]>(&qr[32]);
-          tmem_ld_32x32(tmem_base + lane_off + st_col, q0);
-          tmem_ld_32x32(tmem_base + lane_off + st_col + 32, q1);
-          tmem_ld_wait();
-        }
+        uint32_t qr[32];
+        tmem_ld_32x32(st_addr, qr);
+        tmem_ld_wait();
         tc_fence_before();
         mbar_arrive(&st_free[grp]);      // the next scores may overwrite the columns while the sums leave
         if (r < D) {
-          if (i_lo <= 0 && i_hi >= 64) {
+          float* col = dq_col + (long long)head * (4 * D);
+          const bool whole = i_lo <= 0 && i_hi >= 32 && row0 + 32 <= rows4;
+          if (whole && (row0 & 3) == 0) {
+            float* to = col + row0 * width;
 #pragma unroll
-            for (int i = 0; i < 64; ++i) atomicAdd(col + (long long)i * p.out_ld, __uint_as_float(qr[i]));
+            for (int i = 0; i < 32; i += 4) red_add_f32x4(to + i * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
+          } else if (whole && (row0 & 3) == 2) {
+            float* to = col + (row0 - 2) * width;
+            red_add_f32x2(to + 2, qr[0], qr[1]);
+#pragma unroll
+            for (int i = 2; i < 30; i += 4) red_add_f32x4(to + (i + 2) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
+            red_add_f32x2(to + 32 * width, qr[30], qr[31]);
+          } else if (whole && (row0 & 3) == 1) {
+            float* to = col + (row0 - 1) * width;
+            atomicAdd(to + 1, __uint_as_float(qr[0]));
+            red_add_f32x2(to + 2, qr[1], qr[2]);
+#pragma unroll
+            for (int i = 3; i < 31; i += 4) red_add_f32x4(to + (i + 1) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
+            atomicAdd(to + 32 * width, __uint_as_float(qr[31]));
+          } else if (whole) {
+            float* to = col + (row0 - 3) * width;
+            atomicAdd(to + 3, __uint_as_float(qr[0]));
+#pragma unroll
+            for (int i = 1; i < 29; i += 4) red_add_f32x4(to + (i + 3) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
+            red_add_f32x2(to + 32 * width, qr[29], qr[30]);
+            atomicAdd(to + 32 * width + 2, __uint_as_float(qr[31]));
           } else {
 #pragma unroll
-            for (int i = 0; i < 64; ++i)
-              if (i >= i_lo && i < i_hi) atomicAdd(col + (long long)i * p.out_ld, __uint_as_float(qr[i]));
+            for (int i = 0; i < 32; ++i)
+              if (i >= i_lo && i < i_hi) atomicAdd(p.dq_acc + dq_at(row0 + i, (long long)head * D + r, width, rows4), __uint_as_float(qr[i]));
           }
         }
       }
     }
-    // final dK / dV (warpgroup 0)
-    if (grp == 0 && ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+    // final dK / dV: 32 columns of each per warpgroup
+    if (wg < D / 32 && ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const bool row_ok = kv_idx < doc_len && n_iter > 0;
       const long long grow = (long long)doc_start + kv_idx;  // global kv row
@@ -771,8 +832,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       }
       __nv_bfloat16* krow = base + brow * p.dkv_ld + p.dk_col0 + (long long)kv_head * D;
       __nv_bfloat16* vrow = base + brow * p.dkv_ld + p.dv_col0 + (long long)kv_head * D;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
+      {
+        const int c = wg;
         uint32_t a[32], b[32];
         tmem_ld_32x32(tmem_base + lane_off + C::DK_COL + c * 32, a);
         tmem_ld_32x32(tmem_base + lane_off + C::DV_COL + c * 32, b);
@@ -815,20 +876,30 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   }
 }
 
-// dq (bf16, q block of the fused gradient buffer) = dq_acc (fp32)
-__global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv,
-                                  long long T, int width, long long acc_ld, long long ld,
-                                  int q_col0) {
-  const long long n = T * (width / 4);
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (long long)gridDim.x * blockDim.x) {
-    const long long t = v / (width / 4);
-    const int c = (int)(v % (width / 4)) * 4;
-    const float4 f = *reinterpret_cast<const float4*>(acc + t * acc_ld + c);
-    uint2 u;
-    u.x = pack_bf16x2(f.x, f.y);
-    u.y = pack_bf16x2(f.z, f.w);
-    *reinterpret_cast<uint2*>(dqkv + t * ld + q_col0 + c) = u;
+// dq (bf16, q block of the fused gradient buffer) = dq_acc (fp32): a thread takes 8 columns of the four rows that lie side by side
+__global__ void __launch_bounds__(256) dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv, long long T, int width,
+                                                         long long ld, int q_col0) {
+  const int vecs = width / 8;
+  const long long T4 = T & ~3ll, n = T4 / 4 * vecs + (T - T4) * vecs;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    const long long t = v / vecs;
+    const int c = (int)(v - t * vecs) * 8;
+    if (t < T4 / 4) {
+      const float4* src = reinterpret_cast<const float4*>(acc + t * 4 * width) + c;
+      float4 f[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = src[i];
+      __nv_bfloat16* dst = dqkv + t * 4 * ld + q_col0 + c;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(f[0].x, f[1].x), pack_bf16x2(f[2].x, f[3].x), pack_bf16x2(f[4].x, f[5].x), pack_bf16x2(f[6].x, f[7].x));
+      *reinterpret_cast<uint4*>(dst + ld) = make_uint4(pack_bf16x2(f[0].y, f[1].y), pack_bf16x2(f[2].y, f[3].y), pack_bf16x2(f[4].y, f[5].y), pack_bf16x2(f[6].y, f[7].y));
+      *reinterpret_cast<uint4*>(dst + 2 * ld) = make_uint4(pack_bf16x2(f[0].z, f[1].z), pack_bf16x2(f[2].z, f[3].z), pack_bf16x2(f[4].z, f[5].z), pack_bf16x2(f[6].z, f[7].z));
+      *reinterpret_cast<uint4*>(dst + 3 * ld) = make_uint4(pack_bf16x2(f[0].w, f[1].w), pack_bf16x2(f[2].w, f[3].w), pack_bf16x2(f[4].w, f[5].w), pack_bf16x2(f[6].w, f[7].w));
+    } else {
+      const long long row = T4 + (t - T4 / 4);
+      const float* src = acc + row * width + c;
+      *reinterpret_cast<uint4*>(dqkv + row * ld + q_col0 + c) =
+          make_uint4(pack_bf16x2(src[0], src[1]), pack_bf16x2(src[2], src[3]), pack_bf16x2(src[4], src[5]), pack_bf16x2(src[6], src[7]));
+    }
   }
 }
 
@@ -946,7 +1017,6 @@ int flash_bwd_impl(const AttnGeom& g, const void* dout, const void* out, long lo
   p.q_col0 = q_col0;
   p.k_col0 = k_col0;
   p.v_col0 = v_col0;
-  p.out_ld = (long long)Hq * D;  // leading dimension of dq_acc
   p.lse2 = const_cast<float*>(lse2);
   p.T = T;
   p.kv_rows = g.kv_rows;
@@ -975,10 +1045,9 @@ int flash_bwd_impl(const AttnGeom& g, const void* dout, const void* out, long lo
   for (int i = 0; i < 8; ++i) p.cp_dkv_ptrs[i] = (cp_world > 1 && i < cp_world) ? cp_dkv_ptrs[i] : 0ull;
   int rc = D == 128 ? launch_bwd<128>(tkv, tq, tdo, p, st) : launch_bwd<64>(tkv, tq, tdo, p, st);
   if (rc) return rc;
-  const long long n = T * (long long)(Hq * D / 4);
-  int grid = (int)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
-  dq_convert_kernel<<<grid, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, T, Hq * D, (long long)Hq * D, dqkv_ld,
-                                          dq_col0);
+  const long long n = (T / 4 + T % 4) * (Hq * D / 8);
+  const int grid = (int)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
+  dq_convert_kernel<<<grid, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, T, Hq * D, dqkv_ld, dq_col0);
   return (int)cudaGetLastError();
 }
 
@@ -997,7 +1066,7 @@ extern "C" int axb_flash_varlen_fwd(const void* qkv, long long ld, long long T, 
 }
 
 // Backward. dout/out: [T, o_ld] bf16; dqkv: fused gradient buffer with the layout of qkv (all
-// three blocks are written); dq_acc: fp32 [T, Hq*D] scratch (zeroed here); delta: fp32 [Hq, T]
+// three blocks are written); dq_acc: T * Hq * D fp32 of scratch (zeroed here; 16-byte aligned); delta: fp32 [Hq, T]
 // scratch. tiles must have been built with 128-row tiles.
 extern "C" int axb_flash_varlen_bwd(const void* qkv, long long ld, const void* dout,
                                     const void* out, long long o_ld, const float* lse2,
