@@ -436,34 +436,28 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   if (h < nh && t0 + t < T) delta[(long long)(h0 + h) * T + t0 + t] = s[h][t];
 }
 
-// Where the fp32 sum of dQ[row][col] stands (col = head * D + d, rows of `width`): four rows of a column side by side, so that the
-// thread that owns the column adds them with one 16-byte reduction, and a warp 512 contiguous bytes. The last rows % 4 rows are plain.
+// Where the fp32 sum of dQ[row][col] stands (col = head * D + d, rows of `width`): four rows of a column side by side, so that a
+// warp's 32 columns are 512 contiguous bytes of every group of four rows. The last rows % 4 rows are plain.
 AXB_DEVICE long long dq_at(long long row, long long col, long long width, long long rows4) {
   return row < rows4 ? (row & ~3ll) * width + col * 4 + (row & 3) : row * width + col;
 }
-AXB_DEVICE void red_add_f32x4(float* to, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(__uint_as_float(a)), "f"(__uint_as_float(b)),
-               "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
-               : "memory");
-}
-AXB_DEVICE void red_add_f32x2(float* to, uint32_t a, uint32_t b) {
-  asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(to), "f"(__uint_as_float(a)), "f"(__uint_as_float(b)) : "memory");
-}
-
 // One CTA per (kv tile of 128 rows, kv head). Inner loop over the q heads of the GQA group and
 // over 64-row q tiles at or below the diagonal. Every MMA has M = 128:
 //   S^T  [kv, q]  = K . Q^T        dP^T [kv, q] = V . dO^T
 //   dV   [kv, d] += P^T . dO       dK   [kv, d] += dS^T . Q
-//   dQ^T [d,  q]  = K^T . dS^T     (drained with fp32 atomics into dq_acc)
-// Two softmax warpgroups alternate iterations: S^T / dP^T (TMEM) and P^T / dS^T (shared memory)
-// are double buffered, so the tensor core computes S^T, dP^T of iteration i+1 while warpgroup
-// i % 2 turns S^T(i) into P^T, dS^T and drains dQ^T(i). dQ^T(i) reuses the TMEM columns of S^T(i),
-// which is dead once P^T(i) is written; with D = 128 all 512 columns are in use:
+//   dQ^T [d,  q]  = K^T . dS^T     (drained with fp32 reductions into dq_acc)
+// Two pairs of softmax warpgroups alternate iterations, each warpgroup with 32 of the 64 queries: S^T / dP^T (TMEM) and P^T / dS^T
+// are double buffered, so the tensor core computes S^T, dP^T of iteration i+1 while pair i % 2 turns S^T(i) into P^T, dS^T and
+// drains dQ^T(i). dQ^T(i) reuses the TMEM columns of S^T(i), which is dead once P^T(i) is written; with D = 128 all 512 columns are
+// in use:
 //   [S^T0 | dP^T0 | S^T1 | dP^T1 | dV (D) | dK (D)]
-// What bounds it is the chain of a warpgroup (scores -> P^T, dS^T -> dQ^T -> next scores), not the arithmetic: without its
-// exponentials the kernel took the same time. So nothing waits for memory inside the chain: Q / dO run three stages ahead,
-// lse and delta are requested an iteration early, and the columns of dQ^T are handed back once they are in registers, before
-// the sums leave. One 16384-token document, 32 / 8 heads of 128: 8.60 -> 6.31 ms (872 TFLOP/s), 4 x 2048: 0.71 -> 0.56 ms.
+// What bounds it is the chain of a pair (scores -> P^T, dS^T -> dQ^T -> next scores); the tensor core is busy for 56 % of an
+// iteration (five products of 64 queries, three of them limited by the shared-memory reads of their 64 columns). So nothing waits
+// for memory inside the chain: Q / dO run three stages ahead (with two a quarter slower), lse and delta are requested two iterations
+// early, dQ^T is the first product of its iteration and is drained while dV and dK run, and its sums leave by tile reductions: from
+// registers they filled the load-store queue ahead of the other pair's dS^T (a fifth of the time). One 16384-token document, 32 / 8
+// heads of 128: 8.60 -> 6.31 -> 5.47 ms (1005 TFLOP/s); 4096 tokens, 32 / 4 heads of 64: 258 -> 182 us with delta and conversion;
+// 11 x 707 tokens, 64 / 8 heads of 64, window 128: 338 -> 289.
 constexpr int kBwdThreads = 576;  // TMA warp, MMA warp, 4 x 4 softmax warps
 template <int D>
 struct BwdCfg {
@@ -472,11 +466,18 @@ struct BwdCfg {
   static constexpr int Q_HALF = 64 * 128;               // 64 rows x 128 B
   static constexpr int Q_BYTES = HALVES * Q_HALF;       // Q or dO tile: 64 rows
   static constexpr int PT_BYTES = HALF_BYTES;           // P^T / dS^T: [128 kv x 64 q]
+  // P^T as the TMEM operand of dV where shared memory is full; from shared memory is faster (4096 tokens, 32 heads of 64: 182 against
+  // 235 us; heads of 128 with P^T in shared memory and two stages of Q / dO instead of three: a quarter slower)
+  static constexpr bool PT_TMEM = D == 128;
+  // dQ^T on its way out, per warp that owns rows of it: groups of four queries x 32 columns of d, all nine that 32 queries can touch
+  // where shared memory allows
+  static constexpr int OUT_GROUPS = D == 128 ? 4 : 8;      // rows of the tensor map's box
+  static constexpr int OUT_BYTES = (D == 128 ? 4 : 9) * 512;
   static constexpr int STAGES = 3;                      // Q / dO: the load of a stage hides behind two iterations
-  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + 4 * PT_BYTES + 2048 /*lse+delta*/ + 256;
+  static constexpr int SMEM = 2 * KV_BYTES + STAGES * 2 * Q_BYTES + (PT_TMEM ? 2 : 4) * PT_BYTES + D / 8 * OUT_BYTES + 2048 /*lse+delta*/ + 256;
   static_assert(SMEM <= 227 * 1024, "");
   static constexpr int ST_COL = 0;     // S^T(b) at ST_COL + 128 b, 64 cols; dQ^T(b) aliases it
-  static constexpr int DPT_COL = 64;   // dP^T(b) at DPT_COL + 128 b, 64 cols
+  static constexpr int DPT_COL = 64;   // dP^T(b) at DPT_COL + 128 b, 64 cols; P^T(b) (bf16) in the first half of each 32 (D = 128)
   static constexpr int DV_COL = 256;   // D cols
   static constexpr int DK_COL = 256 + D;
   static constexpr int TMEM_COLS = 512;
@@ -487,6 +488,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 over qkv
                      const __grid_constant__ CUtensorMap tm_q,    // box 64 x 64 over qkv
                      const __grid_constant__ CUtensorMap tm_do,   // box 64 x 64 over dO
+                     const __grid_constant__ CUtensorMap tm_dq,   // box OUT_GROUPS x 128 fp32 over dq_acc, a row per four queries
                      const AttnParams p) {
   using C = BwdCfg<D>;
   const int tile_id = blockIdx.y;
@@ -522,9 +524,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   uint8_t* sV = sK + C::KV_BYTES;
   uint8_t* sQ = sV + C::KV_BYTES;                    // [STAGES]
   uint8_t* sdO = sQ + C::STAGES * C::Q_BYTES;        // [STAGES]
-  uint8_t* sPT = sdO + C::STAGES * C::Q_BYTES;       // [2]
-  uint8_t* sdST = sPT + 2 * C::PT_BYTES;             // [2]
-  float* s_rows = reinterpret_cast<float*>(sdST + 2 * C::PT_BYTES);  // per warpgroup: two buffers of -lse [32], -delta * scale [32]
+  uint8_t* sdST = sdO + C::STAGES * C::Q_BYTES;      // [2]
+  uint8_t* sPT = sdST + 2 * C::PT_BYTES;             // [2], where it is not in TMEM
+  uint8_t* sOut = sPT + (C::PT_TMEM ? 0 : 2 * C::PT_BYTES);   // [4 warpgroups][D / 32 warps]
+  float* s_rows = reinterpret_cast<float*>(sOut + D / 8 * C::OUT_BYTES);  // per warpgroup: two buffers of -lse [32], -delta * scale [32]
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_rows + 4 * 2 * 64);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;    // [STAGES]  (Q and dO of a stage)
@@ -603,7 +606,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     const uint64_t dv_k = make_smem_desc_sw128(smem_u32(sV), 16, 1024);
     const uint64_t dq_k = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dq_mn = make_smem_desc_sw128(smem_u32(sQ), C::Q_HALF, 1024);
     const uint64_t do_k = make_smem_desc_sw128(smem_u32(sdO), 16, 1024), do_mn = make_smem_desc_sw128(smem_u32(sdO), C::Q_HALF, 1024);
-    const uint64_t pt_k = make_smem_desc_sw128(smem_u32(sPT), 16, 1024), ds_k = make_smem_desc_sw128(smem_u32(sdST), 16, 1024);
+    const uint64_t ds_k = make_smem_desc_sw128(smem_u32(sdST), 16, 1024);
+    const uint64_t pt_k = make_smem_desc_sw128(smem_u32(sPT), 16, 1024);
     const uint64_t ds_mn = make_smem_desc_sw128(smem_u32(sdST), HALF_BYTES, 1024);
     bool ok = warp_all(mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL));
     int s_st = 0;             // stage and phase of the next scores
@@ -645,7 +649,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       const uint32_t ph = (it >> 1) & 1;
       if (it + 1 < n_iter && !issue_scores(it + 1)) break;   // keeps the tensor core busy during softmax(it)
       const uint64_t dq = dq_mn + (uint32_t)st * Q16, dd = do_mn + (uint32_t)st * Q16;
-      const uint64_t pt = pt_k + (uint32_t)b * PT16, ds = ds_k + (uint32_t)b * PT16, dst = ds_mn + (uint32_t)b * PT16;
+      const uint32_t pt = tmem_base + C::DPT_COL + 128 * b;
+      const uint64_t ds = ds_k + (uint32_t)b * PT16, dst = ds_mn + (uint32_t)b * PT16;
       if (!warp_all(mbar_wait(&pt_full[b], ph, p.status, AXB_TIMEOUT_GENERIC))) break;
       tc_fence_after();
       if (elect_one()) {
@@ -658,7 +663,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         // reduce over the 64 q rows of this tile: 4 K-steps of 16
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)   // dV += P^T . dO   (B = dO tile, MN-major: chunk stride = one 64x64 half)
-          umma_f16(tmem_base + C::DV_COL, pt + kk * 2, dd + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
+          if (C::PT_TMEM) umma_f16_ts(tmem_base + C::DV_COL, pt + (kk >> 1) * 32 + (kk & 1) * 8, dd + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
+          else umma_f16(tmem_base + C::DV_COL, pt_k + (uint32_t)b * PT16 + kk * 2, dd + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_f16(tmem_base + C::DK_COL, ds + kk * 2, dq + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
@@ -677,8 +683,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
     const uint32_t st_addr = tmem_base + lane_off + C::ST_COL + 128 * grp + c0, dpt_addr = tmem_base + lane_off + C::DPT_COL + 128 * grp + c0;
-    uint8_t* my_pt = sPT + grp * C::PT_BYTES;
     uint8_t* my_dst = sdST + grp * C::PT_BYTES;
+    uint8_t* my_pt = sPT + grp * C::PT_BYTES;
     float* const rows = s_rows + wg * 128;
     bool ok = true;
     // -lse (so that P = exp2(S * sl2 + nlse)) or -delta * scale of one q row of iteration `it`; rows outside the document
@@ -698,9 +704,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     // P^T and dS^T of 32 columns, two at a time (packed fp32 arithmetic rounds like the scalar one)
     const uint64_t sl2 = pack_f32x2(p.sl2, p.sl2), scale2 = pack_f32x2(p.scale, p.scale);
     auto gradients = [&](auto masked, const uint32_t (&sr)[32], const uint32_t (&dr)[32], const float* nlse, int qc0, int q_lo, int q_hi) {
+      uint32_t pk[16];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        uint32_t pk[4], dk[4];
+        uint32_t dk[4];
 #pragma unroll
         for (int i = q * 8; i < q * 8 + 8; i += 4) {
           const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(nlse + i), ds = *reinterpret_cast<const ulonglong2*>(nlse + 32 + i);
@@ -714,17 +721,51 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
               if (qc0 + j + 1 < q_lo || qc0 + j + 1 > q_hi) p1 = 0.f;
             }
             const float2 d = unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), fma_f32x2(pack_b32x2(dr[j], dr[j + 1]), scale2, h ? ds.y : ds.x)));
-            pk[((i & 4) >> 1) + h] = pack_bf16x2(p0, p1);
+            pk[j >> 1] = pack_bf16x2(p0, p1);
             dk[((i & 4) >> 1) + h] = pack_bf16x2(d.x, d.y);
           }
         }
         const uint32_t off = sw128_chunk_off(r, c0 / 8 + q);
-        *reinterpret_cast<uint4*>(my_pt + off) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        if (!C::PT_TMEM) *reinterpret_cast<uint4*>(my_pt + off) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
         *reinterpret_cast<uint4*>(my_dst + off) = make_uint4(dk[0], dk[1], dk[2], dk[3]);
       }
+      if (C::PT_TMEM) tmem_st_32x16(dpt_addr, pk);
     };
-    float* const dq_col = p.dq_acc + ((long long)r << 2);      // four rows of a column lie side by side, see dq_at
+    // The sums of 32 queries (the first one `shift` rows into its group of four) leave through this warp's staging tile and bulk
+    // reductions. As reductions from registers they filled the load-store queue, and the stores of the other warpgroups' dS^T stood
+    // behind them: 1500 of 2800 clocks of an iteration.
+    uint8_t* const out_tile = sOut + (wg * (D / 32) + lg) * C::OUT_BYTES;
     const long long width = (long long)p.Hq * D, rows4 = p.q_rows & ~3;
+    auto put_rows = [&](auto shift, const uint32_t (&v)[32], int group, int col) {
+      constexpr int a = decltype(shift)::value;
+      constexpr bool tail = a != 0;                       // a ninth group: by itself, a 512-byte reduction
+      if (lane == 0) bulk_wait_group_read<0>();           // what was staged before has left
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < 8 + (tail ? 1 : 0); ++g) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = 4 * g + e - a >= 0 && 4 * g + e - a < 32 ? v[(4 * g + e - a) & 31] : 0u;
+        if (C::OUT_GROUPS == 4 && (g == 4 || g == 8)) {   // the tile holds four groups
+          if (lane == 0) bulk_wait_group_read<0>();
+          __syncwarp();
+        }
+        *reinterpret_cast<uint4*>(out_tile + (C::OUT_GROUPS == 4 ? g & 3 : g) * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        if ((C::OUT_GROUPS == 4 && g == 3) || g == 7 || g == 8) {
+          if (g == 7 && tail && C::OUT_GROUPS == 8) continue;   // both leave after the ninth
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (g < 8) tma_reduce_add_2d(&tm_dq, out_tile, col, group + (g & ~(C::OUT_GROUPS - 1)));
+            else {
+              if (C::OUT_GROUPS == 8) tma_reduce_add_2d(&tm_dq, out_tile, col, group);
+              bulk_reduce_add_f32(p.dq_acc + (group + 8) * 4 * width + col, out_tile + (C::OUT_GROUPS == 4 ? 0 : 8) * 512, 512);
+            }
+            bulk_commit_group();
+          }
+        }
+      }
+    };
     float row_val = fetch_row(grp);
     if (st_tid < 64) rows[st_tid] = row_val;
     row_val = fetch_row(grp + 2);
@@ -758,6 +799,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
           gradients(std::false_type{}, sr, dr, nlse, 0, 0, 0);
         }
       }
+      if (C::PT_TMEM) tmem_st_wait();
       tc_fence_before();
       fence_proxy_async_smem();
       mbar_arrive(&pt_full[grp]);
@@ -784,32 +826,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         tc_fence_before();
         mbar_arrive(&st_free[grp]);      // the next scores may overwrite the columns while the sums leave
         if (r < D) {
-          float* col = dq_col + (long long)head * (4 * D);
-          const bool whole = i_lo <= 0 && i_hi >= 32 && row0 + 32 <= rows4;
-          if (whole && (row0 & 3) == 0) {
-            float* to = col + row0 * width;
+          if (row0 >= 0 && ((row0 + 31) | 3) < rows4) {      // every group that these rows touch is one of four whole rows
+            if (i_hi < 32) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) red_add_f32x4(to + i * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
-          } else if (whole && (row0 & 3) == 2) {
-            float* to = col + (row0 - 2) * width;
-            red_add_f32x2(to + 2, qr[0], qr[1]);
-#pragma unroll
-            for (int i = 2; i < 30; i += 4) red_add_f32x4(to + (i + 2) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
-            red_add_f32x2(to + 32 * width, qr[30], qr[31]);
-          } else if (whole && (row0 & 3) == 1) {
-            float* to = col + (row0 - 1) * width;
-            atomicAdd(to + 1, __uint_as_float(qr[0]));
-            red_add_f32x2(to + 2, qr[1], qr[2]);
-#pragma unroll
-            for (int i = 3; i < 31; i += 4) red_add_f32x4(to + (i + 1) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
-            atomicAdd(to + 32 * width, __uint_as_float(qr[31]));
-          } else if (whole) {
-            float* to = col + (row0 - 3) * width;
-            atomicAdd(to + 3, __uint_as_float(qr[0]));
-#pragma unroll
-            for (int i = 1; i < 29; i += 4) red_add_f32x4(to + (i + 3) * width, qr[i], qr[i + 1], qr[i + 2], qr[i + 3]);
-            red_add_f32x2(to + 32 * width, qr[29], qr[30]);
-            atomicAdd(to + 32 * width + 2, __uint_as_float(qr[31]));
+              for (int i = 0; i < 32; ++i) qr[i] = i < i_hi ? qr[i] : 0u;
+            }
+            const int group = (int)(row0 >> 2), col = head * (4 * D) + lg * 128;
+            switch ((int)(row0 & 3)) {
+              case 0: put_rows(std::integral_constant<int, 0>{}, qr, group, col); break;
+              case 1: put_rows(std::integral_constant<int, 1>{}, qr, group, col); break;
+              case 2: put_rows(std::integral_constant<int, 2>{}, qr, group, col); break;
+              default: put_rows(std::integral_constant<int, 3>{}, qr, group, col); break;
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i)
@@ -818,6 +846,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         }
       }
     }
+    if (lane == 0) bulk_wait_group<0>();
     // final dK / dV: 32 columns of each per warpgroup
     if (wg < D / 32 && ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
@@ -921,6 +950,8 @@ template <int D>
 int launch_bwd(const CUtensorMap& tkv, const CUtensorMap& tq, const CUtensorMap& tdo,
                const AttnParams& p, cudaStream_t st) {
   using C = BwdCfg<D>;
+  CUtensorMap tdq;     // without a whole group of four rows nothing goes through it
+  if (axb_make_tmap_2d(&tdq, p.dq_acc, p.T >= 4 ? p.T / 4 : 1, 4ll * p.Hq * D, 4ll * p.Hq * D, C::OUT_GROUPS, 128, 4, false)) return -4;
   auto kern = flash_bwd_kernel<D>;
   static bool attr = false;
   if (!attr) {
@@ -929,7 +960,7 @@ int launch_bwd(const CUtensorMap& tkv, const CUtensorMap& tq, const CUtensorMap&
     attr = true;
   }
   dim3 grid(p.Hk * p.kv_split, p.n_tiles);
-  kern<<<grid, kBwdThreads, C::SMEM, st>>>(tkv, tq, tdo, p);
+  kern<<<grid, kBwdThreads, C::SMEM, st>>>(tkv, tq, tdo, tdq, p);
   return (int)cudaGetLastError();
 }
 }  // namespace
