@@ -23,16 +23,17 @@ USE_GLU_EPILOGUE = os.environ.get("AXB_GLU_EPILOGUE", "1") != "0"
 
 
 # tile width, pair kernel?, rows, tiles at once, microseconds per 64-deep K block, microseconds per tile for bf16 results / fp32
-# results / results added to an operand read by the epilogue (L2 flushed; least squares over 7600 drawn products)
-_TILES = ((256, True, 256, _SM // 2, 0.336, (2.2, 8.7, 25.8)), (256, False, 128, _SM, 0.441, (5.6, 8.6, 24.0)),
-          (128, False, 128, _SM, 0.292, (2.8, 4.3, 11.8)), (64, False, 128, _SM, 0.236, (1.3, 2.1, 5.9)))
+# results / results added to an operand read by the epilogue / results added to the fp32 output by tile reductions (L2 flushed; least
+# squares over 7600 drawn products, the last over 138)
+_TILES = ((256, True, 256, _SM // 2, 0.336, (2.2, 8.7, 25.8, 5.8)), (256, False, 128, _SM, 0.441, (5.6, 8.6, 24.0, 5.4)),
+          (128, False, 128, _SM, 0.292, (2.8, 4.3, 11.8, 2.7)), (64, False, 128, _SM, 0.236, (1.3, 2.1, 5.9, 1.2)))
 
 
 def _pick_tile(M: int, N: int, k_blocks: int = 64, epilogue: int = 0) -> tuple[int, bool]:
     """(tile width, whether the CTA-pair kernel runs it): the choice with the least waves x time per wave. Mostly the number
     of waves decides, 960 x 32000 by 4096 takes 580 / 304 / 200 / 173 us (10, 4, 2, 1 waves with 64, 128, 256, pair); with a
     short K the epilogue does, which the pair kernel has cheapest in bf16 (TMA stores) and wide tiles have dearest where they read
-    and write fp32: 1568 x 88 by 13712 51 / 44 / 42 / 26 us, 1304 x 96 by 3720 added to fp32 46 / 51 / 64 / 70. Within 0.8 % of the best of the four on average, 2.7 % by waves alone.
+    and write an operand: 1568 x 88 by 13712 51 / 44 / 42 / 26 us, 1304 x 96 by 3720 added to fp32 46 / 51 / 64 / 70. Within 0.8 % of the best of the four on average, 2.7 % by waves alone.
     Ties go to the wider tile, which reads less."""
     best = None
     for bn, pair, rows, slots, per_k, per_tile in _TILES:
@@ -135,8 +136,8 @@ def gemm(
         _lib.check_rc(rc, "axb_gemm_bf16")
         return out
     if accumulate and splits <= 1 and out is not None and out.dtype == torch.float32 and c_in is None and a.is_cuda:
-        # a single K pass owns every output tile: plain read-add-write (beta = 1) instead of fp32
-        # atomics, which also makes the launch eligible for the 2-CTA kernel
+        # a single K pass owns every output tile: one sum per element (beta = 1) instead of split-K sums,
+        # which also makes the launch eligible for the 2-CTA kernel
         return gemm(a, b, trans_a=trans_a, trans_b=trans_b, a2=a2, b2=b2, alpha=alpha, beta=1.0, c_in=out, out=out,
                     out_dtype=torch.float32, accumulate=False, splits=1, bn=bn)
     if accumulate:
@@ -171,7 +172,13 @@ def gemm(
     if bn is None and accumulate:
         bn = _pick_bn(M, N)
     elif bn is None:
-        bn, pair = _pick_tile(M, N, (K + 63) // 64 + (K2 + 63) // 64, 2 if c_in is not None and beta != 0.0 else out_mode)
+        epilogue = out_mode
+        if c_in is not None and beta != 0.0:
+            # what the kernels ask before they add by tile reductions (adds_by_tile)
+            tiles = (out_mode == 1 and beta == 1.0 and c_in.data_ptr() == out.data_ptr() and c_in.stride(0) == out.stride(0)
+                     and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0)
+            epilogue = 3 if tiles else 2
+        bn, pair = _pick_tile(M, N, (K + 63) // 64 + (K2 + 63) // 64, epilogue)
     elif not accumulate:
         pair = _use_pair(M, N, bn)
     if pair:

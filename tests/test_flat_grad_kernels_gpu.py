@@ -121,3 +121,25 @@ def test_flat_buffer_leaves_hooks_and_partial_backwards_alone(kind):
     assert not tab._axb_grad.any() and not w._axb_grad.any()
     for a, b in zip(got, want):
         assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 8, 64), (264, 24, 200), (136, 72, 520), (520, 264, 328), (2056, 1040, 136)])
+@pytest.mark.parametrize("bn,splits", [(None, 1), (64, 1), (128, 1), (256, 1), (64, 5), (128, 3)])
+@pytest.mark.parametrize("col", [0, 4, 3])
+def test_product_added_to_an_fp32_slice(M, N, K, bn, splits, col):
+    """dW += dY^T X into columns of a wider buffer, rows and columns that end inside a 32 x 32 tile, aligned slices (tile reductions) and one
+    that is not (added from registers): fp32 sums of bf16 products, in another order; the columns beside the slice stay as they are."""
+    from axolotl_b200.ops.gemm import gemm
+
+    torch.manual_seed(M + K)
+    a, b = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    buf = torch.randn(M, N + 24, device="cuda")
+    old = buf.clone()
+    gemm(a, b, trans_a=True, trans_b=True, out=buf[:, col:col + N], accumulate=True, splits=splits, bn=bn, alpha=0.5)
+    _lib.check_status()
+    want = old.double()
+    want[:, col:col + N] += 0.5 * a.double().t() @ b.double()
+    size = old.double().abs()
+    size[:, col:col + N] += 0.5 * a.double().abs().t() @ b.double().abs()
+    assert ((buf.double() - want).abs() <= 2 ** -20 * size).all()
+    assert torch.equal(buf[:, :col], old[:, :col]) and torch.equal(buf[:, col + N:], old[:, col + N:])

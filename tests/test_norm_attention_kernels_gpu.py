@@ -71,6 +71,47 @@ def test_attention_head_and_token_remainders(D, Hq, Hk, lens, window, causal):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens", [[3], [4], [1, 130], [2, 131, 64], [3, 97, 35], [32, 32, 5, 129]])
+def test_attention_gradient_of_queries_by_row_alignment(D, lens):
+    """The sums of dQ leave in groups of four rows: documents that begin at every place of a group, buffers that end inside one, and the
+    queries of a rank that begin inside a tile (its sums before that row are not its own). Rows of the query gradient against the fp32
+    reference as in test_attention_head_and_token_remainders; nothing behind the scratch is written."""
+    import axolotl_b200.parallel.cp  # noqa: F401  (declares the entry for a rank's rows)
+
+    torch.manual_seed(D + sum(lens))
+    Hq, Hk, T, lib, st = 4, 2, sum(lens), _lib.cuda_lib(), _lib.stream_ptr()
+    qkv, do = torch.randn(T, (Hq + 2 * Hk) * D, device="cuda").bfloat16(), torch.randn(T, Hq * D, device="cuda").bfloat16()
+    cu = np.concatenate([[0], np.cumsum(lens)])
+    meta = Fn.AttnMeta(cu, "cuda")
+    x = qkv.float().requires_grad_(True)
+    q, k, v = (t.reshape(T, -1, D) for t in x.split([Hq * D, Hk * D, Hk * D], -1))
+    (want,) = torch.autograd.grad(Fn._attn_ref(q, k, v, meta.cu_seqlens_host, D ** -0.5, True, 0).reshape(T, -1), x, do.float())
+    out, lse = torch.empty_like(do), torch.empty(Hq, T, device="cuda")
+    word = _lib.status_word(qkv.device).data_ptr()
+    _lib.check_rc(lib.axb_flash_varlen_fwd(qkv.data_ptr(), qkv.stride(0), T, Hq, Hk, D, 0, Hq * D, (Hq + Hk) * D, meta.tiles_fwd.data_ptr(),
+                                           meta.n_tiles, out.data_ptr(), out.stride(0), lse.data_ptr(), D ** -0.5, word, st), "fwd")
+    kv = qkv[:, Hq * D:].contiguous()
+    for off, n in ((0, T), (T // 3, T - T // 3), (T // 2, 1)):
+        acc = torch.full((n * Hq * D + 64,), 5.0, device="cuda")
+        dqkv, delta = torch.zeros(T, qkv.shape[1], device="cuda", dtype=torch.bfloat16), torch.empty(Hq, n, device="cuda")
+        rows = lambda t: t[off:off + n].contiguous()  # noqa: E731
+        ql, dl, ol, ll = rows(qkv), rows(do), rows(out), lse[:, off:off + n].contiguous()
+        if (off, n) == (0, T):
+            rc = lib.axb_flash_varlen_bwd(ql.data_ptr(), ql.stride(0), dl.data_ptr(), ol.data_ptr(), ol.stride(0), ll.data_ptr(), T, Hq, Hk, D, 0,
+                                          Hq * D, (Hq + Hk) * D, meta.tiles_bwd.data_ptr(), meta.n_tiles, dqkv.data_ptr(), dqkv.stride(0),
+                                          acc.data_ptr(), delta.data_ptr(), D ** -0.5, word, st)
+        else:
+            rc = lib.axb_flash_varlen_bwd_cp(ql.data_ptr(), ql.stride(0), n, off, kv.data_ptr(), kv.stride(0), T, dl.data_ptr(), ol.data_ptr(),
+                                             ol.stride(0), ll.data_ptr(), Hq, Hk, D, meta.tiles_bwd.data_ptr(), meta.n_tiles, dqkv.data_ptr(),
+                                             dqkv.stride(0), acc.data_ptr(), delta.data_ptr(), D ** -0.5, 1, T, None, word, st)
+        _lib.check_rc(rc, "bwd")
+        got, ref = dqkv[:n, :Hq * D].float(), want[off:off + n, :Hq * D]
+        _lib.check_status()
+        assert (acc[n * Hq * D:] == 5.0).all()
+        assert ((got - ref).abs() <= 2 ** -6 * want[:, :Hq * D].abs().max()).all()
+
+
 @pytest.mark.parametrize("T,nh,D,rot", [(1, 1, 64, 64), (3, 5, 128, 128), (9, 40, 128, 128), (700, 36, 64, 64), (2500, 10, 256, 128)])
 @pytest.mark.parametrize("sign", [1.0, -1.0])
 def test_rope_head_groups(T, nh, D, rot, sign):
