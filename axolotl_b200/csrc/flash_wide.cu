@@ -15,7 +15,7 @@
 // Takes the place of the reference's flash-attn / SDPA paths for these head sizes
 // (src/axolotl/monkeypatch/attention/flash_attn_4.py:37-111; Gemma attention soft-capping reaches the
 // reference through HF's eager/flash paths selected in src/axolotl/loaders/model.py:560-640).
-#include "axb_common.cuh"
+#include "attn_common.cuh"
 #include <type_traits>
 
 namespace {
@@ -39,21 +39,11 @@ struct WideParams {
   int* status;
   // backward
   const float* delta;  // [Hq, T]
-  float* dq_acc;       // [T, Hq * Dqk] fp32 (atomics)
-  long long dq_ld;
+  float* dq_acc;       // T * Hq * Dqk fp32 in the order of dq_at, accumulated with reductions
   __nv_bfloat16* dkv;  // gradient buffer, same layout as qkv
   long long dkv_ld;
   int dk_col0, dv_col0;
 };
-
-AXB_DEVICE float fast_exp2(float x) {
-  float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-AXB_DEVICE uint32_t sw128_chunk_off(int row, int chunk) {
-  return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4);
-}
 
 // =====================================================================================================
 // Forward: 192 threads = TMA warp, MMA warp, 4 softmax warps. One CTA per (q head, 128-row q tile), all of the v head.
@@ -346,11 +336,11 @@ __global__ void __launch_bounds__(192, 1)
 }
 
 // =====================================================================================================
-// Backward: 320 threads = TMA warp, MMA warp, two softmax warpgroups. One CTA per (kv head, 128-row kv tile,
+// Backward: 576 threads = TMA warp, MMA warp, four softmax warpgroups. One CTA per (kv head, 128-row kv tile,
 // part); loops over the q heads of the GQA group and the 64-row q tiles that see the kv tile. Per iteration
 //   S^T [kv, q] = K . Q^T (over Dqk)      dP^T [kv, q] = V . dO^T (over Dv)
 //   dV[:, part] += P^T . dO[:, part]      dK[:, part] += dS^T . Q[:, part]
-//   dQ^T[part, q] = K[:, part]^T . dS^T   (fp32 atomics into dq_acc; reuses the TMEM columns of S^T)
+//   dQ^T[part, q] = K[:, part]^T . dS^T   (fp32 reductions into dq_acc)
 // A 192-wide q/k head has the parts [0, 128) and [64, 192): the second stores only its upper 64 columns.
 // =====================================================================================================
 template <int DQK, int DV>
@@ -360,14 +350,18 @@ struct WBwd {
   static constexpr int Q_BYTES = (DQK / 64) * QH_BYTES;
   static constexpr int DO_BYTES = (DV / 64) * QH_BYTES;
   static constexpr int PT_BYTES = HALF_BYTES;   // [128 kv x 64 q]
-  static constexpr int SMEM = K_BYTES + V_BYTES + Q_BYTES + DO_BYTES + 2 * PT_BYTES + 512 + 128 + 1024;
-  static constexpr int ST_COL = 0, DPT_COL = 64, DV_COL = 128, DK_COL = 256;
+  static constexpr int SMEM = K_BYTES + V_BYTES + Q_BYTES + DO_BYTES + 2 * PT_BYTES + 1024 /*lse+delta*/ + 128 + 1024;
+  static_assert(SMEM <= 227 * 1024, "");
+  static constexpr int ST_COL = 0, DPT_COL = 64, DV_COL = 128, DK_COL = 256, DQ_COL = 384;
 };
 
-// Two softmax warpgroups share every q tile, 32 columns each: with nothing double-buffered (shared memory is full) an iteration
-// is a chain of scores -> P^T, dS^T -> dQ^T, and the second group halves its middle. lse / delta are requested an iteration
-// early, Q / dO are handed back before dQ^T runs, and the columns of dQ^T once they are in registers.
-constexpr int WBWD_THREADS = 320;
+// Four softmax warpgroups share every q tile, 16 columns each: with nothing double-buffered (shared memory is full) an iteration
+// is a chain of scores -> P^T, dS^T -> products, and more warps shorten its middle. lse / delta are requested two iterations early; dK
+// comes first, so that Q, which the next scores wait for, loads beside dV and dQ^T; dO is handed back by itself; dQ^T has TMEM
+// columns of its own, so that the next scores do not wait for its drain; tiles without a mask have a path of their own; and four rows
+// of a dQ column lie side by side in the fp32 sum, which leaves in 16-byte reductions. 4 x 2048 tokens, 16 / 8 heads of 256, whole
+// backward pass 904 -> 816 us, 300 + 2701 tokens 419 -> 379. Still the chain bounds it: the MMAs are a third of an iteration.
+constexpr int WBWD_THREADS = 576;
 template <int DQK, int DV, bool SOFTCAP>
 __global__ void __launch_bounds__(WBWD_THREADS, 1)
     flash_wide_bwd_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_q,
@@ -402,9 +396,8 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
   uint8_t* sdO = sQ + C::Q_BYTES;
   uint8_t* sPT = sdO + C::DO_BYTES;
   uint8_t* sdST = sPT + C::PT_BYTES;
-  float* s_lse = reinterpret_cast<float*>(sdST + C::PT_BYTES);   // [64]
-  float* s_delta = s_lse + 64;                                   // [64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_delta + 64);
+  float* s_rows = reinterpret_cast<float*>(sdST + C::PT_BYTES);  // per warpgroup: two buffers of -lse [16], -delta * scale [16]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_rows + 4 * 2 * 32);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;
   uint64_t* q_empty = bars + 2;
@@ -413,17 +406,21 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
   uint64_t* dq_full = bars + 5;
   uint64_t* st_free = bars + 6;
   uint64_t* acc_full = bars + 7;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* do_full = bars + 8;
+  uint64_t* do_empty = bars + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
+    mbar_init(do_full, 1);
+    mbar_init(do_empty, 1);
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
     mbar_init(s_full, 1);
-    mbar_init(pt_full, 256);
+    mbar_init(pt_full, 512);
     mbar_init(dq_full, 1);
-    mbar_init(st_free, 256);
+    mbar_init(st_free, 512);
     mbar_init(acc_full, 1);
     mbar_fence_init();
   }
@@ -452,13 +449,18 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
       const int qrow = doc_start + (q_first + qt) * 64;
       if (!warp_all(mbar_wait(q_empty, (it & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
       if (elect_one()) {
-        mbar_expect_tx(q_full, C::Q_BYTES + C::DO_BYTES);
+        mbar_expect_tx(q_full, C::Q_BYTES);
 #pragma unroll
         for (int h = 0; h < DQK / 64; ++h)
           tma_load_2d(sQ + h * QH_BYTES, &tm_q, q_full, p.q_col0 + head * DQK + h * 64, qrow);
+      }
+      __syncwarp();
+      if (!warp_all(mbar_wait(do_empty, (it & 1) ^ 1, p.status, AXB_TIMEOUT_EMPTY))) break;
+      if (elect_one()) {
+        mbar_expect_tx(do_full, C::DO_BYTES);
 #pragma unroll
         for (int h = 0; h < DV / 64; ++h)
-          tma_load_2d(sdO + h * QH_BYTES, &tm_do, q_full, head * DV + h * 64, qrow);
+          tma_load_2d(sdO + h * QH_BYTES, &tm_do, do_full, head * DV + h * 64, qrow);
       }
       __syncwarp();
       if (++qt == n_qt) {
@@ -480,10 +482,7 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
     bool ok = warp_all(mbar_wait(kv_full, 0, p.status, AXB_TIMEOUT_FULL));
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t ph = it & 1;
-      bool fine = mbar_wait(q_full, ph, p.status, AXB_TIMEOUT_FULL);
-      // the S^T columns carried dQ^T of the previous iteration: it must have been drained
-      if (fine && it > 0) fine = mbar_wait(st_free, (it - 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY);
-      if (!warp_all(fine)) break;
+      if (!warp_all(mbar_wait(q_full, ph, p.status, AXB_TIMEOUT_FULL))) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
@@ -491,6 +490,11 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
           const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * QH_BYTES + (kk % 4) * 32) / 16;
           umma_f16(tmem_base + C::ST_COL, dk_k + koff, dq_k + qoff, idesc_st, kk > 0);
         }
+      }
+      __syncwarp();
+      if (!warp_all(mbar_wait(do_full, ph, p.status, AXB_TIMEOUT_FULL))) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < DV / 16; ++kk) {
           const uint32_t koff = ((kk / 4) * HALF_BYTES + (kk % 4) * 32) / 16, qoff = ((kk / 4) * QH_BYTES + (kk % 4) * 32) / 16;
@@ -499,26 +503,30 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
         umma_commit(s_full);
       }
       __syncwarp();
-      if (!warp_all(mbar_wait(pt_full, ph, p.status, AXB_TIMEOUT_GENERIC))) break;
+      // dQ^T of the iteration before is out of its columns (long since), and P^T, dS^T of this one are in place
+      bool fine = mbar_wait(pt_full, ph, p.status, AXB_TIMEOUT_GENERIC);
+      if (fine && it > 0) fine = mbar_wait(st_free, (it - 1) & 1, p.status, AXB_TIMEOUT_TMEM_EMPTY);
+      if (!warp_all(fine)) break;
       tc_fence_after();
       if (elect_one()) {
-        if (has_v) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16(tmem_base + C::DV_COL, pt_k + kk * 2, do_mn + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
-        }
         if (has_k) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
             umma_f16(tmem_base + C::DK_COL, ds_k + kk * 2, dq_mn + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
         }
-        umma_commit(q_empty);   // Q and dO of this iteration are consumed: the next ones load beside dQ^T
+        umma_commit(q_empty);   // the next Q is the first that the next scores wait for: it loads beside dV and dQ^T
+        if (has_v) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16(tmem_base + C::DV_COL, pt_k + kk * 2, do_mn + kk * (2048 / 16), idesc_acc, (it > 0 || kk > 0));
+        }
+        umma_commit(do_empty);
         if (has_k) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_f16(tmem_base + C::ST_COL, dk_mn + kk * (2048 / 16), ds_mn + kk * (2048 / 16), idesc_dq, kk > 0);
+            umma_f16(tmem_base + C::DQ_COL, dk_mn + kk * (2048 / 16), ds_mn + kk * (2048 / 16), idesc_dq, kk > 0);
         }
-        umma_commit(dq_full);   // ... and P^T, dS^T
+        umma_commit(dq_full);
         if (it == n_iter - 1) umma_commit(acc_full);
       }
       __syncwarp();
@@ -526,99 +534,133 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
   } else {
     const int lg = warp & 3;
     const int r = lg * 32 + lane;   // kv row of the tile (S^T, dP^T, dK, dV) or column of the part (dQ^T)
-    const int grp = (warp - 2) >> 2;   // columns [32 grp, 32 grp + 32) of every q tile
+    const int grp = (warp - 2) >> 2, c0 = grp * 16;   // columns [c0, c0 + 16) of every q tile
     const int tid = threadIdx.x - 64 - grp * 128;
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = uint32_t(lg * 32) << 16;
+    float* const rows = s_rows + grp * 64;
     bool ok = true;
-    // -lse or delta * scale of one of this group's 32 q rows, requested an iteration ahead (rows outside: P = 0)
+    // -lse or -delta * scale of one of this group's 16 q rows, requested two iterations ahead (rows outside: P = 0)
     auto fetch_row = [&](int it) -> float {
-      float val = tid < 32 ? -INFINITY : 0.f;
-      if (tid >= 64 || it >= n_iter) return val;
-      const int q = (q_first + it % n_qt) * 64 + grp * 32 + (tid & 31);
+      float val = tid < 16 ? -INFINITY : 0.f;
+      if (tid >= 32 || it >= n_iter) return val;
+      const int q = (q_first + it % n_qt) * 64 + c0 + (tid & 15);
       const long long row = (long long)doc_start + q;
       if (q < doc_len && row < p.T) {
         const long long off = (long long)(head0 + it / n_qt) * p.T + row;
-        val = tid < 32 ? -p.lse2[off] : p.delta[off] * p.scale;
+        val = tid < 16 ? -p.lse2[off] : -p.delta[off] * p.scale;
       }
       return val;
     };
+    auto gradients = [&](auto masked, const uint32_t (&sr)[16], const uint32_t (&dr)[16], const float* nlse, int qc0, int q_lo, int q_hi) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t pk[4], dk[4];
+#pragma unroll
+        for (int i = q * 8; i < q * 8 + 8; i += 2) {
+          float pv[2], dv[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float s = __uint_as_float(sr[i + e]);
+            float g = 1.f;
+            if constexpr (SOFTCAP) {
+              const float t = tanhf(s * p.cap_in);
+              pv[e] = fast_exp2(fmaf(t, p.cap_out2, nlse[i + e]));
+              g = 1.f - t * t;
+            } else {
+              pv[e] = fast_exp2(fmaf(s, p.sl2, nlse[i + e]));
+            }
+            if (decltype(masked)::value && (qc0 + i + e < q_lo || qc0 + i + e > q_hi)) pv[e] = 0.f;
+            dv[e] = pv[e] * fmaf(__uint_as_float(dr[i + e]), p.scale, nlse[16 + i + e]) * g;
+          }
+          pk[(i & 6) >> 1] = pack_bf16x2(pv[0], pv[1]);
+          dk[(i & 6) >> 1] = pack_bf16x2(dv[0], dv[1]);
+        }
+        const uint32_t off = sw128_chunk_off(r, c0 / 8 + q);
+        *reinterpret_cast<uint4*>(sPT + off) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        *reinterpret_cast<uint4*>(sdST + off) = make_uint4(dk[0], dk[1], dk[2], dk[3]);
+      }
+    };
+    const long long width = (long long)p.Hq * DQK, rows4 = p.T & ~3ll;
+    // the sums of 16 queries, the first one `shift` rows into its group of four; whole groups with 16-byte reductions
+    auto add_rows = [&](auto shift, const uint32_t (&v)[16], float* to) {
+      constexpr int a = decltype(shift)::value;
+#pragma unroll
+      for (int g = a ? 1 : 0; g < 4; ++g) red_add_f32x4(to + g * 4 * width, v[(4 * g - a) & 15], v[(4 * g - a + 1) & 15], v[(4 * g - a + 2) & 15], v[(4 * g - a + 3) & 15]);
+      if (a == 1 || a == 3) red_add_f32(to + a, v[0]);
+      if (a == 1 || a == 2) red_add_f32x2(to + 2, v[(2 - a) & 15], v[(3 - a) & 15]);
+      if (a == 2 || a == 3) red_add_f32x2(to + 16 * width, v[(16 - a) & 15], v[(17 - a) & 15]);
+      if (a == 1 || a == 3) red_add_f32(to + 16 * width + a - 1, v[15]);
+    };
     float row_val = fetch_row(0);
+    if (tid < 32) rows[tid] = row_val;
+    row_val = fetch_row(1);
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
     for (int it = 0; it < n_iter && ok; ++it) {
       const uint32_t ph = it & 1;
       const int head = head0 + it / n_qt;
-      const int qt0 = (q_first + it % n_qt) * 64;
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");   // the group finished reading the previous lse / delta
-      if (tid < 64) (tid < 32 ? s_lse : s_delta)[grp * 32 + (tid & 31)] = row_val;
-      row_val = fetch_row(it + 1);
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      const int qc0 = (q_first + it % n_qt) * 64 + c0;      // doc-relative first q row of this group's columns
       if (!mbar_wait(s_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      const bool row_in_doc = kv_idx < doc_len;
-      const int q_lo = row_in_doc ? (bidir ? -(1 << 30) : kv_idx) : (1 << 30);
-      const int q_hi = win > 0 ? kv_idx + win - 1 : (1 << 30);
+      const bool need_mask = (!bidir && qc0 < kv0 + 127) || kv0 + 128 > doc_len || (win > 0 && qc0 + 15 >= kv0 + win);
       {
-        const int c = grp;
-        uint32_t sr[32], dr[32];
-        tmem_ld_32x32(tmem_base + lane_off + C::ST_COL + c * 32, sr);
-        tmem_ld_32x32(tmem_base + lane_off + C::DPT_COL + c * 32, dr);
+        uint32_t sr[16], dr[16];
+        tmem_ld_32x16(tmem_base + lane_off + C::ST_COL + c0, sr);
+        tmem_ld_32x16(tmem_base + lane_off + C::DPT_COL + c0, dr);
         tmem_ld_wait();
-        uint32_t pk[16], dk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float pv[2], dv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float s = __uint_as_float(sr[i + e]);
-            const float nl = s_lse[c * 32 + i + e], dl = s_delta[c * 32 + i + e];
-            float pr, g = 1.f;
-            if constexpr (SOFTCAP) {
-              const float t = tanhf(s * p.cap_in);
-              pr = fast_exp2(fmaf(t, p.cap_out2, nl));
-              g = 1.f - t * t;
-            } else {
-              pr = fast_exp2(fmaf(s, p.sl2, nl));
-            }
-            const int q = qt0 + c * 32 + i + e;
-            if (q < q_lo || q > q_hi) pr = 0.f;
-            pv[e] = pr;
-            dv[e] = pr * fmaf(__uint_as_float(dr[i + e]), p.scale, -dl) * g;
-          }
-          pk[i >> 1] = pack_bf16x2(pv[0], pv[1]);
-          dk[i >> 1] = pack_bf16x2(dv[0], dv[1]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t off = sw128_chunk_off(r, c * 4 + q);
-          *reinterpret_cast<uint4*>(sPT + off) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
-          *reinterpret_cast<uint4*>(sdST + off) = make_uint4(dk[q * 4], dk[q * 4 + 1], dk[q * 4 + 2], dk[q * 4 + 3]);
+        if (need_mask) {
+          const bool row_in_doc = kv_idx < doc_len;
+          const int q_lo = row_in_doc ? (bidir ? -(1 << 30) : kv_idx) : (1 << 30);
+          const int q_hi = win > 0 ? kv_idx + win - 1 : (1 << 30);
+          gradients(std::true_type{}, sr, dr, rows + ph * 32, qc0, q_lo, q_hi);
+        } else {
+          gradients(std::false_type{}, sr, dr, rows + ph * 32, 0, 0, 0);
         }
       }
       tc_fence_before();
       fence_proxy_async_smem();
       mbar_arrive(pt_full);
+      // lse / delta of the next iteration into the other buffer, while the MMAs run; the barrier also says that all warps of the group
+      // have read the present one
+      if (tid < 32) rows[(ph ^ 1) * 32 + tid] = row_val;
+      row_val = fetch_row(it + 2);
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
       if (!mbar_wait(dq_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after();
       if (has_k) {
-        const long long row0 = (long long)doc_start + qt0;
-        int i_hi = min(64, doc_len - qt0);
+        const long long row0 = (long long)doc_start + qc0;
+        int i_hi = min(16, doc_len - qc0);
         if (row0 + i_hi > p.T) i_hi = (int)(p.T - row0);
-        float* col = p.dq_acc + row0 * p.dq_ld + (long long)head * DQK + kpart + r;
-        uint32_t qr[32];
-        tmem_ld_32x32(tmem_base + lane_off + C::ST_COL + grp * 32, qr);
+        uint32_t qr[16];
+        tmem_ld_32x16(tmem_base + lane_off + C::DQ_COL + c0, qr);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(st_free);        // the next scores may overwrite the columns while the sums leave
+        mbar_arrive(st_free);        // the next dQ^T may overwrite the columns while the sums leave
         if (r >= k_lo) {
+          const long long col = (long long)head * DQK + kpart + r;
+          if (((row0 + 15) | 3) < rows4) {      // every group of four rows that these touch is a whole one
+            if (i_hi < 16) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (grp * 32 + i < i_hi) atomicAdd(col + (long long)(grp * 32 + i) * p.dq_ld, __uint_as_float(qr[i]));
+              for (int i = 0; i < 16; ++i) qr[i] = i < i_hi ? qr[i] : 0u;
+            }
+            float* to = p.dq_acc + (row0 & ~3ll) * width + col * 4;
+            switch ((int)(row0 & 3)) {
+              case 0: add_rows(std::integral_constant<int, 0>{}, qr, to); break;
+              case 1: add_rows(std::integral_constant<int, 1>{}, qr, to); break;
+              case 2: add_rows(std::integral_constant<int, 2>{}, qr, to); break;
+              default: add_rows(std::integral_constant<int, 3>{}, qr, to); break;
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (i < i_hi) atomicAdd(p.dq_acc + dq_at(row0 + i, col, width, rows4), __uint_as_float(qr[i]));
+          }
         }
       } else {
         tc_fence_before();
@@ -631,8 +673,8 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
       const long long grow = (long long)doc_start + kv_idx;
       __nv_bfloat16* krow = p.dkv + grow * p.dkv_ld + p.dk_col0 + (long long)kv_head * DQK + kpart;
       __nv_bfloat16* vrow = p.dkv + grow * p.dkv_ld + p.dv_col0 + (long long)kv_head * DV + vpart;
-#pragma unroll 1
-      for (int c = 2 * grp; c < 2 * grp + 2; ++c) {
+      {
+        const int c = grp;
         uint32_t a[32], b[32];
         tmem_ld_32x32(tmem_base + lane_off + C::DK_COL + c * 32, a);
         tmem_ld_32x32(tmem_base + lane_off + C::DV_COL + c * 32, b);
@@ -666,40 +708,6 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
-  }
-}
-
-__global__ void wide_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                  float* __restrict__ delta, long long T, int Hq, int D, long long ld) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= T * Hq) return;
-  const long long t = gw / Hq;
-  const int h = (int)(gw % Hq);
-  const __nv_bfloat16* a = dout + t * ld + (long long)h * D;
-  const __nv_bfloat16* b = out + t * ld + (long long)h * D;
-  float s = 0.f;
-  for (int i = lane * 2; i < D; i += 64) {
-    const float2 x = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(a + i));
-    const float2 y = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(b + i));
-    s += x.x * y.x + x.y * y.y;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) delta[(long long)h * T + t] = s;
-}
-
-__global__ void wide_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv, long long T,
-                                       int width, long long ld, int q_col0) {
-  const long long n = T * (width / 4);
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-    const long long t = v / (width / 4);
-    const int c = (int)(v % (width / 4)) * 4;
-    const float4 f = *reinterpret_cast<const float4*>(acc + t * width + c);
-    uint2 u;
-    u.x = pack_bf16x2(f.x, f.y);
-    u.y = pack_bf16x2(f.z, f.w);
-    *reinterpret_cast<uint2*>(dqkv + t * ld + q_col0 + c) = u;
   }
 }
 
@@ -791,17 +799,13 @@ extern "C" int axb_flash_wide_bwd(const void* qkv, long long ld, const void* dou
   if (axb_make_tmap_2d(&tdo, dout, T, (long long)Hq * Dv, o_ld, 64, 64)) return -4;
   cudaError_t e = cudaMemsetAsync(dq_acc, 0, sizeof(float) * T * Hq * Dqk, st);
   if (e != cudaSuccess) return (int)e;
-  {
-    const long long warps = T * Hq;
-    wide_delta_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(
-        (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, T, Hq, Dv, o_ld);
-  }
+  if (Dv == 256) launch_attn_delta<256>(dout, out, delta, T, Hq, o_ld, st);
+  else launch_attn_delta<128>(dout, out, delta, T, Hq, o_ld, st);
   WideParams p = {};
   fill_common(p, tiles, n_tiles, Hq, Hk, q_col0, k_col0, v_col0, T, softmax_scale, softcap, status);
   p.lse2 = const_cast<float*>(lse2);
   p.delta = delta;
   p.dq_acc = dq_acc;
-  p.dq_ld = (long long)Hq * Dqk;
   p.dkv = reinterpret_cast<__nv_bfloat16*>(dqkv);
   p.dkv_ld = dqkv_ld;
   p.dk_col0 = k_col0;
@@ -811,8 +815,6 @@ extern "C" int axb_flash_wide_bwd(const void* qkv, long long ld, const void* dou
   if (Dqk == 256) rc = sc ? launch_wide_bwd<256, 256, true>(tkv, tq, tdo, p, st) : launch_wide_bwd<256, 256, false>(tkv, tq, tdo, p, st);
   else rc = sc ? launch_wide_bwd<192, 128, true>(tkv, tq, tdo, p, st) : launch_wide_bwd<192, 128, false>(tkv, tq, tdo, p, st);
   if (rc) return rc;
-  const long long n = T * (long long)(Hq * Dqk / 4);
-  const int grid = (int)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
-  wide_dq_convert_kernel<<<grid, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, T, Hq * Dqk, dqkv_ld, q_col0);
+  launch_dq_convert(dq_acc, dqkv, T, Hq * Dqk, dqkv_ld, q_col0, st);
   return (int)cudaGetLastError();
 }
