@@ -112,6 +112,26 @@ def test_attention_gradient_of_queries_by_row_alignment(D, lens):
         assert ((got - ref).abs() <= 2 ** -6 * want[:, :Hq * D].abs().max()).all()
 
 
+@pytest.mark.parametrize("lens", [[3], [17], [1, 130], [2, 131, 64], [3, 97, 35]])
+@pytest.mark.parametrize("window", [0, 20])
+def test_wide_attention_gradient_by_row_alignment(lens, window):
+    """256-wide heads: documents that begin at every place of a group of four rows of the dQ sums, tiles that end inside 16 queries, masked
+    and unmasked tiles; tolerances of test_attention_head_and_token_remainders."""
+    torch.manual_seed(sum(lens))
+    D, Hq, Hk, T = 256, 4, 2, sum(lens)
+    qkv = torch.randn(T, (Hq + 2 * Hk) * D, device="cuda").bfloat16().requires_grad_(True)
+    do = torch.randn(T, Hq * D, device="cuda").bfloat16()
+    meta = Fn.AttnMeta(np.concatenate([[0], np.cumsum(lens)]), "cuda")
+    meta = meta.windowed(window) if window else meta
+    (g,) = torch.autograd.grad(Fn.flash_varlen(qkv, meta, Hq, Hk, D), qkv, do)
+    x = qkv.detach().float().requires_grad_(True)
+    q, k, v = (t.reshape(T, -1, D) for t in x.split([Hq * D, Hk * D, Hk * D], -1))
+    (want,) = torch.autograd.grad(Fn._attn_ref(q, k, v, meta.cu_seqlens_host, D ** -0.5, True, window).reshape(T, -1), x, do.float())
+    _lib.check_status()
+    assert ((g.float() - want).abs() <= 2 ** -6 * want.abs().max()).all()
+    assert ((g.float() - want).norm() / want.norm()).item() < 2 ** -7
+
+
 @pytest.mark.parametrize("T,nh,D,rot", [(1, 1, 64, 64), (3, 5, 128, 128), (9, 40, 128, 128), (700, 36, 64, 64), (2500, 10, 256, 128)])
 @pytest.mark.parametrize("sign", [1.0, -1.0])
 def test_rope_head_groups(T, nh, D, rot, sign):
