@@ -260,10 +260,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_u && ok; ++j) {
-      if (!mbar_wait(&s_full[u], j & 1, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-        ok = false;
-        break;
-      }
+      ok = warp_all(mbar_wait(&s_full[u], j & 1, p.status, AXB_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       tc_fence_after();
       uint32_t sr[4][32];
 #pragma unroll
@@ -326,7 +324,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       mbar_arrive(&p_full[u]);
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
-    if (ok && n_u > 0 && mbar_wait(&o_full[u], 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+    if (ok && n_u > 0 && warp_all(mbar_wait(&o_full[u], 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       const long long lrow = (long long)doc_start + q_idx - p.q_row_off;  // row in the local buffers
@@ -691,13 +689,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     if (st_tid < 64) rows[st_tid] = row_val;
     row_val = fetch_row(grp + 2);
     asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
-    for (int it = grp; it < n_iter && ok; it += 2) {
+    int it = grp;
+    for (; it < n_iter; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int head = head0 + it / n_qt;
       const int qt0 = (q_first + it % n_qt) * 64;  // doc-relative first q row of the tile
       const int qc0 = qt0 + c0;                    // ... and of this group's columns
       const float* nlse = rows + ph * 64;
-      if (!mbar_wait(&s_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      if (!warp_all(mbar_wait(&s_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
         ok = false;
         break;
       }
@@ -730,8 +729,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       row_val = fetch_row(it + 4);
       asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
       // drain dQ^T: this thread owns d = r (only rows < D are meaningful)
-      if (!mbar_wait(&dq_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      if (!warp_all(mbar_wait(&dq_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
         ok = false;
+        it += 2;
         break;
       }
       tc_fence_after();
@@ -767,9 +767,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         }
       }
     }
+    // A warp whose wait ran out does no more work, but meets its group at the barriers that are left.
+#pragma unroll 1
+    for (; it < n_iter; it += 2) asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
     if (lane == 0) bulk_wait_group<0>();
     // final dK / dV: 32 columns of each per warpgroup
-    if (wg < D / 32 && ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+    if (wg < D / 32 && ok && warp_all(mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
       tc_fence_after();
       const bool row_ok = kv_idx < doc_len && n_iter > 0;
       const long long grow = (long long)doc_start + kv_idx;  // global kv row

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(SK_T)
     if (elect_one()) umma_commit(done);
   }
   __syncwarp();
-  mbar_wait(done, 0, p.status, AXB_TIMEOUT_TMEM_FULL);
+  warp_all(mbar_wait(done, 0, p.status, AXB_TIMEOUT_TMEM_FULL));
   tc_fence_after();
   pdl_wait();
   // partial tile, [n][128] fp32 in the ring (every load into it has been consumed by a retired MMA)

@@ -525,10 +525,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int kb1 = (int)((long long)nk_total * (split + 1) / p.splits);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-        ok = false;
-        break;
-      }
+      ok = warp_all(mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       tc_fence_after();
       const long long row = (long long)m_blk * BM + lane_group * 32 + lane;
       const bool row_ok = row < p.M && kb1 > kb0;
@@ -1139,10 +1137,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_load_2d(dst, &tmE2, eb, n_blk * 256, r0);
         tma_load_2d(dst + 2048, &tmE3, eb, n_blk * 256, r0);
       }
-      if (!mbar_wait_backoff(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL, p.epi_sleep_ns)) {
-        ok = false;
-        break;
-      }
+      ok = warp_all(mbar_wait_backoff(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL, p.epi_sleep_ns));
+      if (!ok) break;
       tc_fence_after();
       const long long row = (long long)m_blk * 256 + rank * 128 + lane_group * 32 + lane;
       const bool row_ok = row < p.M;
@@ -1236,10 +1232,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           uint32_t r[32];
           tmem_ld_32x32(t_addr + c * 32, r);
           tmem_ld_wait();
-          if (!mbar_wait(&epi_bar[lane_group * 2 + s_cur], (uint32_t)((q >> 1) & 1), p.status, AXB_TIMEOUT_FULL)) {
-            ok = false;
-            break;
-          }
+          ok = warp_all(mbar_wait(&epi_bar[lane_group * 2 + s_cur], (uint32_t)((q >> 1) & 1), p.status, AXB_TIMEOUT_FULL));
+          if (!ok) break;
           const int sw = (lane >> 1) & 3;
           uint8_t* grow = tile + lane * 64;
           uint8_t* urow = tile + 2048 + lane * 64;

@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         ++it;
-        if (!mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL)) break;
+        if (!warp_all(mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL))) break;
         tc_fence_after();
       } else if (p.out_mode == 2) {
         continue;  // nothing to add

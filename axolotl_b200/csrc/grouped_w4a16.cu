@@ -482,11 +482,8 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
       const int col0 = t.col0() + rank * 128 + lg * 32;      // this warp's columns
       const int cols = pass_cols(ps);
       const int acc = it & 1;
-      if (!wait_sleeping(&tfull_bar[acc], (it >> 1) & 1, 200, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-        ok = false;
-        break;
-      }
-      __syncwarp();
+      ok = warp_all(wait_sleeping(&tfull_bar[acc], (it >> 1) & 1, 200, p.status, AXB_TIMEOUT_TMEM_FULL));
+      if (!ok) break;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (uint32_t(lg * 32) << 16) + acc * 256;
       // the rows that pad a block are written too, as zeros: one staging tile of them serves all their stores

@@ -201,10 +201,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         ++it;
-        if (!mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-          ok = false;
-          break;
-        }
+        ok = warp_all(mbar_wait(&tfull_bar[acc], acc_phase, p.status, AXB_TIMEOUT_TMEM_FULL));
+        if (!ok) break;
         tc_fence_after();
         const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + acc * BM;
         const int key = kt * BN + lane_group * 32 + lane;

@@ -185,10 +185,8 @@ __global__ void __launch_bounds__(LF_THREADS, 1)
       bool ok = true;
       for (int nb = nb0, i = 0; nb < nb1 && ok; ++nb, ++i) {
         const int bb = i & 1;
-        if (!mbar_wait(&db_full[bb], (i >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL)) {
-          ok = false;
-          break;
-        }
+        ok = warp_all(mbar_wait(&db_full[bb], (i >> 1) & 1, p.status, AXB_TIMEOUT_TMEM_FULL));
+        if (!ok) break;
         tc_fence_after();
         const int n = nb * 128 + lg * 32 + lane;   // this thread's column of dY = row of dB
         int r0 = 0, r = 0;
@@ -213,7 +211,7 @@ __global__ void __launch_bounds__(LF_THREADS, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&db_empty[bb]);
       }
-      if (ok && mbar_wait(t_done, 0, p.status, AXB_TIMEOUT_TMEM_FULL)) {
+      if (ok && warp_all(mbar_wait(t_done, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
         tc_fence_after();
         for (int s = 0; s < n_sub; ++s) {
           const int t = row0 + s * 128 + lg * 32 + lane;

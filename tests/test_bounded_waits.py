@@ -1,0 +1,79 @@
+"""The bounded waits of the kernels, read from their sources: what has to hold so that a wait that runs out ends the kernel with a
+status instead of leaving the GPU waiting. (Making one run out in a kernel that is wrong would hang the GPU, so nothing here runs.)"""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "axolotl_b200" / "csrc"
+WAIT = re.compile(r"\b(?:mbar_wait|mbar_wait_spin|mbar_wait_backoff|wait_sleeping)\(")
+SOURCES = sorted(p.name for p in CSRC.glob("*.cu") if WAIT.search(p.read_text()))
+
+
+def _code(name):
+    text = re.sub(r"//[^\n]*", lambda m: " " * len(m.group()), (CSRC / name).read_text())
+    return re.sub(r"/\*.*?\*/", lambda m: re.sub(r"[^\n]", " ", m.group()), text, flags=re.S)
+
+
+def _waits(code):
+    """(position, headers of the enclosing blocks, start of the outermost one) of every wait that is called, not defined."""
+    stack, last = [], 0
+    calls = {m.start() for m in WAIT.finditer(code)}
+    for i, c in enumerate(code):
+        if i in calls:
+            if not code[last:i].strip().endswith("bool") and "bool mbar_wait" not in "".join(h for h, _ in stack):
+                yield i, [h for h, _ in stack], next((at for h, at in stack if not re.match(r"\s*(extern|namespace)", h)), 0)
+        if c == "{":
+            stack.append((code[last:i].strip(), i))
+            last = i + 1
+        elif c == "}":
+            stack.pop()
+            last = i + 1
+        elif c == ";":
+            last = i + 1
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_a_wait_ends_the_same_way_for_all_lanes_of_a_warp(name):
+    """tcgen05.ld, elect.sync and __syncwarp wait for every lane of the warp, without a limit: unless a single lane walks the loop, the
+    outcome of a wait is agreed on (warp_all) before anything depends on it."""
+    code = _code(name)
+    for at, headers, start in _waits(code):
+        line = code.count("\n", 0, at) + 1
+        statement = code[max(code.rfind(c, 0, at) for c in ";{}") + 1:at]
+        held = re.search(r"(\w+) = (?:\w+ && )?$", statement)
+        rest = code[at:at + 400]
+        agreed = "warp_all(" in statement or (held and re.search(r"warp_all\(%s\)" % held.group(1), rest))
+        one_lane = any("lane == 0)" in h or "elect_one()" in h for h in headers) or "lane != 0) return;" in code[start:at]
+        assert agreed or one_lane, f"{name}:{line}: lanes of a warp may leave this wait on different ways"
+
+
+@pytest.mark.parametrize("name", [n for n in SOURCES if "bar.sync" in _code(n)])
+def test_a_warp_that_gives_up_still_meets_its_group(name):
+    """A named barrier has no limit: a warp that leaves a loop with one, because a wait ran out, meets its group at the barriers that
+    are left, in a loop of its own from where it stopped, or it walks on without work (dead)."""
+    code = _code(name)
+    loops = 0
+    for m in re.finditer(r"\bfor \(", code):
+        depth, i = 0, code.index("{", m.end())
+        body = i
+        if ";" in re.sub(r"\([^()]*\)", "", code[m.start():i].split(")", 1)[-1]):     # a loop without braces
+            continue
+        while True:
+            depth += {"{": 1, "}": -1}.get(code[i], 0)
+            i += 1
+            if not depth:
+                break
+        block = code[body:i]
+        if "bar.sync" not in block or not WAIT.search(block):
+            continue
+        loops += 1
+        breaks = [b.start() for b in re.finditer(r"\n\s*break;", block)]              # (not those of a switch)
+        assert breaks or "dead" in block
+        if breaks:
+            step = re.search(r"for \((?:int \w+ = \w+)?; it < n_iter; (it \+= 2|\+\+it)\)$", code[m.start():body].strip()).group(1)
+            assert code[i:i + 400].lstrip().startswith("#pragma unroll 1") and re.match(
+                r"\s*#pragma unroll 1\s*for \(; it < n_iter; %s\) asm volatile\(\"bar.sync" % re.escape(step), code[i:]), name
+        for b in breaks:      # one barrier an iteration: behind it, the next iteration's is the first that is left
+            assert bool(re.search(r"\b%s;\s*$" % re.escape(step), block[:b]) or block[:b].rstrip().endswith(step + ";")) == ("bar.sync" in block[:b]), name
+    assert loops
