@@ -391,11 +391,42 @@ AXB_DEVICE uint32_t mapa_u32(uint32_t smem_addr, uint32_t rank) {
 AXB_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// Arrival on the partner's mbarrier that stands for tiles in THIS CTA's shared memory, which this SM's tensor core reads: the lanes
-// that wrote them have each passed fence.proxy.async, so nothing is left to be made visible to the other CTA, and the default
-// scope of the arrival serves. The release.cluster form waits for every access that the SM has in flight, about 0.3 us of a k block.
+// Arrival on the partner's mbarrier that stands for tiles in THIS CTA's shared memory, and the wait for it: the partner issues the
+// MMA that reads them, so the edge from the writes to its issue needs cluster scope on both sides. The lanes that wrote have each
+// passed fence.proxy.async and met in __syncwarp. The fences are restricted to shared memory: release.cluster on the arrival itself
+// waits for every access in flight, the weight scales requested for the next k blocks included (NVFP4 grouped GEMM, 65536 rows of 128
+// experts, 2048 -> 1536: 500 us with it, 409 with the restricted fence, 397 with the default CTA scope, which orders nothing here).
 AXB_DEVICE void mbar_arrive_partner(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                   cluster_addr)
+               : "memory");
+}
+AXB_DEVICE bool mbar_test_wait_relaxed(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+AXB_DEVICE bool mbar_wait_partner(uint64_t* bar, uint32_t parity, int* status, int code) {
+  if (!mbar_test_wait_relaxed(bar, parity)) {
+    const uint64_t t0 = global_timer_ns();
+    uint32_t spins = 0;
+    while (!mbar_test_wait_relaxed(bar, parity)) {
+      if ((++spins & 0xFFF) == 0 && global_timer_ns() - t0 > AXB_WAIT_BUDGET_NS) {
+        if (status) atomicCAS(status, 0, code);
+        return false;
+      }
+    }
+  }
+  asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+  return true;
 }
 AXB_DEVICE void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr),

@@ -317,12 +317,12 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
       for (Tiles t(p, num_n, total, cluster_id, n_clusters); t.live() && ok; t.next(), ++it) {
         const uint32_t idesc = make_idesc_bf16(256, pass_cols(t.ps), DX ? 1 : 0, 0);
         const int acc = it & 1;
-        if (!warp_all(mbar_wait_spin(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) break;
+        if (!warp_all(mbar_wait_partner(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, AXB_TIMEOUT_TMEM_EMPTY))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * 256;
         for (int kb = 0; kb < nk; ++kb, rx.next(), rw.next()) {
           if (!warp_all(mbar_wait_spin(&x_full[rx.slot], rx.phase, p.status, AXB_TIMEOUT_FULL) &&
-                        mbar_wait_spin(&w_full[rw.slot], rw.phase, p.status, AXB_TIMEOUT_FULL))) {
+                        mbar_wait_partner(&w_full[rw.slot], rw.phase, p.status, AXB_TIMEOUT_FULL))) {
             ok = false;
             break;
           }

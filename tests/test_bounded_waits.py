@@ -6,7 +6,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parents[1] / "axolotl_b200" / "csrc"
-WAIT = re.compile(r"\b(?:mbar_wait|mbar_wait_spin|mbar_wait_backoff|wait_sleeping)\(")
+WAIT = re.compile(r"\b(?:mbar_wait|mbar_wait_spin|mbar_wait_backoff|mbar_wait_partner|wait_sleeping)\(")
 SOURCES = sorted(p.name for p in CSRC.glob("*.cu") if WAIT.search(p.read_text()))
 
 
@@ -77,3 +77,15 @@ def test_a_warp_that_gives_up_still_meets_its_group(name):
         for b in breaks:      # one barrier an iteration: behind it, the next iteration's is the first that is left
             assert bool(re.search(r"\b%s;\s*$" % re.escape(step), block[:b]) or block[:b].rstrip().endswith(step + ";")) == ("bar.sync" in block[:b]), name
     assert loops
+
+
+def test_arrivals_on_another_cta_have_cluster_scope():
+    """The default scope of mbarrier.arrive is the CTA: on the partner's barrier it would order nothing that the arriving CTA wrote
+    before what the other one does. What such an arrival stands for has to be acquired at that scope too."""
+    for name in sorted(p.name for p in CSRC.glob("*.cu*")):
+        for m in re.finditer(r"mbarrier\.arrive[\w.:]*\.shared::cluster[\w.:]*", _code(name)):
+            assert re.search(r"\.(release|relaxed)\.cluster\.", m.group()), f"{name}: {m.group()}"
+    w4a16 = _code("grouped_w4a16.cu")
+    for bar in ("w_full", "tempty_bar"):          # what the partner's converters and epilogue signal
+        waits = re.findall(r"\b(mbar_\w+|wait_\w+)\(&%s\[" % bar, w4a16)
+        assert [w for w in waits if "wait" in w] == ["mbar_wait_partner"], (bar, waits)

@@ -166,3 +166,24 @@ def test_grouped_w4a16_rows_in_use(N, K, r):
         assert torch.equal(got[:used], ref[:used]) and not got[:used][empty].any()
     y32 = grouped_gemm_w4a16(x, q, lay, out_dtype=torch.float32)[:used]
     assert torch.equal(y32.bfloat16(), grouped_gemm(x, W, lay)[:used])
+
+
+def test_grouped_w4a16_repeats_its_bits_under_load():
+    """Several passes on every SM pair, k blocks of every ring position, the LoRA extension and full, half and nearly empty passes side
+    by side, twenty times: a tile that the tensor core read before the other CTA's part of it was in place would change some bit."""
+    E, N, K, r = 48, 1536, 2048, 16
+    counts = [(37 * e) % 600 for e in range(E)]
+    torch.manual_seed(5)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).view(-1, 1).cuda()
+    lay = RoutedLayout(idx, E)
+    q = dict(zip(("qdata", "scale", "pts"), (t.cuda() for t in quantize_nvfp4(torch.randn(E, N, K) * 0.05))))
+    W = dequantize_nvfp4(q["qdata"], q["scale"], q["pts"])
+    pad = lambda c: torch.where(lay.row_slot[:, None] >= 0, torch.randn(lay.max_rows, c, device="cuda"), 0.0).bfloat16()  # noqa: E731
+    x, dy, t = pad(K), pad(N), pad(r)
+    A16, Bt = torch.randn(E, r, K, device="cuda").bfloat16(), torch.randn(E, N, r, device="cuda").bfloat16()
+    used = int(lay.n_blocks) * BLOCK
+    for a, w2, tr in ((x, Bt, False), (dy, A16, True)):
+        want = grouped_gemm(a, W, lay, trans_w=tr, a2=t, w2=w2)[:used]
+        for _ in range(20):
+            assert torch.equal(grouped_gemm_w4a16(a, q, lay, trans_w=tr, a2=t, w2=w2)[:used], want)
+    _lib.check_status()
