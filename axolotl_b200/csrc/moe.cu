@@ -99,23 +99,10 @@ __global__ void __launch_bounds__(RL_T) route_count_kernel(const long long* __re
   for (int e = threadIdx.x; e < E; e += RL_T) hist[(long long)blockIdx.x * E + e] = h[e];
 }
 
-// hist[b][e] becomes the padded row of the first slot of expert e in block b
-__global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__ hist, int blocks, int E, int max_blocks,
-                                                               int* __restrict__ seg_start, int* __restrict__ seg_rows,
-                                                               int* __restrict__ blk_expert, int* __restrict__ n_blocks,
-                                                               int4* __restrict__ passes, int* __restrict__ n_pass) {
-  __shared__ unsigned long long warp_sum[32];
-  __shared__ int first[RL_MAX_E + 1];     // first 128-row block of every expert
-  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-  int count = 0;
-  if (e < E) {
-#pragma unroll 8
-    for (int b = 0; b < blocks; ++b) count += hist[(long long)b * E + e];
-  }
-  // running sums over the experts: blocks of 128 rows (low word), passes of the NVFP4 GEMM over two blocks (high word)
-  const int nb = (count + 127) / 128, np = (nb + 1) / 2;
-  unsigned long long incl = (unsigned long long)np << 32 | (unsigned)nb;
-  const unsigned long long own = incl;
+// Sum of `own` over the threads before this one; warp_sum: 32 words of shared memory. Every thread of a block of 1024 calls it.
+AXB_DEVICE unsigned long long sum_before(unsigned long long own, unsigned long long* warp_sum) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long incl = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -133,7 +120,25 @@ __global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__
     warp_sum[lane] = v;
   }
   __syncthreads();
-  const unsigned long long before = incl - own + (warp ? warp_sum[warp - 1] : 0);
+  return incl - own + (warp ? warp_sum[warp - 1] : 0);
+}
+
+// hist[b][e] becomes the padded row of the first slot of expert e in block b
+__global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__ hist, int blocks, int E, int max_blocks,
+                                                               int* __restrict__ seg_start, int* __restrict__ seg_rows,
+                                                               int* __restrict__ blk_expert, int* __restrict__ n_blocks,
+                                                               int4* __restrict__ passes, int* __restrict__ n_pass) {
+  __shared__ unsigned long long warp_sum[32];
+  __shared__ int first[RL_MAX_E + 1];     // first 128-row block of every expert
+  const int e = threadIdx.x;
+  int count = 0;
+  if (e < E) {
+#pragma unroll 8
+    for (int b = 0; b < blocks; ++b) count += hist[(long long)b * E + e];
+  }
+  // running sums over the experts: blocks of 128 rows (low word), passes of the NVFP4 GEMM over two blocks (high word)
+  const int nb = (count + 127) / 128, np = (nb + 1) / 2;
+  const unsigned long long before = sum_before((unsigned long long)np << 32 | (unsigned)nb, warp_sum);
   const int start = (int)(unsigned)before, pass0 = (int)(before >> 32);
   if (e < E) {
     first[e] = start;
@@ -162,6 +167,36 @@ __global__ void __launch_bounds__(RL_MAX_E) route_place_kernel(int* __restrict__
     }
     blk_expert[b] = lo;
   }
+}
+
+// The passes of the NVFP4 grouped GEMM for a layout given by its rows per expert (any number of experts). A layout that was sized for
+// fewer blocks than its rows need ends at max_blocks; a pass's first block grows with the pass, so those that begin before it are a
+// prefix of the table. Bound: its launch, 10 to 13 us with the two allocations; as tensor operations with a sort the table took 180 to
+// 195 us of the host, half of a forward product over 2664 rows of 128 experts (layout and product 454 -> 300 us, 65536 rows 591 -> 486).
+__global__ void __launch_bounds__(RL_MAX_E) group_passes_kernel(const long long* __restrict__ counts, int E, int max_blocks,
+                                                                int4* __restrict__ passes, int* __restrict__ n_pass) {
+  __shared__ unsigned long long warp_sum[32];
+  __shared__ unsigned long long done;       // blocks (low word) and passes (high word) of the experts before this chunk
+  __shared__ int n;
+  if (threadIdx.x == 0) done = 0, n = 0;
+  __syncthreads();
+  for (int e0 = 0; e0 < E; e0 += RL_MAX_E) {
+    const int e = e0 + threadIdx.x;
+    const int count = e < E ? (int)counts[e] : 0, nb = (count + 127) / 128, np = (nb + 1) / 2;
+    const unsigned long long own = (unsigned long long)np << 32 | (unsigned)nb;
+    const unsigned long long before = done + sum_before(own, warp_sum);
+    const int start = (int)(unsigned)before, pass0 = (int)(before >> 32);
+    int mine = 0;
+    for (; mine < np && start + 2 * mine < max_blocks; ++mine) {
+      const int b = start + 2 * mine, blocks = min(min(2, nb - 2 * mine), max_blocks - b);
+      passes[pass0 + mine] = make_int4(b, e, min(blocks * 128, count - 256 * mine), blocks);
+    }
+    if (mine) atomicAdd(&n, mine);
+    __syncthreads();                        // everyone has read `done`
+    if (threadIdx.x == RL_MAX_E - 1) done = before + own;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *n_pass = n;
 }
 
 __global__ void __launch_bounds__(RL_T) route_scatter_kernel(const long long* __restrict__ expert, const int* __restrict__ base,
@@ -582,6 +617,14 @@ extern "C" int axb_nvfp4_dequant_batched(const void* q, const void* scale, const
 static int rows_grid(long long n_rows) {
   const long long want = (n_rows + 7) / 8;   // 8 warps (rows) per 256-thread block
   return (int)(want > 148 * 8 ? 148 * 8 : (want < 1 ? 1 : want));
+}
+
+// The pass table of axb_grouped_gemm_w4a16 for segments of counts[e] rows (device int64 [E]), each padded to whole 128-row blocks, one
+// behind the other. passes int32 [max_blocks, 4], 16-byte aligned; n_pass [1]. Blocks from max_blocks on are left out.
+extern "C" int axb_group_passes(const long long* counts, int E, int max_blocks, int* passes, int* n_pass, void* stream) {
+  if (E < 1 || max_blocks < 0 || (reinterpret_cast<uintptr_t>(passes) & 15)) return -2;
+  group_passes_kernel<<<1, RL_MAX_E, 0, ST(stream)>>>(counts, E, max_blocks, reinterpret_cast<int4*>(passes), n_pass);
+  return (int)cudaGetLastError();
 }
 
 // Layout of a routed batch. expert [n] (n = T * k slots, expert ids), E <= 1024; slot_row [n], row_slot [max_blocks * 128] (slot of

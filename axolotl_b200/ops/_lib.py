@@ -36,6 +36,8 @@ _CUDA_SIGS = {
     "axb_moe_dispatch_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
     # expert, n, E, max_blocks, slot_row, row_slot, seg_start, seg_rows, blk_expert, n_blocks, passes, n_pass, scratch, status, stream
     "axb_moe_route_layout": [vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
+    # counts, E, max_blocks, passes, n_pass, stream
+    "axb_group_passes": [vp, i32, i32, vp, vp, vp],
     "axb_moe_combine_rows": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_moe_combine_dw": [vp, vp, vp, vp, i64, i32, i32, vp],
     "axb_nf4_dequant": [vp, vp, vp, i64, i32, vp],

@@ -36,12 +36,15 @@ class GroupLayout:
 
     ``dest[i]``: padded row of the i-th expert-sorted compact row; ``blk_expert`` / ``n_blocks`` /
     ``seg_start`` / ``seg_rows`` as consumed by the grouped kernels; ``max_blocks`` is a static
-    upper bound (ceil(rows / 128) + E) so buffer shapes never depend on the routing."""
+    upper bound (ceil(rows / 128) + E) so buffer shapes never depend on the routing. ``counts``: rows in use of
+    every expert (int64), None where only whole blocks are known."""
+
+    counts = None
 
     def __init__(self, counts: torch.Tensor, n_rows: int):
         E = counts.numel()
         dev = counts.device
-        counts = counts.to(torch.int64)
+        self.counts = counts = counts.to(torch.int64).contiguous()
         padded = (counts + (BLOCK - 1)) // BLOCK * BLOCK
         seg_end = padded.cumsum(0)
         seg_start = seg_end - padded
@@ -60,14 +63,13 @@ class GroupLayout:
     @functools.cached_property
     def passes(self):
         """(int32 [max_blocks, 4], count): the passes of the NVFP4 GEMM, (first row block, expert, rows in use, row blocks) of every
-        two row blocks of an expert."""
-        b = torch.arange(self.max_blocks, device=self.blk_expert.device)
-        e = self.blk_expert.long()
-        at = b - self.seg_start[e] // BLOCK                                   # place of the block among its expert's
-        blocks = torch.minimum(self.seg_rows[e] // BLOCK - at, self.n_blocks - b).clamp(max=2)
-        starts = (at % 2 == 0) & (b < self.n_blocks)
-        table = torch.stack([b, e, blocks * BLOCK, blocks], 1).to(torch.int32)
-        return table[torch.argsort(~starts, stable=True)], starts.sum(dtype=torch.int32).view(1)
+        two row blocks of an expert. The rows that pad a segment are zero and not in use."""
+        counts = self.seg_rows.long() if self.counts is None else self.counts
+        table = torch.empty((self.max_blocks, 4), dtype=torch.int32, device=counts.device)
+        n = torch.empty(1, dtype=torch.int32, device=counts.device)
+        _lib.check_rc(_lib.cuda_lib().axb_group_passes(counts.data_ptr(), self.E, self.max_blocks, table.data_ptr(), n.data_ptr(),
+                                                       _lib.stream_ptr()), "group_passes")
+        return table, n
 
     def pad(self, x_sorted):
         out = x_sorted.new_zeros((self.max_rows, x_sorted.shape[1]))

@@ -248,7 +248,7 @@ class ExpertParallelGroup:
         seg_start = seg_end - padded
         first = counts.cumsum(0) - counts
         lay = GroupLayout.__new__(GroupLayout)
-        lay.E, lay.n_rows = El, cap
+        lay.E, lay.n_rows, lay.counts = El, cap, counts
         lay.max_blocks = cap // BLOCK + El
         lay.max_rows = lay.max_blocks * BLOCK
         e_c = e_sorted.clamp(max=El - 1).long()

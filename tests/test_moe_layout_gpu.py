@@ -187,3 +187,56 @@ def test_grouped_w4a16_repeats_its_bits_under_load():
         for _ in range(20):
             assert torch.equal(grouped_gemm_w4a16(a, q, lay, trans_w=tr, a2=t, w2=w2)[:used], want)
     _lib.check_status()
+
+
+def _passes(counts, max_blocks):
+    out, b = [], 0
+    for e, c in enumerate(counts):
+        nb = -(-c // BLOCK)
+        out += [[b + j, e, min(c - j * BLOCK, 256, (max_blocks - b - j) * BLOCK), min(2, nb - j, max_blocks - b - j)]
+                for j in range(0, nb, 2) if b + j < max_blocks]
+        b += nb
+    return out
+
+
+@pytest.mark.parametrize("counts", [[1, 31, 32, 33, 0, 127, 128, 129], [255, 256, 257, 0, 385], [0], [0, 3], [700],
+                                    [(7 * e) % 300 for e in range(1025)], [0] * 1024 + [5, 0, 400] + [1] * 1100])
+def test_passes_of_a_layout_by_counts(counts):
+    """The layouts of the expert-parallel and the general path know their rows too: rows in use, not whole blocks, for any number of
+    experts."""
+    lay = GroupLayout(torch.tensor(counts, device="cuda"), sum(counts))
+    table, n = lay.passes
+    assert table.shape == (lay.max_blocks, 4) and table[: int(n)].tolist() == _passes(counts, lay.max_blocks)
+
+
+@pytest.mark.parametrize("cf", [0.25, 0.6, 4.0])
+def test_passes_of_an_expert_parallel_plan(cf):
+    """The plan that is made on the device, with room for all rows and with too little of it (more rows than the capacity: reported, and
+    the segments end at the last block): every pass inside the blocks that exist."""
+    from axolotl_b200.parallel.ep import ExpertParallelGroup
+
+    world, E, T, k = 4, 16, 512, 2
+    torch.manual_seed(3)
+    g = ExpertParallelGroup.__new__(ExpertParallelGroup)
+    g.device, g.size, g.rank, g.E, g.E_local = torch.device("cuda"), world, 0, E, E // world
+    g.fused, g.dedup, g.overflow, g.capacity_factor = False, True, None, cf
+    all_idx = torch.randint(0, 6, (world * T * k,), dtype=torch.int32, device="cuda")      # mostly this rank's experts
+    lay = g._plan_from_tables(all_idx, torch.ones(world * T * k, device="cuda"), all_idx[: T * k].reshape(T, k), 8).lay
+    counts = [int((all_idx == e).sum()) for e in range(E // world)]
+    want = _passes(counts, lay.max_blocks)
+    assert bool(g.overflow) == (cf < 2) and int(lay.n_blocks) == sum(p[3] for p in want)
+    assert lay.passes[0][: int(lay.passes[1])].tolist() == want
+
+
+def test_rows_in_use_of_a_general_layout():
+    """NVFP4 experts over segments given by their counts, short ones among them: the bits of the bf16 stack, zeros in the padding."""
+    counts, N, K = [1, 31, 0, 33, 129, 255, 257, 64, 0, 128], 136, 192
+    torch.manual_seed(7)
+    lay = GroupLayout(torch.tensor(counts, device="cuda"), sum(counts))
+    q = dict(zip(("qdata", "scale", "pts"), (t.cuda() for t in quantize_nvfp4(torch.randn(len(counts), N, K) * 0.05))))
+    W = dequantize_nvfp4(q["qdata"], q["scale"], q["pts"])
+    used = int(lay.n_blocks) * BLOCK
+    for a, tr in ((lay.pad(torch.randn(sum(counts), K, device="cuda").bfloat16()), False),
+                  (lay.pad(torch.randn(sum(counts), N, device="cuda").bfloat16()), True)):
+        assert torch.equal(grouped_gemm_w4a16(a, q, lay, trans_w=tr)[:used], grouped_gemm(a, W, lay, trans_w=tr)[:used])
+    _lib.check_status()
