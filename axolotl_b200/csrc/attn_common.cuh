@@ -88,6 +88,11 @@ void launch_attn_delta(const void* dout, const void* out, float* delta, long lon
   kern<<<grid, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, T, Hq, ld, ld);
 }
 
+// What the backward passes move 16 bytes at a time, beyond what tensor maps check.
+inline bool attn_bwd_aligned(const void* out, const void* dqkv, const void* dq_acc) {
+  return ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(dq_acc)) & 15) == 0;
+}
+
 // Where the fp32 sum of dQ[row][col] stands (col = head * D + d, rows of `width`): four rows of a column side by side, so that a
 // warp's 32 columns are 512 contiguous bytes of every group of four rows. The last rows % 4 rows are plain.
 AXB_DEVICE long long dq_at(long long row, long long col, long long width, long long rows4) {

@@ -921,6 +921,7 @@ int flash_bwd_impl(const AttnGeom& g, const void* dout, const void* out, long lo
   if (g.q_rows <= 0 || n_tiles <= 0) return 0;
   if (D != 64 && D != 128) return -2;
   if ((g.q_ld & 7) || (g.kv_ld & 7) || (o_ld & 7) || (dqkv_ld & 7) || cp_world > 8) return -3;
+  if (!attn_bwd_aligned(out, dqkv, dq_acc)) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const long long T = g.q_rows;
   CUtensorMap tkv, tq, tdo;

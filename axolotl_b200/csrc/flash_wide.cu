@@ -797,6 +797,7 @@ extern "C" int axb_flash_wide_bwd(const void* qkv, long long ld, const void* dou
   if (T <= 0 || n_tiles <= 0) return 0;
   if (!((Dqk == 256 && Dv == 256) || (Dqk == 192 && Dv == 128))) return -2;
   if ((ld & 7) || (o_ld & 7) || (dqkv_ld & 7) || (q_col0 & 7) || (k_col0 & 7) || (v_col0 & 7) || Hk <= 0 || Hq % Hk) return -3;
+  if (!attn_bwd_aligned(out, dqkv, dq_acc)) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap tkv, tq, tdo;
   if (axb_make_tmap_2d(&tkv, qkv, T, ld, ld, 128, 64)) return -4;

@@ -555,6 +555,12 @@ def _apply_sinks(out, lse2, sinks, Hq):
     return out, lse_new
 
 
+def _aligned_out(out):
+    """The saved attention output for a backward kernel, which reads it 16 bytes at a time; saved-tensor hooks may bring it back at any
+    address."""
+    return out if out.data_ptr() % 16 == 0 else out.clone()
+
+
 class _FlashVarlen(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, meta, Hq, Hk, D, scale, sinks=None):
@@ -586,7 +592,7 @@ class _FlashVarlen(torch.autograd.Function):
         meta = ctx.meta
         T = qkv.shape[0]
         lib = _lib.cuda_lib()
-        dout = dout.contiguous()
+        dout, out = dout.contiguous(), _aligned_out(out)
         dqkv = torch.empty_like(qkv)
         dq_acc = torch.empty((T, Hq * D), dtype=torch.float32, device=qkv.device)
         delta = torch.empty((Hq, T), dtype=torch.float32, device=qkv.device)
@@ -632,7 +638,7 @@ class _FlashWide(torch.autograd.Function):
         Hq, Hk, D, Dv, scale, softcap = ctx.dims
         meta = ctx.meta
         T = qkv.shape[0]
-        dout = dout.contiguous()
+        dout, out = dout.contiguous(), _aligned_out(out)
         dqkv = torch.empty_like(qkv)
         dq_acc = torch.empty((T, Hq * D), dtype=torch.float32, device=qkv.device)
         delta = torch.empty((Hq, T), dtype=torch.float32, device=qkv.device)

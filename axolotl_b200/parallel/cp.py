@@ -156,7 +156,7 @@ class _FlashVarlenCP(torch.autograd.Function):
         lib = _lib.cuda_lib()
         T = qkv.shape[0]
         qw = (Hq + 2 * Hk) * D
-        dout = dout.contiguous()
+        dout, out = dout.contiguous(), Fn._aligned_out(out)
         buf = cp.dkv_bufs[cp.kb & 1]   # zero on every rank since its last use
         cp.kb += 1
         dq_acc = torch.empty((T, Hq * D), dtype=torch.float32, device=qkv.device)
