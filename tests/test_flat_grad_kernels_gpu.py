@@ -143,3 +143,28 @@ def test_product_added_to_an_fp32_slice(M, N, K, bn, splits, col):
     size[:, col:col + N] += 0.5 * a.double().abs().t() @ b.double().abs()
     assert ((buf.double() - want).abs() <= 2 ** -20 * size).all()
     assert torch.equal(buf[:, :col], old[:, :col]) and torch.equal(buf[:, col + N:], old[:, col + N:])
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(136, 72, 64, 64), (136, 168, 64, 128), (72, 264, 128, 256), (2056, 2312, 64, 256)])
+@pytest.mark.parametrize("col,cin_col", [(3, None), (3, 0), (0, 5), (1, 2), (0, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_results_and_operands_off_16_bytes(M, N, K, bn, col, cin_col, dtype):
+    """C and the operand that is added, each on and off a 16-byte boundary while its rows are whole vectors apart, in the single-CTA
+    kernel at its three widths and in the pair kernel: one rounding of an fp32 sum of K products, and the columns beside C stay as they
+    are."""
+    from axolotl_b200.ops import gemm as G
+
+    assert G._use_pair(M, N, bn) == (M > 1000)
+    torch.manual_seed(M + col)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    buf, add = torch.randn(M, N + 24, device="cuda").to(dtype), torch.randn(M, N + 24, device="cuda").to(dtype)
+    old = buf.clone()
+    c_in = None if cin_col is None else add[:, cin_col:cin_col + N]
+    G.gemm(a, b, out=buf[:, col:col + N], out_dtype=dtype, c_in=c_in, beta=0.0 if c_in is None else 0.75, alpha=0.5, bn=bn)
+    _lib.check_status()
+    want, size = 0.5 * a.double() @ b.double().t(), 0.5 * a.double().abs() @ b.double().abs().t()
+    if c_in is not None:
+        want, size = want + 0.75 * c_in.double(), size + 0.75 * c_in.double().abs()
+    got = buf[:, col:col + N].double()
+    assert ((got - want).abs() <= (2 ** -8 if dtype == torch.bfloat16 else 0) * want.abs() + 2 ** -20 * size).all()
+    assert torch.equal(buf[:, :col], old[:, :col]) and torch.equal(buf[:, col + N:], old[:, col + N:])
