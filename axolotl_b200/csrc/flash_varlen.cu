@@ -260,13 +260,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_u && ok; ++j) {
-      ok = warp_all(mbar_wait(&s_full[u], j & 1, p.status, AXB_TIMEOUT_TMEM_FULL));
-      if (!ok) break;
+      ok = mbar_wait(&s_full[u], j & 1, p.status, AXB_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       uint32_t sr[4][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, sr[c]);
+      ok = warp_all(ok);               // beside the loads: before them the vote stands in the chain
       tmem_ld_wait();
+      if (!ok) break;
       const int kv0 = (jb0 + j) * 128;
       if ((j == n_u - 1) || (win > 0 && kv0 < qu0 + 128 - win)) {
         const int lim = (bidir ? doc_len - 1 : min(q_idx, doc_len - 1)) - kv0;  // columns <= lim are visible
