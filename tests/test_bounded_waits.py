@@ -44,6 +44,9 @@ def test_a_wait_ends_the_same_way_for_all_lanes_of_a_warp(name):
         held = re.search(r"(\w+) = (?:\w+ && )?$", statement)
         rest = code[at:at + 400]
         agreed = "warp_all(" in statement or (held and re.search(r"warp_all\(%s\)" % held.group(1), rest))
+        if held and re.search(r"(\w+) = \1 && $", statement):      # remembered: nothing branches on it until the warp agrees
+            agreed = re.search(r"\b(?:if|while|for) \([^{;]*\b%s\b" % held.group(1), code[at:]).group().startswith("if (warp_all(")
+            agreed = agreed and not any(re.match(r"(if|while|for) \(.*\b%s\b" % held.group(1), h) for h in headers[-1:])
         one_lane = any("lane == 0)" in h or "elect_one()" in h for h in headers) or "lane != 0) return;" in code[start:at]
         assert agreed or one_lane, f"{name}:{line}: lanes of a warp may leave this wait on different ways"
 
