@@ -100,7 +100,9 @@ AXB_DEVICE bool elect_one() {
 // about 0.3 us for the four MMAs of a K block (128 x 64 and 128 x 128 tiles took the same time). For that the warp index has
 // to be known uniform, and every wait has to end the same way for all lanes.
 // So has every wait of a warp that goes on to warp-wide instructions (tcgen05.ld, __syncwarp): a lane that gives up alone leaves the
-// others waiting for it without a limit. And a warp that gives up inside a loop with a named barrier still has to meet its group there.
+// others waiting for it without a limit. Either the warp agrees on the outcome (warp_all), or the lane remembers it and walks on with
+// the others without waiting again, which keeps the vote out of a chain, and has to be done where a named barrier of several warps
+// stands in the loop: every thread still comes there.
 AXB_DEVICE int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 AXB_DEVICE bool warp_all(bool x) { return __all_sync(0xffffffffu, x); }
 

@@ -690,17 +690,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     if (st_tid < 64) rows[st_tid] = row_val;
     row_val = fetch_row(grp + 2);
     asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
-    int it = grp;
-    for (; it < n_iter; it += 2) {
+    for (int it = grp; it < n_iter; it += 2) {
       const uint32_t ph = (it >> 1) & 1;
       const int head = head0 + it / n_qt;
       const int qt0 = (q_first + it % n_qt) * 64;  // doc-relative first q row of the tile
       const int qc0 = qt0 + c0;                    // ... and of this group's columns
       const float* nlse = rows + ph * 64;
-      if (!warp_all(mbar_wait(&s_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
-        ok = false;
-        break;
-      }
+      // (a lane whose wait ran out walks on with the others, without waiting again: the group meets at the barrier below)
+      ok = ok && mbar_wait(&s_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       // Only tiles that touch the diagonal or the end of the document need per-element masks
       // (q rows outside the document already carry nlse = -inf, i.e. P = 0).
@@ -730,11 +727,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       row_val = fetch_row(it + 4);
       asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
       // drain dQ^T: this thread owns d = r (only rows < D are meaningful)
-      if (!warp_all(mbar_wait(&dq_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
-        ok = false;
-        it += 2;
-        break;
-      }
+      ok = ok && mbar_wait(&dq_full[grp], ph, p.status, AXB_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       {
         // valid q columns of this group: inside the document and inside this rank's q window
@@ -768,12 +761,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         }
       }
     }
-    // A warp whose wait ran out does no more work, but meets its group at the barriers that are left.
-#pragma unroll 1
-    for (; it < n_iter; it += 2) asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
     if (lane == 0) bulk_wait_group<0>();
     // final dK / dV: 32 columns of each per warpgroup
-    if (wg < D / 32 && ok && warp_all(mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
+    if (warp_all(ok && wg < D / 32 && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
       tc_fence_after();
       const bool row_ok = kv_idx < doc_len && n_iter > 0;
       const long long grow = (long long)doc_start + kv_idx;  // global kv row

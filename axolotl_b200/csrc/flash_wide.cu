@@ -596,15 +596,12 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
     if (tid < 32) rows[tid] = row_val;
     row_val = fetch_row(1);
     asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-    int it = 0;
-    for (; it < n_iter; ++it) {
+    for (int it = 0; it < n_iter; ++it) {
       const uint32_t ph = it & 1;
       const int head = head0 + it / n_qt;
       const int qc0 = (q_first + it % n_qt) * 64 + c0;      // doc-relative first q row of this group's columns
-      if (!warp_all(mbar_wait(s_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
-        ok = false;
-        break;
-      }
+      // (a lane whose wait ran out walks on with the others, without waiting again: the group meets at the barrier below)
+      ok = ok && mbar_wait(s_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       const bool need_mask = (!bidir && qc0 < kv0 + 127) || kv0 + 128 > doc_len || (win > 0 && qc0 + 15 >= kv0 + win);
       {
@@ -629,11 +626,7 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
       if (tid < 32) rows[(ph ^ 1) * 32 + tid] = row_val;
       row_val = fetch_row(it + 2);
       asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-      if (!warp_all(mbar_wait(dq_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL))) {
-        ok = false;
-        ++it;
-        break;
-      }
+      ok = ok && mbar_wait(dq_full, ph, p.status, AXB_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       if (has_k) {
         const long long row0 = (long long)doc_start + qc0;
@@ -669,10 +662,7 @@ __global__ void __launch_bounds__(WBWD_THREADS, 1)
         mbar_arrive(st_free);
       }
     }
-    // A warp whose wait ran out does no more work, but meets its group at the barriers that are left.
-#pragma unroll 1
-    for (; it < n_iter; ++it) asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-    if (ok && warp_all(mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
+    if (warp_all(ok && mbar_wait(acc_full, 0, p.status, AXB_TIMEOUT_TMEM_FULL))) {
       tc_fence_after();
       const bool row_ok = kv_idx < doc_len;
       const long long grow = (long long)doc_start + kv_idx;

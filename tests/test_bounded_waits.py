@@ -53,8 +53,7 @@ def test_a_wait_ends_the_same_way_for_all_lanes_of_a_warp(name):
 
 @pytest.mark.parametrize("name", [n for n in SOURCES if "bar.sync" in _code(n)])
 def test_a_warp_that_gives_up_still_meets_its_group(name):
-    """A named barrier has no limit: a warp that leaves a loop with one, because a wait ran out, meets its group at the barriers that
-    are left, in a loop of its own from where it stopped, or it walks on without work (dead)."""
+    """A named barrier has no limit: a warp never leaves a loop with one because a wait ran out. Its lanes remember that and walk on."""
     code = _code(name)
     loops = 0
     for m in re.finditer(r"\bfor \(", code):
@@ -71,14 +70,10 @@ def test_a_warp_that_gives_up_still_meets_its_group(name):
         if "bar.sync" not in block or not WAIT.search(block):
             continue
         loops += 1
-        breaks = [b.start() for b in re.finditer(r"\n\s*break;", block)]              # (not those of a switch)
-        assert breaks or "dead" in block
-        if breaks:
-            step = re.search(r"for \((?:int \w+ = \w+)?; it < n_iter; (it \+= 2|\+\+it)\)$", code[m.start():body].strip()).group(1)
-            assert code[i:i + 400].lstrip().startswith("#pragma unroll 1") and re.match(
-                r"\s*#pragma unroll 1\s*for \(; it < n_iter; %s\) asm volatile\(\"bar.sync" % re.escape(step), code[i:]), name
-        for b in breaks:      # one barrier an iteration: behind it, the next iteration's is the first that is left
-            assert bool(re.search(r"\b%s;\s*$" % re.escape(step), block[:b]) or block[:b].rstrip().endswith(step + ";")) == ("bar.sync" in block[:b]), name
+        assert not re.search(r"\n\s*(break|return);", block), name                    # (those of a switch stand on its lines)
+        assert "ok" not in re.findall(r"\w+", code[m.start():body]), name
+        for w in WAIT.finditer(block):
+            assert re.search(r"(ok = ok && |if \(!dead\) dead = !warp_all\()$", block[:w.start()]), name
     assert loops
 
 
