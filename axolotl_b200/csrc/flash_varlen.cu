@@ -5,7 +5,7 @@
 // projection buffer [T, (Hq + 2*Hk) * D] (bf16), documents are delimited by a host-built tile
 // table (one entry per (document, 128-row tile)), so no [S,S] mask and no cross-document
 // attention ever exists. Both kernels are warp-specialised:
-//   warp 0: TMA producer, warp 1: tcgen05.mma issuer, warps 2-9: softmax / gradient math
+//   warp 0: TMA producer, warp 1: tcgen05.mma issuer, two (forward) or four (backward) warpgroups: softmax / gradient math
 // with S, P, O (forward) and S^T, dP^T, dK, dV, dQ^T (backward) accumulators living in TMEM.
 //
 // Replaces flash-attn varlen (FA2/FA4) that the reference reaches through HF's
@@ -65,7 +65,8 @@ struct AttnParams {
 // against 64 bits 1.5 % larger for unit normal q and k, 19 % for twice that. Dividing by the sum of the rounded P mends half.
 // Bound: exponentials (16 per clock and SM against 1024 clocks of MMA per 128 x 128 block) and the MMA stream, about level.
 // One 16384-token document, 32 / 8 heads of 128: 3.01 -> 1.89 ms (730 -> 1160 TFLOP/s) against one softmax warpgroup with O in
-// registers and P through shared memory; 4 x 2048 268 -> 180 us; 11 x 707, 64 heads of 64, 279 -> 183 us.
+// registers and P through shared memory; 4 x 2048 268 -> 180 us; 11 x 707, 64 heads of 64, 279 -> 178 us. These are single calls with
+// a cold L2; the long document takes 2.14 ms where calls follow one another and the board's power limit lowers the clock.
 // TMA warp, MMA warp, two idle warps (they complete the warpgroup that gives registers away), 2 x 4 softmax warps. A row of S
 // is held in 128 registers: the 384 x 168 registers of the launch are split 128 x 40 + 256 x 232.
 constexpr int kFwdThreads = 384;
@@ -371,13 +372,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // drains dQ^T(i). dQ^T(i) reuses the TMEM columns of S^T(i), which is dead once P^T(i) is written; with D = 128 all 512 columns are
 // in use:
 //   [S^T0 | dP^T0 | S^T1 | dP^T1 | dV (D) | dK (D)]
-// What bounds it is the chain of a pair (scores -> P^T, dS^T -> dQ^T -> next scores); the tensor core is busy for 56 % of an
-// iteration (five products of 64 queries, three of them limited by the shared-memory reads of their 64 columns). So nothing waits
+// What bounds it is the chain of a pair (scores -> P^T, dS^T -> dQ^T -> next scores); the tensor core is busy for 72 % of the time,
+// 52 % without the operand reads (4 x 2048 tokens, 32 / 8 heads of 128: five products of 64 queries, three of them limited by the
+// shared-memory reads of their 64 columns). 18 warps leave a thread 96 registers, of which heads of 128 spill nine. So nothing waits
 // for memory inside the chain: Q / dO run three stages ahead (with two a quarter slower), lse and delta are requested two iterations
 // early, dQ^T is the first product of its iteration and is drained while dV and dK run, and its sums leave by tile reductions: from
-// registers they filled the load-store queue ahead of the other pair's dS^T (a fifth of the time). One 16384-token document, 32 / 8
-// heads of 128: 8.60 -> 6.31 -> 5.47 ms (1005 TFLOP/s); 4096 tokens, 32 / 4 heads of 64: 258 -> 182 us with delta and conversion;
-// 11 x 707 tokens, 64 / 8 heads of 64, window 128: 338 -> 289.
+// registers they filled the load-store queue ahead of the other pair's dS^T (a fifth of the time). Whole backward pass (zeroing, delta,
+// this kernel, conversion) against the form with two softmax warpgroups and single reductions, cold L2 / eight calls in turn: one
+// 16384-token document, 32 / 8 heads of 128, 6.25 / 6.87 -> 5.18 / 5.99 ms; 4096 tokens, 32 / 4 heads of 64, 437 / 420 -> 330 / 314 us;
+// 11 x 707 tokens, 64 / 8 heads of 64, window 128, 300 / 295 -> 287 / 279 (188 of them this kernel).
 constexpr int kBwdThreads = 576;  // TMA warp, MMA warp, 4 x 4 softmax warps
 template <int D>
 struct BwdCfg {
@@ -386,8 +389,9 @@ struct BwdCfg {
   static constexpr int Q_HALF = 64 * 128;               // 64 rows x 128 B
   static constexpr int Q_BYTES = HALVES * Q_HALF;       // Q or dO tile: 64 rows
   static constexpr int PT_BYTES = HALF_BYTES;           // P^T / dS^T: [128 kv x 64 q]
-  // P^T as the TMEM operand of dV where shared memory is full; from shared memory is faster (4096 tokens, 32 heads of 64: 182 against
-  // 235 us; heads of 128 with P^T in shared memory and two stages of Q / dO instead of three: a quarter slower)
+  // P^T as the TMEM operand of dV where shared memory is full; from shared memory is 1 to 3 % faster (whole backward pass, 32 / 4
+  // heads of 64, 4096 tokens 292 against 295 us, 64 / 8 heads, 11 x 707 tokens 396 against 408; heads of 128 with P^T in shared memory
+  // and two stages of Q / dO instead of three: a quarter slower)
   static constexpr bool PT_TMEM = D == 128;
   // dQ^T on its way out, per warp that owns rows of it: groups of four queries x 32 columns of d, all nine that 32 queries can touch
   // where shared memory allows

@@ -360,7 +360,8 @@ struct WBwd {
 // comes first, so that Q, which the next scores wait for, loads beside dV and dQ^T; dO is handed back by itself; dQ^T has TMEM
 // columns of its own, so that the next scores do not wait for its drain; tiles without a mask have a path of their own; and four rows
 // of a dQ column lie side by side in the fp32 sum, which leaves in 16-byte reductions. 4 x 2048 tokens, 16 / 8 heads of 256, whole
-// backward pass 904 -> 816 us, 300 + 2701 tokens 419 -> 379. Still the chain bounds it: the MMAs are a third of an iteration.
+// backward pass 904 -> 816 us, 300 + 2701 tokens 419 -> 378. Still the chain bounds it: the MMAs are a third of an iteration, half of
+// it with their operand reads.
 constexpr int WBWD_THREADS = 576;
 template <int DQK, int DV, bool SOFTCAP>
 __global__ void __launch_bounds__(WBWD_THREADS, 1)

@@ -16,10 +16,12 @@
 // bf16, with byte permutes, about 2 instructions per value; the products come from a table per expert.
 // What bounds it: one CTA per 128 columns read every tile from shared memory for two MMAs (960 of 1020 clocks of a k block); the pair
 // reads each half once (576). Then the chain of a k block (packed tile seen -> decode -> arrival -> MMA -> slot free), and the decode
-// itself at half rate in the integer pipe (47 % active). 128 experts with the rows of a skewed router, forward / input gradient:
-//   8192 x 8 rows, 2048 -> 1536  517 / 518 -> 389 / 411 us, 768 -> 2048  278 / 276 -> 257 / 212 us
-//    333 x 8 rows, 2048 -> 1536  173 / 159 -> 135 / 142 us, 768 -> 2048   88 /  92 ->  78 /  83 us
-//   32 experts, 2000 x 4 rows, 1024 -> 1024  46 / 46 -> 34 / 34 us
+// itself at half rate in the integer pipe: 3.1 (forward) and 3.7 (input gradient) instructions a value with table reads, addresses and
+// polls, 400 and 470 of the 740 and 760 clocks that a k block takes. 128 experts with the rows of a skewed router, forward / input
+// gradient, one CTA a tile -> pairs (arrivals at cluster scope included, 2 to 3 % of it), cold L2:
+//   8192 x 8 rows, 2048 -> 1536  492 / 488 -> 389 / 404 us, 768 -> 2048  257 / 275 -> 245 / 199 us
+//    333 x 8 rows, 2048 -> 1536  169 / 157 -> 150 / 151 us, 768 -> 2048   84 /  94 ->  87 /  89 us
+//   32 experts, 2000 x 4 rows, 1024 -> 1024  40 / 42 -> 36 / 36 us
 // An L2 prefetch ahead of the packed loads cost 5 % with the twelve-slot ring (it had paid with four); five or six converter groups,
 // eight decoded slots and deeper packed rings changed nothing.
 // The decoded values are bit-identical to nvfp4_dequant_kernel's, so the product equals
@@ -39,7 +41,8 @@ constexpr int W4_THREADS = 192 + 32 * W4_CONV_WARPS + 32;   // TMA (rows), MMA, 
 // its MMA, and the packed weights are small and run twelve k blocks ahead of the decode.
 // The converters work in four groups of four warps, each on a k block of its own, so that four chains (packed tile seen ->
 // decode -> stores -> proxy fence -> arrival) run side by side. Two warps a group left the decode's dependent instructions
-// uncovered: 512 rows of each of 128 experts, 2048 -> 1536 393 -> 366 us, 768 -> 2048 220 -> 199 (one CTA a tile).
+// uncovered: 512 rows of each of 128 experts, 2048 -> 1536 393 -> 366 us, 768 -> 2048 220 -> 199 (measured when one CTA had a tile; six
+// groups changed nothing in the present form).
 constexpr int SX = 5, SW = 4, SR = 12;  // slots: rows, decoded weights, packed weights
 // Every group owns one slot of the decoded ring and three of the packed one (k block i of the whole sequence belongs to group
 // i % 4), so that a slot's waits are made in order by the same warps: a wait for a phase whose predecessor has not completed
